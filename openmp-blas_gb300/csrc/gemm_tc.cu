@@ -1423,15 +1423,54 @@ __global__ void __launch_bounds__(ModeTraits<MODE>::kThreads, 1)
           continue;
         }
       }
-      const int row = m0 + q * 32 + lane;
+      // C += acc by loads and stores; a split-K partial (overwrite) is stored
+      // instead, into dense rows.  Bound by the latency of C's lines, so each
+      // warp keeps 16 loads in flight before the first store (the compiler
+      // cannot see that runtime strides keep the outputs apart: one output at
+      // a time cost 300 of the kernel's 548 us at 3970 x 3475 x 4050).
+      const bool add = !pr.overwrite;
+      const int row0 = m0 + q * 32, cn = n0 + col0;
+      if constexpr (CF::kTmaC) {
+        if (pr.csc == 1) {
+          // contiguous C rows of any alignment: the 32 x 32 blocks go through
+          // shared memory (swizzled as for the TMA update) and the warp
+          // updates one row's 32 columns, 128 bytes, per access
+          const uint32_t skip_rows = __ballot_sync(0xffffffffu, skip_row);
+          float* scr = epi_scratch + (warp - 2) * 1024;
+#pragma unroll
+          for (int cb = 0; cb < kCols; cb += 32) {
+            __syncwarp();
+#pragma unroll
+            for (int c = 0; c < 8; ++c)
+              *reinterpret_cast<float4*>(scr + lane * 32 + ((c ^ (lane & 7)) * 4)) =
+                  make_float4(acc[cb + 4 * c], acc[cb + 4 * c + 1], acc[cb + 4 * c + 2], acc[cb + 4 * c + 3]);
+            __syncwarp();
+            const int col = cn + cb + lane;
+            const bool live = col < pr.N && !(MT::f16 && ((skip_cols >> (cb + lane)) & 1));
+            float* cp = pr.C + (int64_t)row0 * pr.rsc + col;
+#pragma unroll
+            for (int r0 = 0; r0 < 32; r0 += 16) {
+              float old[16];
+#pragma unroll
+              for (int r = 0; r < 16; ++r)
+                old[r] = (add && live && row0 + r0 + r < pr.M) ? cp[(int64_t)(r0 + r) * pr.rsc] : 0.f;
+#pragma unroll
+              for (int r = 0; r < 16; ++r) {
+                const float v = scr[(r0 + r) * 32 + (((lane >> 2) ^ (r & 7)) * 4) + (lane & 3)];
+                if (live && row0 + r0 + r < pr.M && !((skip_rows >> (r0 + r)) & 1))
+                  cp[(int64_t)(r0 + r) * pr.rsc] = old[r] + v;
+              }
+            }
+          }
+          continue;
+        }
+      }
+      // a thread per row (coalesced where C's columns are contiguous)
+      const int row = row0 + lane;
       if (row < pr.M && !skip_row) {
         float* crow = pr.C + (int64_t)row * pr.rsc;
         const bool vec = (pr.csc == 1) && ((pr.rsc & 3) == 0) && ((reinterpret_cast<uintptr_t>(pr.C) & 15) == 0) &&
                          skip_cols == 0;
-        const int cn = n0 + col0;
-        // C += acc; a split-K partial (overwrite) is stored instead, into
-        // dense 16-byte-aligned rows
-        const bool add = !pr.overwrite;
         if (vec && cn + kCols <= pr.N) {
           // 64 bytes at a time: four loads in flight before their stores
 #pragma unroll
@@ -1453,11 +1492,16 @@ __global__ void __launch_bounds__(ModeTraits<MODE>::kThreads, 1)
           }
         } else {
 #pragma unroll
-          for (int j = 0; j < kCols; ++j)
-            if (cn + j < pr.N && !((skip_cols >> j) & 1)) {
-              float* q = crow + (int64_t)(cn + j) * pr.csc;
-              *q = add ? *q + acc[j] : acc[j];
-            }
+          for (int j0 = 0; j0 < kCols; j0 += 16) {
+            float old[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+              old[j] = (add && cn + j0 + j < pr.N) ? crow[(int64_t)(cn + j0 + j) * pr.csc] : 0.f;
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+              if (cn + j0 + j < pr.N && !(MT::f16 && ((skip_cols >> (j0 + j)) & 1)))
+                crow[(int64_t)(cn + j0 + j) * pr.csc] = old[j] + acc[j0 + j];
+          }
         }
       }
     }

@@ -1,0 +1,57 @@
+"""Tensor-core GEMMs whose operands and results sit at awkward places: odd
+leading dimensions, bases off the 16-byte grid, extents that are multiples of
+nothing.  Each case computes the same product from the same values as an
+aligned call, so the results must agree bit for bit, and the memory around C
+must stay as it was."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+BF16X3, FP8, BF16X6, FP16X3 = 1, 2, 4, 8
+
+
+def place(torch, X, pitch, off, col_major=False):
+    """X (numpy, 2-D) in a device buffer: row (column) pitch `pitch`, first
+    element at `off`; returns (buffer, address, row stride, column stride)."""
+    v = X.T if col_major else X
+    buf = np.full(off + v.shape[0] * pitch + 7, np.float32(-77.0), np.float32)
+    at = (off + np.arange(v.shape[0])[:, None] * pitch + np.arange(v.shape[1])[None, :]).ravel()
+    buf[at] = v.ravel()
+    t = torch.from_numpy(buf).cuda()
+    rs, cs = (1, pitch) if col_major else (pitch, 1)
+    return t, t.data_ptr() + 4 * off, rs, cs, at, v.shape
+
+
+def gemm(torch, A, B, C0, acc, pa, pb, pc, la=False, lb=False, lc=False):
+    import gbblas
+    M, K = A.shape
+    N = B.shape[1]
+    a = place(torch, A, (M if la else K) + pa[0], pa[1], la)
+    b = place(torch, B, (K if lb else N) + pb[0], pb[1], lb)
+    c = place(torch, C0, (M if lc else N) + pc[0], pc[1], lc)
+    gbblas.call("gbblas_sgemm", M, N, K, a[1], a[2], a[3], b[1], b[2], b[3], c[1], c[2], c[3], acc, None)
+    gbblas.call("gbblas_check_stream", None)
+    out = c[0].cpu().numpy()
+    rest = np.ones(out.size, bool)
+    rest[c[4]] = False
+    assert np.all(out[rest] == np.float32(-77.0)), "memory beside C changed"
+    got = out[c[4]].reshape(c[5])
+    return got.T if lc else got
+
+
+def values(rng, shape):
+    return rng.uniform(-1, 1, shape).astype(np.float32)
+
+
+# C rows: aligned (the TMA update), pitches and bases that are not (the
+# warp-by-row update); extents at the tile's edges
+@pytest.mark.parametrize("acc", [BF16X3, FP8, BF16X6, FP16X3])
+@pytest.mark.parametrize("M,N,K", [(1, 4, 8), (127, 132, 64), (128, 128, 128), (129, 260, 520), (33, 700, 260)])
+@pytest.mark.parametrize("pad,off", [(1, 0), (2, 0), (3, 3), (0, 1)])
+def test_unaligned_c_same_bits_as_aligned(cuda, acc, M, N, K, pad, off):
+    rng = np.random.default_rng(M * 7 + N + K)
+    A, B, C0 = values(rng, (M, K)), values(rng, (K, N)), values(rng, (M, N))
+    want = gemm(cuda, A, B, C0, acc, (0, 0), (0, 0), (0, 0))
+    got = gemm(cuda, A, B, C0, acc, (0, 0), (0, 0), (pad, off))
+    np.testing.assert_array_equal(got, want)
