@@ -303,6 +303,32 @@ __device__ __forceinline__ void f16_scale_tile_rows(const unsigned (&mx)[16], co
   }
 }
 
+// Widest load (4, 2 or 1 floats) the start of a K-contiguous row allows: the
+// rows of an operand whose leading dimension is no multiple of 4 differ.
+__device__ __forceinline__ int row_width(const float* p) {
+  const unsigned a = (unsigned)reinterpret_cast<uintptr_t>(p);
+  return (a & 15) == 0 ? 4 : ((a & 7) == 0 ? 2 : 1);
+}
+
+// p[0..3], of which the first n exist (the others read as zero), with loads
+// of w = row_width(p) floats.  The narrow forms touch each line of the warp's
+// 512 bytes two or four times, so they go through L1.
+__device__ __forceinline__ float4 load_row4(const float* p, int64_t n, int w) {
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (n >= 4) {
+    if (w == 4) return dev::ld_stream(reinterpret_cast<const float4*>(p));
+    if (w == 2) {
+      const float2 a = __ldg(reinterpret_cast<const float2*>(p)), b = __ldg(reinterpret_cast<const float2*>(p) + 1);
+      return make_float4(a.x, a.y, b.x, b.y);
+    }
+    return make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+  }
+  if (n > 0) v.x = __ldg(p);
+  if (n > 1) v.y = __ldg(p + 1);
+  if (n > 2) v.z = __ldg(p + 2);
+  return v;
+}
+
 // Row exponents are stored biased so that zero (what the launch's one
 // memset writes) means "no nonzero element seen": e[R] = kExpBias + the
 // frexp exponent of the row's largest magnitude, emin[R] = ~(magnitude bits
@@ -489,9 +515,13 @@ __device__ __forceinline__ int prep_slot(int r, int k) {
   return r * LD + 4 * ((k >> 2) ^ ((r >> 2) & 7)) + (k & 3);
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(256) prep_group_kernel(PrepSide side_a, PrepSide side_b, int njobs, int64_t pitch,
-                                                         int64_t scale_stride) {
+// VEC: every operand prepared by this launch takes the 128-bit loads
+// throughout (prep_vec).  The general form's 16 scalar loads in flight need
+// registers that would cost the 128-bit form occupancy: with both in one
+// kernel an aligned 8192^2 pair of FP8 operands took 240 us instead of 192.
+template <int MODE, bool VEC>
+__global__ void __launch_bounds__(256, VEC ? 1 : 4) prep_group_kernel(PrepSide side_a, PrepSide side_b, int njobs,
+                                                                      int64_t pitch, int64_t scale_stride) {
   using PT = PrepTile<MODE>;
   constexpr int TK = PT::TK, TR = PT::TR, LD = PT::LD;
   __shared__ __align__(16) float tile[TR * LD];
@@ -526,7 +556,7 @@ __global__ void __launch_bounds__(256) prep_group_kernel(PrepSide side_a, PrepSi
   // edge tiles too where that dimension's extent is a multiple of 4 (each
   // float4 then lies wholly inside or wholly outside the operand)
   const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (al16 && j.cs == 1 && (j.rs & 3) == 0 && (full || (j.K & 3) == 0)) {  // along K
+  if (VEC ? j.cs == 1 : (al16 && j.cs == 1 && (j.rs & 3) == 0 && (full || (j.K & 3) == 0))) {  // along K
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int idx = tid + 256 * i, r = idx / (TK / 4), k4 = idx % (TK / 4);
@@ -535,7 +565,7 @@ __global__ void __launch_bounds__(256) prep_group_kernel(PrepSide side_a, PrepSi
                            : zero4;
       *reinterpret_cast<float4*>(&tile[prep_slot<LD>(r, 4 * k4)]) = v;
     }
-  } else if (al16 && j.rs == 1 && (j.cs & 3) == 0 && (full || (j.rows & 3) == 0)) {  // along rows
+  } else if (VEC || (al16 && j.rs == 1 && (j.cs & 3) == 0 && (full || (j.rows & 3) == 0))) {  // along rows
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int idx = tid + 256 * i, k = idx / (TR / 4), r4 = idx % (TR / 4);
@@ -547,19 +577,24 @@ __global__ void __launch_bounds__(256) prep_group_kernel(PrepSide side_a, PrepSi
       tile[prep_slot<LD>(4 * r4 + 2, k)] = v.z;
       tile[prep_slot<LD>(4 * r4 + 3, k)] = v.w;
     }
-  } else if (j.cs == 1) {  // K contiguous: consecutive threads along k
-#pragma unroll 4
-    for (int i = 0; i < 16; ++i) {
-      const int idx = tid + 256 * i, r = idx / TK, k = idx % TK;
-      tile[prep_slot<LD>(r, k)] = (r0 + r < j.rows && k0 + k < j.K) ? __ldg(j.src + (r0 + r) * j.rs + k0 + k) : 0.f;
-    }
-  } else {  // rows contiguous (or general): consecutive threads along r
-#pragma unroll 4
-    for (int i = 0; i < 16; ++i) {
-      const int idx = tid + 256 * i, r = idx % TR, k = idx / TR;
-      tile[prep_slot<LD>(r, k)] =
-          (r0 + r < j.rows && k0 + k < j.K) ? __ldg(j.src + (r0 + r) * j.rs + (k0 + k) * j.cs) : 0.f;
-    }
+  } else {
+    // other alignments and strides, element by element (consecutive threads
+    // along k where K is contiguous, else along r): all 16 loads of a thread
+    // in flight before its shared-memory stores
+    const bool kc = j.cs == 1;
+    const int r = kc ? tid / TK : tid % TR, k = kc ? tid % TK : tid / TR;  // element i: r (k) + i * stride
+    constexpr int SR = 256 / TK, SK = 256 / TR;
+    const float* __restrict__ p = j.src + (r0 + r) * j.rs + (k0 + k) * j.cs;
+    const int64_t step = kc ? SR * j.rs : SK * j.cs;
+    // elements 0 .. n - 1 exist
+    const int64_t left = kc ? (k0 + k < j.K ? (j.rows - r0 - r + SR - 1) / SR : 0)
+                            : (r0 + r < j.rows ? (j.K - k0 - k + SK - 1) / SK : 0);
+    const int n = (int)min(left, (int64_t)16);
+    float v[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = i < n ? __ldg(p + i * step) : 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) tile[prep_slot<LD>(kc ? r + SR * i : r, kc ? k : k + SK * i)] = v[i];
   }
   __syncthreads();
   const int warp = tid >> 5, lane = tid & 31;
@@ -659,12 +694,14 @@ __global__ void __launch_bounds__(256) prep_group_kernel(PrepSide side_a, PrepSi
 
 // Row exponents of the FP16 split for operands whose rows are contiguous
 // (row-major B seen as B^T, column-major A): f16_scale_kernel's results by
-// a column reduction.  A CTA covers 1024 consecutive rows (4 per thread, as
-// one float4) and `kblk` (kColScaleK) of K; each thread keeps 8 loads in flight and
-// its rows' extremes in registers, then atomicMax-es them into e[R] and
-// emin[R] once.  Conditions (host side, per operand): every job has rows
-// contiguous, 16-byte aligned columns and a row count that is a multiple of
-// 4 (each float4 wholly inside or outside the operand).
+// a column reduction.  A CTA covers 1024 consecutive rows (4 per thread: one
+// float4 where every column of the job starts on a 16-byte boundary and the
+// row count is a multiple of 4, else rows tid, tid + 256, ... one by one) and
+// `kblk` (kColScaleK) of K; each thread keeps 8 K's loads in flight and its
+// rows' extremes in registers, then atomicMax-es them into e[R] and emin[R]
+// once.  Bound by HBM.  A 4050 x 3475 row-major B: 44 us through
+// f16_scale_kernel's scalar tiles, see the launch rule for this kernel's.
+// Condition (host side, per operand): every job has rows contiguous.
 constexpr int kColScaleK = 128;
 
 __global__ void __launch_bounds__(256, 4) f16_col_scale_kernel(ScaleSide side_a, ScaleSide side_b, int njobs,
@@ -683,18 +720,34 @@ __global__ void __launch_bounds__(256, 4) f16_col_scale_kernel(ScaleSide side_a,
   const SplitJob& j = sd.jobs[lo];
   const int local = t - j.col_start;
   const int kblocks = (int)((j.K + kblk - 1) / kblk);
-  const int64_t r = (int64_t)(local / kblocks) * 1024 + 4 * threadIdx.x;  // this thread's first row
+  const bool vec = (reinterpret_cast<uintptr_t>(j.src) & 15) == 0 && (j.cs & 3) == 0 && (j.rows & 3) == 0;
+  // this thread's rows: r, r + step, r + 2 step, r + 3 step
+  const int step = vec ? 1 : 256;
+  const int64_t r = (int64_t)(local / kblocks) * 1024 + (vec ? 4 * threadIdx.x : threadIdx.x);
   const int64_t k0 = (int64_t)(local % kblocks) * kblk;
   const int64_t k1 = min(k0 + kblk, j.K);
   if (r >= j.rows) return;
+  const int nrow = vec ? 4 : (int)min((j.rows - r + 255) / 256, (int64_t)4);  // of which this many exist
   const float* __restrict__ src = j.src + r;
   unsigned w[4] = {0u, 0u, 0u, 0u}, v[4] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu};
   for (int64_t k = k0; k < k1; k += 8) {
     float4 x[8];
+    if (vec) {
 #pragma unroll
-    for (int u = 0; u < 8; ++u)
-      x[u] = k + u < k1 ? dev::ld_stream(reinterpret_cast<const float4*>(src + (k + u) * j.cs))
-                        : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int u = 0; u < 8; ++u)
+        x[u] = k + u < k1 ? dev::ld_stream(reinterpret_cast<const float4*>(src + (k + u) * j.cs))
+                          : make_float4(0.f, 0.f, 0.f, 0.f);
+    } else {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const float* p = src + (k + u) * j.cs;
+        const int n = k + u < k1 ? nrow : 0;
+        x[u].x = n > 0 ? __ldg(p) : 0.f;
+        x[u].y = n > 1 ? __ldg(p + 256) : 0.f;
+        x[u].z = n > 2 ? __ldg(p + 512) : 0.f;
+        x[u].w = n > 3 ? __ldg(p + 768) : 0.f;
+      }
+    }
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       w[0] = max(w[0], mag_bits(x[u].x));
@@ -709,7 +762,8 @@ __global__ void __launch_bounds__(256, 4) f16_col_scale_kernel(ScaleSide side_a,
   }
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    const int64_t row = j.dst_row + r + q;
+    const int64_t row = j.dst_row + r + q * step;
+    if (q >= nrow) break;
     if (w[q] != 0u) {
       // frexp's exponent of a positive finite float (subnormals included):
       // floor(log2 x) + 1; Inf / NaN take the top exponent, as elsewhere
@@ -721,11 +775,11 @@ __global__ void __launch_bounds__(256, 4) f16_col_scale_kernel(ScaleSide side_a,
 }
 
 // Split-BF16 preparation of operands whose K is contiguous (row-major A,
-// column-major B; 16-byte aligned rows, K a multiple of 4): a warp per
-// arena row at a time, each lane 4 consecutive K per 128-bit load (four loads in
-// flight), its P pieces written as 8-byte stores - the same pieces as
-// prep_group_kernel, without the shared-memory tile or its barriers.
-// Padding rows and the K padding get zeros.
+// column-major B), any alignment: a warp per arena row at a time, each lane 4
+// consecutive K per step (load_row4; four steps' loads in flight), its P
+// pieces written as 8-byte stores - the same pieces as prep_group_kernel,
+// without the shared-memory tile or its barriers.  Padding rows and the K
+// padding get zeros.
 struct RowSplitSide {
   const SplitJob* jobs;
   int rows;  // arena rows prepared here (0: this operand takes the tile kernel)
@@ -769,14 +823,14 @@ __global__ void __launch_bounds__(256) split_rows_kernel(RowSplitSide side_a, Ro
   const int64_t kp = (int64_t)j.tiles_k * PrepTile<P>::TK;  // the job's padded K
   const int64_t K = local < j.rows ? j.K : 0;                // padding rows: all zeros
   const float* __restrict__ src = j.src + (local < j.rows ? local : 0) * j.rs;
+  const int w = row_width(src);
   __nv_bfloat16* __restrict__ dst = sd.out + R * pitch;
-  const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int64_t k0 = 4 * lane; k0 < kp; k0 += 4 * 128) {
     float4 x[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int64_t k = k0 + 128 * u;
-      x[u] = k < K ? dev::ld_stream(reinterpret_cast<const float4*>(src + k)) : zero4;
+      x[u] = load_row4(src + k, K - k, w);
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
@@ -803,18 +857,19 @@ __global__ void __launch_bounds__(256) split_rows_kernel(RowSplitSide side_a, Ro
 }
 
 // Split-FP16 preparation in one pass for operands whose K is contiguous
-// (row-major A, column-major B): one CTA per arena row reads the row once
-// into registers (kRowPrepNV float4 per thread), finds its largest and its
-// smallest nonzero magnitude (warp shuffles, then the 8 warps' values in
-// shared memory), records e[R] (and, under the guard, emin[R] and the
+// (row-major A, column-major B), any alignment: TPR threads per arena row
+// (a CTA of 256, or a warp where no row is longer than 1024) read the row
+// once into registers (kRowPrepNV x 4 floats per thread), find its largest
+// and its smallest nonzero magnitude (warp shuffles, then the 8 warps' values
+// in shared memory), record e[R] (and, under the guard, emin[R] and the
 // row's out-of-span decision) exactly as f16_scale_kernel and
-// prep_group_kernel do, then scales the row by 2^(15 - e) and writes its two
+// prep_group_kernel do, then scale the row by 2^(15 - e) and write its two
 // FP16 pieces - the same bits as the two-kernel path, from one read of the
 // operand instead of two.  Padding rows (beyond the job's rows) get zero
-// pieces.  Conditions (host side, per operand): every job K contiguous,
-// 16-byte aligned rows, K a multiple of 4 and at most 1024 kRowPrepNV.
+// pieces.  Bound by HBM (4 B read and 4 B written per element).
+// Conditions (host side, per operand): every job K contiguous, padded K at
+// most 4 kRowPrepNV TPR.
 constexpr int kRowPrepNV = 8;
-constexpr int64_t kRowPrepMinK = 1024;  // shorter rows: the tile kernels (a CTA per row would idle)
 
 struct RowPrepSide {
   const SplitJob* jobs;
@@ -825,15 +880,18 @@ struct RowPrepSide {
   F16Guard guard;
 };
 
+template <int TPR>
 __global__ void __launch_bounds__(256) f16_row_prep_kernel(RowPrepSide side_a, RowPrepSide side_b, int njobs,
                                                            int64_t pitch) {
   constexpr int NV = kRowPrepNV;
+  constexpr int RPC = 256 / TPR;  // rows per CTA (of one job: its rows are padded to a multiple of 128)
   __shared__ unsigned red_max[8], red_min[8];
   __shared__ int sh_shift;
-  const bool on_b = (int)blockIdx.x >= side_a.rows;
+  const int a_ctas = side_a.rows / RPC;
+  const bool on_b = (int)blockIdx.x >= a_ctas;
   const RowPrepSide& sd = on_b ? side_b : side_a;
-  const int64_t R = (int64_t)blockIdx.x - (on_b ? side_a.rows : 0);  // arena row
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x % TPR, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t R = ((int64_t)blockIdx.x - (on_b ? a_ctas : 0)) * RPC + threadIdx.x / TPR;  // arena row
   int lo = 0, hi = njobs - 1;  // job: the last whose first arena row is <= R
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
@@ -847,7 +905,7 @@ __global__ void __launch_bounds__(256) f16_row_prep_kernel(RowPrepSide side_a, R
   const int64_t kp = (int64_t)j.tiles_k * PrepTile<kModeF16>::TK;  // the job's padded K
   __half* __restrict__ ph = sd.out + R * pitch;
   if (local >= j.rows) {  // padding row of the job's last tile
-    for (int64_t k = 4 * tid; k < kp; k += 1024) {
+    for (int64_t k = 4 * tid; k < kp; k += 4 * TPR) {
       *reinterpret_cast<uint2*>(ph + k) = make_uint2(0u, 0u);
       *reinterpret_cast<uint2*>(ph + sd.piece_stride + k) = make_uint2(0u, 0u);
     }
@@ -855,12 +913,12 @@ __global__ void __launch_bounds__(256) f16_row_prep_kernel(RowPrepSide side_a, R
     return;
   }
   const float* __restrict__ src = j.src + local * j.rs;
-  const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+  const int width = row_width(src);
   float4 x[NV];
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
-    const int64_t k = 4 * (tid + 256 * i);
-    x[i] = k < j.K ? dev::ld_stream(reinterpret_cast<const float4*>(src + k)) : zero4;
+    const int64_t k = 4 * (tid + TPR * i);
+    x[i] = load_row4(src + k, j.K - k, width);
   }
   unsigned mx = 0u, mn = 0xFFFFFFFFu;
 #pragma unroll
@@ -873,18 +931,8 @@ __global__ void __launch_bounds__(256) f16_row_prep_kernel(RowPrepSide side_a, R
     mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
   }
-  if (lane == 0) {
-    red_max[warp] = mx;
-    red_min[warp] = mn;
-  }
-  __syncthreads();
-  if (tid == 0) {
-    unsigned w = red_max[0], v = red_min[0];
-#pragma unroll
-    for (int i = 1; i < 8; ++i) {
-      w = max(w, red_max[i]);
-      v = min(v, red_min[i]);
-    }
+  // the row's records by one thread; its shift (15 - e) to all of them
+  auto record = [&](unsigned w, unsigned v) {
     int e_store = 0;  // what f16_scale_kernel leaves: kExpBias + exponent, 0 for an all-zero row
     if (w != 0u) {
       int e;
@@ -900,13 +948,33 @@ __global__ void __launch_bounds__(256) f16_row_prep_kernel(RowPrepSide side_a, R
       sd.guard.flags[R] = out_of_span;
       if (out_of_span) sd.guard.list[atomicAdd(sd.guard.count, 1)] = (int)R;
     }
-    sh_shift = kF16ScaleTop - e;
+    return kF16ScaleTop - e;
+  };
+  int sh = 0;
+  if constexpr (TPR == 32) {
+    if (lane == 0) sh = record(mx, mn);
+    sh = __shfl_sync(0xffffffffu, sh, 0);
+  } else {
+    if (lane == 0) {
+      red_max[warp] = mx;
+      red_min[warp] = mn;
+    }
+    __syncthreads();
+    if (tid == 0) {
+      unsigned w = red_max[0], v = red_min[0];
+#pragma unroll
+      for (int i = 1; i < 8; ++i) {
+        w = max(w, red_max[i]);
+        v = min(v, red_min[i]);
+      }
+      sh_shift = record(w, v);
+    }
+    __syncthreads();
+    sh = sh_shift;
   }
-  __syncthreads();
-  const int sh = sh_shift;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
-    const int64_t k = 4 * (tid + 256 * i);
+    const int64_t k = 4 * (tid + TPR * i);
     if (k < kp) {
       float4 v = make_float4(scale_pow2(x[i].x, sh), scale_pow2(x[i].y, sh), scale_pow2(x[i].z, sh),
                              scale_pow2(x[i].w, sh));
@@ -1733,6 +1801,7 @@ struct TcGroupPlan {
   bool row_prep_a = false, row_prep_b = false;  // FP16 split: operand prepared by f16_row_prep_kernel
   bool col_scale_a = false, col_scale_b = false;  // FP16 split: exponents by f16_col_scale_kernel
   bool row_split_a = false, row_split_b = false;  // BF16 split: operand prepared by split_rows_kernel
+  bool prep_vec_a = false, prep_vec_b = false;    // prep_group_kernel: 128-bit loads for every job of the operand
   int a_col_ctas = 0, b_col_ctas = 0, col_kblk = 128;
   size_t off_gmin = 0, off_gflag = 0, off_glist = 0;  // guard arrays: A rows then B rows each
   size_t off_init_end = 0;  // the launch clears [kTileCounterOffset, off_init_end)
@@ -1850,29 +1919,31 @@ gbblas_status plan_group(int mode, const gbblas_gemm_desc* d, int64_t count, TcG
     pl.b_rows += Np;
   }
   pl.nprob = (int)pl.probs.size();
+  // (each float4 then lies wholly inside or wholly outside the operand)
+  auto vec_ok = [](const SplitJob& j) {
+    return (reinterpret_cast<uintptr_t>(j.src) & 15) == 0 &&
+           ((j.cs == 1 && (j.rs & 3) == 0 && (j.K & 3) == 0) || (j.rs == 1 && (j.cs & 3) == 0 && (j.rows & 3) == 0));
+  };
+  pl.prep_vec_a = std::all_of(pl.ajobs.begin(), pl.ajobs.end(), vec_ok);
+  pl.prep_vec_b = std::all_of(pl.bjobs.begin(), pl.bjobs.end(), vec_ok);
   if (pl.mode == 2 || pl.mode == 3) {
     // the BF16 split's pieces straight from registers where every job of an
-    // operand has K contiguous, 16-byte aligned rows and K a multiple of 4
-    auto split_ok = [](const SplitJob& j) {
-      return j.cs == 1 && (j.rs & 3) == 0 && (reinterpret_cast<uintptr_t>(j.src) & 15) == 0 && (j.K & 3) == 0;
-    };
+    // operand has K contiguous
+    auto split_ok = [](const SplitJob& j) { return j.cs == 1; };
     pl.row_split_a = std::all_of(pl.ajobs.begin(), pl.ajobs.end(), split_ok);
     pl.row_split_b = std::all_of(pl.bjobs.begin(), pl.bjobs.end(), split_ok);
   }
   if (pl.f16()) {
-    // one-pass preparation where every job of an operand has K contiguous,
-    // 16-byte aligned rows, K a multiple of 4 within the kernel's reach
+    // one-pass preparation where every job of an operand has K contiguous
+    // and within the kernel's reach
     auto row_ok = [](const SplitJob& j) {
-      return j.cs == 1 && (j.rs & 3) == 0 && (reinterpret_cast<uintptr_t>(j.src) & 15) == 0 && (j.K & 3) == 0 &&
-             j.K >= kRowPrepMinK && (int64_t)j.tiles_k * PrepTile<kModeF16>::TK <= 1024 * kRowPrepNV;
+      return j.cs == 1 && (int64_t)j.tiles_k * PrepTile<kModeF16>::TK <= 1024 * kRowPrepNV;
     };
     pl.row_prep_a = std::all_of(pl.ajobs.begin(), pl.ajobs.end(), row_ok);
     pl.row_prep_b = std::all_of(pl.bjobs.begin(), pl.bjobs.end(), row_ok);
     // the exponents of an operand whose rows are contiguous by a column
     // reduction (its pieces still come from the tile kernel)
-    auto col_ok = [](const SplitJob& j) {
-      return j.rs == 1 && (j.cs & 3) == 0 && (reinterpret_cast<uintptr_t>(j.src) & 15) == 0 && (j.rows & 3) == 0;
-    };
+    auto col_ok = [](const SplitJob& j) { return j.rs == 1; };
     auto number = [](std::vector<SplitJob>& jobs, int kblk) {
       int64_t n = 0;
       for (SplitJob& j : jobs) {
@@ -2087,7 +2158,12 @@ gbblas_status launch_bound(DeviceCtx* c, const TcGroupPlan& pl, cudaStream_t str
       const RowPrepSide rb{djobs + pl.njobs, pl.row_prep_b ? (int)pl.b_rows : 0,
                            reinterpret_cast<__half*>(arena_b(pl)), (int64_t)(pl.b_rows * pl.pitch),
                            reinterpret_cast<int*>(scales_b(pl)), gb};
-      f16_row_prep_kernel<<<ra.rows + rb.rows, 256, 0, stream>>>(ra, rb, pl.njobs, pl.pitch);
+      // a warp per row while the group's longest row fits its registers (a
+      // CTA per row would leave most of its threads without an element)
+      if (pl.kpad <= 128 * kRowPrepNV)
+        f16_row_prep_kernel<32><<<(ra.rows + rb.rows) / 8, 256, 0, stream>>>(ra, rb, pl.njobs, pl.pitch);
+      else
+        f16_row_prep_kernel<256><<<ra.rows + rb.rows, 256, 0, stream>>>(ra, rb, pl.njobs, pl.pitch);
       GB_TRY(check_launch("f16_row_prep_kernel"));
     }
     // per-row exponents of A's and B^T's arena rows (and the guard's
@@ -2115,7 +2191,10 @@ gbblas_status launch_bound(DeviceCtx* c, const TcGroupPlan& pl, cudaStream_t str
   if (prep_ctas > 0) {
     const PrepSide pa{djobs, a_tiles, arena_a(pl), (int64_t)(pl.a_rows * pl.pitch), scales_a(pl), ga};
     const PrepSide pb{djobs + pl.njobs, b_tiles, arena_b(pl), (int64_t)(pl.b_rows * pl.pitch), scales_b(pl), gb};
-    prep_group_kernel<MODE><<<prep_ctas, 256, 0, stream>>>(pa, pb, pl.njobs, pl.pitch, pl.kpad);
+    if ((a_tiles == 0 || pl.prep_vec_a) && (b_tiles == 0 || pl.prep_vec_b))
+      prep_group_kernel<MODE, true><<<prep_ctas, 256, 0, stream>>>(pa, pb, pl.njobs, pl.pitch, pl.kpad);
+    else
+      prep_group_kernel<MODE, false><<<prep_ctas, 256, 0, stream>>>(pa, pb, pl.njobs, pl.pitch, pl.kpad);
     GB_TRY(check_launch("prep_group_kernel"));
   }
   // the GEMM, as `slices` launches over consecutive ranges of whole waves of

@@ -11,15 +11,16 @@ pytestmark = pytest.mark.gpu
 BF16X3, FP8, BF16X6, FP16X3 = 1, 2, 4, 8
 
 
-def place(torch, X, pitch, off, col_major=False):
+def place(torch, X, pitch, off, col_major=False, step=1):
     """X (numpy, 2-D) in a device buffer: row (column) pitch `pitch`, first
-    element at `off`; returns (buffer, address, row stride, column stride)."""
+    element at `off`, neighbours `step` apart; returns (buffer, address, row
+    stride, column stride, the elements' places, their shape)."""
     v = X.T if col_major else X
-    buf = np.full(off + v.shape[0] * pitch + 7, np.float32(-77.0), np.float32)
-    at = (off + np.arange(v.shape[0])[:, None] * pitch + np.arange(v.shape[1])[None, :]).ravel()
+    buf = np.full(off + v.shape[0] * pitch * step + 7, np.float32(-77.0), np.float32)
+    at = (off + np.arange(v.shape[0])[:, None] * pitch * step + np.arange(v.shape[1])[None, :] * step).ravel()
     buf[at] = v.ravel()
     t = torch.from_numpy(buf).cuda()
-    rs, cs = (1, pitch) if col_major else (pitch, 1)
+    rs, cs = (step, pitch * step) if col_major else (pitch * step, step)
     return t, t.data_ptr() + 4 * off, rs, cs, at, v.shape
 
 
@@ -27,8 +28,8 @@ def gemm(torch, A, B, C0, acc, pa, pb, pc, la=False, lb=False, lc=False):
     import gbblas
     M, K = A.shape
     N = B.shape[1]
-    a = place(torch, A, (M if la else K) + pa[0], pa[1], la)
-    b = place(torch, B, (K if lb else N) + pb[0], pb[1], lb)
+    a = place(torch, A, (M if la else K) + pa[0], pa[1], la, *pa[2:])
+    b = place(torch, B, (K if lb else N) + pb[0], pb[1], lb, *pb[2:])
     c = place(torch, C0, (M if lc else N) + pc[0], pc[1], lc)
     gbblas.call("gbblas_sgemm", M, N, K, a[1], a[2], a[3], b[1], b[2], b[3], c[1], c[2], c[3], acc, None)
     gbblas.call("gbblas_check_stream", None)
@@ -54,4 +55,23 @@ def test_unaligned_c_same_bits_as_aligned(cuda, acc, M, N, K, pad, off):
     A, B, C0 = values(rng, (M, K)), values(rng, (K, N)), values(rng, (M, N))
     want = gemm(cuda, A, B, C0, acc, (0, 0), (0, 0), (0, 0))
     got = gemm(cuda, A, B, C0, acc, (0, 0), (0, 0), (pad, off))
+    np.testing.assert_array_equal(got, want)
+
+
+# Operands: every preparation route (K contiguous at 16-, 8- and 4-byte
+# aligned rows, one pass per row or per warp; rows contiguous, aligned or not)
+# against the strided tile route (neighbours two apart) on the same values
+@pytest.mark.parametrize("acc", [BF16X3, BF16X6, FP16X3, FP8])
+@pytest.mark.parametrize("M,N,K", [(130, 135, 1), (129, 260, 67), (140, 1030, 1023), (65, 129, 1025), (40, 30, 8191),
+                                   (16, 20, 8200)])
+@pytest.mark.parametrize("pad,off", [(0, 0), (1, 0), (2, 2), (3, 1)])
+@pytest.mark.parametrize("cols", [False, True])
+def test_operand_routes_same_bits(cuda, acc, M, N, K, pad, off, cols):
+    rng = np.random.default_rng(M + N * 3 + K)
+    A = (values(rng, (M, K)) * np.float32(2.0) ** rng.integers(-6, 7, (M, K))).astype(np.float32)
+    B = (values(rng, (K, N)) * np.float32(2.0) ** rng.integers(-6, 7, (K, N))).astype(np.float32)
+    A[M // 2] = 0.0
+    C0 = values(rng, (M, N))
+    want = gemm(cuda, A, B, C0, acc, (0, 0, 2), (0, 0, 2), (0, 0), False, False)
+    got = gemm(cuda, A, B, C0, acc, (pad, off), (pad, off), (0, 0), cols, not cols)
     np.testing.assert_array_equal(got, want)
