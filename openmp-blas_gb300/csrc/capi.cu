@@ -287,7 +287,7 @@ gbblas_status gemm_any(DeviceCtx* c, int64_t M, int64_t N, int64_t K, const T* A
     if (mode != 0) return launch_gemm_tc(c, mode, M, N, K, A, rsa, csa, B, rsb, csb, C, rsc, csc, s);
     // FP32 on the FMA pipe: the tile shape the autotuner measured faster
     return launch_gemm_fma<T>(c, M, N, K, A, rsa, csa, B, rsb, csb, C, rsc, csc, s, 0,
-                              tuned_fma_tile(c, M, N, K, s));
+                              tuned_fma_tile(c, {M, N, K, A, rsa, csa, B, rsb, csb, C, rsc, csc}, s));
   }
   return launch_gemm_fma<T>(c, M, N, K, A, rsa, csa, B, rsb, csb, C, rsc, csc, s);
 }

@@ -133,15 +133,19 @@ gbblas_status launch_dot(DeviceCtx* c, int64_t n, const T* a, const T* b, T* res
 
 // max_ctas > 0 caps the grid (the kernel loops over tiles), leaving SMs to
 // other streams.
-// tile (FP32 only): 3 = TMA-fed, stream-K (K blocks shared out equally among the SMs),
-// 2 = TMA-fed 128 x 128 kernel (gemm_fma_tma.cu; where
-// sgemm_tma_eligible), 1 = 128 x 128 CTA tiles, 0 = 64 x 64, -1 = by the
-// tile count (TMA-fed for a row-major B once the 128 x 128 tiles fill the
-// SMs, register-staged 128 x 128 from twice that, else 64 x 64).
+// tile (FP32 only): 0 = 64 x 64 CTA tiles, 1 = 128 x 128, 2 = TMA-fed 128 x
+// 128 kernel (gemm_fma_tma.cu; where sgemm_tma_eligible, else 1), 3 = that
+// with stream-K (K blocks shared out equally among the SMs), 4 = that in
+// cluster pairs, 5 / 6 = 64 x 64 / 128 x 128 with K cut over the CTAs of a
+// cluster where the tiles leave SMs idle, -1 = by the tile count (TMA-fed for
+// a row-major B once the 128 x 128 tiles fill the SMs, 128 x 128 from twice
+// that, else 5).  Double: 64 x 64, K cut likewise.
 template <typename T>
 gbblas_status launch_gemm_fma(DeviceCtx* c, int64_t M, int64_t N, int64_t K, const T* A, int64_t rsa,
                               int64_t csa, const T* B, int64_t rsb, int64_t csb, T* C, int64_t rsc,
                               int64_t csc, cudaStream_t stream, int max_ctas = 0, int tile = -1);
+
+void gemm_fma_prepare(DeviceCtx* c);  // kernel attributes, before any stream capture
 
 // FP32 C += A*B on the FMA pipes with TMA-fed operands (gemm_fma_tma.cu):
 // A and B each row- or column-major, 16-byte aligned, row / column pitch a
@@ -243,7 +247,7 @@ int tuned_gemm_auto(DeviceCtx* c, int64_t M, int64_t N, int64_t K);
 // Autotuner: split-K parts and CTA form of one tensor-core GEMM.
 TcLaunchOpts tuned_tc_opts(DeviceCtx* c, int mode, int64_t M, int64_t N, int64_t K, cudaStream_t stream);
 // Autotuner: FP32 FMA tile (launch_gemm_fma's `tile`).
-int tuned_fma_tile(DeviceCtx* c, int64_t M, int64_t N, int64_t K, cudaStream_t stream);
+int tuned_fma_tile(DeviceCtx* c, const gbblas_gemm_desc& g, cudaStream_t stream);
 
 // Streaming operations beside the hot path (stream_ops.cu).
 // C[r*ld + l] += u[r] * v[l] (rows of C contiguous).

@@ -2267,6 +2267,7 @@ size_t tc_arena_bytes(int mode, int64_t M, int64_t N, int64_t K) {
 }
 
 void tc_prepare(DeviceCtx* c) {
+  gemm_fma_prepare(c);
   sgemm_tma_prepare(c);
   dgemm_digits_prepare(c);
   kernel_setup<2, false>(c);

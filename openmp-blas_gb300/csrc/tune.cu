@@ -24,10 +24,12 @@
 //                    the output tiles fill at most half the SMs) and the CTA
 //                    form (single CTAs or CTA pairs, split-BF16 only);
 //                    GBBLAS_TC_SPLITK=n forces n parts;
-//   gemm_fma_tile    FP32 FMA kernel and CTA tile per bucket: 64 x 64 or
-//                    128 x 128 register-staged, the TMA-fed 128 x 128, or
-//                    that in stream-K form where whole tiles fill the SMs badly;
-//                    GBBLAS_FMA_TILE=0 / 1 / 2 / 3 forces one.
+//   gemm_fma_tile    FP32 FMA kernel and CTA tile per bucket, operand
+//                    layouts and alignment: 64 x 64 or 128 x 128 (K cut over
+//                    a cluster's CTAs where those leave SMs idle), the TMA-fed
+//                    128 x 128, that in stream-K form where whole tiles fill
+//                    the SMs badly, or in cluster pairs;
+//                    GBBLAS_FMA_TILE=0 .. 6 forces one (launch_gemm_fma's list).
 // Nothing is timed while the caller's stream is being captured into a graph
 // (the defaults apply); single-call paths consult the tuner, grouped,
 // batched and served launches use the defaults.
@@ -151,11 +153,14 @@ bool capturing(cudaStream_t s) {
 
 // Scratch FP32 operands (zeros) for timing one GEMM shape on the tuner's own
 // stream; each candidate runs once to warm up, then 3 times between events.
+// a_col / b_col: column-major operands (C is row-major); pad: leading
+// dimensions that much longer than they need be.
 class GemmBench {
  public:
-  GemmBench(DeviceCtx* c, int64_t m, int64_t n, int64_t k) : c_(c), m_(m), n_(n), k_(k) {
+  GemmBench(DeviceCtx* c, int64_t m, int64_t n, int64_t k, bool a_col = false, bool b_col = false, int64_t pad = 0)
+      : c_(c), m_(m), n_(n), k_(k), a_col_(a_col), b_col_(b_col), pad_(pad) {
     if (cudaStreamCreateWithFlags(&s_, cudaStreamNonBlocking) != cudaSuccess) return;
-    const size_t bytes = sizeof(float) * (size_t)(m * k + k * n + m * n);
+    const size_t bytes = sizeof(float) * (size_t)(a_elems() + b_elems() + m * n);
     if (cudaMallocAsync(&mem_, bytes, s_) != cudaSuccess) {
       mem_ = nullptr;
       return;
@@ -177,9 +182,11 @@ class GemmBench {
   bool ok() const { return mem_ != nullptr; }
   gbblas_gemm_desc desc() const {
     float* A = static_cast<float*>(mem_);
-    float* B = A + m_ * k_;
-    float* C = B + k_ * n_;
-    return gbblas_gemm_desc{m_, n_, k_, A, k_, 1, B, n_, 1, C, n_, 1};
+    float* B = A + a_elems();
+    float* C = B + b_elems();
+    const int64_t lda = (a_col_ ? m_ : k_) + pad_, ldb = (b_col_ ? k_ : n_) + pad_;
+    return gbblas_gemm_desc{m_, n_, k_, A, a_col_ ? 1 : lda, a_col_ ? lda : 1, B, b_col_ ? 1 : ldb, b_col_ ? ldb : 1,
+                            C, n_, 1};
   }
   cudaStream_t stream() const { return s_; }
   // ms per call of run(stream), or a huge value if it failed
@@ -197,8 +204,14 @@ class GemmBench {
   }
 
  private:
+  // (rounded so that B and C start on 16-byte boundaries)
+  int64_t a_elems() const { return ((a_col_ ? k_ * (m_ + pad_) : m_ * (k_ + pad_)) + 3) / 4 * 4; }
+  int64_t b_elems() const { return ((b_col_ ? n_ * (k_ + pad_) : k_ * (n_ + pad_)) + 3) / 4 * 4; }
+
   DeviceCtx* c_;
   int64_t m_, n_, k_;
+  bool a_col_, b_col_;
+  int64_t pad_;
   cudaStream_t s_ = nullptr;
   void* mem_ = nullptr;
   cudaEvent_t e0_ = nullptr, e1_ = nullptr;
@@ -370,28 +383,42 @@ TcLaunchOpts tuned_tc_opts(DeviceCtx* c, int mode, int64_t M, int64_t N, int64_t
   return best;
 }
 
-int tuned_fma_tile(DeviceCtx* c, int64_t M, int64_t N, int64_t K, cudaStream_t stream) {
-  if (const char* e = std::getenv("GBBLAS_FMA_TILE"); e && e[0] >= '0' && e[0] <= '4') return e[0] - '0';
+int tuned_fma_tile(DeviceCtx* c, const gbblas_gemm_desc& g, cudaStream_t stream) {
+  if (const char* e = std::getenv("GBBLAS_FMA_TILE"); e && e[0] >= '0' && e[0] <= '6') return e[0] - '0';
+  if ((double)g.M * g.N * g.K < 1.0e8) return -1;  // small: the tile-count rule
+  // a column-major C runs as its transpose (launch_gemm_fma): tune that
+  const bool flip = g.csc != 1 && g.rsc == 1;
+  const int64_t M = flip ? g.N : g.M, N = flip ? g.M : g.N, K = g.K;
+  const int64_t rsa = flip ? g.csb : g.rsa, csa = flip ? g.rsb : g.csa;
+  const int64_t rsb = flip ? g.csa : g.rsb, csb = flip ? g.rsa : g.csb;
+  const float *A = flip ? g.B : g.A, *B = flip ? g.A : g.B;
+  const bool a_col = rsa == 1 && csa != 1, b_col = rsb == 1 && csb != 1;
+  // operands TMA cannot fetch never take its kernels, and are timed with
+  // leading dimensions off the 16-byte grid
+  const bool tma = sgemm_tma_eligible(M, N, K, A, rsa, csa, B, rsb, csb);
   Tuner& t = Tuner::get();
   const int bm = log2_bucket(M), bn = log2_bucket(N), bk = log2_bucket(K);
   const std::string key = "gemm_fma_tile|" + device_tag(c) + "|m" + std::to_string(bm) + "|n" + std::to_string(bn) +
-                          "|k" + std::to_string(bk) + "|f32";
+                          "|k" + std::to_string(bk) + (a_col ? "|ac" : "|ar") + (b_col ? "|bc" : "|br") +
+                          (tma ? "|t" : "|u") + "|f32";
   const int v = t.lookup(key);
   if (v >= 0) return v;
-  if (!t.enabled() || capturing(stream) || (double)M * N * K < 1.0e8) return -1;  // small: the tile-count rule
+  if (!t.enabled() || capturing(stream)) return -1;
   int64_t m, n, k;
   bucket_shape(bm, bn, bk, m, n, k);
-  GemmBench b(c, m, n, k);
+  GemmBench b(c, m, n, k, a_col, b_col, tma ? 0 : 1);
   if (!b.ok()) return -1;
   const gbblas_gemm_desc d = b.desc();
-  // 0 = 64 x 64, 1 = 128 x 128 (register-staged), 2 = TMA-fed 128 x 128,
-  // 3 = TMA-fed stream-K, offered where whole tiles fill the SMs badly, 4 =
-  // TMA-fed cluster pairs, offered where two CTAs per tile fill the SMs in
-  // one wave (the TMA kernels' eligibility is the caller's operands': an
-  // ineligible call falls back)
-  std::vector<int> tiles{0, 1, 2};
-  if (sgemm_tma_streamk_useful(c, m, n, k)) tiles.push_back(3);
-  if (sgemm_tma_pairs_useful(c, m, n, k)) tiles.push_back(4);
+  // 5 / 6 = 64 x 64 / 128 x 128 CTA tiles, K cut over the CTAs of a cluster
+  // where they leave SMs idle; 2 = TMA-fed 128 x 128, 3 = TMA-fed stream-K,
+  // offered where whole tiles fill the SMs badly, 4 = TMA-fed cluster pairs,
+  // offered where two CTAs per tile fill the SMs in one wave
+  std::vector<int> tiles{5, 6};
+  if (tma) {
+    tiles.push_back(2);
+    if (sgemm_tma_streamk_useful(c, m, n, k)) tiles.push_back(3);
+    if (sgemm_tma_pairs_useful(c, m, n, k)) tiles.push_back(4);
+  }
   int best = -1;
   float best_ms = 1e30f;
   for (int tile : tiles) {
