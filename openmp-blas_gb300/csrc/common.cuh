@@ -273,7 +273,38 @@ gbblas_status check_stream_errors(DeviceCtx* c, cudaStream_t stream);
 
 // ----------------------------------------------------------- device helpers
 #ifdef __CUDACC__
+namespace gbblas {
+
+// Launch `kernel` behind this library's previous kernel on the stream without
+// waiting for its end (programmatic dependent launch): its CTAs may be set up
+// while the previous kernel's last CTAs run, which takes the launch gap
+// (about 1 us) off a chain of short kernels.  Only for a kernel whose every
+// CTA calls dev::grid_wait() before it touches memory, and only directly
+// behind a kernel of this library that does the same or was launched plainly.
+template <typename... P, typename... A>
+cudaError_t launch_after(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+}  // namespace gbblas
+
 namespace gbblas::dev {
+
+// Programmatic dependent launch (launch_after): let the next kernel's CTAs be
+// set up from here on / wait until the kernels before this one have finished
+// and their writes are visible (at once in a plain launch).
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Streaming loads: read-only path, no L1 allocation (data is used once).
 __device__ __forceinline__ float4 ld_stream(const float4* p) {

@@ -83,6 +83,7 @@
 #include <cstring>
 #include <mutex>
 #include <numeric>
+#include <utility>
 #include <vector>
 
 #include "common.cuh"
@@ -203,20 +204,22 @@ struct TcProblem {
   CUtensorMap c_map;  // FP8 with c_tma: C as a float tensor, 32 x 32 boxes, 128-byte swizzle
   int c_tma;          // 1: the epilogue adds into C with TMA reduce-add stores
   int M, N;
-  int num_kt;      // K stages of this (sub)problem: 64 of K (BF16) or 256 (FP8) each
-  int kt0;         // its first K stage (a split-K part covers stages kt0 .. kt0 + num_kt - 1)
+  int num_kt;      // K stages: 64 of K (BF16) or 256 (FP8) each
+  int parts;       // split-K parts: part p covers stages num_kt p / parts .. num_kt (p + 1) / parts - 1
   int a_row;       // first row of this problem in the A arena (piece 0)
   int b_row;       // first row in the B^T arena (piece 0)
   int tiles_m, tiles_n;
-  int tile_start;  // first global tile index of this problem
-  int overwrite;   // 1: the epilogue stores (a split-K partial), 0: C += result
-  float* C;
+  int tile_start;  // first global tile index of this problem (parts x tiles_m x tiles_n tiles)
+  float* C;        // parts = 1: C += result
   int64_t rsc, csc;
+  float* ws;       // parts > 1: part p stores its sums at ws + p * ws_plane, contiguous where C is
+  int64_t ws_rs, ws_cs, ws_plane;
 };
 
 // One split-K problem's final step: C += sum over s of part[s] (in order of
 // s, so the result does not depend on which part finished first); parts are
-// M x pitch row-major, `parts` x M x pitch floats in all.
+// M x pitch row-major, `parts` x M x pitch floats in all (M and N are those of
+// C^T where C is column-major).
 struct SplitReduce {
   float* C;
   int64_t rsc, csc;
@@ -350,6 +353,8 @@ struct ScaleSide {
 // rows' extremes of a tile combined in shared memory, then atomicMax-ed
 // into the encodings above.
 __global__ void __launch_bounds__(256) f16_scale_kernel(ScaleSide side_a, ScaleSide side_b, int njobs) {
+  dev::grid_release();
+  dev::grid_wait();
   constexpr int TK = 64, TR = 64;
   __shared__ unsigned int rmax[TR], rmin[TR];
   __shared__ int sjob;
@@ -522,6 +527,8 @@ __device__ __forceinline__ int prep_slot(int r, int k) {
 template <int MODE, bool VEC>
 __global__ void __launch_bounds__(256, VEC ? 1 : 4) prep_group_kernel(PrepSide side_a, PrepSide side_b, int njobs,
                                                                       int64_t pitch, int64_t scale_stride) {
+  dev::grid_release();
+  dev::grid_wait();
   using PT = PrepTile<MODE>;
   constexpr int TK = PT::TK, TR = PT::TR, LD = PT::LD;
   __shared__ __align__(16) float tile[TR * LD];
@@ -706,6 +713,8 @@ constexpr int kColScaleK = 128;
 
 __global__ void __launch_bounds__(256, 4) f16_col_scale_kernel(ScaleSide side_a, ScaleSide side_b, int njobs,
                                                                int kblk) {
+  dev::grid_release();
+  dev::grid_wait();
   const bool on_b = (int)blockIdx.x >= side_a.tiles;
   const ScaleSide& sd = on_b ? side_b : side_a;
   const int t = (int)blockIdx.x - (on_b ? side_a.tiles : 0);
@@ -794,9 +803,14 @@ struct RowSplitSide {
 // once for all of them.
 constexpr int kSplitRowsPerCtaMax = 32;
 
+// blockIdx.y: which `kseg` K (a multiple of 512) of the rows (all of K unless
+// the rows alone would leave most SMs without a CTA: 32 rows of 7066 took 14
+// us, a serial chain of loads in 16 CTAs).
 template <int P>
 __global__ void __launch_bounds__(256) split_rows_kernel(RowSplitSide side_a, RowSplitSide side_b, int njobs,
-                                                         int64_t pitch, int rows_per_cta) {
+                                                         int64_t pitch, int rows_per_cta, int64_t kseg) {
+  dev::grid_release();
+  dev::grid_wait();
   __shared__ int sjob;
   const int a_ctas = side_a.rows / rows_per_cta;
   const bool on_b = (int)blockIdx.x >= a_ctas;
@@ -825,7 +839,8 @@ __global__ void __launch_bounds__(256) split_rows_kernel(RowSplitSide side_a, Ro
   const float* __restrict__ src = j.src + (local < j.rows ? local : 0) * j.rs;
   const int w = row_width(src);
   __nv_bfloat16* __restrict__ dst = sd.out + R * pitch;
-  for (int64_t k0 = 4 * lane; k0 < kp; k0 += 4 * 128) {
+  const int64_t kbeg = (int64_t)blockIdx.y * kseg, kend = min(kp, kbeg + kseg);
+  for (int64_t k0 = kbeg + 4 * lane; k0 < kend; k0 += 4 * 128) {
     float4 x[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
@@ -883,6 +898,8 @@ struct RowPrepSide {
 template <int TPR>
 __global__ void __launch_bounds__(256) f16_row_prep_kernel(RowPrepSide side_a, RowPrepSide side_b, int njobs,
                                                            int64_t pitch) {
+  dev::grid_release();
+  dev::grid_wait();
   constexpr int NV = kRowPrepNV;
   constexpr int RPC = 256 / TPR;  // rows per CTA (of one job: its rows are padded to a multiple of 128)
   __shared__ unsigned red_max[8], red_min[8];
@@ -1009,20 +1026,38 @@ __device__ __forceinline__ int find_problem(const TcProblem* __restrict__ probs,
   return lo;
 }
 
-// Output tile of global index t (BMT rows x 128 columns): grouped raster
-// inside its problem (consecutive tiles walk 8 row-tiles of one column band
+// One tile's work: output tile (BMT rows x 128 columns) at (m0, n0), K
+// stages kt0 .. kt0 + nkt - 1 (those of its split-K part).
+struct TileWork {
+  int m0, n0, kt0, nkt, part;
+};
+
+// Global tile index t: the parts of a split problem one after another, each
+// in a grouped raster (consecutive tiles walk 8 row-tiles of one column band
 // for L2 reuse).
 template <int BMT>
-__device__ __forceinline__ void tile_coords(const TcProblem& p, int t, int& m0, int& n0) {
+__device__ __forceinline__ TileWork tile_work(const TcProblem& p, int t) {
   constexpr int kGroup = 8;
-  const int local = t - p.tile_start;
+  TileWork w;
+  int local = t - p.tile_start;
+  w.part = 0;
+  w.kt0 = 0;
+  w.nkt = p.num_kt;
+  if (p.parts > 1) {
+    const int tiles = p.tiles_m * p.tiles_n;
+    w.part = local / tiles;
+    local %= tiles;
+    w.kt0 = (int)((int64_t)p.num_kt * w.part / p.parts);
+    w.nkt = (int)((int64_t)p.num_kt * (w.part + 1) / p.parts) - w.kt0;
+  }
   const int group_span = kGroup * p.tiles_n;
   const int g = local / group_span;
   const int first_m = g * kGroup;
   const int gm = min(p.tiles_m - first_m, kGroup);
   const int in_g = local % group_span;
-  m0 = (first_m + in_g % gm) * BMT;
-  n0 = (in_g / gm) * kBN;
+  w.m0 = (first_m + in_g % gm) * BMT;
+  w.n0 = (in_g / gm) * kBN;
+  return w;
 }
 
 // PAIR = false: one CTA per SM computes 128 x 128 tiles (tcgen05 .cta_group::1).
@@ -1112,6 +1147,7 @@ __global__ void __launch_bounds__(ModeTraits<MODE>::kThreads, 1)
   __syncthreads();
   if constexpr (PAIR) cluster_sync_all();  // the peer's barriers exist before anyone signals them
   tc_fence_after();
+  dev::grid_wait();  // the set-up above overlapped the preparation's last CTAs
   const uint32_t tmem = *tmem_slot;
 
   auto fail = [&]() {
@@ -1140,17 +1176,16 @@ __global__ void __launch_bounds__(ModeTraits<MODE>::kThreads, 1)
         mbar_arrive(&ring_full[slot]);  // release: consumers see ring[slot]
         if (t < 0) break;
         const TcProblem& pr = probs[find_problem(probs, nprob, t)];
-        int m0, n0;
-        tile_coords<BMT>(pr, t, m0, n0);
-        const int own_m0 = m0 + (int)rank * kBM;  // this CTA's rows
-        for (int kt = 0; kt < pr.num_kt; ++kt) {
+        const TileWork tw = tile_work<BMT>(pr, t);
+        const int n0 = tw.n0, own_m0 = tw.m0 + (int)rank * kBM;  // this CTA's rows
+        for (int kt = 0; kt < tw.nkt; ++kt) {
           const int s = issued % ST, round = issued / ST;
           if (round > 0 && !mbar_wait_bounded(&empty[s], (round - 1) & 1, abort_flag, kWaitLimitNs)) {
             fail();
             stop = true;
             break;
           }
-          const int kx = (pr.kt0 + kt) * MT::kBKe;  // first K element of the stage
+          const int kx = (tw.kt0 + kt) * MT::kBKe;  // first K element of the stage
           // one 3-D copy per operand brings all P piece planes of the tile
           if constexpr (PAIR) {
             if (rank == 0) {
@@ -1198,16 +1233,16 @@ __global__ void __launch_bounds__(ModeTraits<MODE>::kThreads, 1)
         mbar_arrive(&ring_empty[slot]);
         if (t < 0) break;
         const TcProblem& pr = probs[find_problem(probs, nprob, t)];
-        int m0, n0;
-        tile_coords<BMT>(pr, t, m0, n0);
-        for (int kt = 0; kt < pr.num_kt; ++kt) {
+        const TileWork tw = tile_work<BMT>(pr, t);
+        const int n0 = tw.n0;
+        for (int kt = 0; kt < tw.nkt; ++kt) {
           const int s = bissued % ST, round = bissued / ST;
           if (round > 0 && !mbar_wait_bounded(&empty[s], (round - 1) & 1, abort_flag, kWaitLimitNs)) {
             fail();
             stop = true;
             break;
           }
-          const int kx = (pr.kt0 + kt) * MT::kBKe;
+          const int kx = (tw.kt0 + kt) * MT::kBKe;
           mbar_arrive_expect_tx(&full[s], CF::kBStageBytes);
           if constexpr (MT::fp8) {
 #pragma unroll
@@ -1255,7 +1290,7 @@ __global__ void __launch_bounds__(ModeTraits<MODE>::kThreads, 1)
         const int t = ring[slot];
         mbar_arrive(&ring_empty[slot]);
         if (t < 0) break;
-        const int num_kt = probs[find_problem(probs, nprob, t)].num_kt;
+        const int num_kt = tile_work<BMT>(probs[find_problem(probs, nprob, t)], t).nkt;
         for (int kt = 0; kt < num_kt; ++kt) {
           const int s = consumed % ST, round = consumed / ST;
           const bool chunk_first = (kt % MT::kChunk) == 0;
@@ -1373,10 +1408,9 @@ __global__ void __launch_bounds__(ModeTraits<MODE>::kThreads, 1)
       if (lane == 0) mbar_arrive(&ring_empty[slot]);
       if (t < 0) break;
       const TcProblem& pr = probs[find_problem(probs, nprob, t)];
-      int m0, n0;
-      tile_coords<BMT>(pr, t, m0, n0);
-      m0 += (int)rank * kBM;  // this CTA's rows
-      const int nchunks = (pr.num_kt + MT::kChunk - 1) / MT::kChunk;
+      const TileWork tw = tile_work<BMT>(pr, t);
+      const int n0 = tw.n0, m0 = tw.m0 + (int)rank * kBM;  // this CTA's rows
+      const int nchunks = (tw.nkt + MT::kChunk - 1) / MT::kChunk;
       float acc[kCols];
 #pragma unroll
       for (int j = 0; j < kCols; ++j) acc[j] = 0.f;
@@ -1454,6 +1488,15 @@ __global__ void __launch_bounds__(ModeTraits<MODE>::kThreads, 1)
 #pragma unroll
           for (int c = 0; c < kCols; ++c)
             if (__ldg(guard_b + (int64_t)pr.b_row + n0 + col0 + c)) skip_cols |= uint64_t(1) << c;
+          // a split-K partial takes -0.0 there, which leaves C as it was when
+          // the parts are added into it
+          if (pr.parts > 1 && (skip_row || skip_cols)) {
+#pragma unroll
+            for (int c = 0; c < kCols; ++c)
+              if (skip_row || ((skip_cols >> c) & 1)) acc[c] = -0.0f;
+            skip_row = false;
+            skip_cols = 0;
+          }
         }
       }
       if constexpr (CF::kTmaC) {
@@ -1472,6 +1515,7 @@ __global__ void __launch_bounds__(ModeTraits<MODE>::kThreads, 1)
             }
           }
           float* scr = epi_scratch + (warp - 2) * 1024;
+          if (lane == 0) fence_tensormap(&pr.c_map);  // the tables were written after the driver last saw them
 #pragma unroll
           for (int cb = 0; cb < kCols; cb += 32) {
 #pragma unroll
@@ -1496,10 +1540,12 @@ __global__ void __launch_bounds__(ModeTraits<MODE>::kThreads, 1)
       // warp keeps 16 loads in flight before the first store (the compiler
       // cannot see that runtime strides keep the outputs apart: one output at
       // a time cost 300 of the kernel's 548 us at 3970 x 3475 x 4050).
-      const bool add = !pr.overwrite;
+      const bool add = pr.parts == 1;
+      float* Cd = add ? pr.C : pr.ws + (int64_t)tw.part * pr.ws_plane;
+      const int64_t rsc = add ? pr.rsc : pr.ws_rs, csc = add ? pr.csc : pr.ws_cs;
       const int row0 = m0 + q * 32, cn = n0 + col0;
       if constexpr (CF::kTmaC) {
-        if (pr.csc == 1) {
+        if (csc == 1) {
           // contiguous C rows of any alignment: the 32 x 32 blocks go through
           // shared memory (swizzled as for the TMA update) and the warp
           // updates one row's 32 columns, 128 bytes, per access
@@ -1514,19 +1560,19 @@ __global__ void __launch_bounds__(ModeTraits<MODE>::kThreads, 1)
                   make_float4(acc[cb + 4 * c], acc[cb + 4 * c + 1], acc[cb + 4 * c + 2], acc[cb + 4 * c + 3]);
             __syncwarp();
             const int col = cn + cb + lane;
-            const bool live = col < pr.N && !(MT::f16 && ((skip_cols >> (cb + lane)) & 1));
-            float* cp = pr.C + (int64_t)row0 * pr.rsc + col;
+            // rows r < rows of the block exist for this lane's column
+            const int rows = col < pr.N && !(MT::f16 && ((skip_cols >> (cb + lane)) & 1)) ? min(pr.M - row0, 32) : 0;
+            float* cp = Cd + (int64_t)row0 * rsc + col;
 #pragma unroll
             for (int r0 = 0; r0 < 32; r0 += 16) {
               float old[16];
+              const float* lp = cp;
 #pragma unroll
-              for (int r = 0; r < 16; ++r)
-                old[r] = (add && live && row0 + r0 + r < pr.M) ? cp[(int64_t)(r0 + r) * pr.rsc] : 0.f;
+              for (int r = 0; r < 16; ++r, lp += rsc) old[r] = (add && r0 + r < rows) ? *lp : 0.f;
 #pragma unroll
-              for (int r = 0; r < 16; ++r) {
+              for (int r = 0; r < 16; ++r, cp += rsc) {
                 const float v = scr[(r0 + r) * 32 + (((lane >> 2) ^ (r & 7)) * 4) + (lane & 3)];
-                if (live && row0 + r0 + r < pr.M && !((skip_rows >> (r0 + r)) & 1))
-                  cp[(int64_t)(r0 + r) * pr.rsc] = old[r] + v;
+                if (r0 + r < rows && !((skip_rows >> (r0 + r)) & 1)) *cp = add ? old[r] + v : v;
               }
             }
           }
@@ -1536,9 +1582,9 @@ __global__ void __launch_bounds__(ModeTraits<MODE>::kThreads, 1)
       // a thread per row (coalesced where C's columns are contiguous)
       const int row = row0 + lane;
       if (row < pr.M && !skip_row) {
-        float* crow = pr.C + (int64_t)row * pr.rsc;
-        const bool vec = (pr.csc == 1) && ((pr.rsc & 3) == 0) && ((reinterpret_cast<uintptr_t>(pr.C) & 15) == 0) &&
-                         skip_cols == 0;
+        float* crow = Cd + (int64_t)row * rsc;
+        // (contiguous rows get here in CTA pairs only)
+        const bool vec = PAIR && (csc == 1) && ((rsc & 3) == 0) && ((reinterpret_cast<uintptr_t>(Cd) & 15) == 0);
         if (vec && cn + kCols <= pr.N) {
           // 64 bytes at a time: four loads in flight before their stores
 #pragma unroll
@@ -1546,7 +1592,7 @@ __global__ void __launch_bounds__(ModeTraits<MODE>::kThreads, 1)
             float4* p = reinterpret_cast<float4*>(crow + cn + j0);
             float4 cv[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) cv[u] = add ? p[u] : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int u = 0; u < 4; ++u) cv[u] = add ? p[u] : make_float4(-0.f, -0.f, -0.f, -0.f);
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
               const int j = j0 + 4 * u;
@@ -1559,16 +1605,17 @@ __global__ void __launch_bounds__(ModeTraits<MODE>::kThreads, 1)
             for (int u = 0; u < 4; ++u) p[u] = cv[u];
           }
         } else {
+          float* p = crow + (int64_t)cn * csc;
+          const int cols = pr.N - cn;  // columns j < cols exist
 #pragma unroll
           for (int j0 = 0; j0 < kCols; j0 += 16) {
             float old[16];
+            const float* lp = p;
 #pragma unroll
-            for (int j = 0; j < 16; ++j)
-              old[j] = (add && cn + j0 + j < pr.N) ? crow[(int64_t)(cn + j0 + j) * pr.csc] : 0.f;
+            for (int j = 0; j < 16; ++j, lp += csc) old[j] = (add && j0 + j < cols) ? *lp : -0.f;
 #pragma unroll
-            for (int j = 0; j < 16; ++j)
-              if (cn + j0 + j < pr.N && !(MT::f16 && ((skip_cols >> (j0 + j)) & 1)))
-                crow[(int64_t)(cn + j0 + j) * pr.csc] = old[j] + acc[j0 + j];
+            for (int j = 0; j < 16; ++j, p += csc)
+              if (j0 + j < cols && !(MT::f16 && ((skip_cols >> (j0 + j)) & 1))) *p = old[j] + acc[j0 + j];
           }
         }
       }
@@ -1585,6 +1632,7 @@ __global__ void __launch_bounds__(ModeTraits<MODE>::kThreads, 1)
   // waits for the consumer that needs both halves) get the missing arrival,
   // so every issued slice's stage completes once its copies have landed.
   if constexpr (!PAIR) __syncthreads();
+  dev::grid_release();
   if (warp == 0 && lane == 0 && rank == 0 && *abort_flag) {
     int never = 0;
     int hi = issued;
@@ -1631,14 +1679,15 @@ __global__ void __launch_bounds__(ModeTraits<MODE>::kThreads, 1)
 // then the lanes' sums meet in a fixed shuffle tree.  Error at most
 // (K / 32 + 5) eps32 (|A||B|)_ij, order fixed: the same bits on every run.
 // CTAs take the listed rows in turn; with empty lists every CTA returns at
-// once.  jobs: the A jobs then the B^T jobs of a group without split-K
-// (problem i = job i).
+// once.  jobs: the A jobs then the B^T jobs of a group (problem i = job i).
 __global__ void __launch_bounds__(256) f16_guard_fixup_kernel(const SplitJob* __restrict__ jobs, int njobs,
                                                               const TcProblem* __restrict__ probs,
                                                               const int* __restrict__ list_a,
                                                               const int* __restrict__ list_b,
                                                               const int* __restrict__ counts,
                                                               const int* __restrict__ flags_a) {
+  dev::grid_release();
+  dev::grid_wait();
   const int na = counts[0], nb = counts[1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   auto job_of = [&](const SplitJob* js, int64_t row) {  // last job with dst_row <= row
@@ -1684,17 +1733,44 @@ __global__ void __launch_bounds__(256) f16_guard_fixup_kernel(const SplitJob* __
 }
 
 // Split-K: C += part[0] + part[1] + ... (in that order) for every element of
-// every split problem; blockIdx.y = problem, grid-stride over its elements.
+// every split problem; blockIdx.y = problem, warps walk its rows' 32-column
+// blocks.  Bound by the L2 the partials were just written to.
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(const SplitReduce* __restrict__ jobs) {
+  dev::grid_release();
+  dev::grid_wait();
   const SplitReduce j = jobs[blockIdx.y];
-  const int64_t total = (int64_t)j.M * j.N, plane = (int64_t)j.M * j.pitch;
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = e / j.N, c = e % j.N;
+  const int lane = threadIdx.x & 31, blocks = (j.N + 31) / 32;
+  const int64_t plane = (int64_t)j.M * j.pitch, items = (int64_t)j.M * blocks;
+  const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t w = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < items; w += nw) {
+    const int64_t r = w / blocks;
+    const int c = (int)(w % blocks) * 32 + lane;
+    if (c >= j.N) continue;
     const float* p = j.part + r * j.pitch + c;
-    float sum = p[0];
-    for (int s = 1; s < j.parts; ++s) sum += p[s * plane];
-    j.C[r * j.rsc + c * j.csc] += sum;
+    float* cp = j.C + r * j.rsc + c * j.csc;
+    const float old = *cp;
+    float sum = __ldcg(p);
+#pragma unroll 4
+    for (int s = 1; s < j.parts; ++s) sum += __ldcg(p + s * plane);
+    *cp = old + sum;
   }
+}
+
+// The launch's tables (one host image of the plan's problems, jobs and
+// reductions) as a kernel parameter: copied to the scratch, and the words the
+// launch starts from cleared, by one small kernel - a pageable host-to-device
+// copy and a memset cost a single call several us of host and stream time.
+constexpr int kInitBytes = 2048;
+struct InitTables {
+  uint4 words[kInitBytes / 16];
+};
+__global__ void __launch_bounds__(256) tc_init_kernel(const __grid_constant__ InitTables t, int table_bytes,
+                                                      unsigned char* __restrict__ dst, uint4* __restrict__ zero,
+                                                      int64_t zero_words) {
+  dev::grid_release();
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i * 16 < table_bytes) reinterpret_cast<uint4*>(dst)[i] = t.words[i];
+  for (int64_t z = i; z < zero_words; z += (int64_t)gridDim.x * blockDim.x) zero[z] = make_uint4(0u, 0u, 0u, 0u);
 }
 
 }  // namespace
@@ -1781,7 +1857,7 @@ inline size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 // the operand arena live on the device, and the two arena tensor maps.
 struct TcGroupPlan {
   int mode = 2;  // 2 / 3 BF16 pieces, kModeFp8
-  int nprob = 0;  // tile problems (a split-K problem counts once per part)
+  int nprob = 0;  // problems (of which reds.size() are cut along K)
   int njobs = 0;  // operand preparations (one per problem of the group)
   int64_t a_rows = 0, b_rows = 0, tiles = 0;
   int64_t kpad = 0;   // longest padded K of the group (elements)
@@ -1790,12 +1866,13 @@ struct TcGroupPlan {
   std::vector<TcProblem> probs;
   std::vector<SplitJob> ajobs, bjobs;
   std::vector<SplitReduce> reds;     // split-K problems' final sums
-  std::vector<int64_t> part_off;     // per tile problem: byte offset of its partial in the workspace, or -1
+  std::vector<int64_t> part_off;     // per problem: byte offset of its first partial in the workspace, or -1
   std::vector<int64_t> red_off;      // per reduction: byte offset of its first partial
   size_t off_probs = 0, off_jobs = 0, off_red = 0, off_arena = 0, off_sa = 0, off_sb = 0, off_ws = 0, bytes = 0;
   char* base = nullptr;  // device: zeroed header | problems | jobs | reductions | arena | FP8 scales | partials
   bool owned = false;    // base allocated by the plan (graph plans)
   CUtensorMap map_a, map_b;
+  bool cleared = false;  // the launch's start words are clear already (tc_init_kernel)
   bool pair = false;  // CTA pairs computing 256 x 128 tiles (see gemm_split_kernel)
   bool guard = false;  // FP16 split with the AUTO guard (F16Guard, f16_guard_fixup_kernel)
   bool row_prep_a = false, row_prep_b = false;  // FP16 split: operand prepared by f16_row_prep_kernel
@@ -1822,7 +1899,7 @@ namespace {
 // Host-side planning (no device work): problem order (largest K first),
 // arena rows, tile numbering, split jobs, device layout.  opt.split > 1
 // cuts every problem's K into that many parts (at most one per K stage),
-// each a tile problem of its own that stores a partial; a reduction then adds
+// each with tiles of its own that store a partial; a reduction then adds
 // the parts into C in order.  opt.pair forces the CTA form (-1: the
 // GBBLAS_TC_PAIR setting).
 gbblas_status plan_group(int mode, const gbblas_gemm_desc* d, int64_t count, TcGroupPlan& pl,
@@ -1874,42 +1951,48 @@ gbblas_status plan_group(int mode, const gbblas_gemm_desc* d, int64_t count, TcG
     const gbblas_gemm_desc& g = d[order[i]];
     const int64_t Mp = round_up(g.M, bmt), Np = round_up(g.N, kBN), Kp = round_up(g.K, pk);
     const int num_kt = (int)(Kp / sk);  // pk is a multiple of sk
-    // (the guard's fixup pairs problem i with job i: no split-K under it)
-    const int parts = pl.guard ? 1 : std::max(1, std::min(opt.split, num_kt));
-    const int64_t ppitch = round_up(g.N, 4);  // partial rows stay 16-byte aligned
+    const int parts = std::max(1, std::min(opt.split, num_kt));
+    // partials lie the way C does, so that both the epilogue and the
+    // reduction run along contiguous elements; their rows stay 16-byte aligned
+    const bool c_cols = g.csc != 1 && g.rsc == 1;
+    const int64_t ppitch = round_up(c_cols ? g.M : g.N, 4), pplane = ppitch * (c_cols ? g.N : g.M);
+    TcProblem p;
+    p.M = (int)g.M;
+    p.N = (int)g.N;
+    p.num_kt = num_kt;
+    p.parts = parts;
+    p.a_row = (int)pl.a_rows;
+    p.b_row = (int)pl.b_rows;
+    p.tiles_m = (int)(Mp / bmt);
+    p.tiles_n = (int)(Np / kBN);
+    p.tile_start = (int)pl.tiles;
+    p.C = g.C;
+    p.rsc = g.rsc;
+    p.csc = g.csc;
+    p.ws = nullptr;  // pointed into the workspace when bound
+    p.ws_rs = c_cols ? 1 : ppitch;
+    p.ws_cs = c_cols ? ppitch : 1;
+    p.ws_plane = pplane;
+    p.c_tma = 0;
+    // single CTAs add their results into C with TMA reduce-add stores where
+    // C rows are contiguous, 16-byte aligned and 16-byte-multiple apart
+    // (split-K partials are stored by the register path)
+    if (!pl.pair && parts == 1 && g.csc == 1 && g.rsc >= g.N && (g.rsc % 4) == 0 &&
+        (reinterpret_cast<uintptr_t>(g.C) & 15) == 0 &&
+        make_map_f32_2d(&p.c_map, g.C, (uint64_t)g.N, (uint64_t)g.M, (uint64_t)g.rsc, 32, 32, true) ==
+            GBBLAS_STATUS_SUCCESS)
+      p.c_tma = 1;
+    pl.probs.push_back(p);
+    pl.part_off.push_back(parts > 1 ? ws : -1);
     if (parts > 1) {
-      pl.reds.push_back({g.C, g.rsc, g.csc, nullptr, (int)g.M, (int)g.N, (int)ppitch, parts});
+      if (c_cols)
+        pl.reds.push_back({g.C, g.csc, g.rsc, nullptr, (int)g.N, (int)g.M, (int)ppitch, parts});
+      else
+        pl.reds.push_back({g.C, g.rsc, g.csc, nullptr, (int)g.M, (int)g.N, (int)ppitch, parts});
       pl.red_off.push_back(ws);
+      ws += (int64_t)parts * pplane * (int64_t)sizeof(float);
     }
-    for (int part = 0; part < parts; ++part) {
-      TcProblem p;
-      p.M = (int)g.M;
-      p.N = (int)g.N;
-      p.kt0 = (int)((int64_t)num_kt * part / parts);
-      p.num_kt = (int)((int64_t)num_kt * (part + 1) / parts) - p.kt0;
-      p.a_row = (int)pl.a_rows;
-      p.b_row = (int)pl.b_rows;
-      p.tiles_m = (int)(Mp / bmt);
-      p.tiles_n = (int)(Np / kBN);
-      p.tile_start = (int)pl.tiles;
-      p.overwrite = parts > 1 ? 1 : 0;
-      p.C = parts > 1 ? nullptr : g.C;  // partials: pointed into the workspace when bound
-      p.rsc = parts > 1 ? ppitch : g.rsc;
-      p.csc = parts > 1 ? 1 : g.csc;
-      p.c_tma = 0;
-      // single CTAs add their results into C with TMA reduce-add stores
-      // where C rows are contiguous, 16-byte aligned and 16-byte-multiple
-      // apart (split-K partials are stored by the register path)
-      if (!pl.pair && parts == 1 && g.csc == 1 && g.rsc >= g.N && (g.rsc % 4) == 0 &&
-          (reinterpret_cast<uintptr_t>(g.C) & 15) == 0 &&
-          make_map_f32_2d(&p.c_map, g.C, (uint64_t)g.N, (uint64_t)g.M, (uint64_t)g.rsc, 32, 32, true) ==
-              GBBLAS_STATUS_SUCCESS)
-        p.c_tma = 1;
-      pl.probs.push_back(p);
-      pl.part_off.push_back(parts > 1 ? ws : -1);
-      if (parts > 1) ws += (int64_t)g.M * ppitch * (int64_t)sizeof(float);
-      pl.tiles += (int64_t)p.tiles_m * p.tiles_n;
-    }
+    pl.tiles += (int64_t)parts * p.tiles_m * p.tiles_n;
     pl.ajobs[i] = {g.A, g.M, g.K, g.rsa, g.csa, pl.a_rows, (int)(Mp / jr), (int)(Kp / jk), pl.a_tiles};
     pl.a_tiles += pl.ajobs[i].tiles_r * pl.ajobs[i].tiles_k;
     // B^T: element (n, k) = B[k*rsb + n*csb]
@@ -2012,11 +2095,13 @@ uint32_t* scales_b(const TcGroupPlan& pl) { return reinterpret_cast<uint32_t*>(p
 
 // Point the plan at device memory `base` (>= pl.bytes, header zeroed), copy
 // the tables there on `stream`, and encode the arena tensor maps.
-gbblas_status bind_group(TcGroupPlan& pl, char* base, cudaStream_t stream) {
+// per_call: the plan is launched once, right after: small tables go with the
+// words that launch clears, by tc_init_kernel (pl.cleared).
+gbblas_status bind_group(TcGroupPlan& pl, char* base, cudaStream_t stream, bool per_call) {
   pl.base = base;
   if (pl.nprob == 0) return GBBLAS_STATUS_SUCCESS;
   for (int i = 0; i < pl.nprob; ++i)
-    if (pl.part_off[i] >= 0) pl.probs[i].C = reinterpret_cast<float*>(base + pl.off_ws + pl.part_off[i]);
+    if (pl.part_off[i] >= 0) pl.probs[i].ws = reinterpret_cast<float*>(base + pl.off_ws + pl.part_off[i]);
   for (size_t r = 0; r < pl.reds.size(); ++r)
     pl.reds[r].part = reinterpret_cast<const float*>(base + pl.off_ws + pl.red_off[r]);
   // problems, jobs and reductions as one host image and one copy (the image
@@ -2029,7 +2114,21 @@ gbblas_status bind_group(TcGroupPlan& pl, char* base, cudaStream_t stream) {
               sizeof(SplitJob) * pl.njobs);
   if (!pl.reds.empty())
     std::memcpy(h + (pl.off_red - pl.off_probs), pl.reds.data(), sizeof(SplitReduce) * pl.reds.size());
-  GB_CUDA_TRY(cudaMemcpyAsync(base + pl.off_probs, h, pl.tables.size(), cudaMemcpyHostToDevice, stream));
+  if (per_call && pl.tables.size() <= (size_t)kInitBytes) {
+    InitTables t;
+    std::memcpy(&t, h, pl.tables.size());
+    // (from the tile counter on; the header and the arrays are 16-byte multiples)
+    const int64_t zero_words = (int64_t)(pl.off_init_end - kTileCounterOffset) / 16;
+    const int64_t most = std::max<int64_t>(zero_words, (int64_t)pl.tables.size() / 16);
+    const int64_t ctas = std::min<int64_t>((most + 255) / 256, 256);
+    tc_init_kernel<<<(unsigned)ctas, 256, 0, stream>>>(t, (int)pl.tables.size(),
+                                                       reinterpret_cast<unsigned char*>(base + pl.off_probs),
+                                                       reinterpret_cast<uint4*>(base + kTileCounterOffset), zero_words);
+    GB_TRY(check_launch("tc_init_kernel"));
+    pl.cleared = true;
+  } else {
+    GB_CUDA_TRY(cudaMemcpyAsync(base + pl.off_probs, h, pl.tables.size(), cudaMemcpyHostToDevice, stream));
+  }
   GB_TRY(make_map(&pl.map_a, arena_a(pl), (uint64_t)pl.a_rows, (uint64_t)pl.pitch, (uint64_t)pl.planes(), kBM,
                   pl.fp8(), pl.row_bytes()));
   GB_TRY(make_map(&pl.map_b, arena_b(pl), (uint64_t)pl.b_rows, (uint64_t)pl.pitch, (uint64_t)pl.planes(),
@@ -2074,7 +2173,7 @@ int kernel_setup(DeviceCtx* c) {
 
 template <int MODE, bool PAIR>
 gbblas_status launch_gemm_kernel(DeviceCtx* c, const TcGroupPlan& pl, cudaStream_t stream, int max_ctas,
-                                 int tile_begin, int tile_end) {
+                                 int tile_begin, int tile_end, bool chained) {
   using CF = TcCfg<MODE, PAIR>;
   int* err = reinterpret_cast<int*>(pl.base + kErrWordOffset);
   int* counter = reinterpret_cast<int*>(pl.base + kTileCounterOffset);
@@ -2087,9 +2186,15 @@ gbblas_status launch_gemm_kernel(DeviceCtx* c, const TcGroupPlan& pl, cudaStream
   }
   if constexpr (!PAIR) {
     const int* ga = pl.guard ? reinterpret_cast<const int*>(pl.base + pl.off_gflag) : nullptr;
-    gemm_split_kernel<MODE, false><<<units, ModeTraits<MODE>::kThreads, CF::kSmem, stream>>>(
-        pl.map_a, pl.map_b, dprobs, pl.nprob, tile_begin, tile_end, pl.kpad, counter, err, scales_a(pl), scales_b(pl), ga,
-        ga ? ga + pl.a_rows : nullptr);
+    const int* gb = ga ? ga + pl.a_rows : nullptr;
+    if (chained)
+      GB_CUDA_TRY(launch_after(gemm_split_kernel<MODE, false>, dim3(units), ModeTraits<MODE>::kThreads, CF::kSmem,
+                               stream, pl.map_a, pl.map_b, dprobs, pl.nprob, tile_begin, tile_end, pl.kpad, counter,
+                               err, scales_a(pl), scales_b(pl), ga, gb));
+    else
+      gemm_split_kernel<MODE, false><<<units, ModeTraits<MODE>::kThreads, CF::kSmem, stream>>>(
+          pl.map_a, pl.map_b, dprobs, pl.nprob, tile_begin, tile_end, pl.kpad, counter, err, scales_a(pl), scales_b(pl),
+          ga, gb);
     return check_launch("gemm_split_kernel");
   } else {
   cudaLaunchConfig_t cfg = {};
@@ -2117,13 +2222,26 @@ gbblas_status launch_gemm_kernel(DeviceCtx* c, const TcGroupPlan& pl, cudaStream
   }
 }
 
+// A 256-thread kernel of a call's chain, or launched plainly.
+template <typename... P, typename... A>
+cudaError_t launch_chain(bool chained, void (*kernel)(P...), dim3 grid, cudaStream_t stream, A&&... args) {
+  if (chained) return launch_after(kernel, grid, 256, 0, stream, std::forward<A>(args)...);
+  kernel<<<grid, 256, 0, stream>>>(std::forward<A>(args)...);
+  return cudaSuccess;
+}
+
 template <int MODE>
 gbblas_status launch_bound(DeviceCtx* c, const TcGroupPlan& pl, cudaStream_t stream, int max_ctas, int slices) {
   if (pl.nprob == 0) return GBBLAS_STATUS_SUCCESS;
   const auto* djobs = reinterpret_cast<const SplitJob*>(pl.base + pl.off_jobs);
+  // a single call's kernels follow one another directly, the first behind
+  // tc_init_kernel: they are launched as a chain.  A plan captured into a
+  // graph, or whose tables came by a copy, takes plain launches.
+  const bool chained = pl.cleared;
   // the tile counter, the guard's counts and (FP16 split) the row exponents
   // and minima: zero, in one memset
-  GB_CUDA_TRY(cudaMemsetAsync(pl.base + kTileCounterOffset, 0, pl.off_init_end - kTileCounterOffset, stream));
+  if (!pl.cleared)
+    GB_CUDA_TRY(cudaMemsetAsync(pl.base + kTileCounterOffset, 0, pl.off_init_end - kTileCounterOffset, stream));
   F16Guard ga, gb;  // AUTO guard arrays (A rows, then B^T rows)
   int* gcounts = reinterpret_cast<int*>(pl.base + kGuardCountOffset);
   if (pl.guard) {
@@ -2147,7 +2265,11 @@ gbblas_status launch_bound(DeviceCtx* c, const TcGroupPlan& pl, cudaStream_t str
       // arena rows come in multiples of 128 per job: whole CTAs of 8 or 32 rows
       const int64_t rows = (int64_t)ra.rows + rb.rows;
       const int rpc = rows / kSplitRowsPerCtaMax >= 4 * (int64_t)c->num_sms ? kSplitRowsPerCtaMax : 8;
-      split_rows_kernel<MODE><<<(unsigned)(rows / rpc), 256, 0, stream>>>(ra, rb, pl.njobs, pl.pitch, rpc);
+      const int64_t steps = (pl.kpad + 511) / 512;  // of K per row, to share out until there are 4 CTAs per SM
+      const int64_t segs = std::max<int64_t>(1, std::min<int64_t>(steps, 4 * (int64_t)c->num_sms * rpc / rows));
+      const int64_t kseg = (steps + segs - 1) / segs * 512;
+      const dim3 grid((unsigned)(rows / rpc), (unsigned)((steps * 512 + kseg - 1) / kseg));
+      GB_CUDA_TRY(launch_chain(chained, split_rows_kernel<MODE>, grid, stream, ra, rb, pl.njobs, pl.pitch, rpc, kseg));
       GB_TRY(check_launch("split_rows_kernel"));
     }
   }
@@ -2161,9 +2283,11 @@ gbblas_status launch_bound(DeviceCtx* c, const TcGroupPlan& pl, cudaStream_t str
       // a warp per row while the group's longest row fits its registers (a
       // CTA per row would leave most of its threads without an element)
       if (pl.kpad <= 128 * kRowPrepNV)
-        f16_row_prep_kernel<32><<<(ra.rows + rb.rows) / 8, 256, 0, stream>>>(ra, rb, pl.njobs, pl.pitch);
+        GB_CUDA_TRY(launch_chain(chained, f16_row_prep_kernel<32>, dim3((ra.rows + rb.rows) / 8), stream, ra, rb,
+                                 pl.njobs, pl.pitch));
       else
-        f16_row_prep_kernel<256><<<ra.rows + rb.rows, 256, 0, stream>>>(ra, rb, pl.njobs, pl.pitch);
+        GB_CUDA_TRY(launch_chain(chained, f16_row_prep_kernel<256>, dim3(ra.rows + rb.rows), stream, ra, rb, pl.njobs,
+                                 pl.pitch));
       GB_TRY(check_launch("f16_row_prep_kernel"));
     }
     // per-row exponents of A's and B^T's arena rows (and the guard's
@@ -2174,7 +2298,8 @@ gbblas_status launch_bound(DeviceCtx* c, const TcGroupPlan& pl, cudaStream_t str
       const ScaleSide sa{djobs, a_cols, reinterpret_cast<int*>(scales_a(pl)), const_cast<unsigned*>(ga.emin)};
       const ScaleSide sb{djobs + pl.njobs, b_cols, reinterpret_cast<int*>(scales_b(pl)),
                          const_cast<unsigned*>(gb.emin)};
-      f16_col_scale_kernel<<<a_cols + b_cols, 256, 0, stream>>>(sa, sb, pl.njobs, pl.col_kblk);
+      GB_CUDA_TRY(
+          launch_chain(chained, f16_col_scale_kernel, dim3(a_cols + b_cols), stream, sa, sb, pl.njobs, pl.col_kblk));
       GB_TRY(check_launch("f16_col_scale_kernel"));
     }
     const int a_st = pl.col_scale_a ? 0 : a_tiles, b_st = pl.col_scale_b ? 0 : b_tiles;
@@ -2182,7 +2307,7 @@ gbblas_status launch_bound(DeviceCtx* c, const TcGroupPlan& pl, cudaStream_t str
       const ScaleSide sa{djobs, a_st, reinterpret_cast<int*>(scales_a(pl)), const_cast<unsigned*>(ga.emin)};
       const ScaleSide sb{djobs + pl.njobs, b_st, reinterpret_cast<int*>(scales_b(pl)),
                          const_cast<unsigned*>(gb.emin)};
-      f16_scale_kernel<<<a_st + b_st, 256, 0, stream>>>(sa, sb, pl.njobs);
+      GB_CUDA_TRY(launch_chain(chained, f16_scale_kernel, dim3(a_st + b_st), stream, sa, sb, pl.njobs));
       GB_TRY(check_launch("f16_scale_kernel"));
     }
   }
@@ -2192,9 +2317,11 @@ gbblas_status launch_bound(DeviceCtx* c, const TcGroupPlan& pl, cudaStream_t str
     const PrepSide pa{djobs, a_tiles, arena_a(pl), (int64_t)(pl.a_rows * pl.pitch), scales_a(pl), ga};
     const PrepSide pb{djobs + pl.njobs, b_tiles, arena_b(pl), (int64_t)(pl.b_rows * pl.pitch), scales_b(pl), gb};
     if ((a_tiles == 0 || pl.prep_vec_a) && (b_tiles == 0 || pl.prep_vec_b))
-      prep_group_kernel<MODE, true><<<prep_ctas, 256, 0, stream>>>(pa, pb, pl.njobs, pl.pitch, pl.kpad);
+      GB_CUDA_TRY(launch_chain(chained, prep_group_kernel<MODE, true>, dim3(prep_ctas), stream, pa, pb, pl.njobs,
+                               pl.pitch, pl.kpad));
     else
-      prep_group_kernel<MODE, false><<<prep_ctas, 256, 0, stream>>>(pa, pb, pl.njobs, pl.pitch, pl.kpad);
+      GB_CUDA_TRY(launch_chain(chained, prep_group_kernel<MODE, false>, dim3(prep_ctas), stream, pa, pb, pl.njobs,
+                               pl.pitch, pl.kpad));
     GB_TRY(check_launch("prep_group_kernel"));
   }
   // the GEMM, as `slices` launches over consecutive ranges of whole waves of
@@ -2212,25 +2339,27 @@ gbblas_status launch_bound(DeviceCtx* c, const TcGroupPlan& pl, cudaStream_t str
     if (sl > 0)
       GB_CUDA_TRY(cudaMemsetAsync(pl.base + kTileCounterOffset, 0, sizeof(int), stream));
     if constexpr (MODE != kModeFp8 && MODE != kModeF16) {
-      st = pl.pair ? launch_gemm_kernel<MODE, true>(c, pl, stream, max_ctas, tb, te)
-                   : launch_gemm_kernel<MODE, false>(c, pl, stream, max_ctas, tb, te);
+      st = pl.pair ? launch_gemm_kernel<MODE, true>(c, pl, stream, max_ctas, tb, te, chained)
+                   : launch_gemm_kernel<MODE, false>(c, pl, stream, max_ctas, tb, te, chained && sl == 0);
     } else {
-      st = launch_gemm_kernel<MODE, false>(c, pl, stream, max_ctas, tb, te);
+      st = launch_gemm_kernel<MODE, false>(c, pl, stream, max_ctas, tb, te, chained && sl == 0);
     }
   }
+  if (st == GBBLAS_STATUS_SUCCESS && !pl.reds.empty()) {
+    int64_t most = 0;  // 32-column blocks of the largest split C
+    for (const SplitReduce& r : pl.reds) most = std::max<int64_t>(most, (int64_t)r.M * ((r.N + 31) / 32));
+    const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((most + 7) / 8, 8 * (int64_t)c->num_sms));
+    GB_CUDA_TRY(launch_chain(chained, splitk_reduce_kernel, dim3(blocks, (unsigned)pl.reds.size()), stream,
+                             reinterpret_cast<const SplitReduce*>(pl.base + pl.off_red)));
+    st = check_launch("splitk_reduce_kernel");
+  }
   if (st == GBBLAS_STATUS_SUCCESS && pl.guard) {
-    f16_guard_fixup_kernel<<<2 * c->num_sms, 256, 0, stream>>>(
-        djobs, pl.njobs, reinterpret_cast<const TcProblem*>(pl.base + pl.off_probs), ga.list, gb.list, gcounts,
-        ga.flags);
+    GB_CUDA_TRY(launch_chain(chained, f16_guard_fixup_kernel, dim3(2 * c->num_sms), stream, djobs, pl.njobs,
+                             reinterpret_cast<const TcProblem*>(pl.base + pl.off_probs), ga.list, gb.list, gcounts,
+                             ga.flags));
     st = check_launch("f16_guard_fixup_kernel");
   }
-  if (st != GBBLAS_STATUS_SUCCESS || pl.reds.empty()) return st;
-  int64_t most = 0;
-  for (const SplitReduce& r : pl.reds) most = std::max<int64_t>(most, (int64_t)r.M * r.N);
-  const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((most + 255) / 256, 4 * (int64_t)c->num_sms));
-  splitk_reduce_kernel<<<dim3(blocks, (unsigned)pl.reds.size()), 256, 0, stream>>>(
-      reinterpret_cast<const SplitReduce*>(pl.base + pl.off_red));
-  return check_launch("splitk_reduce_kernel");
+  return st;
 }
 
 }  // namespace
@@ -2306,7 +2435,7 @@ gbblas_status tc_group_create(DeviceCtx* c, int mode, const gbblas_gemm_desc* de
   pl->owned = true;
   e = cudaMemset(p, 0, kScratchZeroBytes);
   if (e == cudaSuccess) {
-    st = bind_group(*pl, static_cast<char*>(p), nullptr);
+    st = bind_group(*pl, static_cast<char*>(p), nullptr, false);
     if (st == GBBLAS_STATUS_SUCCESS && cudaDeviceSynchronize() != cudaSuccess) st = GBBLAS_STATUS_CUDA_ERROR;
   } else {
     st = GBBLAS_STATUS_CUDA_ERROR;
@@ -2337,7 +2466,7 @@ gbblas_status launch_gemm_tc_group(DeviceCtx* c, int mode, const gbblas_gemm_des
   if (pl.nprob == 0) return GBBLAS_STATUS_SUCCESS;
   void* s = nullptr;
   GB_TRY(get_scratch(c, stream, pl.bytes, &s));
-  GB_TRY(bind_group(pl, static_cast<char*>(s), stream));
+  GB_TRY(bind_group(pl, static_cast<char*>(s), stream, true));
   return tc_group_launch(c, &pl, stream, max_ctas, slices);
 }
 
@@ -2348,7 +2477,7 @@ gbblas_status launch_gemm_tc_opts(DeviceCtx* c, int mode, const gbblas_gemm_desc
   if (pl.nprob == 0) return GBBLAS_STATUS_SUCCESS;
   void* s = nullptr;
   GB_TRY(get_scratch(c, stream, pl.bytes, &s));
-  GB_TRY(bind_group(pl, static_cast<char*>(s), stream));
+  GB_TRY(bind_group(pl, static_cast<char*>(s), stream, true));
   return tc_group_launch(c, &pl, stream, 0, gemm_slices_env());
 }
 
@@ -2357,9 +2486,7 @@ gbblas_status launch_gemm_tc(DeviceCtx* c, int mode, int64_t M, int64_t N, int64
                              int64_t csc, cudaStream_t stream) {
   if (M == 0 || N == 0 || K == 0) return GBBLAS_STATUS_SUCCESS;
   gbblas_gemm_desc d{M, N, K, A, rsa, csa, B, rsb, csb, C, rsc, csc};
-  // (the guarded FP16 split runs single CTAs without split-K: nothing to tune)
-  return launch_gemm_tc_opts(c, mode, d, mode == kModeF16Guard ? TcLaunchOpts() : tuned_tc_opts(c, mode, M, N, K, stream),
-                             stream);
+  return launch_gemm_tc_opts(c, mode, d, tuned_tc_opts(c, mode, d.M, d.N, d.K, stream), stream);
 }
 
 }  // namespace gbblas

@@ -117,6 +117,12 @@ __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
 
+// Acquire a tensor map that lies in global memory (written by another kernel
+// or a copy) for this thread's TMA instructions.
+__device__ __forceinline__ void fence_tensormap(const CUtensorMap* map) {
+  asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
+}
+
 // ------------------------------------------------------------ TMEM / MMA
 // Allocate `ncols` (power of two >= 32) TMEM columns; whole warp executes.
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst_smem, uint32_t ncols) {

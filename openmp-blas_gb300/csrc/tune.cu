@@ -19,10 +19,8 @@
 //   gemm_auto        for GBBLAS_ACCURACY_AUTO, FP32 FMA kernel or the guarded
 //                    FP16 split (three products) - both FP32-accurate -
 //                    bucketed by log2 M, N, K;
-//   gemm_tc          per tensor-core mode and log2 M, N, K bucket: split-K
-//                    parts (1, 2, 4, 8, 16; offered when K >= 4 max(M, N) and
-//                    the output tiles fill at most half the SMs) and the CTA
-//                    form (single CTAs or CTA pairs, split-BF16 only);
+//   gemm_tc          per split-BF16 mode and log2 M, N, K bucket: the CTA form
+//                    (single CTAs, with split-K by rule, or CTA pairs);
 //                    GBBLAS_TC_SPLITK=n forces n parts;
 //   gemm_fma_tile    FP32 FMA kernel and CTA tile per bucket, operand
 //                    layouts and alignment: 64 x 64 or 128 x 128 (K cut over
@@ -269,7 +267,7 @@ int tuned_gemm_auto(DeviceCtx* c, int64_t M, int64_t N, int64_t K) {
   const int fallback = (M >= 256 && N >= 256 && K >= 256 && (double)M * N * K >= 1.0e9) ? 1 : 0;
   Tuner& t = Tuner::get();
   const int bm = log2_bucket(M), bn = log2_bucket(N), bk = log2_bucket(K);
-  const std::string key = "gemm_auto_f16g|" + device_tag(c) + "|m" + std::to_string(bm) + "|n" + std::to_string(bn) +
+  const std::string key = "gemm_auto_f16s|" + device_tag(c) + "|m" + std::to_string(bm) + "|n" + std::to_string(bn) +
                           "|k" + std::to_string(bk) + "|f32";
   int v = t.lookup(key);
   if (v >= 0) return v;
@@ -292,11 +290,12 @@ int tuned_gemm_auto(DeviceCtx* c, int64_t M, int64_t N, int64_t K) {
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
+  const int fma_tile = tuned_fma_tile(c, {m, n, k, A, k, 1, B, n, 1, C, n, 1}, s);
   float best_ms[2] = {1e30f, 1e30f};
   for (int choice = 0; choice < 2; ++choice) {
     auto run = [&]() {
       return choice == 1 ? launch_gemm_tc(c, kTcModeF16Guard, m, n, k, A, k, 1, B, n, 1, C, n, 1, s)
-                         : launch_gemm_fma<float>(c, m, n, k, A, k, 1, B, n, 1, C, n, 1, s);
+                         : launch_gemm_fma<float>(c, m, n, k, A, k, 1, B, n, 1, C, n, 1, s, 0, fma_tile);
     };
     if (run() != GBBLAS_STATUS_SUCCESS) continue;  // warm-up
     cudaEventRecord(e0, s);
@@ -320,17 +319,37 @@ int tuned_gemm_auto(DeviceCtx* c, int64_t M, int64_t N, int64_t K) {
   return best;
 }
 
-// Split-K parts worth trying for an M x N x K tensor-core GEMM: K at least
-// four times the larger output side, output tiles filling at most half the
-// SMs, every part at least 8 K stages, parts x tiles at most twice the SMs.
-static std::vector<int> split_candidates(DeviceCtx* c, int mode, int64_t M, int64_t N, int64_t K) {
-  std::vector<int> out;
+// Split-K parts of an M x N x K tensor-core GEMM on single CTAs: the number
+// with the least estimated time, waves of tiles x K stages each (us per stage
+// as measured at 8192^3) plus, for more than one part, the reduction (its
+// launch, and the partials' bytes at about 3 TB/s).  A rule and not a
+// measurement per bucket: whether tiles x parts fit the SMs in one wave turns
+// on the shape itself (4880 x 249 x 4096, 78 tiles: 137 us unsplit, 178 in the
+// two parts that suit its bucket's 64 tiles).  The BF16 splits and FP8 keep to
+// K at least four times the larger output side, so that a product of ordinary
+// proportions gives the same bits alone as in a group (whose problems are not
+// split); AUTO, whose arithmetic is the library's choice per shape, splits any
+// of them, and the FP16 split it stands for goes with it.
+static int split_parts(DeviceCtx* c, int mode, int64_t M, int64_t N, int64_t K) {
+  const int64_t sms = c->num_sms;
   const int64_t tiles = ((M + 127) / 128) * ((N + 127) / 128);
   const int64_t stages = (K + tc_stage_k(mode) - 1) / tc_stage_k(mode);
-  if (K < 4 * std::max(M, N) || 2 * tiles > c->num_sms) return out;
-  for (int s : {2, 4, 8, 16})
-    if (stages >= 8 * s && tiles * s <= 2 * (int64_t)c->num_sms) out.push_back(s);
-  return out;
+  const bool f16 = mode == kTcModeF16Guard || mode == tc_mode(GBBLAS_ACCURACY_FP16X3);
+  if (tiles >= sms || (!f16 && K < 4 * std::max(M, N))) return 1;
+  const double stage_us = mode == tc_mode(GBBLAS_ACCURACY_BF16X6) ? 1.25 : 0.7;
+  int best = 1;
+  double best_us = 1e30;
+  for (int s : {1, 2, 3, 4, 6, 8, 12, 16}) {
+    if (s > 1 && stages < 4 * s) break;
+    const int64_t waves = (tiles * s + sms - 1) / sms;
+    const double us = (double)waves * (double)((stages + s - 1) / s) * stage_us +
+                      (s > 1 ? 3.0 + (double)(s + 1) * (double)M * (double)N * 4.0 / 3e6 : 0.0);
+    if (us < (s > 1 ? 0.9 : 1.0) * best_us) {  // (each step up has to be worth 10 %)
+      best_us = us;
+      best = s;
+    }
+  }
+  return best;
 }
 
 TcLaunchOpts tuned_tc_opts(DeviceCtx* c, int mode, int64_t M, int64_t N, int64_t K, cudaStream_t stream) {
@@ -339,48 +358,38 @@ TcLaunchOpts tuned_tc_opts(DeviceCtx* c, int mode, int64_t M, int64_t N, int64_t
     def.split = std::atoi(e);
     return def;
   }
-  const std::vector<int> splits = split_candidates(c, mode, M, N, K);
+  def.split = split_parts(c, mode, M, N, K);
   // GBBLAS_TC_PAIR, when set, fixes the CTA form; otherwise the tuner picks it
   // (pairs only where padding M to 256 rows adds at most 10 % of the work)
   const char* pe = std::getenv("GBBLAS_TC_PAIR");
   const bool pair_env = pe && pe[0];
-  const int single = pair_env ? -1 : 0;
+  def.pair = pair_env ? -1 : 0;
   const bool pairs = !pair_env && mode != tc_mode(GBBLAS_ACCURACY_FP8) && mode != tc_mode(GBBLAS_ACCURACY_FP16X3) &&
+                     mode != kTcModeF16Guard &&
                      M >= 256 &&
                      (double)((M + 255) / 256 * 256) <= 1.1 * (double)((M + 127) / 128 * 128);
-  // without measurements: the largest listed split (the tiles alone leave
-  // most SMs idle) and the GBBLAS_TC_PAIR setting
-  TcLaunchOpts fallback = def;
-  if (!splits.empty()) fallback.split = splits.back();
-  if (splits.empty() && !pairs) return def;
+  if (!pairs) return def;
   Tuner& t = Tuner::get();
   const int bm = log2_bucket(M), bn = log2_bucket(N), bk = log2_bucket(K);
   const std::string key = "gemm_tc|" + device_tag(c) + "|mode" + std::to_string(mode) + "|m" + std::to_string(bm) +
-                          "|n" + std::to_string(bn) + "|k" + std::to_string(bk);
+                          "|n" + std::to_string(bn) + "|k" + std::to_string(bk) + "|pair";
   const int v = t.lookup(key);
-  if (v >= 0) return TcLaunchOpts{std::max(1, v / 4), pair_env ? -1 : v % 4 - 1};
-  if (!t.enabled() || capturing(stream)) return fallback;
+  if (v >= 0) return v == 1 ? TcLaunchOpts{1, 1} : def;
+  if (!t.enabled() || capturing(stream)) return def;
   int64_t m, n, k;
   bucket_shape(bm, bn, bk, m, n, k);
-  std::vector<TcLaunchOpts> cands{TcLaunchOpts{1, single}};
-  for (int s : split_candidates(c, mode, m, n, k)) cands.push_back(TcLaunchOpts{s, single});
-  if (pairs && m >= 256) cands.push_back(TcLaunchOpts{1, 1});
-  if (cands.size() == 1) return fallback;
+  if (m < 256) return def;
   GemmBench b(c, m, n, k);
-  if (!b.ok()) return fallback;
+  if (!b.ok()) return def;
   const gbblas_gemm_desc d = b.desc();
-  TcLaunchOpts best = fallback;
-  float best_ms = 1e30f;
-  for (const TcLaunchOpts& o : cands) {
-    const float ms = b.time([&](cudaStream_t s) { return launch_gemm_tc_opts(c, mode, d, o, s); });
-    if (ms < best_ms) {
-      best_ms = ms;
-      best = o;
-    }
-  }
-  if (best_ms >= 1e30f) return fallback;
-  t.store(key, best.split * 4 + best.pair + 1);
-  return best;
+  float ms[2];
+  const TcLaunchOpts cands[2] = {TcLaunchOpts{split_parts(c, mode, m, n, k), 0}, TcLaunchOpts{1, 1}};
+  for (int i = 0; i < 2; ++i)
+    ms[i] = b.time([&](cudaStream_t s) { return launch_gemm_tc_opts(c, mode, d, cands[i], s); });
+  if (ms[0] >= 1e30f && ms[1] >= 1e30f) return def;
+  const int best = ms[1] < ms[0] ? 1 : 0;
+  t.store(key, best);
+  return best == 1 ? cands[1] : def;
 }
 
 int tuned_fma_tile(DeviceCtx* c, const gbblas_gemm_desc& g, cudaStream_t stream) {

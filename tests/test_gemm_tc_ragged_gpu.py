@@ -75,3 +75,26 @@ def test_operand_routes_same_bits(cuda, acc, M, N, K, pad, off, cols):
     want = gemm(cuda, A, B, C0, acc, (0, 0, 2), (0, 0, 2), (0, 0), False, False)
     got = gemm(cuda, A, B, C0, acc, (pad, off), (pad, off), (0, 0), cols, not cols)
     np.testing.assert_array_equal(got, want)
+
+
+# K cut into parts under AUTO's guard: outputs in out-of-span rows and columns
+# are left out of the partials and computed once by the fix-up; everything
+# stays inside the guard's bound (2^-19 + 2 K eps32) (|A||B|) plus the addition
+# into C, and repeats bit for bit
+@pytest.mark.parametrize("parts", [1, 2, 3, 16])
+@pytest.mark.parametrize("M,N,K", [(40, 30, 1025), (129, 257, 4100), (300, 64, 2048)])
+@pytest.mark.parametrize("lc", [False, True])
+def test_split_k_under_the_guard(cuda, monkeypatch, parts, M, N, K, lc):
+    monkeypatch.setenv("GBBLAS_GEMM_AUTO", "1")
+    monkeypatch.setenv("GBBLAS_TC_SPLITK", str(parts))
+    rng = np.random.default_rng(parts + M)
+    A, B, C0 = values(rng, (M, K)), values(rng, (K, N)), values(rng, (M, N))
+    A[M // 3] *= np.float32(2.0 ** -30)  # a row and a column whose magnitudes span too far
+    A[M // 3, 0] = 1.0
+    B[:, N // 2] *= np.float32(2.0 ** -30)
+    B[0, N // 2] = 1.0
+    got = gemm(cuda, A, B, C0, 3, (1, 0), (0, 0), (1, 0), False, False, lc)
+    exact = A.astype(np.float64) @ B.astype(np.float64) + C0
+    mag = np.abs(A).astype(np.float64) @ np.abs(B)
+    assert np.all(np.abs(got - exact) <= (2.0 ** -19 + 2 * K * 2.0 ** -23) * mag + 2.0 ** -23 * (np.abs(C0) + mag))
+    np.testing.assert_array_equal(gemm(cuda, A, B, C0, 3, (1, 0), (0, 0), (1, 0), False, False, lc), got)
