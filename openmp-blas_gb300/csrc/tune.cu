@@ -41,6 +41,7 @@
 #include <regex>
 #include <sstream>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "common.cuh"
@@ -59,6 +60,20 @@ class Tuner {
   }
 
   bool enabled() const { return enabled_; }
+
+  // Choices this process has looked up or made, by a packed key: every call
+  // asks, and building the text key and searching for it took 1.5 us of a
+  // call's host time.
+  int recall(uint64_t packed) {
+    std::lock_guard<std::mutex> lk(mu_);
+    auto it = memo_.find(packed);
+    return it == memo_.end() ? -1 : it->second;
+  }
+  int remember(uint64_t packed, int value) {
+    std::lock_guard<std::mutex> lk(mu_);
+    memo_[packed] = value;
+    return value;
+  }
 
   // Cached choice for `key`, or -1.
   int lookup(const std::string& key) {
@@ -125,6 +140,7 @@ class Tuner {
 
   std::mutex mu_;
   std::map<std::string, int> cache_;
+  std::unordered_map<uint64_t, int> memo_;  // bounded by the number of keys
   bool loaded_ = false;
   bool enabled_ = true;
   std::string path_;
@@ -137,6 +153,13 @@ std::string device_tag(DeviceCtx* c) {
   std::replace(name.begin(), name.end(), ' ', '_');
   return name + "_sm" + std::to_string(c->num_sms);
 }
+
+// Packed form of a key: what is chosen (op), mode or layout flags, device, buckets.
+uint64_t pack_key(int op, int flags, DeviceCtx* c, int bm, int bn, int bk) {
+  return (uint64_t)op | (uint64_t)flags << 4 | (uint64_t)c->device << 12 | (uint64_t)bm << 20 | (uint64_t)bn << 28 |
+         (uint64_t)bk << 36;
+}
+enum : int { kOpAuto = 1, kOpPair = 2, kOpFma = 3 };
 
 int log2_bucket(int64_t v) { return v <= 1 ? 0 : (int)std::lround(std::log2((double)v)); }
 
@@ -267,10 +290,12 @@ int tuned_gemm_auto(DeviceCtx* c, int64_t M, int64_t N, int64_t K) {
   const int fallback = (M >= 256 && N >= 256 && K >= 256 && (double)M * N * K >= 1.0e9) ? 1 : 0;
   Tuner& t = Tuner::get();
   const int bm = log2_bucket(M), bn = log2_bucket(N), bk = log2_bucket(K);
+  const uint64_t packed = pack_key(kOpAuto, 0, c, bm, bn, bk);
+  if (const int m = t.recall(packed); m >= 0) return m;
   const std::string key = "gemm_auto_f16s|" + device_tag(c) + "|m" + std::to_string(bm) + "|n" + std::to_string(bn) +
                           "|k" + std::to_string(bk) + "|f32";
   int v = t.lookup(key);
-  if (v >= 0) return v;
+  if (v >= 0) return t.remember(packed, v);
   if (!t.enabled()) return fallback;
   // representative shape of the bucket, capped so tuning stays cheap
   const int64_t m = std::min<int64_t>(int64_t(1) << bm, 8192), n = std::min<int64_t>(int64_t(1) << bn, 8192),
@@ -316,7 +341,7 @@ int tuned_gemm_auto(DeviceCtx* c, int64_t M, int64_t N, int64_t K) {
   if (best_ms[0] >= 1e30f && best_ms[1] >= 1e30f) return fallback;
   const int best = best_ms[1] < best_ms[0] ? 1 : 0;
   t.store(key, best);
-  return best;
+  return t.remember(packed, best);
 }
 
 // Split-K parts of an M x N x K tensor-core GEMM on single CTAs: the number
@@ -371,10 +396,12 @@ TcLaunchOpts tuned_tc_opts(DeviceCtx* c, int mode, int64_t M, int64_t N, int64_t
   if (!pairs) return def;
   Tuner& t = Tuner::get();
   const int bm = log2_bucket(M), bn = log2_bucket(N), bk = log2_bucket(K);
+  const uint64_t packed = pack_key(kOpPair, mode, c, bm, bn, bk);
+  if (const int m = t.recall(packed); m >= 0) return m == 1 ? TcLaunchOpts{1, 1} : def;
   const std::string key = "gemm_tc|" + device_tag(c) + "|mode" + std::to_string(mode) + "|m" + std::to_string(bm) +
                           "|n" + std::to_string(bn) + "|k" + std::to_string(bk) + "|pair";
   const int v = t.lookup(key);
-  if (v >= 0) return v == 1 ? TcLaunchOpts{1, 1} : def;
+  if (v >= 0) return t.remember(packed, v) == 1 ? TcLaunchOpts{1, 1} : def;
   if (!t.enabled() || capturing(stream)) return def;
   int64_t m, n, k;
   bucket_shape(bm, bn, bk, m, n, k);
@@ -389,7 +416,7 @@ TcLaunchOpts tuned_tc_opts(DeviceCtx* c, int mode, int64_t M, int64_t N, int64_t
   if (ms[0] >= 1e30f && ms[1] >= 1e30f) return def;
   const int best = ms[1] < ms[0] ? 1 : 0;
   t.store(key, best);
-  return best == 1 ? cands[1] : def;
+  return t.remember(packed, best) == 1 ? cands[1] : def;
 }
 
 int tuned_fma_tile(DeviceCtx* c, const gbblas_gemm_desc& g, cudaStream_t stream) {
@@ -407,11 +434,13 @@ int tuned_fma_tile(DeviceCtx* c, const gbblas_gemm_desc& g, cudaStream_t stream)
   const bool tma = sgemm_tma_eligible(M, N, K, A, rsa, csa, B, rsb, csb);
   Tuner& t = Tuner::get();
   const int bm = log2_bucket(M), bn = log2_bucket(N), bk = log2_bucket(K);
+  const uint64_t packed = pack_key(kOpFma, (a_col ? 1 : 0) | (b_col ? 2 : 0) | (tma ? 4 : 0), c, bm, bn, bk);
+  if (const int m = t.recall(packed); m >= 0) return m;
   const std::string key = "gemm_fma_tile|" + device_tag(c) + "|m" + std::to_string(bm) + "|n" + std::to_string(bn) +
                           "|k" + std::to_string(bk) + (a_col ? "|ac" : "|ar") + (b_col ? "|bc" : "|br") +
                           (tma ? "|t" : "|u") + "|f32";
   const int v = t.lookup(key);
-  if (v >= 0) return v;
+  if (v >= 0) return t.remember(packed, v);
   if (!t.enabled() || capturing(stream)) return -1;
   int64_t m, n, k;
   bucket_shape(bm, bn, bk, m, n, k);
@@ -442,7 +471,7 @@ int tuned_fma_tile(DeviceCtx* c, const gbblas_gemm_desc& g, cudaStream_t stream)
   }
   if (best < 0) return -1;
   t.store(key, best);
-  return best;
+  return t.remember(packed, best);
 }
 
 }  // namespace gbblas

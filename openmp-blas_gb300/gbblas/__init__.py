@@ -157,7 +157,9 @@ def _check(fn: str, status: int) -> None:
 
 def call(name: str, *args) -> None:
     """Call a C-ABI function by name and raise GbblasError on a non-zero status."""
-    _check(name, getattr(lib(), name)(*args))
+    status = getattr(_lib if _lib is not None else lib(), name)(*args)
+    if status != 0:
+        _check(name, status)
 
 
 def status_of(name: str, *args) -> int:
@@ -167,19 +169,39 @@ def status_of(name: str, *args) -> int:
 
 # ---------------------------------------------------------------- torch helpers
 
+# These helpers run on every call, and a small call's time is its host time:
+# torch is looked up once, and the current stream's handle is read without
+# building a torch.cuda.Stream (2.9 us of a dot's 8.0; 0.2 this way).
+
+_torch = None
+_raw_stream = None  # device index -> the current stream's handle
+
+
+def _torch_module():
+    global _torch, _raw_stream
+    if _torch is None:
+        import torch
+        get = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        _raw_stream = get if get is not None else (lambda device: torch.cuda.current_stream(device).cuda_stream)
+        _torch = torch
+    return _torch
+
+
 def _stream_ptr(stream) -> int | None:
-    import torch
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return s.cuda_stream or None
+    if stream is not None:
+        return stream.cuda_stream or None
+    torch = _torch if _torch is not None else _torch_module()
+    return _raw_stream(torch.cuda.current_device()) or None
 
 
 def _pfx(t) -> str:
-    import torch
-    if t.dtype == torch.float32:
+    torch = _torch if _torch is not None else _torch_module()
+    d = t.dtype
+    if d is torch.float32:
         return "s"
-    if t.dtype == torch.float64:
+    if d is torch.float64:
         return "d"
-    raise TypeError(f"unsupported dtype {t.dtype}")
+    raise TypeError(f"unsupported dtype {d}")
 
 
 def _dev(t) -> int:
@@ -196,8 +218,8 @@ def gemm(A, B, C, accuracy: int = ACCURACY_FP32, stream=None):
     M, K = A.shape
     N = B.shape[1]
     p = _pfx(A)
-    args = [M, N, K, _dev(A), A.stride(0), A.stride(1), _dev(B), B.stride(0), B.stride(1),
-            _dev(C), C.stride(0), C.stride(1)]
+    (rsa, csa), (rsb, csb), (rsc, csc) = A.stride(), B.stride(), C.stride()
+    args = (M, N, K, _dev(A), rsa, csa, _dev(B), rsb, csb, _dev(C), rsc, csc)
     if p == "s":
         call("gbblas_sgemm", *args, accuracy, _stream_ptr(stream))
     elif accuracy == ACCURACY_FP32:
@@ -226,7 +248,8 @@ def gemv(layout: int, transpose: bool, M: int, N: int, A, x, y, accumulate: bool
 
 def dot(a, b, out, stream=None):
     """out[0] = a . b (out is a 1-element device tensor)."""
-    call(f"gbblas_{_pfx(a)}dot", a.numel(), _dev(a), _dev(b), _dev(out), _stream_ptr(stream))
+    call("gbblas_sdot" if _pfx(a) == "s" else "gbblas_ddot", a.numel(), _dev(a), _dev(b), _dev(out),
+         _stream_ptr(stream))
     return out
 
 
