@@ -14,8 +14,11 @@
 //
 // Accuracy: FP32 partials are Kahan-compensated (products and sums rounded
 // with __fmul_rn / __fadd_rn so the compiler cannot contract them into FMAs
-// and lose the compensation) and are combined in FP64; FP64 dots use plain
+// and lose the compensation), are combined as unevaluated pairs of floats
+// within a warp (46 bits) and in FP64 beyond it; FP64 dots use plain
 // FMA partials.  Roofline: HBM bandwidth, 2*n*sizeof(T) bytes per call.
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace gbblas {
@@ -28,6 +31,39 @@ constexpr int kDotUnroll = 4;
 // pairs stream as fast as unclustered CTAs (f32 0.303 ms, f64 0.629 vs 0.623),
 // clusters of 4 / 8 lose 15-30 % of the bandwidth.
 constexpr int kDotCluster = 2;
+// Short vectors: latency - launch, one round of loads, the reduction - is all
+// they cost, and the partials' last-CTA step adds 2 us to it.  Up to kDotOne
+// bytes of an operand go to one CTA, up to eight times that to one cluster of
+// CTAs, which adds through distributed shared memory and touches no scratch;
+// FP64 takes fewer bytes per CTA, its products being bound by the FP64 pipes
+// (16 cycles per warp and SM).  us per call, back to back, before and after
+// (FP64 totals per thread, pairs of CTAs throughout): f32 1000 elements 6.2 ->
+// 4.1, 8192 6.2 -> 4.6, 65536 8.2 -> 6.2, 1567544 12.3 -> 8.2, 13466139 20.5 ->
+// 14.4; f64 1000 6.2 -> 5.2, 16384 8.2 -> 6.2, 1000000 13.5 -> 10.3.
+constexpr int kDotOneThreads = 512;
+template <typename T>
+constexpr int64_t kDotOne = sizeof(T) == 4 ? 32768 : 16384;
+
+// A sum as an unevaluated pair of floats, hi + lo with |lo| <= ulp(hi) / 2.
+// Two of them add with about 2^-46 of relative error (Knuth's TwoSum on the
+// leading parts, the trailing parts added to its error term, renormalised):
+// FP32 instructions, where GB300's FP64 pipes take 16 cycles per warp
+// instruction and SM - a CTA of 256 threads spent 1000 cycles adding its
+// threads' FP64 totals.
+struct FloatPair {
+  float hi, lo;
+};
+__device__ __forceinline__ FloatPair two_sum(float a, float b) {
+  const float s = __fadd_rn(a, b);
+  const float t = __fsub_rn(s, a);
+  return {s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t))};
+}
+__device__ __forceinline__ FloatPair add(FloatPair a, FloatPair b) {
+  const FloatPair s = two_sum(a.hi, b.hi);
+  const FloatPair e = two_sum(a.lo, b.lo);
+  const FloatPair u = two_sum(s.hi, __fadd_rn(s.lo, e.hi));
+  return two_sum(u.hi, __fadd_rn(u.lo, e.lo));
+}
 
 // Per-thread accumulator.  FP32: four Kahan lanes.  FP64: four FMA lanes.
 template <typename T>
@@ -50,9 +86,19 @@ struct DotAcc<float> {
     add(2, a.z, b.z);
     add(3, a.w, b.w);
   }
-  __device__ __forceinline__ double total() const {
+  // Whether a warp's lanes might not add up in FP32: 128 of them below 2^120
+  // stay below 2^127.  (Also true of Inf and NaN.)
+  __device__ __forceinline__ bool wide() const {
+    const float most = 0x1p120f;
+    return !(fabsf(s[0]) < most && fabsf(s[1]) < most && fabsf(s[2]) < most && fabsf(s[3]) < most);
+  }
+  __device__ __forceinline__ double total64() const {
     return (((double)s[0] - (double)c[0]) + ((double)s[1] - (double)c[1])) +
            (((double)s[2] - (double)c[2]) + ((double)s[3] - (double)c[3]));
+  }
+  __device__ __forceinline__ FloatPair total() const {
+    return gbblas::add(gbblas::add(two_sum(s[0], -c[0]), two_sum(s[1], -c[1])),
+                       gbblas::add(two_sum(s[2], -c[2]), two_sum(s[3], -c[3])));
   }
 };
 
@@ -92,17 +138,60 @@ __device__ __forceinline__ void acc_vec<double>(DotAcc<double>& acc, double2 a, 
   acc.add4(a, b, u & 1);
 }
 
+// The sum of the CTA's threads' doubles, in thread 0 (fixed order): through
+// shared memory, added by one warp - 12 FP64 warp instructions for 256
+// threads in place of five per warp.  `sh` holds NT doubles.
+template <int NT>
+__device__ __forceinline__ double cta_sum(double v, double* sh) {
+  sh[threadIdx.x] = v;
+  __syncthreads();
+  double t = 0.0;
+  if (threadIdx.x < 32) {
+    t = sh[threadIdx.x];
+#pragma unroll
+    for (int i = 32; i < NT; i += 32) t += sh[threadIdx.x + i];
+    t = dev::warp_sum(t);
+  }
+  return t;
+}
+
+// The CTA's total, in thread 0.  FP32: pairs of floats through the warp
+// shuffles (FP64 in a warp whose lanes could overflow), then the warps' totals
+// in FP64.
+template <int NT>
+__device__ __forceinline__ double cta_total_of(const DotAcc<float>& acc, double* sh) {
+  double w;
+  if (__any_sync(0xffffffffu, acc.wide())) {
+    w = dev::warp_sum(acc.total64());
+  } else {
+    FloatPair v = acc.total();
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+      v = add(v, FloatPair{__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)});
+    w = (double)v.hi + (double)v.lo;
+  }
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = w;
+  __syncthreads();
+  double t = 0.0;
+  if (threadIdx.x < 32) t = dev::warp_sum(threadIdx.x < NT / 32 ? sh[threadIdx.x] : 0.0);
+  return t;
+}
+template <int NT>
+__device__ __forceinline__ double cta_total_of(const DotAcc<double>& acc, double* sh) {
+  return cta_sum<NT>(acc.total(), sh);
+}
+
 // One pass over a[0:n) . b[0:n).  VEC: both pointers 16-byte aligned.
 // partials[gridDim.x / kDotCluster] (FP64) and *counter live in scratch;
 // with one cluster they are not touched.  No thread leaves before the two
-// cluster barriers.
-template <typename T, bool VEC>
-__global__ void __launch_bounds__(kDotThreads, kDotCtasPerSm)
+// cluster barriers.  NT threads per CTA.
+template <typename T, bool VEC, int NT>
+__global__ void __launch_bounds__(NT, kDotCtasPerSm * kDotThreads / NT)
     dot_kernel(const T* __restrict__ a, const T* __restrict__ b, int64_t n, double* __restrict__ partials,
                unsigned* __restrict__ counter, T* __restrict__ result) {
   using V = typename Vec<T>::type;
   constexpr int W = Vec<T>::width;
-  __shared__ double sh[32];
+  __shared__ double sh[NT];
   __shared__ double cta_total;  // read by the cluster's rank 0
   __shared__ bool is_last;
 
@@ -130,7 +219,7 @@ __global__ void __launch_bounds__(kDotThreads, kDotCtasPerSm)
   }
   for (int64_t i = tail_start + tid; i < n; i += nthr) acc.add(0, dev::ld_stream(a + i), dev::ld_stream(b + i));
 
-  const double block_total = dev::block_sum<double>(acc.total(), sh);
+  const double block_total = cta_total_of<NT>(acc, sh);  // thread 0's
 
   // cluster step: rank 0 adds the cluster's CTA totals in rank order
   const unsigned csize = dev::cluster_size();
@@ -163,31 +252,31 @@ __global__ void __launch_bounds__(kDotThreads, kDotCtasPerSm)
   if (!is_last) return;
   __threadfence();
   double t = 0.0;
-  for (int i = threadIdx.x; i < nclusters; i += blockDim.x) t += __ldcg(partials + i);
-  t = dev::block_sum<double>(t, sh);
+  for (int i = threadIdx.x; i < nclusters; i += NT) t += __ldcg(partials + i);
+  t = cta_sum<NT>(t, sh);
   if (threadIdx.x == 0) {
     *result = (T)t;
     *counter = 0u;  // ready for the next call on this scratch
   }
 }
 
-// grid: a multiple of kDotCluster; clusters of kDotCluster CTAs.
-template <typename T>
-cudaError_t launch_dot_kernel(bool vec, int grid, cudaStream_t stream, const T* a, const T* b, int64_t n,
+// grid: a multiple of `cluster`; clusters of that many CTAs.
+template <typename T, int NT = kDotThreads>
+cudaError_t launch_dot_kernel(bool vec, int grid, int cluster, cudaStream_t stream, const T* a, const T* b, int64_t n,
                               double* partials, unsigned* counter, T* result) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3(kDotThreads);
+  cfg.blockDim = dim3(NT);
   cfg.stream = stream;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = kDotCluster;
+  at[0].val.clusterDim.x = (unsigned)cluster;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = kDotCluster > 1 ? 1 : 0;
-  return vec ? cudaLaunchKernelEx(&cfg, dot_kernel<T, true>, a, b, n, partials, counter, result)
-             : cudaLaunchKernelEx(&cfg, dot_kernel<T, false>, a, b, n, partials, counter, result);
+  cfg.numAttrs = cluster > 1 ? 1 : 0;
+  return vec ? cudaLaunchKernelEx(&cfg, dot_kernel<T, true, NT>, a, b, n, partials, counter, result)
+             : cudaLaunchKernelEx(&cfg, dot_kernel<T, false, NT>, a, b, n, partials, counter, result);
 }
 
 }  // namespace
@@ -195,20 +284,25 @@ cudaError_t launch_dot_kernel(bool vec, int grid, cudaStream_t stream, const T* 
 template <typename T>
 gbblas_status launch_dot(DeviceCtx* c, int64_t n, const T* a, const T* b, T* result, cudaStream_t stream) {
   const bool vec = aligned16(a) && aligned16(b);
+  const int64_t bytes = n * (int64_t)sizeof(T);
+  if (bytes <= 8 * kDotOne<T>) {
+    const int ctas = (int)std::max<int64_t>(1, (bytes + kDotOne<T> - 1) / kDotOne<T>);
+    GB_CUDA_TRY((launch_dot_kernel<T, kDotOneThreads>(vec, ctas, ctas, stream, a, b, n, nullptr, nullptr, result)));
+    return check_launch("dot_kernel");
+  }
   const int64_t per_cta = (int64_t)kDotThreads * kDotUnroll * Vec<T>::width;
   int64_t want = (n + per_cta - 1) / per_cta;
   const int64_t full = (int64_t)c->num_sms * kDotCtasPerSm;
-  int grid = (int)(want < full ? (want < 1 ? 1 : want) : full);
-  grid = (grid + kDotCluster - 1) / kDotCluster * kDotCluster;  // whole clusters
-  double* partials = nullptr;
-  unsigned* counter = nullptr;
-  if (grid > kDotCluster) {
-    void* s = nullptr;
-    GB_TRY(get_scratch(c, stream, kScratchZeroBytes + sizeof(double) * (grid / kDotCluster), &s));
-    counter = reinterpret_cast<unsigned*>(s);
-    partials = reinterpret_cast<double*>(static_cast<char*>(s) + kScratchZeroBytes);
-  }
-  GB_CUDA_TRY(launch_dot_kernel<T>(vec, grid, stream, a, b, n, partials, counter, result));
+  // clusters only once the grid is full (fewer partials for the last one to
+  // add); below that their barriers only add latency
+  const int cluster = want >= full ? kDotCluster : 1;
+  int grid = (int)std::min(want, full);
+  grid = (grid + cluster - 1) / cluster * cluster;  // whole clusters
+  void* s = nullptr;
+  GB_TRY(get_scratch(c, stream, kScratchZeroBytes + sizeof(double) * (grid / cluster), &s));
+  unsigned* counter = reinterpret_cast<unsigned*>(s);
+  double* partials = reinterpret_cast<double*>(static_cast<char*>(s) + kScratchZeroBytes);
+  GB_CUDA_TRY(launch_dot_kernel<T>(vec, grid, cluster, stream, a, b, n, partials, counter, result));
   return check_launch("dot_kernel");
 }
 
@@ -314,6 +408,6 @@ extern "C" gbblas_status gbblas_sdot_noalloc(int64_t n, const float* a, const fl
   double* partials = reinterpret_cast<double*>(static_cast<char*>(d->scratch) + kScratchZeroBytes);
   // The counter must start at zero; partials are fully rewritten by each call.
   GB_CUDA_TRY(cudaMemsetAsync(counter, 0, sizeof(unsigned), s));
-  GB_CUDA_TRY(launch_dot_kernel<float>(vec, (int)grid, s, a, b, n, partials, counter, result));
+  GB_CUDA_TRY(launch_dot_kernel<float>(vec, (int)grid, kDotCluster, s, a, b, n, partials, counter, result));
   return check_launch("dot_kernel (noalloc)");
 }
