@@ -13,16 +13,25 @@
 //              simd_loop.hpp:52-78, accumulates into y) and vtm with
 //              row-major A.
 //
-// Both stream A from HBM exactly once with 128-bit read-only loads and keep
-// x in L1/L2.  When the grid would be too small to fill the 152 SMs the
-// reduction dimension is split across CTAs.  Two splits, or up to 8 on a
-// small matrix, run as one thread-block cluster per row block: each CTA
-// leaves its partials in its shared memory and the cluster's rank 0 adds
-// them in split order through distributed shared memory.  Otherwise the
-// partials go to per-stream scratch and a second small kernel adds them in
-// split order.  Either way
-// the additions are in the same order and deterministic (no atomics).
-// Roofline: HBM, (rows*cols + rows + cols) * sizeof(T) bytes per call.
+// Both stream A from HBM once with 128-bit read-only loads at any leading
+// dimension and keep x in L1 / shared memory.  When the grid would be too
+// small to fill the 152 SMs the reduction dimension is split across CTAs.
+// Up to 8 splits of a small matrix run as one thread-block cluster per row
+// block: each CTA leaves its partials in its shared memory and the
+// cluster's rank 0 adds them in split order through distributed shared
+// memory.  Otherwise the partials go to per-stream scratch and a second small
+// kernel, chained to the first, adds them.  Either way the order of additions
+// is fixed by the shape and the alignment (no atomics).
+// Roofline: HBM, (rows*cols + rows + cols) * sizeof(T) bytes per call; for
+// double the FP64 pipes (2 multiply-adds per clock and SM: 4.6 TB/s of A),
+// so that sums over threads are kept few.  us per call, cold, before (scalar
+// loads at odd leading dimensions, a CTA per four rows, a thread per row of a
+// column) and now: rows f32 16384^2 153.9 -> 148, 8191 x 6001 48.3 -> 35.4,
+// 25596 x 256 16.4 -> 8.5; f64 18652 x 947 86 -> 45, 25596 x 256 82 -> 20;
+// columns f32 16384^2 156.4 -> 154, 10001 x 10003 166 -> 69, 256 x 25596 36 -> 12;
+// f64 8191 x 6001 95 -> 92, 10001 x 10003 205 -> 177, 512 x 6552 33 -> 15.
+#include <algorithm>
+#include <type_traits>
 #include <utility>
 
 #include "common.cuh"
@@ -57,201 +66,315 @@ __device__ __forceinline__ float4 ldg_vec(const float4* p) { return __ldg(p); }
 __device__ __forceinline__ double2 ldg_vec(const double2* p) { return __ldg(p); }
 
 constexpr int kRowsThreads = 256;
+constexpr int kWarps = kRowsThreads / 32;
 
 constexpr int kMaxClusterSplits = 8;  // portable cluster size
 
-// Whether the ksplit CTAs of a row block reduce as one cluster.  Measured on
-// split shapes: clusters of two stream as fast as separate CTAs; up to 8 pay
-// off while the matrix is small (12-60 MB: 17-24 % faster, the second launch
-// saved); on large matrices clusters of 3-4 lose up to 17 % of the bandwidth.
+// Whether the ksplit CTAs of a row block reduce as one cluster: on a small
+// matrix, where a second launch is a good part of the call (512 x 512
+// column-major: f32 4.1 us, 5.2 through scratch; f64 6.2 and 7.3).  On larger
+// ones the CTAs of a cluster waiting for one another cost more than the
+// chained finish (20069 x 264 f64: 20.4 us in clusters, 17.7 through scratch;
+// 256 x 25596 f32 12.3 and 10.7).
 inline bool cluster_splits(int64_t ksplit, int64_t rows, int64_t cols, size_t elem) {
-  return ksplit >= 2 && ksplit <= kMaxClusterSplits && (ksplit == 2 || (double)rows * cols * elem <= 64.0e6);
+  return ksplit >= 2 && ksplit <= kMaxClusterSplits && (double)rows * cols * elem <= 8.0e6;
 }
 
-// grid = (ceil(rows / R), ksplit); CTA = 8 warps splitting its column range.
+// The sums of a warp's R values per lane: lane 32 / R * j ends up with the
+// total of value j.  The halves of the warp first trade values, so R = 4 takes
+// 6 additions where a butterfly per value takes 20 (the same pairs are added,
+// so the same bits) - on the FP64 pipes 96 cycles against 320.
+template <typename T>
+__device__ __forceinline__ T warp_totals(const T (&v)[1], int) {
+  return dev::warp_sum(v[0]);
+}
+template <typename T>
+__device__ __forceinline__ T warp_totals(const T (&v)[4], int lane) {
+  const bool h = lane & 16, q = lane & 8;
+  T a = (h ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, h ? v[0] : v[2], 16);
+  T b = (h ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, h ? v[1] : v[3], 16);
+  T t = (q ? b : a) + __shfl_xor_sync(0xffffffffu, q ? a : b, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  return t;
+}
+
+// Row-streaming form.  A CTA's 8 warps are 8 / wc row groups of wc warps; a
+// group computes R rows, its warps sharing the columns out 32 vectors at a
+// time.  The R rows of a group lie `period` apart, the distance at which every
+// row starts at the same offset from a 16-byte boundary: the group's `head`
+// elements up to it and its last few are added one by one, everything between
+// by 128-bit loads, and x is read once for all R rows (by vectors where it
+// shares their alignment).  grid = (groups / groups per CTA, ksplit); split p
+// covers vectors p * vps .. + vps - 1.
 // CL: the ksplit CTAs of a row block form a cluster (1, ksplit, 1).
-template <typename T, int R, bool VEC, bool CL>
-__global__ void __launch_bounds__(kRowsThreads) gemv_rows_kernel(int64_t rows, int64_t cols,
-                                                                 const T* __restrict__ A, int64_t lda,
-                                                                 const T* __restrict__ x, T* __restrict__ y,
-                                                                 bool accumulate, T* __restrict__ partials,
-                                                                 int64_t cols_per_split) {
+template <typename T, int R, bool CL>
+__global__ void __launch_bounds__(kRowsThreads, R == 4 ? 3 : 4)
+    gemv_rows_kernel(int64_t rows, int64_t cols, const T* __restrict__ A, int64_t lda, const T* __restrict__ x,
+                     T* __restrict__ y, bool accumulate, T* __restrict__ partials, int64_t vps, int lperiod, int lwc) {
   using VT = typename V<T>::t;
   constexpr int W = V<T>::w;
-  __shared__ T red[kRowsThreads / 32][R];
-  __shared__ T split_part[R];  // CL: this split's row sums, read by the cluster's rank 0
-  const int64_t r0 = (int64_t)blockIdx.x * R;
-  const int64_t c0 = (int64_t)blockIdx.y * cols_per_split;
-  int64_t c1 = c0 + cols_per_split;
-  if (c1 > cols) c1 = cols;
-  const int nr = (int)((rows - r0) < R ? (rows - r0) : R);
-
+  constexpr int U = R == 4 ? 2 : 4;  // vectors per row and lane in flight
+  __shared__ T red[kWarps][R];
+  __shared__ T split_part[kWarps * R];  // CL: this split's row sums, read by the cluster's rank 0
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int period = 1 << lperiod, wc = 1 << lwc;  // powers of two: no division on the way to the first load
+  const int wr = warp >> lwc, wi = warp & (wc - 1);
+  const int groups = kWarps >> lwc;  // of this CTA
+  // first row of a group (its others follow `period` apart)
+  auto first_row = [&](int w) {
+    const int64_t g = (int64_t)blockIdx.x * groups + w;
+    return ((g >> lperiod) * R << lperiod) + (g & (period - 1));
+  };
+  const int64_t r0 = first_row(wr);
+  const int nr = r0 < rows ? (int)min((rows - r0 + period - 1) >> lperiod, (int64_t)R) : 0;
+  const T* __restrict__ row = A + (nr > 0 ? r0 : 0) * lda;
+  const int64_t rstep = lda << lperiod;
+  int64_t head = (int64_t)(((16 - (reinterpret_cast<uintptr_t>(row) & 15)) & 15) / sizeof(T));
+  if (head > cols) head = cols;
+  const int64_t nv = (cols - head) / W;
+  const int64_t v1 = min(((int64_t)blockIdx.y + 1) * vps, nv);
+  const T* __restrict__ xb = x + head;
+  const bool xvec = (reinterpret_cast<uintptr_t>(xb) & 15) == 0;
+  auto xload = [&](int64_t v) {
+    VT r;
+    if (xvec) {
+      r = ldg_vec(reinterpret_cast<const VT*>(xb) + v);
+    } else {
+      T* e = reinterpret_cast<T*>(&r);
+#pragma unroll
+      for (int i = 0; i < W; ++i) e[i] = __ldg(xb + v * W + i);
+    }
+    return r;
+  };
   T acc[R];
 #pragma unroll
-  for (int r = 0; r < R; ++r) acc[r] = T(0);
+  for (int j = 0; j < R; ++j) acc[j] = T(0);
 
-  int64_t scalar_from = c0;
-  if (VEC) {
-    const int64_t v0 = c0 / W, v1 = c1 / W;  // c0 is a multiple of W
-    const VT* xv = reinterpret_cast<const VT*>(x);
-    int64_t v = v0 + threadIdx.x;
-    if (nr == R) {
-      for (; v + kRowsThreads < v1; v += 2 * kRowsThreads) {
-        VT xa = ldg_vec(xv + v), xb = ldg_vec(xv + v + kRowsThreads);
-        VT aa[R], ab[R];
+  const int64_t step = 32 * wc;
+  int64_t v = (int64_t)blockIdx.y * vps + wi * 32 + lane;
+  if (nr == R) {
+    for (; v + (U - 1) * step < v1; v += U * step) {
+      VT a[U][R], xv[U];
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const VT* row = reinterpret_cast<const VT*>(A + (r0 + r) * lda);
-          aa[r] = dev::ld_stream(row + v);
-          ab[r] = dev::ld_stream(row + v + kRowsThreads);
-        }
+      for (int u = 0; u < U; ++u)
 #pragma unroll
-        for (int r = 0; r < R; ++r) acc[r] = vdot(ab[r], xb, vdot(aa[r], xa, acc[r]));
-      }
+        for (int j = 0; j < R; ++j)
+          a[u][j] = dev::ld_stream(reinterpret_cast<const VT*>(row + head + j * rstep) + v + u * step);
+#pragma unroll
+      for (int u = 0; u < U; ++u) xv[u] = xload(v + u * step);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int j = 0; j < R; ++j) acc[j] = vdot(a[u][j], xv[u], acc[j]);
     }
-    for (; v < v1; v += kRowsThreads) {
-      VT xa = ldg_vec(xv + v);
+  }
+  for (; v < v1; v += step) {
+    const VT xv = xload(v);
 #pragma unroll
-      for (int r = 0; r < R; ++r)
-        if (r < nr) acc[r] = vdot(dev::ld_stream(reinterpret_cast<const VT*>(A + (r0 + r) * lda) + v), xa, acc[r]);
+    for (int j = 0; j < R; ++j)
+      if (j < nr) acc[j] = vdot(dev::ld_stream(reinterpret_cast<const VT*>(row + head + j * rstep) + v), xv, acc[j]);
+  }
+  if (blockIdx.y == 0 && wi == 0) {  // the elements before the first vector and after the last
+    const int64_t tail = cols - head - nv * W;
+    const int64_t c = lane < head ? lane : (lane >= 8 && lane - 8 < tail ? head + nv * W + lane - 8 : -1);
+    if (c >= 0) {
+      const T xc = __ldg(x + c);
+#pragma unroll
+      for (int j = 0; j < R; ++j)
+        if (j < nr) acc[j] = fma(dev::ld_stream(row + j * rstep + c), xc, acc[j]);
     }
-    scalar_from = v1 * W;
   }
-  for (int64_t c = scalar_from + threadIdx.x; c < c1; c += kRowsThreads) {
-    T xc = __ldg(x + c);
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-      if (r < nr) acc[r] = fma(dev::ld_stream(A + (r0 + r) * lda + c), xc, acc[r]);
-  }
+  dev::grid_release();  // a chained finish_splits_kernel may be set up
 
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    T s = dev::warp_sum(acc[r]);
-    if (lane == 0) red[warp][r] = s;
-  }
+  const T t = warp_totals(acc, lane);
+  if (lane % (32 / R) == 0) red[warp][lane / (32 / R)] = t;
   __syncthreads();
-  if (threadIdx.x < nr) {
-    const int r = threadIdx.x;
-    T s = T(0);
-#pragma unroll
-    for (int w = 0; w < kRowsThreads / 32; ++w) s += red[w][r];
-    if (CL) {
-      split_part[r] = s;
-    } else if (gridDim.y == 1) {
-      y[r0 + r] = accumulate ? y[r0 + r] + s : s;
-    } else {
-      partials[(int64_t)blockIdx.y * rows + r0 + r] = s;
-    }
+  const int fw = (int)threadIdx.x / R, fj = (int)threadIdx.x % R;  // this thread's group and row of it
+  const int64_t r = fw < groups ? first_row(fw) + (int64_t)fj * period : rows;
+  T sum = T(0);
+  if (r < rows) {
+    for (int w = 0; w < wc; ++w) sum += red[fw * wc + w][fj];
+    if (CL)
+      split_part[threadIdx.x] = sum;
+    else if (gridDim.y == 1)
+      y[r] = accumulate ? y[r] + sum : sum;
+    else
+      partials[(int64_t)blockIdx.y * rows + r] = sum;
   }
   if constexpr (CL) {
+    __syncwarp();
     dev::cluster_sync();
-    if (blockIdx.y == 0 && threadIdx.x < nr) {  // rank 0 of the cluster: splits in order
-      const int r = threadIdx.x;
+    if (blockIdx.y == 0 && r < rows) {  // rank 0 of the cluster: splits in order
       T s = T(0);
-      for (unsigned k = 0; k < gridDim.y; ++k) s += dev::dsmem_ld(&split_part[r], k);
-      y[r0 + r] = accumulate ? y[r0 + r] + s : s;
+      for (unsigned k = 0; k < gridDim.y; ++k) s += dev::dsmem_ld(&split_part[threadIdx.x], k);
+      y[r] = accumulate ? y[r] + s : s;
     }
+    __syncwarp();
     dev::cluster_sync();  // the other splits stay resident until rank 0 has read them
   }
 }
 
-// y[r] = (accumulate ? y[r] : 0) + sum_s partials[s*rows + r], s in order.
+// y[r] = (accumulate ? y[r] : 0) + sum_s partials[s*rows + r].  Up to 16
+// splits: a thread per row, in split order.  More: 8 threads per row, thread
+// g adding splits g, g + 8, ..., their sums then added in order of g (a
+// thread alone waited for one load after another: 8191 rows of 38 splits took
+// 10.6 us).
+__device__ __forceinline__ int finish_group(int ksplit) { return ksplit > 16 ? 8 : 1; }
+
 template <typename T>
-__global__ void finish_splits_kernel(int64_t rows, int ksplit, const T* __restrict__ partials, T* __restrict__ y,
-                                     bool accumulate) {
-  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= rows) return;
+__global__ void __launch_bounds__(256) finish_splits_kernel(int64_t rows, int ksplit, const T* __restrict__ partials,
+                                                            T* __restrict__ y, bool accumulate) {
+  dev::grid_wait();
+  __shared__ T part[256];
+  const int groups = finish_group(ksplit), per = 256 / groups;
+  const int g = (int)threadIdx.x / per;
+  const int64_t r = (int64_t)blockIdx.x * per + threadIdx.x % per;
   T s = T(0);
-  for (int k = 0; k < ksplit; ++k) s += partials[(int64_t)k * rows + r];
-  y[r] = accumulate ? y[r] + s : s;
+  if (r < rows) {
+    const T* p = partials + r;
+    int k = g;
+    for (; k + 7 * groups < ksplit; k += 8 * groups) {
+      T v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = __ldcg(p + (int64_t)(k + u * groups) * rows);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) s += v[u];
+    }
+    for (; k < ksplit; k += groups) s += __ldcg(p + (int64_t)k * rows);
+  }
+  if (groups > 1) {
+    part[threadIdx.x] = s;
+    __syncthreads();
+    if (g > 0) return;
+    for (int i = 1; i < groups; ++i) s += part[i * per + threadIdx.x];
+  }
+  if (r < rows) y[r] = accumulate ? y[r] + s : s;
 }
 
+// Column-streaming form.  A warp owns 32 VW consecutive rows (a 16-byte
+// vector of VW rows a lane, or one row), a CTA's 8 warps take the columns of
+// its range 8 at a time in turn, and their sums meet in shared memory.
+// SHIFT (VW > 1, columns that do not all start on a 16-byte boundary): column
+// c is read from the boundary at or before its first row of the block, m(c)
+// elements early; columns 4 apart share m, so a lane keeps one set of sums
+// per c % 4 and the sets are shifted back when they meet.  A block then owns
+// the 32 VW - 4 rows that every shift covers.
+// grid = (row blocks, ksplit); split p covers cps columns (a multiple of 64).
+// CL: the ksplit CTAs of a row block form a cluster (1, ksplit, 1).
 constexpr int kColsUnroll = 8;
 
-// grid = (ceil(rows / (threads*W)), ksplit).  Each thread owns W (VEC) or 1
-// consecutive rows and walks its CTA's column range.  CL: the ksplit CTAs of
-// a row block form a cluster (1, ksplit, 1); no thread leaves early then.
-template <typename T, bool VEC, bool CL>
-__global__ void __launch_bounds__(256) gemv_cols_kernel(int64_t rows, int64_t cols, const T* __restrict__ A,
-                                                        int64_t lda, const T* __restrict__ x, T* __restrict__ y,
-                                                        bool accumulate, T* __restrict__ partials,
-                                                        int64_t cols_per_split) {
-  using VT = typename V<T>::t;
-  constexpr int W = VEC ? V<T>::w : 1;
-  __shared__ T split_part[CL ? 256 * W : 1];
-  const int64_t rbase = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * W;
-  if (!CL && rbase >= rows) return;
-  const int64_t c0 = (int64_t)blockIdx.y * cols_per_split;
-  int64_t c1 = c0 + cols_per_split;
-  if (c1 > cols) c1 = cols;
-  T acc[W];
+template <int VW, bool SHIFT>
+struct ColsCfg {
+  static constexpr int kSpan = 32 * VW;                    // rows a warp reads
+  static constexpr int kRows = SHIFT ? kSpan - 4 : kSpan;  // rows a block owns
+  static constexpr int kSets = SHIFT ? 4 : 1;
+};
+
+template <typename T, int VW, bool SHIFT, bool CL>
+__global__ void __launch_bounds__(256, 3)
+    gemv_cols_kernel(int64_t rows, int64_t cols, const T* __restrict__ A, int64_t lda, const T* __restrict__ x,
+                     T* __restrict__ y, bool accumulate, T* __restrict__ partials, int64_t cps, int rw) {
+  using VT = std::conditional_t<VW == 1, T, typename V<T>::t>;
+  using CF = ColsCfg<VW, SHIFT>;
+  constexpr int U = kColsUnroll, SETS = CF::kSets, SPAN = CF::kSpan;
+  static_assert(VW == 1 || VW == V<T>::w, "one row or a 16-byte vector of rows");
+  __shared__ T part[kWarps][SETS][SPAN];
+  __shared__ T split_part[CL ? kWarps * SPAN : 1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int wc = kWarps / rw;  // warps that share a row block's columns
+  const int64_t cta_rb = (int64_t)blockIdx.x * rw * CF::kRows;   // the CTA's first row
+  const int64_t rb = cta_rb + (int64_t)(warp % rw) * CF::kRows;  // this warp's
+  const int64_t c0 = (int64_t)blockIdx.y * cps;
+  const int64_t c1 = min(c0 + cps, cols);
+  T acc[SETS][VW];
 #pragma unroll
-  for (int i = 0; i < W; ++i) acc[i] = T(0);
-  const bool full = rbase + W <= rows;
-  if (rbase >= rows) {
-    // CL only: nothing to add, but the thread still meets the cluster barriers
-  } else if (VEC && full) {
-    const T* base = A + rbase;
-    int64_t c = c0;
-    for (; c + kColsUnroll <= c1; c += kColsUnroll) {
-      VT a[kColsUnroll];
-      T xc[kColsUnroll];
+  for (int q = 0; q < SETS; ++q)
 #pragma unroll
-      for (int u = 0; u < kColsUnroll; ++u) {
-        a[u] = dev::ld_stream(reinterpret_cast<const VT*>(base + (c + u) * lda));
-        xc[u] = __ldg(x + c + u);
+    for (int i = 0; i < VW; ++i) acc[q][i] = T(0);
+  // elements from the 16-byte boundary to column c's row rb (columns 4 apart agree)
+  auto shift_of = [&](int64_t c) {
+    return SHIFT ? (int)((reinterpret_cast<uintptr_t>(A + rb + c * lda) & 15) / sizeof(T)) : 0;
+  };
+  int m[SETS];
+#pragma unroll
+  for (int q = 0; q < SETS; ++q) m[q] = shift_of(c0 + q);  // c0 is a multiple of 4
+
+  // a block whose every vector lies inside its column (not the first or last)
+  const bool inside = (rb >= 4 || !SHIFT) && rb + SPAN <= rows;
+  for (int64_t c = c0 + warp / rw * U; c < c1; c += wc * U) {
+    const T* p = A + rb + VW * lane + c * lda;
+    if (inside && c + U <= c1) {
+      VT a[U];
+      T xv[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) a[u] = dev::ld_stream(reinterpret_cast<const VT*>(p + u * lda - m[u % SETS]));
+#pragma unroll
+      for (int u = 0; u < U; ++u) xv[u] = __ldg(x + c + u);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const T* e = reinterpret_cast<const T*>(&a[u]);
+#pragma unroll
+        for (int i = 0; i < VW; ++i) acc[u % SETS][i] = fma(e[i], xv[u], acc[u % SETS][i]);
+      }
+    } else {
+      T a[U][VW];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int64_t rv = rb + VW * lane - m[u % SETS];  // the vector's first row
+#pragma unroll
+        for (int i = 0; i < VW; ++i)
+          a[u][i] = (c + u < c1 && rv + i >= 0 && rv + i < rows) ? dev::ld_stream(p + u * lda - m[u % SETS] + i) : T(0);
       }
 #pragma unroll
-      for (int u = 0; u < kColsUnroll; ++u) {
-        const T* av = reinterpret_cast<const T*>(&a[u]);
+      for (int u = 0; u < U; ++u)
+        if (c + u < c1) {
+          const T xc = __ldg(x + c + u);
 #pragma unroll
-        for (int i = 0; i < W; ++i) acc[i] = fma(av[i], xc[u], acc[i]);
-      }
-    }
-    for (; c < c1; ++c) {
-      VT a = dev::ld_stream(reinterpret_cast<const VT*>(base + c * lda));
-      T xc = __ldg(x + c);
-      const T* av = reinterpret_cast<const T*>(&a);
-#pragma unroll
-      for (int i = 0; i < W; ++i) acc[i] = fma(av[i], xc, acc[i]);
-    }
-  } else {
-    for (int64_t c = c0; c < c1; ++c) {
-      T xc = __ldg(x + c);
-#pragma unroll
-      for (int i = 0; i < W; ++i)
-        if (rbase + i < rows) acc[i] = fma(dev::ld_stream(A + rbase + i + c * lda), xc, acc[i]);
+          for (int i = 0; i < VW; ++i) acc[u % SETS][i] = fma(a[u][i], xc, acc[u % SETS][i]);
+        }
     }
   }
-  if constexpr (CL) {
+  dev::grid_release();  // a chained finish_splits_kernel may be set up
 #pragma unroll
-    for (int i = 0; i < W; ++i) split_part[threadIdx.x * W + i] = acc[i];
+  for (int q = 0; q < SETS; ++q)
+#pragma unroll
+    for (int i = 0; i < VW; ++i) part[warp][q][VW * lane + i] = acc[q][i];
+  __syncthreads();
+  // the CTA's rows: their sums over the column warps and sets, in order
+  for (int t = threadIdx.x; t < rw * CF::kRows; t += kRowsThreads) {
+    const int64_t r = cta_rb + t;
+    if (r >= rows) break;
+    const int blk = t / CF::kRows, i = t % CF::kRows;
+    const int64_t brow = cta_rb + (int64_t)blk * CF::kRows;
+    T sum = T(0);
+#pragma unroll
+    for (int q = 0; q < SETS; ++q) {
+      const int mq = SHIFT ? (int)((reinterpret_cast<uintptr_t>(A + brow + (c0 + q) * lda) & 15) / sizeof(T)) : 0;
+      for (int w = 0; w < wc; ++w) {
+        const T v = part[w * rw + blk][q][i + mq];
+        sum = q + w == 0 ? v : sum + v;
+      }
+    }
+    if (CL)
+      split_part[t] = sum;
+    else if (gridDim.y == 1)
+      y[r] = accumulate ? y[r] + sum : sum;
+    else
+      partials[(int64_t)blockIdx.y * rows + r] = sum;
+  }
+  if constexpr (CL) {
     __syncwarp();  // lanes past the last row rejoin before the aligned cluster barrier
     dev::cluster_sync();
     if (blockIdx.y == 0) {  // rank 0 of the cluster: splits in order
-#pragma unroll
-      for (int i = 0; i < W; ++i) {
-        const int64_t r = rbase + i;
-        if (r < rows) {
-          T s = T(0);
-          for (unsigned k = 0; k < gridDim.y; ++k) s += dev::dsmem_ld(&split_part[threadIdx.x * W + i], k);
-          y[r] = accumulate ? y[r] + s : s;
-        }
+      for (int t = threadIdx.x; t < rw * CF::kRows && cta_rb + t < rows; t += kRowsThreads) {
+        T s = T(0);
+        for (unsigned k = 0; k < gridDim.y; ++k) s += dev::dsmem_ld(&split_part[t], k);
+        y[cta_rb + t] = accumulate ? y[cta_rb + t] + s : s;
       }
     }
+    __syncwarp();
     dev::cluster_sync();  // the other splits stay resident until rank 0 has read them
-  } else {
-#pragma unroll
-    for (int i = 0; i < W; ++i) {
-      const int64_t r = rbase + i;
-      if (r < rows) {
-        if (gridDim.y == 1)
-          y[r] = accumulate ? y[r] + acc[i] : acc[i];
-        else
-          partials[(int64_t)blockIdx.y * rows + r] = acc[i];
-      }
-    }
   }
 }
 
@@ -276,41 +399,20 @@ cudaError_t launch_split_clusters(void (*kernel)(P...), dim3 grid, int threads, 
 
 }  // namespace
 
-template <typename T>
-gbblas_status launch_gemv_rows(DeviceCtx* c, int64_t rows, int64_t cols, const T* A, int64_t lda, const T* x,
-                               T* y, bool accumulate, cudaStream_t stream) {
-  if (rows <= 0) return GBBLAS_STATUS_SUCCESS;
-  constexpr int W = V<T>::w;
-  const bool vec = aligned16(A) && aligned16(x) && (lda % W) == 0;
-  const int64_t target = (int64_t)c->num_sms * 8;  // 8 CTAs of 256 threads fill an SM
-  const bool use_r4 = rows >= 4 * (int64_t)c->num_sms * 4;
-  const int R = use_r4 ? 4 : 1;
-  const int64_t groups = cdiv(rows, R);
-  int64_t ksplit = 1;
-  if (groups < target && cols > 4096) {
-    ksplit = cdiv(target, groups);
-    int64_t max_split = cdiv(cols, 2048);
-    if (ksplit > max_split) ksplit = max_split;
-    if (ksplit > 65535) ksplit = 65535;
-  }
-  int64_t cps = cdiv(cdiv(cols, ksplit), 256) * 256;  // multiple of the vector width
-  ksplit = cdiv(cols, cps);
-  if (ksplit < 1) ksplit = 1;
-  dim3 grid((unsigned)groups, (unsigned)ksplit);
+namespace {
+
+// The kernel over `grid` with its splits as clusters, or with partials in
+// scratch and the finish behind it.
+template <typename T, typename K, typename... A>
+gbblas_status launch_split(DeviceCtx* c, K clustered, K plain, dim3 grid, int64_t rows, int64_t cols, T* y,
+                           bool accumulate, cudaStream_t stream, const char* what, const T* mat, int64_t lda,
+                           const T* x, A... more) {
+  const int64_t ksplit = grid.y;
   T* partials = nullptr;
   if (cluster_splits(ksplit, rows, cols, sizeof(T))) {
-    cudaError_t e;
-    if (R == 4)
-      e = vec ? launch_split_clusters(gemv_rows_kernel<T, 4, true, true>, grid, kRowsThreads, stream, rows, cols, A,
-                                      lda, x, y, accumulate, partials, cps)
-              : launch_split_clusters(gemv_rows_kernel<T, 4, false, true>, grid, kRowsThreads, stream, rows, cols, A,
-                                      lda, x, y, accumulate, partials, cps);
-    else
-      e = vec ? launch_split_clusters(gemv_rows_kernel<T, 1, true, true>, grid, kRowsThreads, stream, rows, cols, A,
-                                      lda, x, y, accumulate, partials, cps)
-              : launch_split_clusters(gemv_rows_kernel<T, 1, false, true>, grid, kRowsThreads, stream, rows, cols, A,
-                                      lda, x, y, accumulate, partials, cps);
-    if (e == cudaSuccess) return check_launch("gemv_rows_kernel (split clusters)");
+    if (launch_split_clusters(clustered, grid, kRowsThreads, stream, rows, cols, mat, lda, x, y, accumulate, partials,
+                              more...) == cudaSuccess)
+      return check_launch(what);
     cudaGetLastError();  // the cluster launch was refused: partials in scratch instead
   }
   if (ksplit > 1) {
@@ -318,28 +420,59 @@ gbblas_status launch_gemv_rows(DeviceCtx* c, int64_t rows, int64_t cols, const T
     GB_TRY(get_scratch(c, stream, kScratchZeroBytes + sizeof(T) * ksplit * rows, &s));
     partials = reinterpret_cast<T*>(static_cast<char*>(s) + kScratchZeroBytes);
   }
-  if (R == 4) {
-    if (vec)
-      gemv_rows_kernel<T, 4, true, false><<<grid, kRowsThreads, 0, stream>>>(rows, cols, A, lda, x, y, accumulate,
-                                                                             partials, cps);
-    else
-      gemv_rows_kernel<T, 4, false, false><<<grid, kRowsThreads, 0, stream>>>(rows, cols, A, lda, x, y, accumulate,
-                                                                              partials, cps);
-  } else {
-    if (vec)
-      gemv_rows_kernel<T, 1, true, false><<<grid, kRowsThreads, 0, stream>>>(rows, cols, A, lda, x, y, accumulate,
-                                                                             partials, cps);
-    else
-      gemv_rows_kernel<T, 1, false, false><<<grid, kRowsThreads, 0, stream>>>(rows, cols, A, lda, x, y, accumulate,
-                                                                              partials, cps);
-  }
-  GB_TRY(check_launch("gemv_rows_kernel"));
+  plain<<<grid, kRowsThreads, 0, stream>>>(rows, cols, mat, lda, x, y, accumulate, partials, more...);
+  GB_TRY(check_launch(what));
   if (ksplit > 1) {
-    finish_splits_kernel<T><<<(unsigned)cdiv(rows, 256), 256, 0, stream>>>(rows, (int)ksplit, partials, y,
-                                                                           accumulate);
+    const int64_t per = 256 / (ksplit > 16 ? 8 : 1);
+    GB_CUDA_TRY(launch_after(finish_splits_kernel<T>, dim3((unsigned)cdiv(rows, per)), 256, 0, stream, rows,
+                             (int)ksplit, (const T*)partials, y, accumulate));
     GB_TRY(check_launch("finish_splits_kernel"));
   }
   return GBBLAS_STATUS_SUCCESS;
+}
+
+// Log2 of the number of rows after which a row starts at the same offset from
+// a 16-byte boundary again: 1, 2 or 4 rows.
+template <typename T>
+int align_period(int64_t lda) {
+  const int64_t off = lda * (int64_t)sizeof(T) % 16;
+  return off == 0 ? 0 : (off == 8 ? 1 : 2);
+}
+
+}  // namespace
+
+template <typename T>
+gbblas_status launch_gemv_rows(DeviceCtx* c, int64_t rows, int64_t cols, const T* A, int64_t lda, const T* x,
+                               T* y, bool accumulate, cudaStream_t stream) {
+  if (rows <= 0) return GBBLAS_STATUS_SUCCESS;
+  constexpr int W = V<T>::w;
+  const int64_t nv = cols / W, sms = c->num_sms;
+  const int odd = align_period<T>(lda);
+  // warps per row group: as many as leave each 2 vectors a lane (4 where the
+  // rows are few and the call is all latency: 944 x 1024 f32 4.1 us, 6.2 with 1)
+  const int64_t least = rows >= 16 * sms ? 64 : 128;
+  int lwc = 3;
+  while (lwc > 0 && (nv >> lwc) < least) --lwc;
+  // 4 rows a group once those groups make 3 CTAs per SM (2 where the 4 rows
+  // share x read element by element, or the FP64 additions of their sums):
+  // 1488 x 16384 f32 takes 21 us as 372 CTAs of 4 rows, 18-20 as 1488 of one
+  const int R = (rows << lwc) >= (odd > 0 || sizeof(T) == 8 ? 64 : 96) * sms ? 4 : 1;
+  const int lperiod = R == 1 ? 0 : odd;
+  const int64_t groups = cdiv(rows, (int64_t)R << lperiod) << lperiod;
+  const int64_t ctas = cdiv(groups, kWarps >> lwc);
+  // split the columns while the CTAs do not fill the SMs and each warp has
+  // more than 8 vectors a lane
+  int64_t ksplit = 1;
+  if (ctas * kWarps < 32 * sms) ksplit = std::min(cdiv(48 * sms, ctas * kWarps), nv >> (lwc + 8));
+  ksplit = std::max<int64_t>(1, std::min<int64_t>(ksplit, 65535));
+  const int64_t vps = cdiv(cdiv(nv, ksplit), 32) * 32;
+  if (vps > 0) ksplit = std::max<int64_t>(1, cdiv(nv, vps));
+  const dim3 grid((unsigned)ctas, (unsigned)ksplit);
+  if (R == 4)
+    return launch_split<T>(c, gemv_rows_kernel<T, 4, true>, gemv_rows_kernel<T, 4, false>, grid, rows, cols, y,
+                           accumulate, stream, "gemv_rows_kernel", A, lda, x, vps, lperiod, lwc);
+  return launch_split<T>(c, gemv_rows_kernel<T, 1, true>, gemv_rows_kernel<T, 1, false>, grid, rows, cols, y,
+                         accumulate, stream, "gemv_rows_kernel", A, lda, x, vps, lperiod, lwc);
 }
 
 template <typename T>
@@ -348,50 +481,31 @@ gbblas_status launch_gemv_cols(DeviceCtx* c, int64_t rows, int64_t cols, const T
   if (rows <= 0) return GBBLAS_STATUS_SUCCESS;
   constexpr int W = V<T>::w;
   const bool vec = aligned16(A) && (lda % W) == 0;
-  const int w = vec ? W : 1;
-  int threads = 256;
-  const int64_t thr_needed = cdiv(rows, w);
-  if (thr_needed < 256) threads = (int)cdiv(thr_needed, 32) * 32;
-  const int64_t rblocks = cdiv(thr_needed, threads);
-  const int64_t target = (int64_t)c->num_sms * (2048 / threads);
-  int64_t ksplit = 1;
-  if (rblocks < target && cols > 64) {
-    ksplit = cdiv(target, rblocks);
-    int64_t max_split = cdiv(cols, 64);
-    if (ksplit > max_split) ksplit = max_split;
-    if (ksplit > 65535) ksplit = 65535;
-  }
-  int64_t cps = cdiv(cols, ksplit);
-  ksplit = cdiv(cols, cps);
-  if (ksplit < 1) ksplit = 1;
-  dim3 grid((unsigned)rblocks, (unsigned)ksplit);
-  T* partials = nullptr;
-  if (cluster_splits(ksplit, rows, cols, sizeof(T))) {
-    const cudaError_t e = vec ? launch_split_clusters(gemv_cols_kernel<T, true, true>, grid, threads, stream, rows,
-                                                      cols, A, lda, x, y, accumulate, partials, cps)
-                              : launch_split_clusters(gemv_cols_kernel<T, false, true>, grid, threads, stream, rows,
-                                                      cols, A, lda, x, y, accumulate, partials, cps);
-    if (e == cudaSuccess) return check_launch("gemv_cols_kernel (split clusters)");
-    cudaGetLastError();  // the cluster launch was refused: partials in scratch instead
-  }
-  if (ksplit > 1) {
-    void* s = nullptr;
-    GB_TRY(get_scratch(c, stream, kScratchZeroBytes + sizeof(T) * ksplit * rows, &s));
-    partials = reinterpret_cast<T*>(static_cast<char*>(s) + kScratchZeroBytes);
-  }
+  // unaligned columns: shifted vectors for float; for double, bound by the
+  // FP64 pipes, one row a lane (no row is computed twice)
+  constexpr bool kShift = sizeof(T) == 4;
+  using Odd = ColsCfg<kShift ? W : 1, kShift>;
+  // two row blocks a CTA from 2048 rows (their pieces of a column adjoin: at
+  // 16384^2 f32 159 us with one, 154-156 with two, 160 with eight), one below
+  const int rw = rows > 2048 ? 2 : 1;
+  const int64_t blocks = cdiv(rows, (vec ? ColsCfg<W, false>::kRows : Odd::kRows) * (int64_t)rw);
+  // columns per CTA: enough CTAs for 16 per SM, at least 64 columns, a whole
+  // number of rounds (8 columns a warp); double, whose time is its FP64 work,
+  // shares short rows out evenly instead (20069 x 264: 20 us, 23 in 64s and a
+  // rest; float 11.0 and 10.3)
+  const int64_t want = std::min<int64_t>(cdiv(16 * (int64_t)c->num_sms, blocks), 65535), round = 8 * (kWarps / rw);
+  const int64_t even = cdiv(cols, std::max<int64_t>(1, std::min(want, cols / 64)));
+  const int64_t cps = cdiv(sizeof(T) == 8 ? even : std::max<int64_t>(cdiv(cols, want), 64), round) * round;
+  const dim3 grid((unsigned)blocks, (unsigned)std::max<int64_t>(1, cdiv(cols, cps)));
   if (vec)
-    gemv_cols_kernel<T, true, false><<<grid, threads, 0, stream>>>(rows, cols, A, lda, x, y, accumulate, partials,
-                                                                   cps);
+    return launch_split<T>(c, gemv_cols_kernel<T, W, false, true>, gemv_cols_kernel<T, W, false, false>, grid, rows,
+                           cols, y, accumulate, stream, "gemv_cols_kernel", A, lda, x, cps, rw);
+  if constexpr (kShift)
+    return launch_split<T>(c, gemv_cols_kernel<T, W, true, true>, gemv_cols_kernel<T, W, true, false>, grid, rows,
+                           cols, y, accumulate, stream, "gemv_cols_kernel", A, lda, x, cps, rw);
   else
-    gemv_cols_kernel<T, false, false><<<grid, threads, 0, stream>>>(rows, cols, A, lda, x, y, accumulate, partials,
-                                                                    cps);
-  GB_TRY(check_launch("gemv_cols_kernel"));
-  if (ksplit > 1) {
-    finish_splits_kernel<T><<<(unsigned)cdiv(rows, 256), 256, 0, stream>>>(rows, (int)ksplit, partials, y,
-                                                                           accumulate);
-    GB_TRY(check_launch("finish_splits_kernel"));
-  }
-  return GBBLAS_STATUS_SUCCESS;
+    return launch_split<T>(c, gemv_cols_kernel<T, 1, false, true>, gemv_cols_kernel<T, 1, false, false>, grid, rows,
+                           cols, y, accumulate, stream, "gemv_cols_kernel", A, lda, x, cps, rw);
 }
 
 #define GB_INST(T)                                                                                          \
