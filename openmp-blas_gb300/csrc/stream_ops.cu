@@ -8,6 +8,8 @@
 // All three move each byte of their operands once; their roofline is HBM
 // bandwidth.  Algorithmic bytes: outer 2*M*N*s (read and write C) plus the
 // vectors; transpose 2*M*N*s; element-wise 3*n*s.
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace gbblas {
@@ -108,6 +110,88 @@ __global__ void __launch_bounds__(kThreads, 3) transpose_kernel(int64_t M, int64
         if (full || (i0 + ii < M && j0 + jj < N)) pc[k * ck + h * ch] = tile[ii][jj];
       }
     __syncthreads();
+  }
+}
+
+// The same for large matrices where C's contiguous rows do not all start on a
+// 128-byte line; C(j, i) at C[j*rsc + i] (the launch turns a C of the other
+// layout round).  Tile by tile every row of a tile then ends in two partly
+// written lines, and those bound the kernel: 9001 x 7003 f32 took 107 us, 86
+// with a padded C.  Here a CTA takes kTJ columns j of A and walks down a strip
+// of its rows i, kCI at a time: the rows' 256-byte pieces go to registers while
+// the previous chunk is written, then to a shared-memory ring of two chunks,
+// from which each of the kTJ rows of C is written in whole lines - what a
+// chunk leaves of a row's last line waits for the next chunk.  94 us; 16383 x
+// 16001 f32 529 -> 375, f64 838 -> 677 (chunks of 32 rows and twice the CTAs:
+// 98 us for the first).
+// KCONTIG: A's columns are contiguous as C's rows are (rsa = 1): no exchange
+// of indexes, the pieces run along i.
+constexpr int kCI = 64;
+
+template <typename T>
+struct TransCfg {
+  static constexpr int kTJ = 256 / (int)sizeof(T);    // 64 floats / 32 doubles: 256 bytes of a row of A
+  static constexpr int kLine = 128 / (int)sizeof(T);  // elements per line
+};
+
+template <typename T, bool KCONTIG>
+__global__ void __launch_bounds__(kThreads, 4) transpose_lines_kernel(int64_t M, int64_t N, const T* __restrict__ A,
+                                                                int64_t rsa, int64_t csa, T* __restrict__ C,
+                                                                int64_t rsc, int64_t jblocks, int strip) {
+  constexpr int TJ = TransCfg<T>::kTJ, LINE = TransCfg<T>::kLine;
+  constexpr int PER = kCI * TJ / kThreads;  // elements of a chunk per thread
+  __shared__ T ring[2 * kCI][TJ + 1];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int64_t j0 = (int64_t)(blockIdx.x % jblocks) * TJ;
+  const int64_t i0 = (int64_t)(blockIdx.x / jblocks) * strip * kCI;
+  const int64_t i1 = min(i0 + (int64_t)strip * kCI, M);  // the strip's rows
+  // element e of this thread lies at (ii(e), jj(e)) of a chunk
+  auto ii = [&](int e) { return KCONTIG ? tx + 32 * (e % (kCI / 32)) : ty + 8 * (e / (TJ / 32)); };
+  auto jj = [&](int e) { return KCONTIG ? ty + 8 * (e / (kCI / 32)) : tx + 32 * (e % (TJ / 32)); };
+  T r[PER];
+  auto load = [&](int64_t ic) {
+    const T* p = A + ic * rsa + j0 * csa;
+    if (ic + kCI <= i1 && j0 + TJ <= N) {
+#pragma unroll
+      for (int e = 0; e < PER; ++e) r[e] = p[ii(e) * rsa + jj(e) * csa];
+    } else {
+#pragma unroll
+      for (int e = 0; e < PER; ++e)
+        r[e] = (ic + ii(e) < i1 && j0 + jj(e) < N) ? p[ii(e) * rsa + jj(e) * csa] : T(0);
+    }
+  };
+  load(i0);
+  int half = 0;
+  for (int64_t ic = i0; ic < i1; ic += kCI, half ^= kCI) {
+#pragma unroll
+    for (int e = 0; e < PER; ++e) ring[half + ii(e)][jj(e)] = r[e];
+    __syncthreads();
+    const bool last = ic + kCI >= i1;
+    if (!last) load(ic + kCI);
+    // row j of C: from where the last chunk stopped to the last whole line
+    // (to the end of the strip in its last chunk)
+    if (ic != i0 && !last && j0 + TJ <= N) {
+      // kCI elements from the line boundary at or before (j, ic), all of them
+      T* __restrict__ crow = C + (j0 + ty) * rsc + ic;
+#pragma unroll 4
+      for (int j = ty; j < TJ; j += 8, crow += 8 * rsc) {
+        const int i = tx - (int)((reinterpret_cast<uintptr_t>(crow) / sizeof(T)) % LINE);
+        crow[i] = ring[(half + i) & (2 * kCI - 1)][j];
+        if (kCI > 32) crow[i + 32] = ring[(half + i + 32) & (2 * kCI - 1)][j];
+      }
+    } else {
+      for (int j = ty; j < TJ && j0 + j < N; j += 8) {
+        T* __restrict__ crow = C + (j0 + j) * rsc + ic;
+        const int off = (int)((reinterpret_cast<uintptr_t>(crow) / sizeof(T)) % LINE);
+        const int beg = ic == i0 ? 0 : -off, end = last ? (int)(i1 - ic) : kCI - off;
+#pragma unroll
+        for (int h = 0; h < kCI / 32 + 1; ++h) {
+          const int i = tx - off + 32 * h;
+          if (i >= beg && i < end) crow[i] = ring[(half + i) & (2 * kCI - 1)][j];
+        }
+      }
+    }
+    __syncthreads();  // the next chunk overwrites the one before this
   }
 }
 
@@ -235,6 +319,26 @@ template <typename T>
 gbblas_status launch_transpose(DeviceCtx* c, int64_t M, int64_t N, const T* A, int64_t rsa, int64_t csa, T* C,
                                int64_t rsc, int64_t csc, cudaStream_t s) {
   if (M == 0 || N == 0) return GBBLAS_STATUS_SUCCESS;
+  // Large matrices whose written rows do not all start on a line: strips, 12
+  // CTAs per SM.  From 200 MB moved (below it the writes of neighbouring tiles
+  // meet in L2 before they leave it: 4501 x 4499 f32, 162 MB, 33.5 us by tiles
+  // and 35.0 in strips; 6001 x 5003, 240 MB, 51.2 and 47.4).
+  const bool c_rows = csc == 1;
+  const int64_t ldc = c_rows ? rsc : csc, ra = c_rows ? rsa : csa, ca = c_rows ? csa : rsa;
+  const int64_t m = c_rows ? M : N, n = c_rows ? N : M;  // C has n contiguous rows of m
+  constexpr int TJ = TransCfg<T>::kTJ, LINE = TransCfg<T>::kLine;
+  const int64_t jblocks = (n + TJ - 1) / TJ, chunks = (m + kCI - 1) / kCI;
+  if ((c_rows || rsc == 1) && (ra == 1 || ca == 1) && 2.0 * (double)M * (double)N * sizeof(T) >= 200e6 &&
+      (ldc % LINE != 0 || (reinterpret_cast<uintptr_t>(C) & 127) != 0) && jblocks * chunks <= 0x7fffffff / kCI) {
+    const int64_t strips = std::min(chunks, std::max<int64_t>(1, (12 * (int64_t)c->num_sms + jblocks - 1) / jblocks));
+    const int64_t strip = (chunks + strips - 1) / strips;
+    const unsigned lgrid = (unsigned)(jblocks * ((chunks + strip - 1) / strip));
+    if (ca != 1)
+      transpose_lines_kernel<T, true><<<lgrid, kThreads, 0, s>>>(m, n, A, ra, ca, C, ldc, jblocks, (int)strip);
+    else
+      transpose_lines_kernel<T, false><<<lgrid, kThreads, 0, s>>>(m, n, A, ra, ca, C, ldc, jblocks, (int)strip);
+    return check_launch("transpose_lines_kernel");
+  }
   constexpr int TILE = 64;  // 16 (f32) / 32 (f64) KB of shared memory per CTA
   const int64_t tm = (M + TILE - 1) / TILE, tn = (N + TILE - 1) / TILE, nt = tm * tn;
   int64_t grid = nt;
