@@ -2,6 +2,7 @@
 // runtime behind it: per-device context, per-stream scratch, host staging,
 // argument checking and status/error reporting.
 #include <atomic>
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <string>
@@ -234,16 +235,18 @@ gbblas_status gemv_any(DeviceCtx* c, gbblas_layout la, bool transpose, int64_t M
 
 // Shapes where AUTO takes the guarded tensor-core digits for a double GEMM:
 // K of at least 32 (and within the digit kernels' limit) where the digits'
-// estimated time is the shorter.  FP64 pipes: about 4000 multiply-adds per
-// us per SM (GB300: 2 DFMA per cycle per SM), over as many SMs as there are
-// 64 x 64 tiles; measured 0.27 ms at 256^3 (16 tiles).  Digits: about 50 us
-// of operand preparation and launches, then ~38 TFLOP/s.
+// estimated time is the shorter.  FP64 pipes: about 4000 multiply-adds per us
+// per SM (GB300: 2 DFMA per cycle per SM), in rounds of one 64 x 64 tile per
+// SM; 72 us at 5387 x 133 x 32 (255 tiles, 2 rounds), where the digits take
+// 36.  Digits: at least 25 us of operand preparation and launches (46 keeps
+// products of a tile and a short K, which the pipes finish first, on them),
+// then ~38 TFLOP/s.
 bool dgemm_auto_digits(int64_t M, int64_t N, int64_t K, int num_sms) {
   if (K < 32 || K > dgemm_digits_max_k(7)) return false;
   const double macs = (double)M * (double)N * (double)K;
   const double tiles = (double)((M + 63) / 64) * (double)((N + 63) / 64);
-  const double pipes_us = 5.0 + macs / (4000.0 * std::min(tiles, (double)std::max(num_sms, 1)));
-  const double digits_us = 50.0 + 2.0 * macs / 38e6;
+  const double pipes_us = 5.0 + macs / (4000.0 * tiles) * std::ceil(tiles / (double)std::max(num_sms, 1));
+  const double digits_us = 46.0 + 2.0 * macs / 38e6;
   return digits_us < pipes_us;
 }
 

@@ -128,7 +128,12 @@ struct DgCfg {
 // One GEMM (device-side view).
 struct DgProblem {
   int M, N, num_kt, tiles_m, tiles_n, total_tiles;
-  int tile_begin, tile_end;  // this launch's tiles (a slice of 0 .. total_tiles - 1)
+  int tile_begin;            // this launch's first tile (a slice of 0 .. total_tiles - 1)
+  int full;                  // its tiles computed whole ...
+  int rest, parts;           // ... and the last ones, whose K is cut into `parts` (see dg_work)
+  longlong2* slots;          // parts > 1: each part's exact sums, 512 per epilogue warp's block
+  int* gslots;               // and guard sums
+  unsigned* arrived;         // parts in, per block of a cut tile (starts at kArrivedBase)
   double* C;
   int64_t rsc, csc;
   const int* ea;  // [rows of A, padded] row scales
@@ -183,7 +188,17 @@ __device__ __forceinline__ unsigned long long abs_bits(const double* p) {
   return (unsigned long long)__double_as_longlong(__ldg(p)) & kAbsMask;
 }
 
+// First kernel of a call's chain: the arrival counts and row scales start as
+// the byte 0x80 throughout.
+__global__ void __launch_bounds__(256) dg_init_kernel(uint4* __restrict__ words, int n) {
+  dev::grid_release();
+  for (int i = (int)(blockIdx.x * blockDim.x + threadIdx.x); i < n; i += (int)(gridDim.x * blockDim.x))
+    words[i] = make_uint4(0x80808080u, 0x80808080u, 0x80808080u, 0x80808080u);
+}
+
 __global__ void __launch_bounds__(256) row_scale_kernel(const DgOperand oa, const DgOperand ob, int* fix_count) {
+  dev::grid_release();
+  dev::grid_wait();
   __shared__ unsigned long long part_max[8][33];
   const bool is_a = (int)blockIdx.x < oa.blocks;
   const DgOperand& o = is_a ? oa : ob;
@@ -305,6 +320,8 @@ __device__ __forceinline__ void f64_digits(double a, int e, int (&d)[S]) {
 // one row and writes 8 bytes per plane.
 template <int S, int G>
 __global__ void __launch_bounds__(256) digits_kernel(const DgOperand oa, const DgOperand ob) {
+  dev::grid_release();
+  dev::grid_wait();
   __shared__ double tile[32][33];
   const bool is_a = (int)blockIdx.x < oa.blocks;
   const DgOperand& o = is_a ? oa : ob;
@@ -392,7 +409,33 @@ __device__ __forceinline__ double i128_scaled_to_double(long long hi, long long 
                               (long long)(mant & ((1ull << 52) - 1)));
 }
 
-// Output tile t (static round-robin over the CTAs): grouped raster, 8 tile
+// Work item w of a launch (static round-robin over the CTAs): whole tiles
+// first, as many as make full rounds of the grid; what is left over would
+// occupy a round with part of the CTAs, so its tiles are cut along K, at chunk
+// boundaries, into as many parts as the grid has CTAs for.  The sums are
+// integers, so the parts add up to the same bits in any order: each part's
+// epilogue warps leave theirs in slots, and a block's last one adds them and
+// finishes it.  A whole call, before and after: 48 x 640 x 2363 (20 tiles) 100
+// -> 60 us, 1568 x 396 x 3536 (169 tiles) 274 -> 208, 1531 x 1400 x 1601 (528
+// tiles) 254 -> 245; chaining the call's kernels took another 9-12 us off each.
+constexpr unsigned kArrivedBase = 0x80808080u;  // the fill byte 0x80
+
+struct DgWork {
+  int tile, kt0, nkt, part, rest;  // rest: index among the cut tiles, -1 if whole
+};
+template <int CHUNK>
+__device__ __forceinline__ DgWork dg_work(const DgProblem& p, int w) {
+  if (w < p.full) return {p.tile_begin + w, 0, p.num_kt, 0, -1};
+  const int r = (w - p.full) / p.parts, part = (w - p.full) % p.parts;
+  if (p.parts == 1) return {p.tile_begin + w, 0, p.num_kt, 0, -1};
+  const int nc = (p.num_kt + CHUNK - 1) / CHUNK;
+  const int b = (int)((int64_t)nc * part / p.parts) * CHUNK;
+  const int e = min((int)((int64_t)nc * (part + 1) / p.parts) * CHUNK, p.num_kt);
+  return {p.tile_begin + p.full + r, b, e - b, part, r};
+}
+__device__ __forceinline__ int dg_items(const DgProblem& p) { return p.full + p.rest * p.parts; }
+
+// Output tile t: grouped raster, 8 tile
 // rows per band, so the CTAs running at one time share A's and B's digit
 // tiles in L2.
 __device__ __forceinline__ void dg_tile(const DgProblem& p, int t, int& m0, int& n0) {
@@ -462,22 +505,26 @@ __global__ void __launch_bounds__(kThreads, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  dev::grid_wait();  // the set-up above overlapped the preparation's last CTAs
   const uint32_t tmem = *tmem_slot;
   auto fail = [&]() {
     *abort_flag = 1;
     atomicExch(err, (int)GBBLAS_STATUS_TIMEOUT);
   };
 
+  const int items = dg_items(p);
   int issued = 0;  // A producer: stages whose copies were issued
   if ((warp == 0 || warp == kBProdWarp) && lane == 0) {
     // producers: warp 0 brings A's digit planes, warp 10 B's, into the same stages
     const bool is_a = warp == 0;
     int n_issued = 0, g_issued = 0;
     bool stop = false;
-    for (int t = p.tile_begin + (int)blockIdx.x; t < p.tile_end && !stop; t += gridDim.x) {
+    for (int w = (int)blockIdx.x; w < items && !stop; w += gridDim.x) {
+      const DgWork dw = dg_work<CF::kChunk>(p, w);
       int m0, n0;
-      dg_tile(p, t, m0, n0);
-      for (int kt = 0; kt < p.num_kt; ++kt) {
+      dg_tile(p, dw.tile, m0, n0);
+      for (int kt = 0; kt < dw.nkt; ++kt) {
+        const int kx = (dw.kt0 + kt) * kBK;
         if (G && kt % CF::kChunk == 0) {
           // the guard planes' first 32 K of this chunk, once the MMAs of the
           // previous chunk's guard product have read the slot
@@ -488,10 +535,10 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
           if (is_a) {
             mbar_arrive_expect_tx(gfull, CF::kATile);
-            tma_load_3d(guard_a, &tm_ga, gfull, kt * kBK, m0, 0);
+            tma_load_3d(guard_a, &tm_ga, gfull, kx, m0, 0);
           } else {
             mbar_arrive_expect_tx(gfull, CF::kBTile);
-            tma_load_3d(guard_b, &tm_gb, gfull, kt * kBK, n0, 0);
+            tma_load_3d(guard_b, &tm_gb, gfull, kx, n0, 0);
           }
           ++g_issued;
         }
@@ -503,10 +550,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         if (is_a) {
           mbar_arrive_expect_tx(&full[s], CF::kAStage);
-          tma_load_3d(a_tile(s, 0), &tm_a, &full[s], kt * kBK, m0, 0);
+          tma_load_3d(a_tile(s, 0), &tm_a, &full[s], kx, m0, 0);
         } else {
           mbar_arrive_expect_tx(&full[s], CF::kBStage);
-          tma_load_3d(b_tile(s), &tm_b, &full[s], kt * kBK, n0, 0);
+          tma_load_3d(b_tile(s), &tm_b, &full[s], kx, n0, 0);
         }
         ++n_issued;
       }
@@ -516,11 +563,12 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (lane == 0) {
       int consumed = 0, chunk_g = 0, g_used = 0;
       bool stop = false;
-      for (int t = p.tile_begin + (int)blockIdx.x; t < p.tile_end && !stop; t += gridDim.x) {
-        for (int kt = 0; kt < p.num_kt; ++kt) {
+      for (int w = (int)blockIdx.x; w < items && !stop; w += gridDim.x) {
+        const int nkt = dg_work<CF::kChunk>(p, w).nkt;
+        for (int kt = 0; kt < nkt; ++kt) {
           const int s = consumed % ST, round = consumed / ST;
           const bool chunk_first = (kt % CF::kChunk) == 0;
-          const bool chunk_last = ((kt + 1) % CF::kChunk) == 0 || kt + 1 == p.num_kt;
+          const bool chunk_last = ((kt + 1) % CF::kChunk) == 0 || kt + 1 == nkt;
           if (chunk_first) ++chunk_g;
           const int chunk = chunk_g - 1, b = chunk & 1;
           if (chunk_first && chunk >= 2) {  // buffer b drained by the epilogue
@@ -581,12 +629,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     // columns (half h) of each group's 32
     const int q = warp & 3, h = (warp - 2) >> 2;
     const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(16 * h);
-    const int nchunks = (p.num_kt + CF::kChunk - 1) / CF::kChunk;
     int chunk_g = 0;
     bool ok = true;
-    for (int t = p.tile_begin + (int)blockIdx.x; t < p.tile_end && ok; t += gridDim.x) {
-      int m0, n0;
-      dg_tile(p, t, m0, n0);
+    for (int wk = (int)blockIdx.x; wk < items && ok; wk += gridDim.x) {
+      const int nchunks = (dg_work<CF::kChunk>(p, wk).nkt + CF::kChunk - 1) / CF::kChunk;
       // sum_w G_w 2^(8(S-1-w)) = hi 2^32 + lo, exactly: groups w < S-4 go
       // into hi (shifted by 8(S-5-w)), the last four into lo (8(S-1-w))
       long long hi[16], lo[16];
@@ -640,6 +686,42 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
       if (!ok) break;
       if (__shfl_sync(0xffffffffu, *abort_flag, 0)) break;
+      // (the item's place is worked out again: kept over the chunks it spills)
+      const DgWork dw = dg_work<CF::kChunk>(p, wk);
+      const int t = dw.tile;
+      int m0, n0;
+      dg_tile(p, t, m0, n0);
+      if (dw.rest >= 0) {
+        // a part of a cut tile: its sums to this block's slot (16 bytes a lane
+        // and output, consecutive); the block's last part adds the others'
+        const int blk = dw.rest * kEpiWarps + (warp - 2);
+        const int64_t pstride = (int64_t)p.rest * (kEpiWarps * 512);  // from a part's slots to the next's
+        longlong2* sp = p.slots + blk * 512 + lane;
+        int* gp = p.gslots + blk * 512 + lane;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          __stcg(sp + dw.part * pstride + 32 * j, make_longlong2(hi[j], lo[j]));
+          if (G) __stcg(gp + dw.part * pstride + 32 * j, gsum[j]);
+        }
+        __threadfence();
+        __syncwarp();
+        unsigned before = 0;
+        if (lane == 0) before = atomicAdd(p.arrived + blk, 1u) - kArrivedBase;
+        before = __shfl_sync(0xffffffffu, before, 0);
+        if (before != (unsigned)p.parts - 1) continue;  // another part finishes the block
+        __threadfence();
+        for (int o = 0; o < p.parts; ++o, sp += pstride, gp += pstride) {
+          if (o == dw.part) continue;
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            const longlong2 v = __ldcg(sp + 32 * j);
+            hi[j] += v.x;
+            lo[j] += v.y;
+            if (G) gsum[j] = min(gsum[j] + min(__ldcg(gp + 32 * j), kGuardCap - 1), kGuardCap);
+            if (j % 4 == 3) __syncwarp();  // four loads at a time: all 16 would spill
+          }
+        }
+      }
       const int row = m0 + q * 32 + lane;
       if constexpr (G) {
         // every output of this warp's 32 x 16 block must pass, else the
@@ -716,6 +798,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
   tc_fence_before();
   __syncthreads();
+  dev::grid_release();
   if (warp == 1) {
     __syncwarp();
     tc_fence_after();
@@ -729,6 +812,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 // (row lane, column pair) sums its two outputs over k in order with fused
 // multiply-adds and adds them into C (the FP64 FMA kernel's arithmetic).
 __global__ void __launch_bounds__(256) dgemm_fixup_kernel(const DgProblem p) {
+  dev::grid_wait();
   const int n = *p.fix_count;
   const int lane = threadIdx.x & 31, pair = threadIdx.x >> 5;
   for (int i = blockIdx.x; i < n; i += gridDim.x) {
@@ -759,6 +843,16 @@ __global__ void __launch_bounds__(256) dgemm_fixup_kernel(const DgProblem p) {
 inline int64_t round_up(int64_t a, int64_t b) { return (a + b - 1) / b * b; }
 inline size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 
+// The last, incomplete round's tiles and their K parts on `ctas` CTAs: at
+// least two chunks (of 128 K) a part, at most one part per CTA in all.
+constexpr int kMaxCtas = 256;
+constexpr size_t kArrivedBytes = (size_t)kMaxCtas * kEpiWarps * sizeof(unsigned);
+constexpr size_t kSlotBytes = (size_t)kEpiWarps * 512 * sizeof(longlong2);   // one part's sums
+constexpr size_t kGSlotBytes = (size_t)kEpiWarps * 512 * sizeof(int);        // and guard sums
+inline int rest_parts(int64_t rest, int64_t chunks, int ctas) {
+  return rest > 0 ? (int)std::max<int64_t>(1, std::min<int64_t>(ctas / rest, chunks / 2)) : 1;
+}
+
 template <int S, int G>
 void dg_setup(DeviceCtx* c) {
   static std::mutex mu;
@@ -786,14 +880,21 @@ gbblas_status launch_digits(DeviceCtx* c, int64_t M, int64_t N, int64_t K, const
     return GBBLAS_STATUS_NOT_SUPPORTED;
   }
   const int64_t Mp = round_up(M, kBM), Np = round_up(N, kBN), Kp = round_up(K, kBK);
-  const size_t off_ea = kScratchZeroBytes;
+  const size_t off_arr = kScratchZeroBytes;  // arrival counts of cut tiles, filled with 0x80 as the scales are
+  const size_t off_ea = off_arr + kArrivedBytes;
   const size_t off_eb = off_ea + align256(sizeof(int) * (size_t)Mp);
   const size_t off_a = off_eb + align256(sizeof(int) * (size_t)Np);
   const size_t a_plane = (size_t)(Mp * Kp), b_plane = (size_t)(Np * Kp);
   const size_t off_b = off_a + align256((size_t)NP * a_plane * sizeof(__nv_bfloat16));
   const int64_t tiles = (Mp / kBM) * (Np / kBN);
   const size_t off_fix = off_b + align256((size_t)NP * b_plane * sizeof(__nv_bfloat16));
-  const size_t bytes = off_fix + (G ? align256(sizeof(int) * (size_t)(1 + tiles * kEpiWarps)) : 0);
+  const size_t off_slots = off_fix + (G ? align256(sizeof(int) * (size_t)(1 + tiles * kEpiWarps)) : 0);
+  int ctas = std::min(c->num_sms, kMaxCtas);
+  if (max_ctas > 0 && ctas > max_ctas) ctas = max_ctas;
+  const int64_t chunks = (Kp / kBK + CF::kChunk - 1) / CF::kChunk, rest = tiles % ctas;
+  const int parts = rest_parts(rest, chunks, ctas);
+  const size_t nslots = parts > 1 ? (size_t)rest * parts : 0;
+  const size_t bytes = off_slots + nslots * (kSlotBytes + (G ? kGSlotBytes : 0));
   void* scratch = nullptr;
   GB_TRY(get_scratch(c, stream, bytes, &scratch));
   char* base = static_cast<char*>(scratch);
@@ -805,7 +906,11 @@ gbblas_status launch_digits(DeviceCtx* c, int64_t M, int64_t N, int64_t K, const
 
   // scales: rows of A over K; columns of B (element (n, k) = B[k*rsb + n*csb])
   int* fix_count = G ? reinterpret_cast<int*>(base + off_fix) : nullptr;
-  GB_CUDA_TRY(cudaMemsetAsync(ea, 0x80, off_a - off_ea, stream));  // kZeroExp everywhere (ea and eb)
+  // kZeroExp everywhere (ea and eb), and kArrivedBase
+  const int words = (int)((off_a - off_arr) / sizeof(uint4));
+  dg_init_kernel<<<std::min((words + 255) / 256, c->num_sms), 256, 0, stream>>>(
+      reinterpret_cast<uint4*>(base + off_arr), words);
+  GB_TRY(check_launch("dg_init_kernel"));
   const int stk = (int)((K + kScaleTK - 1) / kScaleTK);
   const int tiles_k = (int)(Kp / 32);
   DgOperand oa{A, M, K, rsa, csa, ea, da, (int64_t)a_plane, Kp, stk, (int)((Mp / 32) * stk)};
@@ -814,12 +919,13 @@ gbblas_status launch_digits(DeviceCtx* c, int64_t M, int64_t N, int64_t K, const
     set_error("dgemm (FP64 digits): operands too large for one preparation launch");
     return GBBLAS_STATUS_NOT_SUPPORTED;
   }
-  row_scale_kernel<<<(unsigned)(oa.blocks + ob.blocks), 256, 0, stream>>>(oa, ob, fix_count);
+  // (each behind the one before without waiting for its end: launch_after)
+  GB_CUDA_TRY(launch_after(row_scale_kernel, dim3((unsigned)(oa.blocks + ob.blocks)), 256, 0, stream, oa, ob, fix_count));
   GB_TRY(check_launch("row_scale_kernel"));
   oa.tiles_k = ob.tiles_k = tiles_k;
   oa.blocks = (int)((Mp / 32) * tiles_k);
   ob.blocks = (int)((Np / 32) * tiles_k);
-  digits_kernel<S, G><<<(unsigned)(oa.blocks + ob.blocks), 256, 0, stream>>>(oa, ob);
+  GB_CUDA_TRY(launch_after(digits_kernel<S, G>, dim3((unsigned)(oa.blocks + ob.blocks)), 256, 0, stream, oa, ob));
   GB_TRY(check_launch("digits_kernel"));
 
   CUtensorMap ma, mb;
@@ -856,22 +962,31 @@ gbblas_status launch_digits(DeviceCtx* c, int64_t M, int64_t N, int64_t K, const
   p.csb = csb;
   p.K = K;
   dg_setup<S, G>(c);
-  int grid = (int)std::min<int64_t>(tiles, c->num_sms);
-  if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
+  p.slots = reinterpret_cast<longlong2*>(base + off_slots);
+  p.gslots = reinterpret_cast<int*>(base + off_slots + nslots * kSlotBytes);
+  p.arrived = reinterpret_cast<unsigned*>(base + off_arr);
   // slices: consecutive tile ranges of whole waves, one launch each (higher-
-  // priority work on other streams gets the SMs between them)
-  const int64_t waves = (tiles + grid - 1) / grid;
+  // priority work on other streams gets the SMs between them); the tiles of
+  // the last, incomplete wave are cut along K (dg_work)
+  const int64_t waves = (tiles + ctas - 1) / ctas;
   const int64_t nsl = std::max<int64_t>(1, std::min<int64_t>(slices, waves));
   for (int64_t sl = 0; sl < nsl; ++sl) {
-    p.tile_begin = (int)(grid * (waves * sl / nsl));
-    p.tile_end = (int)std::min<int64_t>(tiles, grid * (waves * (sl + 1) / nsl));
-    dgemm_digits_kernel<S, G><<<grid, kThreads, CF::kSmem, stream>>>(ma, mb, mga, mgb, p, err);
+    const int64_t tb = ctas * (waves * sl / nsl), te = std::min<int64_t>(tiles, ctas * (waves * (sl + 1) / nsl));
+    p.tile_begin = (int)tb;
+    p.full = (int)((te - tb) / ctas * ctas);
+    p.rest = (int)(te - tb - p.full);
+    p.parts = p.rest ? parts : 1;
+    const int grid = (int)std::min<int64_t>(ctas, p.full + (int64_t)p.rest * p.parts);
+    if (sl == 0)
+      GB_CUDA_TRY(launch_after(dgemm_digits_kernel<S, G>, dim3(grid), kThreads, CF::kSmem, stream, ma, mb, mga, mgb, p, err));
+    else
+      dgemm_digits_kernel<S, G><<<grid, kThreads, CF::kSmem, stream>>>(ma, mb, mga, mgb, p, err);
     GB_TRY(check_launch("dgemm_digits_kernel"));
   }
   if constexpr (G) {
     // the rejected blocks (usually none: the kernel reads the count and returns)
-    dgemm_fixup_kernel<<<(unsigned)(max_ctas > 0 ? std::min(max_ctas, 2 * c->num_sms) : 2 * c->num_sms), 256, 0,
-                         stream>>>(p);
+    const int fctas = max_ctas > 0 ? std::min(max_ctas, 2 * c->num_sms) : 2 * c->num_sms;
+    GB_CUDA_TRY(launch_after(dgemm_fixup_kernel, dim3(fctas), 256, 0, stream, p));
     GB_TRY(check_launch("dgemm_fixup_kernel"));
   }
   return GBBLAS_STATUS_SUCCESS;
@@ -890,7 +1005,8 @@ size_t dgemm_digits_scratch_bytes(int digits, bool guarded, int64_t M, int64_t N
   const int64_t Mp = round_up(M, kBM), Np = round_up(N, kBN), Kp = round_up(K, kBK);
   const int64_t np = digits + (guarded ? 1 : 0);
   const int64_t tiles = (Mp / kBM) * (Np / kBN);
-  return kScratchZeroBytes + align256(sizeof(int) * (size_t)Mp) + align256(sizeof(int) * (size_t)Np) +
+  return kScratchZeroBytes + kArrivedBytes + (size_t)kMaxCtas * (kSlotBytes + kGSlotBytes) + align256(sizeof(int) * (size_t)Mp) +
+         align256(sizeof(int) * (size_t)Np) +
          align256((size_t)(np * Mp * Kp) * 2) + align256((size_t)(np * Np * Kp) * 2) +
          (guarded ? align256(sizeof(int) * (size_t)(1 + tiles * kEpiWarps)) : 0);
 }
