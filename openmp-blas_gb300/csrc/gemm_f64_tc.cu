@@ -36,7 +36,8 @@
 //
 // The guard (7 digits, G = 1; what AUTO runs): one more plane per operand,
 // P = max(|D_0| - 1, 0) <= |x| 2^7, whose products summed over the first
-// 32 of K of every 128-K chunk bound sum_k |a_ik||b_kj| from below.  An
+// 32 of K of every 128-K chunk (over all of K where that sample is too thin)
+// bound sum_k |a_ik||b_kj| from below.  An
 // epilogue warp keeps its 32 x 16 block only where that bound makes the
 // digit error smaller than the FP64 pipes' bound; other blocks leave C
 // alone and are recomputed on the FP64 pipes by dgemm_fixup_kernel.
@@ -53,7 +54,7 @@
 // accumulator columns of groups s..S-1 (group w at column 32 w of a
 // 256-column TMEM buffer; two buffers, so the epilogue folds one 128-K chunk
 // while the MMAs fill the next).  Warp roles as in gemm_tc.cu: warp 0
-// streams A, warp 10 B, warp 1 allocates TMEM and issues the MMAs, warps
+// streams A, warp 10 B, warp 11 the guard planes, warp 1 allocates TMEM and issues the MMAs, warps
 // 2-9 fold (warp w: TMEM lane quarter w % 4 = 32 tile rows, 16 of the 32
 // columns).  Every wait is bounded; a wait that gives up records
 // GBBLAS_STATUS_TIMEOUT, and the CTA drains its copies and MMAs, frees TMEM
@@ -85,13 +86,15 @@ constexpr int kBM = 128;  // tile rows (TMEM lanes)
 constexpr int kBN = 32;   // tile columns per digit group
 constexpr int kBK = 32;   // K per stage: one 64-byte row of BF16
 constexpr int kEpiWarps = 8;
-constexpr int kThreads = 32 * (3 + kEpiWarps);  // A producer, MMA, 8 epilogue, B producer
+constexpr int kThreads = 32 * (4 + kEpiWarps);  // A producer, MMA, 8 epilogue, B producer, guard producer
 constexpr int kBProdWarp = 2 + kEpiWarps;
+constexpr int kGuardWarp = kBProdWarp + 1;
 constexpr uint32_t kBufCols = 256;  // one TMEM buffer: S <= 8 groups x 32 columns
 constexpr uint64_t kWaitLimitNs = 2000000000ull;  // 2 s
 constexpr size_t kSmemLimit = 232448;             // 227 KB per CTA
 constexpr int kBadExp = INT_MAX;                  // scale marker: the row / column holds Inf or NaN
 constexpr int kZeroExp = (int)0x80808080;          // scale of an all-zero row (the fill byte 0x80)
+constexpr unsigned kArrivedBase = 0x80808080u;     // where counts start: the fill byte 0x80
 
 // S digits; G = 1 adds the guard plane (P = max(|D_0| - 1, 0), whose
 // product sum bounds sum_k |a_ik||b_kj| from below) and its accumulator in
@@ -122,7 +125,7 @@ struct DgCfg {
   static_assert(kStages >= 2, "need a double-buffered stage ring");
   static_assert((uint64_t)S * kChunk * kBK * 16384 < (1u << 24), "chunk sums must stay exact in FP32");
   static_assert(kStageBytes % 1024 == 0, "stages stay 1024-byte aligned");
-  static_assert((2 * 4 + 2 * 2 + 2 + 1) * 8 + 8 <= kBarBytes, "barrier area too small");
+  static_assert((2 * 4 + 2 * 2 + 2 + 1) * 8 + 8 + 8 <= kBarBytes, "barrier area too small");
 };
 
 // One GEMM (device-side view).
@@ -138,6 +141,8 @@ struct DgProblem {
   int64_t rsc, csc;
   const int* ea;  // [rows of A, padded] row scales
   const int* eb;  // [columns of B, padded] column scales
+  const unsigned* ga;  // guarded form: the rows' (columns') sampled sums of the guard plane, from kArrivedBase
+  const unsigned* gb;
   // guarded form: the 32 x 16 blocks the guard rejected (block b of tile t
   // = t * 8 + epilogue warp), recomputed on the FP64 pipes from A and B
   int* fix_count;
@@ -172,6 +177,7 @@ struct DgOperand {
   const double* src;
   int64_t rows, K, rs, cs;  // element (r, k) at src[r*rs + k*cs]
   int* e;                   // row scales
+  unsigned* gsum;           // guard: the rows' sampled sums of the guard plane (start at kArrivedBase)
   __nv_bfloat16* out;       // digit planes
   int64_t plane_stride, pitch;
   int tiles_k;              // CTAs per 32 rows (K tiles of the kernel at hand)
@@ -329,6 +335,7 @@ __global__ void __launch_bounds__(256) digits_kernel(const DgOperand oa, const D
   const double* __restrict__ src = o.src;
   const int64_t rows = o.rows, K = o.K, rs = o.rs, cs = o.cs, plane_stride = o.plane_stride, pitch = o.pitch;
   const int* __restrict__ e_row = o.e;
+  unsigned* __restrict__ gsum_row = o.gsum;
   __nv_bfloat16* __restrict__ out = o.out;
   const int tid = threadIdx.x;
   const int64_t r0 = (int64_t)(blk / o.tiles_k) * 32, k0 = (int64_t)(blk % o.tiles_k) * 32;
@@ -369,6 +376,14 @@ __global__ void __launch_bounds__(256) digits_kernel(const DgOperand oa, const D
     w.x = *reinterpret_cast<const uint32_t*>(&h01);
     w.y = *reinterpret_cast<const uint32_t*>(&h23);
     *reinterpret_cast<uint2*>(dst + S * plane_stride) = w;
+    // the row's sum over the first 32 of every 128 K (8 threads a row), for the
+    // GEMM's choice of how much of K the guard samples
+    if (k0 % 128 == 0) {
+      int sum = (int)(g(d[0][0]) + g(d[1][0]) + g(d[2][0]) + g(d[3][0]));
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      if ((tid & 7) == 0 && r0 + r < rows && sum) atomicAdd(gsum_row + r0 + r, (unsigned)sum);
+    }
   }
 }
 
@@ -418,8 +433,6 @@ __device__ __forceinline__ double i128_scaled_to_double(long long hi, long long 
 // finishes it.  A whole call, before and after: 48 x 640 x 2363 (20 tiles) 100
 // -> 60 us, 1568 x 396 x 3536 (169 tiles) 274 -> 208, 1531 x 1400 x 1601 (528
 // tiles) 254 -> 245; chaining the call's kernels took another 9-12 us off each.
-constexpr unsigned kArrivedBase = 0x80808080u;  // the fill byte 0x80
-
 struct DgWork {
   int tile, kt0, nkt, part, rest;  // rest: index among the cut tiles, -1 if whole
 };
@@ -470,11 +483,13 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint64_t* empty = full + 4;   // [ST]  MMA -> TMA
   uint64_t* tfull = empty + 4;  // [2]   MMA -> epilogue: chunk in TMEM buffer b
   uint64_t* tempty = tfull + 2;  // [2]  epilogue -> MMA: buffer b drained
-  uint64_t* gfull = tempty + 2;  // [1]  TMA -> MMA: the guard slot (both producers)
+  uint64_t* gfull = tempty + 2;  // [1]  TMA -> MMA: the guard slot (A's and B's guard tiles)
   uint64_t* gempty = gfull + 1;  // [1]  MMA -> TMA
   uint64_t* accf = gempty + 1;   // [1]  every MMA of this CTA finished
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accf + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  uint64_t* gready = accf + 2;   // [1] the guard's minima are in `least`
+  __shared__ unsigned least[2];  // guard: smallest row sum of A, column sum of B
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
@@ -486,9 +501,11 @@ __global__ void __launch_bounds__(kThreads, 1)
       mbar_init(&tfull[b], 1);
       mbar_init(&tempty[b], kEpiWarps);
     }
-    mbar_init(gfull, 2);
+    mbar_init(gfull, 1);
     mbar_init(gempty, 1);
     mbar_init(accf, 1);
+    mbar_init(gready, kEpiWarps);
+    least[0] = least[1] = 0xFFFFFFFFu;
     *abort_flag = 0;
     fence_mbar_init();
     prefetch_tensormap(&tm_a);
@@ -513,11 +530,25 @@ __global__ void __launch_bounds__(kThreads, 1)
   };
 
   const int items = dg_items(p);
+  // The guard's sampling: the first 32 of every 128 K, or, where the guard
+  // planes' sums over those say that some output's lower bound may fall short,
+  // all of K.  (The smallest row sum times the smallest column sum over the
+  // number of K sampled estimates an output's sum; it has to be four times
+  // the limit.)  Either sum is a lower bound; the full one takes a third more
+  // shared-memory traffic and keeps operands whose magnitudes spread over
+  // many binades, few of them large at once, off the FP64 pipes: exponents of
+  // +-10 at 1531 x 1400 x 1601, 6435 us with the quarter, 275 with all.
+  // The epilogue warps find the two minima while the first stage is under way;
+  // the MMA lane and the guard producer wait for them after it (the wait up
+  // front took 3 us of every call).
+  auto sample_all = [&]() {
+    return (float)least[0] * (float)least[1] < 4.0f * (float)kGuardMin * 32.0f * (float)((p.K + 127) / 128);
+  };
   int issued = 0;  // A producer: stages whose copies were issued
   if ((warp == 0 || warp == kBProdWarp) && lane == 0) {
     // producers: warp 0 brings A's digit planes, warp 10 B's, into the same stages
     const bool is_a = warp == 0;
-    int n_issued = 0, g_issued = 0;
+    int n_issued = 0;
     bool stop = false;
     for (int w = (int)blockIdx.x; w < items && !stop; w += gridDim.x) {
       const DgWork dw = dg_work<CF::kChunk>(p, w);
@@ -525,23 +556,6 @@ __global__ void __launch_bounds__(kThreads, 1)
       dg_tile(p, dw.tile, m0, n0);
       for (int kt = 0; kt < dw.nkt; ++kt) {
         const int kx = (dw.kt0 + kt) * kBK;
-        if (G && kt % CF::kChunk == 0) {
-          // the guard planes' first 32 K of this chunk, once the MMAs of the
-          // previous chunk's guard product have read the slot
-          if (g_issued > 0 && !mbar_wait_bounded(gempty, (g_issued - 1) & 1, abort_flag, kWaitLimitNs)) {
-            fail();
-            stop = true;
-            break;
-          }
-          if (is_a) {
-            mbar_arrive_expect_tx(gfull, CF::kATile);
-            tma_load_3d(guard_a, &tm_ga, gfull, kx, m0, 0);
-          } else {
-            mbar_arrive_expect_tx(gfull, CF::kBTile);
-            tma_load_3d(guard_b, &tm_gb, gfull, kx, n0, 0);
-          }
-          ++g_issued;
-        }
         const int s = n_issued % ST, round = n_issued / ST;
         if (round > 0 && !mbar_wait_bounded(&empty[s], (round - 1) & 1, abort_flag, kWaitLimitNs)) {
           fail();
@@ -559,10 +573,42 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
     }
     if (is_a) issued = n_issued;
+  } else if (G && warp == kGuardWarp) {
+    // guard producer: the guard planes' 32 K of every sampled stage into the
+    // guard slot, once the guard product before has read it.  A warp of its
+    // own, so that waiting for the one slot does not hold back the stages.
+    if (lane == 0) {
+      int g_issued = 0;
+      bool stop = false, guard_all = false;
+      for (int w = (int)blockIdx.x; w < items && !stop; w += gridDim.x) {
+        const DgWork dw = dg_work<CF::kChunk>(p, w);
+        int m0, n0;
+        dg_tile(p, dw.tile, m0, n0);
+        for (int kt = 0; kt < dw.nkt; kt += guard_all ? 1 : CF::kChunk, ++g_issued) {
+          if (g_issued > 0 && !mbar_wait_bounded(gempty, (g_issued - 1) & 1, abort_flag, kWaitLimitNs)) {
+            fail();
+            stop = true;
+            break;
+          }
+          const int kx = (dw.kt0 + kt) * kBK;
+          mbar_arrive_expect_tx(gfull, CF::kATile + CF::kBTile);
+          tma_load_3d(guard_a, &tm_ga, gfull, kx, m0, 0);
+          tma_load_3d(guard_b, &tm_gb, gfull, kx, n0, 0);
+          if (g_issued == 0) {  // (the first stage is sampled either way)
+            if (!mbar_wait_bounded(gready, 0, abort_flag, kWaitLimitNs)) {
+              fail();
+              stop = true;
+              break;
+            }
+            guard_all = sample_all();
+          }
+        }
+      }
+    }
   } else if (warp == 1) {
     if (lane == 0) {
       int consumed = 0, chunk_g = 0, g_used = 0;
-      bool stop = false;
+      bool stop = false, guard_all = false;
       for (int w = (int)blockIdx.x; w < items && !stop; w += gridDim.x) {
         const int nkt = dg_work<CF::kChunk>(p, w).nkt;
         for (int kt = 0; kt < nkt; ++kt) {
@@ -587,8 +633,8 @@ __global__ void __launch_bounds__(kThreads, 1)
           tc_fence_after();
           const uint32_t acc = tmem + (uint32_t)b * kBufCols;
           const uint32_t b0 = smem_u32(b_tile(s));
-          if (G && chunk_first) {
-            // guard plane x guard plane over the chunk's first 32 K -> slot S
+          if (G && (guard_all || chunk_first)) {
+            // guard plane x guard plane over these 32 K -> slot S
             if (!mbar_wait_bounded(gfull, g_used & 1, abort_flag, kWaitLimitNs)) {
               fail();
               stop = true;
@@ -598,7 +644,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
             for (int kk = 0; kk < kBK / 16; ++kk)
               mma_f16(acc + 32u * S, sw64_kmajor_desc(smem_u32(guard_a) + kk * 32),
-                      sw64_kmajor_desc(smem_u32(guard_b) + kk * 32), idesc_bf16_f32(kBM, kBN), kk == 0 ? 0u : 1u);
+                      sw64_kmajor_desc(smem_u32(guard_b) + kk * 32), idesc_bf16_f32(kBM, kBN),
+                      chunk_first && kk == 0 ? 0u : 1u);
             mma_commit(gempty);
             ++g_used;
           }
@@ -615,6 +662,14 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
           mma_commit(&empty[s]);
           if (chunk_last) mma_commit(&tfull[b]);
+          if (G && consumed == 0) {  // (the first stage is sampled either way)
+            if (!mbar_wait_bounded(gready, 0, abort_flag, kWaitLimitNs)) {
+              fail();
+              stop = true;
+              break;
+            }
+            guard_all = sample_all();
+          }
           ++consumed;
         }
       }
@@ -629,6 +684,21 @@ __global__ void __launch_bounds__(kThreads, 1)
     // columns (half h) of each group's 32
     const int q = warp & 3, h = (warp - 2) >> 2;
     const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(16 * h);
+    if constexpr (G) {
+      unsigned la = 0xFFFFFFFFu, lb = 0xFFFFFFFFu;
+      const int tid = threadIdx.x - 64;
+#pragma unroll 8
+      for (int i = tid; i < p.M; i += 32 * kEpiWarps) la = min(la, __ldcg(p.ga + i) - kArrivedBase);
+#pragma unroll 8
+      for (int i = tid; i < p.N; i += 32 * kEpiWarps) lb = min(lb, __ldcg(p.gb + i) - kArrivedBase);
+      la = __reduce_min_sync(0xffffffffu, la);
+      lb = __reduce_min_sync(0xffffffffu, lb);
+      if (lane == 0) {
+        atomicMin(&least[0], la);
+        atomicMin(&least[1], lb);
+        mbar_arrive(gready);  // release: the waiters see both
+      }
+    }
     int chunk_g = 0;
     bool ok = true;
     for (int wk = (int)blockIdx.x; wk < items && ok; wk += gridDim.x) {
@@ -883,7 +953,9 @@ gbblas_status launch_digits(DeviceCtx* c, int64_t M, int64_t N, int64_t K, const
   const size_t off_arr = kScratchZeroBytes;  // arrival counts of cut tiles, filled with 0x80 as the scales are
   const size_t off_ea = off_arr + kArrivedBytes;
   const size_t off_eb = off_ea + align256(sizeof(int) * (size_t)Mp);
-  const size_t off_a = off_eb + align256(sizeof(int) * (size_t)Np);
+  const size_t off_ga = off_eb + align256(sizeof(int) * (size_t)Np);
+  const size_t off_gb = off_ga + (G ? align256(sizeof(int) * (size_t)Mp) : 0);
+  const size_t off_a = off_gb + (G ? align256(sizeof(int) * (size_t)Np) : 0);
   const size_t a_plane = (size_t)(Mp * Kp), b_plane = (size_t)(Np * Kp);
   const size_t off_b = off_a + align256((size_t)NP * a_plane * sizeof(__nv_bfloat16));
   const int64_t tiles = (Mp / kBM) * (Np / kBN);
@@ -913,8 +985,10 @@ gbblas_status launch_digits(DeviceCtx* c, int64_t M, int64_t N, int64_t K, const
   GB_TRY(check_launch("dg_init_kernel"));
   const int stk = (int)((K + kScaleTK - 1) / kScaleTK);
   const int tiles_k = (int)(Kp / 32);
-  DgOperand oa{A, M, K, rsa, csa, ea, da, (int64_t)a_plane, Kp, stk, (int)((Mp / 32) * stk)};
-  DgOperand ob{B, N, K, csb, rsb, eb, db, (int64_t)b_plane, Kp, stk, (int)((Np / 32) * stk)};
+  unsigned* gsa = reinterpret_cast<unsigned*>(base + off_ga);
+  unsigned* gsb = reinterpret_cast<unsigned*>(base + off_gb);
+  DgOperand oa{A, M, K, rsa, csa, ea, gsa, da, (int64_t)a_plane, Kp, stk, (int)((Mp / 32) * stk)};
+  DgOperand ob{B, N, K, csb, rsb, eb, gsb, db, (int64_t)b_plane, Kp, stk, (int)((Np / 32) * stk)};
   if ((double)(Mp + Np) / 32 * tiles_k >= 2.0e9) {
     set_error("dgemm (FP64 digits): operands too large for one preparation launch");
     return GBBLAS_STATUS_NOT_SUPPORTED;
@@ -952,6 +1026,8 @@ gbblas_status launch_digits(DeviceCtx* c, int64_t M, int64_t N, int64_t K, const
   p.csc = csc;
   p.ea = ea;
   p.eb = eb;
+  p.ga = gsa;
+  p.gb = gsb;
   p.fix_count = fix_count;  // cleared by row_scale_kernel
   p.fix_list = G ? fix_count + 1 : nullptr;
   p.A = A;
@@ -1005,7 +1081,8 @@ size_t dgemm_digits_scratch_bytes(int digits, bool guarded, int64_t M, int64_t N
   const int64_t Mp = round_up(M, kBM), Np = round_up(N, kBN), Kp = round_up(K, kBK);
   const int64_t np = digits + (guarded ? 1 : 0);
   const int64_t tiles = (Mp / kBM) * (Np / kBN);
-  return kScratchZeroBytes + kArrivedBytes + (size_t)kMaxCtas * (kSlotBytes + kGSlotBytes) + align256(sizeof(int) * (size_t)Mp) +
+  return kScratchZeroBytes + kArrivedBytes + (size_t)kMaxCtas * (kSlotBytes + kGSlotBytes) +
+         (guarded ? align256(sizeof(int) * (size_t)Mp) + align256(sizeof(int) * (size_t)Np) : 0) + align256(sizeof(int) * (size_t)Mp) +
          align256(sizeof(int) * (size_t)Np) +
          align256((size_t)(np * Mp * Kp) * 2) + align256((size_t)(np * Np * Kp) * 2) +
          (guarded ? align256(sizeof(int) * (size_t)(1 + tiles * kEpiWarps)) : 0);
