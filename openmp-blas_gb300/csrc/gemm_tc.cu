@@ -510,6 +510,28 @@ struct PrepSide {
   F16Guard guard;
 };
 
+// FP8: the 128 K of one row's block, 4 consecutive ones per lane, as E4M3
+// bytes; `scale` = the block's scale word (every lane).
+__device__ __forceinline__ uint32_t fp8_block(float4 v, uint32_t& scale) {
+  // the largest magnitude by its bits (a NaN does not count)
+  const float m = fmaxf(fmaxf(fmaxf(0.f, fabsf(v.x)), fabsf(v.y)), fmaxf(fmaxf(0.f, fabsf(v.z)), fabsf(v.w)));
+  const float amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
+  int e = 0;
+  if (amax > 0.f) {
+    int ex;
+    const float f = frexpf(amax, &ex);  // amax = f * 2^ex, f in [0.5, 1); 448 = 0.875 * 2^9
+    e = ex - 9 + (f > 0.875f ? 1 : 0);
+    e = e < -126 ? -126 : (e > 126 ? 126 : e);
+  }
+  const float inv = __int_as_float((127 - e) << 23);  // 2^-e, a normal float for |e| <= 126
+  const __nv_fp8x2_storage_t lo =
+      __nv_cvt_float2_to_fp8x2(make_float2(v.x * inv, v.y * inv), __NV_SATFINITE, __NV_E4M3);
+  const __nv_fp8x2_storage_t hi =
+      __nv_cvt_float2_to_fp8x2(make_float2(v.z * inv, v.w * inv), __NV_SATFINITE, __NV_E4M3);
+  scale = (uint32_t)(127 + e) * 0x01010101u;
+  return (uint32_t)lo | ((uint32_t)hi << 16);
+}
+
 // Shared-memory slot of (row r, K element k) of a preparation tile: the
 // 16-byte chunks of a row are permuted by the row's group of four (chunk c
 // stored at c ^ ((r / 4) & 7)), so the transposing stores of the
@@ -612,26 +634,11 @@ __global__ void __launch_bounds__(256, VEC ? 1 : 4) prep_group_kernel(PrepSide s
     for (int rr = 0; rr < 4; ++rr) {
       const int r = warp * 4 + rr;
       const float4 v = *reinterpret_cast<const float4*>(&tile[prep_slot<LD>(r, lane * 4)]);
-      float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-      int e = 0;
-      if (amax > 0.f) {
-        int ex;
-        const float m = frexpf(amax, &ex);  // amax = m * 2^ex, m in [0.5, 1); 448 = 0.875 * 2^9
-        e = ex - 9 + (m > 0.875f ? 1 : 0);
-        e = e < -126 ? -126 : (e > 126 ? 126 : e);
-      }
-      const float inv = __int_as_float((127 - e) << 23);  // 2^-e, a normal float for |e| <= 126
-      const __nv_fp8x2_storage_t lo =
-          __nv_cvt_float2_to_fp8x2(make_float2(v.x * inv, v.y * inv), __NV_SATFINITE, __NV_E4M3);
-      const __nv_fp8x2_storage_t hi =
-          __nv_cvt_float2_to_fp8x2(make_float2(v.z * inv, v.w * inv), __NV_SATFINITE, __NV_E4M3);
+      uint32_t scale;
+      const uint32_t bytes = fp8_block(v, scale);
       const int64_t row = j.dst_row + r0 + r;
-      *reinterpret_cast<uint32_t*>(q8 + row * pitch + k0 + lane * 4) = (uint32_t)lo | ((uint32_t)hi << 16);
-      if (lane == 0)
-        scales[(row >> 7) * scale_stride + k0 + 4 * (row & 31) + ((row >> 5) & 3)] =
-            (uint32_t)(127 + e) * 0x01010101u;
+      *reinterpret_cast<uint32_t*>(q8 + row * pitch + k0 + lane * 4) = bytes;
+      if (lane == 0) scales[(row >> 7) * scale_stride + k0 + 4 * (row & 31) + ((row >> 5) & 3)] = scale;
     }
   } else if constexpr (MODE == kModeF16) {
     // half-warp per row as below; the row scaled by 2^(15 - e) (exact), then
@@ -868,6 +875,71 @@ __global__ void __launch_bounds__(256) split_rows_kernel(RowSplitSide side_a, Ro
       }
     }
   }
+  }
+}
+
+// FP8 preparation of operands whose K is contiguous, any alignment: a warp per
+// arena row, a 128-K block per step, four steps' loads in flight - the same
+// bytes and scales as prep_group_kernel, without the shared-memory tile.
+// Grid as split_rows_kernel's.  Bound by HBM (4 B read, 1 written per element):
+// of an 8192^2 pair's 192 us by tiles A's half took 90, see launch_bound.
+struct RowFp8Side {
+  const SplitJob* jobs;
+  int rows;  // arena rows prepared here (0: this operand takes the tile kernel)
+  uint8_t* out;
+  uint32_t* scales;
+};
+
+__global__ void __launch_bounds__(256) fp8_rows_kernel(RowFp8Side side_a, RowFp8Side side_b, int njobs, int64_t pitch,
+                                                       int64_t scale_stride, int rows_per_cta, int64_t kseg) {
+  dev::grid_release();
+  dev::grid_wait();
+  __shared__ int sjob;
+  const int a_ctas = side_a.rows / rows_per_cta;
+  const bool on_b = (int)blockIdx.x >= a_ctas;
+  const RowFp8Side& sd = on_b ? side_b : side_a;
+  const int64_t R0 = (int64_t)((int)blockIdx.x - (on_b ? a_ctas : 0)) * rows_per_cta;  // first arena row
+  if (threadIdx.x == 0) {
+    int lo = 0, hi = njobs - 1;  // job: the last whose first arena row is <= R0
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (sd.jobs[mid].dst_row <= R0)
+        lo = mid;
+      else
+        hi = mid - 1;
+    }
+    sjob = lo;
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const SplitJob& j = sd.jobs[sjob];
+  const int per_warp = rows_per_cta / 8;
+  for (int rr = 0; rr < per_warp; ++rr) {
+    const int64_t R = R0 + (threadIdx.x >> 5) * per_warp + rr;  // arena row
+    const int64_t local = R - j.dst_row;
+    const int64_t kp = (int64_t)j.tiles_k * PrepTile<kModeFp8>::TK;  // the job's padded K
+    const int64_t K = local < j.rows ? j.K : 0;                      // padding rows: all zeros
+    const float* __restrict__ src = j.src + (local < j.rows ? local : 0) * j.rs;
+    const int w = row_width(src);
+    const int64_t kbeg = (int64_t)blockIdx.y * kseg, kend = min(kp, kbeg + kseg);
+    uint32_t* __restrict__ srow = sd.scales + (R >> 7) * scale_stride + 4 * (R & 31) + ((R >> 5) & 3);
+    for (int64_t k0 = kbeg; k0 < kend; k0 += 512) {
+      float4 x[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int64_t k = k0 + 128 * u + 4 * lane;
+        x[u] = load_row4(src + k, K - k, w);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int64_t kb = k0 + 128 * u;
+        if (kb >= kend) break;
+        uint32_t scale;
+        const uint32_t bytes = fp8_block(x[u], scale);
+        *reinterpret_cast<uint32_t*>(sd.out + R * pitch + kb + 4 * lane) = bytes;
+        if (lane == 0) srow[kb] = scale;
+      }
+    }
   }
 }
 
@@ -1877,7 +1949,7 @@ struct TcGroupPlan {
   bool guard = false;  // FP16 split with the AUTO guard (F16Guard, f16_guard_fixup_kernel)
   bool row_prep_a = false, row_prep_b = false;  // FP16 split: operand prepared by f16_row_prep_kernel
   bool col_scale_a = false, col_scale_b = false;  // FP16 split: exponents by f16_col_scale_kernel
-  bool row_split_a = false, row_split_b = false;  // BF16 split: operand prepared by split_rows_kernel
+  bool row_split_a = false, row_split_b = false;  // BF16 split, FP8: operand prepared row by row
   bool prep_vec_a = false, prep_vec_b = false;    // prep_group_kernel: 128-bit loads for every job of the operand
   int a_col_ctas = 0, b_col_ctas = 0, col_kblk = 128;
   size_t off_gmin = 0, off_gflag = 0, off_glist = 0;  // guard arrays: A rows then B rows each
@@ -2009,8 +2081,8 @@ gbblas_status plan_group(int mode, const gbblas_gemm_desc* d, int64_t count, TcG
   };
   pl.prep_vec_a = std::all_of(pl.ajobs.begin(), pl.ajobs.end(), vec_ok);
   pl.prep_vec_b = std::all_of(pl.bjobs.begin(), pl.bjobs.end(), vec_ok);
-  if (pl.mode == 2 || pl.mode == 3) {
-    // the BF16 split's pieces straight from registers where every job of an
+  if (pl.mode == 2 || pl.mode == 3 || pl.fp8()) {
+    // (FP8: the bytes and scales) the BF16 split's pieces straight from registers where every job of an
     // operand has K contiguous
     auto split_ok = [](const SplitJob& j) { return j.cs == 1; };
     pl.row_split_a = std::all_of(pl.ajobs.begin(), pl.ajobs.end(), split_ok);
@@ -2256,21 +2328,30 @@ gbblas_status launch_bound(DeviceCtx* c, const TcGroupPlan& pl, cudaStream_t str
   const int a_tiles = (pl.row_prep_a || pl.row_split_a) ? 0 : pl.a_tiles,
             b_tiles = (pl.row_prep_b || pl.row_split_b) ? 0 : pl.b_tiles;
   const int prep_ctas = a_tiles + b_tiles;
-  if constexpr (MODE == 2 || MODE == 3) {
+  if constexpr (MODE != kModeF16) {
     if (pl.row_split_a || pl.row_split_b) {
-      const RowSplitSide ra{djobs, pl.row_split_a ? (int)pl.a_rows : 0,
-                            reinterpret_cast<__nv_bfloat16*>(arena_a(pl)), (int64_t)(pl.a_rows * pl.pitch)};
-      const RowSplitSide rb{djobs + pl.njobs, pl.row_split_b ? (int)pl.b_rows : 0,
-                            reinterpret_cast<__nv_bfloat16*>(arena_b(pl)), (int64_t)(pl.b_rows * pl.pitch)};
       // arena rows come in multiples of 128 per job: whole CTAs of 8 or 32 rows
-      const int64_t rows = (int64_t)ra.rows + rb.rows;
+      const int ra_rows = pl.row_split_a ? (int)pl.a_rows : 0, rb_rows = pl.row_split_b ? (int)pl.b_rows : 0;
+      const int64_t rows = (int64_t)ra_rows + rb_rows;
       const int rpc = rows / kSplitRowsPerCtaMax >= 4 * (int64_t)c->num_sms ? kSplitRowsPerCtaMax : 8;
       const int64_t steps = (pl.kpad + 511) / 512;  // of K per row, to share out until there are 4 CTAs per SM
       const int64_t segs = std::max<int64_t>(1, std::min<int64_t>(steps, 4 * (int64_t)c->num_sms * rpc / rows));
       const int64_t kseg = (steps + segs - 1) / segs * 512;
       const dim3 grid((unsigned)(rows / rpc), (unsigned)((steps * 512 + kseg - 1) / kseg));
-      GB_CUDA_TRY(launch_chain(chained, split_rows_kernel<MODE>, grid, stream, ra, rb, pl.njobs, pl.pitch, rpc, kseg));
-      GB_TRY(check_launch("split_rows_kernel"));
+      if constexpr (MODE == kModeFp8) {
+        const RowFp8Side ra{djobs, ra_rows, reinterpret_cast<uint8_t*>(arena_a(pl)), scales_a(pl)};
+        const RowFp8Side rb{djobs + pl.njobs, rb_rows, reinterpret_cast<uint8_t*>(arena_b(pl)), scales_b(pl)};
+        GB_CUDA_TRY(
+            launch_chain(chained, fp8_rows_kernel, grid, stream, ra, rb, pl.njobs, pl.pitch, pl.kpad, rpc, kseg));
+        GB_TRY(check_launch("fp8_rows_kernel"));
+      } else {
+        const RowSplitSide ra{djobs, ra_rows, reinterpret_cast<__nv_bfloat16*>(arena_a(pl)),
+                              (int64_t)(pl.a_rows * pl.pitch)};
+        const RowSplitSide rb{djobs + pl.njobs, rb_rows, reinterpret_cast<__nv_bfloat16*>(arena_b(pl)),
+                              (int64_t)(pl.b_rows * pl.pitch)};
+        GB_CUDA_TRY(launch_chain(chained, split_rows_kernel<MODE>, grid, stream, ra, rb, pl.njobs, pl.pitch, rpc, kseg));
+        GB_TRY(check_launch("split_rows_kernel"));
+      }
     }
   }
   if constexpr (MODE == kModeF16) {
