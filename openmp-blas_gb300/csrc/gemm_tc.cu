@@ -238,12 +238,15 @@ struct SplitJob {
 };
 
 // ------------------------------------------------------ operand preparation
-// Tile of one preparation CTA: TR rows x TK along K (16 KB of FP32).
+// Tile of one preparation CTA: 64 rows x TK along K, 16 or (FP8) 32 KB of FP32
+// (FP8 with 32 rows: 128-byte reads of a row-contiguous operand, 83 us for
+// 8192^2 against 74 with 64).
 template <int MODE>
 struct PrepTile {
   static constexpr int TK = MODE == kModeFp8 ? 128 : 64;  // one FP8 scale block / one BF16 slice
-  static constexpr int TR = 4096 / TK;                    // 32 / 64 rows
-  static constexpr int LD = TK + 4;                       // shared row pitch (floats), 16-byte multiple
+  static constexpr int TR = 64;
+  static constexpr int NV = TR * TK / 1024;  // 16-byte vectors per thread
+  static constexpr int LD = TK + 4;          // shared row pitch (floats), 16-byte multiple
 };
 
 // For every job, writes its rows_pad x k_pad operand into the arena (row pitch
@@ -262,8 +265,10 @@ struct PrepTile {
 //    a * scale_stride + 128 kb + 4 i + j  (scale_stride = 128 x the K-blocks;
 //    each atom in the layout tmem_cp_scales expects).
 // One CTA per tile.  Interior tiles of 16-byte-aligned sources are read with
-// 128-bit loads along whichever dimension is contiguous; edge tiles and other
-// strides element by element (still coalesced along the contiguous side).
+// 128-bit loads along whichever dimension is contiguous, all of a thread's in
+// flight before its shared-memory stores (8192^2, split-FP16: 95 us with the
+// stores between them, 87 so); edge tiles and other strides element by
+// element (still coalesced along the contiguous side).
 // FP16 split: every row is scaled by 2^(15 - e), e the frexp exponent of its
 // largest magnitude (f16_scale_kernel), so it lies below 2^15 and inside
 // FP16's range.
@@ -586,25 +591,35 @@ __global__ void __launch_bounds__(256, VEC ? 1 : 4) prep_group_kernel(PrepSide s
   // float4 then lies wholly inside or wholly outside the operand)
   const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
   if (VEC ? j.cs == 1 : (al16 && j.cs == 1 && (j.rs & 3) == 0 && (full || (j.K & 3) == 0))) {  // along K
+    float4 v[PT::NV];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < PT::NV; ++i) {
       const int idx = tid + 256 * i, r = idx / (TK / 4), k4 = idx % (TK / 4);
-      const float4 v = (full || (r0 + r < j.rows && k0 + 4 * k4 < j.K))
-                           ? dev::ld_stream(reinterpret_cast<const float4*>(j.src + (r0 + r) * j.rs + k0 + 4 * k4))
-                           : zero4;
-      *reinterpret_cast<float4*>(&tile[prep_slot<LD>(r, 4 * k4)]) = v;
+      v[i] = (full || (r0 + r < j.rows && k0 + 4 * k4 < j.K))
+                 ? dev::ld_stream(reinterpret_cast<const float4*>(j.src + (r0 + r) * j.rs + k0 + 4 * k4))
+                 : zero4;
+    }
+#pragma unroll
+    for (int i = 0; i < PT::NV; ++i) {
+      const int idx = tid + 256 * i, r = idx / (TK / 4), k4 = idx % (TK / 4);
+      *reinterpret_cast<float4*>(&tile[prep_slot<LD>(r, 4 * k4)]) = v[i];
     }
   } else if (VEC || (al16 && j.rs == 1 && (j.cs & 3) == 0 && (full || (j.rows & 3) == 0))) {  // along rows
+    float4 v[PT::NV];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < PT::NV; ++i) {
       const int idx = tid + 256 * i, k = idx / (TR / 4), r4 = idx % (TR / 4);
-      const float4 v = (full || (k0 + k < j.K && r0 + 4 * r4 < j.rows))
-                           ? dev::ld_stream(reinterpret_cast<const float4*>(j.src + (k0 + k) * j.cs + r0 + 4 * r4))
-                           : zero4;
-      tile[prep_slot<LD>(4 * r4 + 0, k)] = v.x;
-      tile[prep_slot<LD>(4 * r4 + 1, k)] = v.y;
-      tile[prep_slot<LD>(4 * r4 + 2, k)] = v.z;
-      tile[prep_slot<LD>(4 * r4 + 3, k)] = v.w;
+      v[i] = (full || (k0 + k < j.K && r0 + 4 * r4 < j.rows))
+                 ? dev::ld_stream(reinterpret_cast<const float4*>(j.src + (k0 + k) * j.cs + r0 + 4 * r4))
+                 : zero4;
+    }
+#pragma unroll
+    for (int i = 0; i < PT::NV; ++i) {
+      const int idx = tid + 256 * i, k = idx / (TR / 4), r4 = idx % (TR / 4);
+      tile[prep_slot<LD>(4 * r4 + 0, k)] = v[i].x;
+      tile[prep_slot<LD>(4 * r4 + 1, k)] = v[i].y;
+      tile[prep_slot<LD>(4 * r4 + 2, k)] = v[i].z;
+      tile[prep_slot<LD>(4 * r4 + 3, k)] = v[i].w;
     }
   } else {
     // other alignments and strides, element by element (consecutive threads
@@ -618,21 +633,25 @@ __global__ void __launch_bounds__(256, VEC ? 1 : 4) prep_group_kernel(PrepSide s
     // elements 0 .. n - 1 exist
     const int64_t left = kc ? (k0 + k < j.K ? (j.rows - r0 - r + SR - 1) / SR : 0)
                             : (r0 + r < j.rows ? (j.K - k0 - k + SK - 1) / SK : 0);
-    const int n = (int)min(left, (int64_t)16);
-    float v[16];
+    const int n = (int)min(left, (int64_t)(4 * PT::NV));
+#pragma unroll 1
+    for (int i0 = 0; i0 < 4 * PT::NV; i0 += 16) {
+      float v[16];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = i < n ? __ldg(p + i * step) : 0.f;
+      for (int i = 0; i < 16; ++i) v[i] = i0 + i < n ? __ldg(p + (i0 + i) * step) : 0.f;
 #pragma unroll
-    for (int i = 0; i < 16; ++i) tile[prep_slot<LD>(kc ? r + SR * i : r, kc ? k : k + SK * i)] = v[i];
+      for (int i = 0; i < 16; ++i)
+        tile[prep_slot<LD>(kc ? r + SR * (i0 + i) : r, kc ? k : k + SK * (i0 + i))] = v[i];
+    }
   }
   __syncthreads();
   const int warp = tid >> 5, lane = tid & 31;
   if constexpr (MODE == kModeFp8) {
-    // warp w: rows 4w..4w+3, lane: 4 consecutive K of the row's 128
+    // warp w: rows 8w..8w+7, lane: 4 consecutive K of the row's 128
     uint8_t* q8 = static_cast<uint8_t*>(out);
 #pragma unroll
-    for (int rr = 0; rr < 4; ++rr) {
-      const int r = warp * 4 + rr;
+    for (int rr = 0; rr < TR / 8; ++rr) {
+      const int r = warp * (TR / 8) + rr;
       const float4 v = *reinterpret_cast<const float4*>(&tile[prep_slot<LD>(r, lane * 4)]);
       uint32_t scale;
       const uint32_t bytes = fp8_block(v, scale);
@@ -1983,7 +2002,7 @@ gbblas_status plan_group(int mode, const gbblas_gemm_desc* d, int64_t count, TcG
   pl.guard = mode == kModeF16Guard;
   if (pl.guard) mode = kModeF16;
   pl.mode = mode;
-  const int64_t sk = pl.slice_k(), pk = pl.pad_k(), jk = pl.job_k(), jr = 4096 / jk;
+  const int64_t sk = pl.slice_k(), pk = pl.pad_k(), jk = pl.job_k(), jr = 64;
   std::vector<int64_t> order;
   order.reserve(count);
   for (int64_t i = 0; i < count; ++i) {
