@@ -22,10 +22,10 @@
 //        prep_group_kernel on tiles.  All routes give the same bits.
 //      prep_group_kernel, FP8: every 128-element K-block of a row becomes
 //        128 E4M3 values and one power-of-two scale, kept as its UE8M0
-//        exponent byte in 512-byte atoms (128 rows of one K-block) beside
+//        exponent byte in 512-byte atoms (128 rows of four K-blocks) beside
 //        the arena, laid out the way tcgen05.cp moves them into TMEM.
 //   2. gemm_split_kernel (persistent, one CTA per SM): a device-side tile
-//      scheduler hands out 128 x 128 output tiles of all problems (largest K
+//      scheduler hands out 128 x 128 (FP8 also 128 x 256) output tiles of all problems (largest K
 //      first) through an atomic counter.  K is walked in chunks: each chunk
 //      accumulates in one of two TMEM buffers while the epilogue warps fold
 //      the previous chunk into FP32 registers with round-to-nearest adds; the
@@ -44,24 +44,28 @@
 //      accurate as FP32 FMA arithmetic.  bf16x3 keeps about 16 bits.
 //      FP8 (tcgen05.mma kind::mxf8f6f4 block_scale, E4M3 in, FP32
 //      accumulate): the tensor core applies the row and column block scales
-//      itself (UE8M0 scales copied from the stage into TMEM by tcgen05.cp
-//      ahead of each slice's MMAs); chunks of 512 K as for the split.
+//      itself (UE8M0 scales copied from the stage into TMEM by tcgen05.cp,
+//      those of 512 of K at once); chunks of 512 K as for the split.
 //
-// Warp roles (320 threads; FP8: 192):
-//   warp 0      tile scheduler + TMA producer: takes the next tile from the
-//               global counter, publishes it in a shared-memory tile ring,
-//               then streams its K slices (128 bytes of K of all P pieces of
-//               A and of B: one 3-D tiled bulk copy per operand, 128-byte
-//               swizzle; FP8 adds the two 512-byte scale atoms) into a
-//               stage ring;
-//   warp 1      allocates TMEM and issues the MMAs (one elected lane);
+// Warp roles (384 threads; FP8 on narrow tiles 256), B producer and scheduler
+// last:
+//   scheduler   takes the next tile from the global counter while the A
+//               producer loads the last stages of the one before, finds its
+//               problem and publishes both in a shared-memory tile ring;
+//   warp 0      TMA producer of A: streams the tile's K slices (128 bytes of
+//               K of all P pieces: one 3-D tiled bulk copy, 128-byte swizzle;
+//               FP8 adds a 512-byte scale atom every 512 of K) into a stage
+//               ring; the B producer does the same for B (CTA pairs: warp 0
+//               loads both);
+//   warp 1      allocates TMEM and issues the MMAs (one elected lane of a
+//               warp whose control flow stays uniform);
 //               tcgen05.commit frees a stage once its MMAs have read it and
 //               signals a TMEM chunk buffer as full;
 //   warps 2-9   epilogue: tcgen05.ld each finished chunk (warp w reads TMEM
-//   (FP8: 2-5)  lanes 32*(w%4)..+31 = tile rows; with 8 warps, warps 2-5
-//               take the first 64 columns, 6-9 the other 64) into FP32
+//   (narrow     lanes 32*(w%4)..+31 = tile rows; with 8 warps, warps 2-5
+//   FP8: 2-5)   take the first half of the columns, 6-9 the other) into FP32
 //               registers, release the buffer, add the registers into C
-//               (single CTAs: 32 x 32 blocks staged in shared memory and
+//               (single CTAs: 32-column blocks staged in shared memory and
 //               added by TMA reduce-add stores where C's layout allows).
 // Every mbarrier wait is bounded (2 s by %globaltimer); a wait that gives up
 // records GBBLAS_STATUS_TIMEOUT in the stream's error word, the CTA drains
@@ -97,6 +101,7 @@ using namespace tc;
 
 constexpr int kBM = 128;
 constexpr int kBN = 128;
+constexpr int kBNWide = 256;  // FP8: tile columns where they leave enough tiles, see fp8_wide
 constexpr int kBK = 64;  // K padding of the BF16 arenas: 64 bf16 = one 128-byte row
 // K slices folded into FP32 registers per chunk: three-product split every
 // 512 of K, six-product split every 128 (the tensor core's accumulation over
@@ -113,6 +118,7 @@ constexpr int kChunkTiles6 = 2;
 constexpr int kChunkTilesF16 = 2;
 constexpr int kChunkTilesFp8 = 2;  // FP8 stages are 256 K deep
 constexpr int kTileRing = 4;     // tiles in flight between scheduler and consumers
+constexpr int kAhead = 4;        // stages of a tile left to load when the next is taken
 constexpr int kMaxStages = 8;    // operand stages in flight (as many as shared memory holds, up to this)
 constexpr uint64_t kWaitLimitNs = 2000000000ull;  // 2 s
 constexpr size_t kSmemLimit = 232448;             // 227 KB per CTA
@@ -126,10 +132,13 @@ constexpr int kModeF16 = 12;
 // kModeF16 with the AUTO guard (host-side plan mode; the kernels run kModeF16)
 constexpr int kModeF16Guard = kTcModeF16Guard;
 
-template <int MODE>
+// BN: tile columns (kBN; FP8 also kBNWide).
+template <int MODE, int BN = kBN>
 struct ModeTraits {
   static constexpr bool fp8 = MODE == kModeFp8;
   static constexpr bool f16 = MODE == kModeF16;
+  static constexpr bool wide = BN == kBNWide;
+  static_assert(BN == kBN || (wide && fp8), "256 tile columns are FP8's");
   static constexpr int P = fp8 ? 1 : (f16 ? 2 : MODE);  // operand planes per operand
   // Bytes of K per operand row in one K sub-tile (128-byte swizzle).  The
   // six-product split measured slower with 64-byte rows (32-K stages, 4 in
@@ -138,59 +147,72 @@ struct ModeTraits {
   static constexpr int kKSteps = kRowBytes / 32;  // MMAs of 32 bytes of K per sub-tile
   // K sub-tiles per stage: one for the split, two for FP8 (256 E4M3: twice
   // the MMAs per barrier round trip, the per-stage hand-offs being what
-  // bounds the four-MMA FP8 stage).
-  static constexpr int kSub = fp8 ? 2 : 1;
+  // bounds the four-MMA FP8 stage; a wide tile's MMAs last twice as long).
+  static constexpr int kSub = fp8 && !wide ? 2 : 1;
   static constexpr int kBKe = fp8 ? 128 * kSub : kRowBytes / 2;  // K elements per stage
   // slices per TMEM chunk (the six-product and the FP16 split every 128 of
   // K, the three-product split and FP8 every 512)
-  static constexpr int kChunk = fp8 ? kChunkTilesFp8 : (MODE == 2 ? kChunkTiles3 : (f16 ? kChunkTilesF16 : kChunkTiles6));
+  static constexpr int kChunk = fp8 ? kChunkTilesFp8 * (wide ? 2 : 1) : (MODE == 2 ? kChunkTiles3 : (f16 ? kChunkTilesF16 : kChunkTiles6));
   // Epilogue warps: 8 for the split, each 32 tile rows x 64 columns (with
   // 128 FP32 accumulators per thread the kernel ran out of registers and
-  // spilled); 4 for FP8, each 32 rows x 128 columns (no spills).
-  static constexpr int kEpiWarps = fp8 ? 4 : 8;
-  static constexpr int kCols = kBN * 4 / kEpiWarps;  // tile columns per epilogue thread
+  // spilled); 4 for FP8 (8 in wide tiles), each 32 rows x 128 columns (no
+  // spills).
+  static constexpr int kEpiWarps = fp8 && !wide ? 4 : 8;
+  static constexpr int kCols = BN * 4 / kEpiWarps;  // tile columns per epilogue thread
   // Single CTAs load B with a second producer warp (after the epilogue
   // warps): one thread issuing every copy caps what TMA delivers into the
   // SM (measured 43-46 B/cycle for 64 KB stages from one issuing thread,
   // 66-68 from two).  CTA pairs keep one producer; the warp then idles.
   static constexpr int kBProdWarp = 2 + kEpiWarps;
-  static constexpr int kThreads = 64 + 32 * kEpiWarps + 32;
+  static constexpr int kSchedWarp = kBProdWarp + 1;  // the tile scheduler
+  static constexpr int kThreads = 64 + 32 * kEpiWarps + 64;
   // TMEM: two chunk buffers (the MMAs may run one chunk ahead of the
   // epilogue), main + correction accumulators for the split (2 x 256
-  // columns), one accumulator for FP8 (2 x 128 columns, then one 8-column
-  // scale slot per stage from column 256).
+  // columns), one accumulator for FP8 (2 x 128 columns, then a ring of
+  // scale slots from column 256, one per stage in flight).  Wide tiles have one
+  // chunk buffer, whose halves of 128 columns are filled and drained in turn.
   static constexpr int kBufs = 2;
   static constexpr uint32_t kBufCols = fp8 ? kBN : 2 * kBN;
   static constexpr uint32_t kSfCol0 = 2 * kBN;
+  static constexpr uint32_t kSfB = wide ? 8 : 4;            // B's scales within a slot (256 rows: 8 columns)
+  static constexpr uint32_t kSfSlot = wide ? 16 : 8;        // columns of a slot
+  // FP8: stages that one pair of scale atoms (512 of K) covers.  A stage that
+  // begins one brings it.
+  static constexpr int kAtomStages = fp8 ? 512 / kBKe : 1;
 };
 
-template <int MODE, bool PAIR>
+template <int MODE, bool PAIR, int BN = kBN>
 struct TcCfg {
-  static constexpr int P = ModeTraits<MODE>::P;
-  static constexpr uint32_t kRow = ModeTraits<MODE>::kRowBytes;
+  using MT = ModeTraits<MODE, BN>;
+  static constexpr int P = MT::P;
+  static constexpr uint32_t kRow = MT::kRowBytes;
   static constexpr uint32_t kABytes = kBM * kRow;  // one K sub-tile of A (this CTA's rows)
-  static constexpr uint32_t kBBytes = (PAIR ? kBN / 2 : kBN) * kRow;  // B^T rows this CTA stages
-  static constexpr int kSub = ModeTraits<MODE>::kSub;
-  // FP8: the stage's scale atoms (512 bytes per 128-K block) of A, then of B
-  static constexpr uint32_t kSfBytes = ModeTraits<MODE>::fp8 ? 2 * 512 * kSub : 0;
+  static constexpr uint32_t kBBytes = (PAIR ? kBN / 2 : BN) * kRow;  // B^T rows this CTA stages
+  static constexpr int kSub = MT::kSub;
+  // FP8: a scale atom (128 rows x 512 of K) of A, then those of B
+  static constexpr uint32_t kSfABytes = MT::fp8 ? 512 : 0, kSfBBytes = kSfABytes * (BN / 128);
+  static constexpr uint32_t kSfBytes = (kSfABytes + kSfBBytes + 1023) / 1024 * 1024;
   static constexpr uint32_t kStageBytes = P * kSub * (kABytes + kBBytes) + kSfBytes;
-  // what each producer of a single CTA brings per stage (A part, B part)
-  static constexpr uint32_t kAStageBytes = P * kSub * kABytes + kSfBytes / 2;
-  static constexpr uint32_t kBStageBytes = P * kSub * kBBytes + kSfBytes / 2;
+  // what each producer of a single CTA brings per stage (A part, B part),
+  // besides the scale atoms
+  static constexpr uint32_t kAStageBytes = P * kSub * kABytes;
+  static constexpr uint32_t kBStageBytes = P * kSub * kBBytes;
   static constexpr uint32_t kTmemCols = 512;
   static constexpr size_t kBarBytes = 1024;  // mbarriers, tile ring, TMEM slot, abort flag
-  // Single CTAs: per epilogue warp one 32 x 32 float block (4 KB, 1024-aligned)
-  // that a TMA reduce-add store adds into C (where C's layout allows it)
+  // Single CTAs: per epilogue warp one block of 32 (wide tiles, for a fourth
+  // stage: 16) rows x 32 floats, 1024-aligned, that a TMA reduce-add store
+  // adds into C (where C's layout allows it)
   static constexpr bool kTmaC = !PAIR;
-  static constexpr size_t kEpiScratch = kTmaC ? (size_t)ModeTraits<MODE>::kEpiWarps * 4096 : 0;
+  static constexpr int kScrRows = MT::wide ? 16 : 32;
+  static constexpr size_t kEpiScratch = kTmaC ? (size_t)MT::kEpiWarps * kScrRows * 128 : 0;
   static constexpr int kStagesFit = (int)((kSmemLimit - 1024 - kBarBytes - kEpiScratch) / kStageBytes);
   static constexpr int kStages = kStagesFit > kMaxStages ? kMaxStages : kStagesFit;
   static constexpr size_t kSmem = 1024 /*alignment slack*/ + (size_t)kStages * kStageBytes + kEpiScratch + kBarBytes;
-  static_assert(!(PAIR && ModeTraits<MODE>::fp8), "FP8 runs on single CTAs");
-  static_assert(ModeTraits<MODE>::kBufs * ModeTraits<MODE>::kBufCols <= kTmemCols, "chunk buffers exceed TMEM");
-  static_assert(!ModeTraits<MODE>::fp8 || ModeTraits<MODE>::kSfCol0 + 8 * kSub * kStages <= kTmemCols,
+  static_assert(!(PAIR && MT::fp8), "FP8 runs on single CTAs");
+  static_assert(MT::kBufs * MT::kBufCols <= kTmemCols, "chunk buffers exceed TMEM");
+  static_assert(!MT::fp8 || MT::kSfCol0 + MT::kSfSlot * kStages <= kTmemCols,
                 "scale slots exceed TMEM");
-  static_assert((2 * kMaxStages + 2 * 4 + 2 * kTileRing + 1) * 8 + (kTileRing + 3) * 4 <= kBarBytes,
+  static_assert((2 * kMaxStages + 2 * 4 + 2 * kTileRing + 2) * 8 + (8 * kTileRing + 3) * 4 <= kBarBytes,
                 "barrier area too small");
   static_assert(kStages >= 2, "need at least a double-buffered stage ring");
   static_assert(kSmem <= kSmemLimit, "exceeds the 227 KB per-CTA shared memory limit");
@@ -201,7 +223,7 @@ struct TcCfg {
 
 // One GEMM of a group, as the kernel sees it (device memory).
 struct TcProblem {
-  CUtensorMap c_map;  // FP8 with c_tma: C as a float tensor, 32 x 32 boxes, 128-byte swizzle
+  CUtensorMap c_map;  // with c_tma: C as a float tensor, boxes of 32 columns x TcCfg::kScrRows rows, 128-byte swizzle
   int c_tma;          // 1: the epilogue adds into C with TMA reduce-add stores
   int M, N;
   int num_kt;      // K stages: 64 of K (BF16) or 256 (FP8) each
@@ -258,12 +280,12 @@ struct PrepTile {
 //    amax * 2^-e <= 448 (the largest finite E4M3), so v * 2^-e is exact and
 //    only the E4M3 rounding (nearest-even, saturating) loses bits.  All-zero
 //    (and padding) blocks get s = 1.  The scale is stored as its UE8M0 byte
-//    e + 127, repeated in the four bytes of a 32-bit word (one per 32-K
-//    sub-block of the MMA), words in 512-byte atoms of 128 arena rows and
-//    one K-block, the atoms of a row block consecutive along K:
-//    row R = 128 a + 32 j + i of K-block kb at word
-//    a * scale_stride + 128 kb + 4 i + j  (scale_stride = 128 x the K-blocks;
-//    each atom in the layout tmem_cp_scales expects).
+//    e + 127, those of four K-blocks in one 32-bit word (an MMA names the
+//    byte it takes), words in 512-byte atoms of 128 arena rows and 512 of K,
+//    the atoms of a row block consecutive along K: row R = 128 a + 32 j + i of
+//    K-block kb at byte kb % 4 of word
+//    a * scale_stride + 128 (kb / 4) + 4 i + j  (scale_stride = 128 x the
+//    atoms along K; each atom in the layout tmem_cp_scales expects).
 // One CTA per tile.  Interior tiles of 16-byte-aligned sources are read with
 // 128-bit loads along whichever dimension is contiguous, all of a thread's in
 // flight before its shared-memory stores (8192^2, split-FP16: 95 us with the
@@ -516,7 +538,7 @@ struct PrepSide {
 };
 
 // FP8: the 128 K of one row's block, 4 consecutive ones per lane, as E4M3
-// bytes; `scale` = the block's scale word (every lane).
+// bytes; `scale` = the block's scale byte (every lane).
 __device__ __forceinline__ uint32_t fp8_block(float4 v, uint32_t& scale) {
   // the largest magnitude by its bits (a NaN does not count)
   const float m = fmaxf(fmaxf(fmaxf(0.f, fabsf(v.x)), fabsf(v.y)), fmaxf(fmaxf(0.f, fabsf(v.z)), fabsf(v.w)));
@@ -533,7 +555,7 @@ __device__ __forceinline__ uint32_t fp8_block(float4 v, uint32_t& scale) {
       __nv_cvt_float2_to_fp8x2(make_float2(v.x * inv, v.y * inv), __NV_SATFINITE, __NV_E4M3);
   const __nv_fp8x2_storage_t hi =
       __nv_cvt_float2_to_fp8x2(make_float2(v.z * inv, v.w * inv), __NV_SATFINITE, __NV_E4M3);
-  scale = (uint32_t)(127 + e) * 0x01010101u;
+  scale = (uint32_t)(127 + e);
   return (uint32_t)lo | ((uint32_t)hi << 16);
 }
 
@@ -657,7 +679,10 @@ __global__ void __launch_bounds__(256, VEC ? 1 : 4) prep_group_kernel(PrepSide s
       const uint32_t bytes = fp8_block(v, scale);
       const int64_t row = j.dst_row + r0 + r;
       *reinterpret_cast<uint32_t*>(q8 + row * pitch + k0 + lane * 4) = bytes;
-      if (lane == 0) scales[(row >> 7) * scale_stride + k0 + 4 * (row & 31) + ((row >> 5) & 3)] = scale;
+      if (lane == 0) {
+        uint32_t* word = scales + (row >> 7) * scale_stride + (k0 >> 9) * 128 + 4 * (row & 31) + ((row >> 5) & 3);
+        reinterpret_cast<uint8_t*>(word)[(k0 >> 7) & 3] = (uint8_t)scale;
+      }
     }
   } else if constexpr (MODE == kModeF16) {
     // half-warp per row as below; the row scaled by 2^(15 - e) (exact), then
@@ -949,6 +974,7 @@ __global__ void __launch_bounds__(256) fp8_rows_kernel(RowFp8Side side_a, RowFp8
         const int64_t k = k0 + 128 * u + 4 * lane;
         x[u] = load_row4(src + k, K - k, w);
       }
+      uint32_t word = 0;  // the four K-blocks' scale bytes (kseg is a multiple of 512)
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int64_t kb = k0 + 128 * u;
@@ -956,8 +982,9 @@ __global__ void __launch_bounds__(256) fp8_rows_kernel(RowFp8Side side_a, RowFp8
         uint32_t scale;
         const uint32_t bytes = fp8_block(x[u], scale);
         *reinterpret_cast<uint32_t*>(sd.out + R * pitch + kb + 4 * lane) = bytes;
-        if (lane == 0) srow[kb] = scale;
+        word |= scale << (8 * u);
       }
+      if (lane == 0) srow[(k0 >> 9) * 128] = word;
     }
   }
 }
@@ -1117,16 +1144,23 @@ __device__ __forceinline__ int find_problem(const TcProblem* __restrict__ probs,
   return lo;
 }
 
-// One tile's work: output tile (BMT rows x 128 columns) at (m0, n0), K
+// One tile's work: output tile (BMT rows x BN columns) at (m0, n0), K
 // stages kt0 .. kt0 + nkt - 1 (those of its split-K part).
 struct TileWork {
   int m0, n0, kt0, nkt, part;
 };
 
+// What the scheduler publishes of a tile in shared memory: its problem (-1: no
+// more work), its work, and its first rows in the arenas.
+struct alignas(16) RingTile {
+  int prob, kt0, nkt, part;
+  int m0, n0, a_row, b_row;
+};
+
 // Global tile index t: the parts of a split problem one after another, each
 // in a grouped raster (consecutive tiles walk 8 row-tiles of one column band
 // for L2 reuse).
-template <int BMT>
+template <int BMT, int BN>
 __device__ __forceinline__ TileWork tile_work(const TcProblem& p, int t) {
   constexpr int kGroup = 8;
   TileWork w;
@@ -1147,7 +1181,7 @@ __device__ __forceinline__ TileWork tile_work(const TcProblem& p, int t) {
   const int gm = min(p.tiles_m - first_m, kGroup);
   const int in_g = local % group_span;
   w.m0 = (first_m + in_g % gm) * BMT;
-  w.n0 = (in_g / gm) * kBN;
+  w.n0 = (in_g / gm) * BN;
   return w;
 }
 
@@ -1160,16 +1194,22 @@ __device__ __forceinline__ TileWork tile_work(const TcProblem& p, int t) {
 // stages and signal both CTAs' epilogues, and both epilogues report drained
 // TMEM buffers to it.  Pairs walk tiles in a static order (cluster i takes
 // tiles i, i + clusters, ...), so both CTAs see the same sequence.
-template <int MODE, bool PAIR>
-__global__ void __launch_bounds__(ModeTraits<MODE>::kThreads, 1)
+// BN = 256 (FP8): 128 x 256 tiles.  At FP8's rate a tile of 128 columns is
+// bound by what TMA delivers (64 KB per 1050 cycles of its MMAs, 62 bytes a
+// cycle); a wide tile needs three quarters of those bytes, and reads A from
+// shared memory once for twice the columns.  TMEM then holds one chunk only:
+// the MMAs of a chunk's first and last K stage are issued by column halves, so
+// that the epilogue drains one half while the other's run.  What is left is
+// that wait (530 of 3590 cycles a chunk) and the halves' own pace.
+template <int MODE, bool PAIR, int BN>
+__global__ void __launch_bounds__(ModeTraits<MODE, BN>::kThreads, 1)
     gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                       const TcProblem* __restrict__ probs, int nprob, int tile_begin, int total_tiles,
-                      int64_t sf_stride,
-                      int* __restrict__ tile_counter, int* __restrict__ err,
+                      int64_t sf_stride, int sfb_blocks, int* __restrict__ tile_counter, int* __restrict__ err,
                       const uint32_t* __restrict__ sa, const uint32_t* __restrict__ sb,
                       const int* __restrict__ guard_a, const int* __restrict__ guard_b) {
-  using MT = ModeTraits<MODE>;
-  using CF = TcCfg<MODE, PAIR>;
+  using MT = ModeTraits<MODE, BN>;
+  using CF = TcCfg<MODE, PAIR, BN>;
   constexpr int P = MT::P;
   constexpr int ST = CF::kStages;
   constexpr int BMT = PAIR ? 2 * kBM : kBM;  // output tile rows (both CTAs of a pair)
@@ -1183,10 +1223,14 @@ __global__ void __launch_bounds__(ModeTraits<MODE>::kThreads, 1)
   auto b_tile = [&](int s, int p) {
     return smem + (size_t)s * CF::kStageBytes + (size_t)NT * CF::kABytes + (size_t)p * CF::kBBytes;
   };
-  // FP8: the stage's scale atoms of A (op 0) / of B^T (op 1), kSub x 512 bytes each
+  // FP8: the scale atom of A (op 0) / the BN / 128 of B^T (op 1), if the stage brings them
   auto sf_atom = [&](int s, int op) {
     return smem + (size_t)s * CF::kStageBytes + (size_t)NT * (CF::kABytes + CF::kBBytes) +
-           (size_t)op * 512 * MT::kSub;
+           (size_t)op * 512;
+  };
+  // does K stage kt of a tile bring scale atoms (the tile's first one, or the first of 512 of K)?
+  auto brings_atoms = [](const RingTile& w, int kt) {
+    return MT::fp8 && (kt == 0 || (w.kt0 + kt) % MT::kAtomStages == 0);
   };
   float* epi_scratch = reinterpret_cast<float*>(smem + (size_t)ST * CF::kStageBytes);  // single CTAs, 1024-aligned
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (size_t)ST * CF::kStageBytes + CF::kEpiScratch);
@@ -1197,7 +1241,10 @@ __global__ void __launch_bounds__(ModeTraits<MODE>::kThreads, 1)
   uint64_t* ring_full = tempty + 4;        // [kTileRing] scheduler -> consumers
   uint64_t* ring_empty = ring_full + kTileRing;  // [kTileRing] consumers -> scheduler
   uint64_t* accf = ring_empty + kTileRing;       // [1] every MMA of this CTA finished
-  int* ring = reinterpret_cast<int*>(accf + 1);  // [kTileRing] tile ids, -1 = no more work
+  uint64_t* want = accf + 1;                     // [1] A producer -> scheduler: the next tile, please
+  // [kTileRing] (the barrier area is 1024-aligned)
+  RingTile* ring =
+      reinterpret_cast<RingTile*>((reinterpret_cast<uintptr_t>(want + 1) + 15) & ~uintptr_t(15));
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ring + kTileRing);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* b_issued_slot = abort_flag + 1;  // single CTAs: K slices the B producer issued (teardown)
@@ -1212,13 +1259,15 @@ __global__ void __launch_bounds__(ModeTraits<MODE>::kThreads, 1)
     }
     for (int b = 0; b < MT::kBufs; ++b) {
       mbar_init(&tfull[b], 1);
-      mbar_init(&tempty[b], MT::kEpiWarps * (PAIR ? 2 : 1));  // one arrival per epilogue warp (of both CTAs)
+      // one arrival per epilogue warp (of both CTAs; of the half's four in a wide tile)
+      mbar_init(&tempty[b], MT::wide ? 4 : MT::kEpiWarps * (PAIR ? 2 : 1));
     }
     for (int r = 0; r < kTileRing; ++r) {
       mbar_init(&ring_full[r], 1);
-      mbar_init(&ring_empty[r], 1 + MT::kEpiWarps + (PAIR ? 0 : 1));  // MMA lane, epilogue warps, B producer
+      mbar_init(&ring_empty[r], 2 + MT::kEpiWarps + (PAIR ? 0 : 1));  // A producer, MMA lane, epilogue warps, B producer
     }
     mbar_init(accf, 1);
+    mbar_init(want, 1);
     *abort_flag = 0;
     *b_issued_slot = 0;
     fence_mbar_init();
@@ -1247,29 +1296,56 @@ __global__ void __launch_bounds__(ModeTraits<MODE>::kThreads, 1)
   };
 
   int issued = 0;  // producer: K slices whose copies were issued (all tiles)
-  if (warp == 0) {
+  if (warp == MT::kSchedWarp) {
+    // Tile scheduler.  It takes a tile when the A producer has kAhead stages
+    // of the one before left to load: early enough that no role waits for the
+    // counter or the search through the problems, late enough that no CTA
+    // holds tiles that another could have begun.
     if (lane == 0) {
-      bool stop = false;
-      for (int it = 0; !stop; ++it) {
+      for (int it = 0;; ++it) {
         const int slot = it % kTileRing, use = it / kTileRing;
+        if (it > 0 && !mbar_wait_bounded(want, (it - 1) & 1, abort_flag, kWaitLimitNs)) {
+          fail();
+          break;
+        }
         int t;
         // this launch's tiles: tile_begin .. total_tiles - 1
         if constexpr (PAIR)
           t = tile_begin + (int)(blockIdx.x >> 1) + it * (int)(gridDim.x >> 1);
         else
           t = tile_begin + atomicAdd(tile_counter, 1);
-        if (t >= total_tiles) t = -1;
+        RingTile rt = {-1, 0, 0, 0, 0, 0, 0, 0};
+        if (t < total_tiles) {
+          rt.prob = find_problem(probs, nprob, t);
+          const TcProblem& pr = probs[rt.prob];
+          const TileWork tw = tile_work<BMT, BN>(pr, t);
+          rt = RingTile{rt.prob, tw.kt0, tw.nkt, tw.part, tw.m0, tw.n0, pr.a_row + tw.m0, pr.b_row + tw.n0};
+        }
         if (use > 0 && !mbar_wait_bounded(&ring_empty[slot], (use - 1) & 1, abort_flag, kWaitLimitNs)) {
           fail();
           break;
         }
-        ring[slot] = t;
+        ring[slot] = rt;
         mbar_arrive(&ring_full[slot]);  // release: consumers see ring[slot]
-        if (t < 0) break;
-        const TcProblem& pr = probs[find_problem(probs, nprob, t)];
-        const TileWork tw = tile_work<BMT>(pr, t);
-        const int n0 = tw.n0, own_m0 = tw.m0 + (int)rank * kBM;  // this CTA's rows
+        if (rt.prob < 0) break;
+      }
+    }
+  } else if (warp == 0) {
+    if (lane == 0) {
+      bool stop = false;
+      for (int it = 0; !stop; ++it) {
+        const int slot = it % kTileRing, use = it / kTileRing;
+        if (!mbar_wait_bounded(&ring_full[slot], use & 1, abort_flag, kWaitLimitNs)) {
+          fail();
+          break;
+        }
+        const RingTile tw = ring[slot];
+        mbar_arrive(&ring_empty[slot]);
+        if (tw.prob < 0) break;
+        const int own_row = tw.a_row + (int)rank * kBM;  // this CTA's rows
+        const int ask = max(0, tw.nkt - kAhead);
         for (int kt = 0; kt < tw.nkt; ++kt) {
+          if (kt == ask) mbar_arrive(want);
           const int s = issued % ST, round = issued / ST;
           if (round > 0 && !mbar_wait_bounded(&empty[s], (round - 1) & 1, abort_flag, kWaitLimitNs)) {
             fail();
@@ -1281,27 +1357,26 @@ __global__ void __launch_bounds__(ModeTraits<MODE>::kThreads, 1)
           if constexpr (PAIR) {
             if (rank == 0) {
               mbar_arrive_expect_tx(&full[s], 2 * CF::kStageBytes);  // both CTAs' copies
-              tma_load_3d(a_tile(s, 0), &tm_a, &full[s], kx, pr.a_row + own_m0, 0);
-              tma_load_3d(b_tile(s, 0), &tm_b, &full[s], kx, pr.b_row + n0, 0);
+              tma_load_3d(a_tile(s, 0), &tm_a, &full[s], kx, own_row, 0);
+              tma_load_3d(b_tile(s, 0), &tm_b, &full[s], kx, tw.b_row, 0);
             } else {
               const uint32_t fb = mapa_shared(smem_u32(&full[s]), 0);
-              tma_load_3d_pair(a_tile(s, 0), &tm_a, fb, kx, pr.a_row + own_m0, 0);
-              tma_load_3d_pair(b_tile(s, 0), &tm_b, fb, kx, pr.b_row + n0 + kBN / 2, 0);
+              tma_load_3d_pair(a_tile(s, 0), &tm_a, fb, kx, own_row, 0);
+              tma_load_3d_pair(b_tile(s, 0), &tm_b, fb, kx, tw.b_row + kBN / 2, 0);
             }
           } else {
             // A's part of the stage; the B producer warp brings the rest
-            mbar_arrive_expect_tx(&full[s], CF::kAStageBytes);
+            const bool atoms = brings_atoms(tw, kt);
+            mbar_arrive_expect_tx(&full[s], CF::kAStageBytes + (atoms ? CF::kSfABytes : 0));
             if constexpr (MT::fp8) {
 #pragma unroll
               for (int u = 0; u < MT::kSub; ++u)
-                tma_load_3d(a_tile(s, u), &tm_a, &full[s], kx + u * 128, pr.a_row + own_m0, 0);
-              // the stage's K-blocks' scale atoms of these 128 rows of A:
-              // consecutive in the scale array (one run)
-              const int64_t kb0 = kx;  // 128 words per K-block of 128 = one word per K element
-              bulk_load(sf_atom(s, 0), sa + (int64_t)((pr.a_row + own_m0) >> 7) * sf_stride + kb0, 512 * MT::kSub,
-                        &full[s]);
+                tma_load_3d(a_tile(s, u), &tm_a, &full[s], kx + u * 128, own_row, 0);
+              if (atoms)
+                bulk_load(sf_atom(s, 0), sa + (int64_t)((own_row) >> 7) * sf_stride + (kx >> 9) * 128, 512,
+                          &full[s]);
             } else {
-              tma_load_3d(a_tile(s, 0), &tm_a, &full[s], kx, pr.a_row + own_m0, 0);
+              tma_load_3d(a_tile(s, 0), &tm_a, &full[s], kx, own_row, 0);
             }
           }
           ++issued;
@@ -1320,12 +1395,9 @@ __global__ void __launch_bounds__(ModeTraits<MODE>::kThreads, 1)
           fail();
           break;
         }
-        const int t = ring[slot];
+        const RingTile tw = ring[slot];
         mbar_arrive(&ring_empty[slot]);
-        if (t < 0) break;
-        const TcProblem& pr = probs[find_problem(probs, nprob, t)];
-        const TileWork tw = tile_work<BMT>(pr, t);
-        const int n0 = tw.n0;
+        if (tw.prob < 0) break;
         for (int kt = 0; kt < tw.nkt; ++kt) {
           const int s = bissued % ST, round = bissued / ST;
           if (round > 0 && !mbar_wait_bounded(&empty[s], (round - 1) & 1, abort_flag, kWaitLimitNs)) {
@@ -1334,15 +1406,23 @@ __global__ void __launch_bounds__(ModeTraits<MODE>::kThreads, 1)
             break;
           }
           const int kx = (tw.kt0 + kt) * MT::kBKe;
-          mbar_arrive_expect_tx(&full[s], CF::kBStageBytes);
+          const bool atoms = brings_atoms(tw, kt);
+          mbar_arrive_expect_tx(&full[s], CF::kBStageBytes + (atoms ? CF::kSfBBytes : 0));
           if constexpr (MT::fp8) {
 #pragma unroll
             for (int u = 0; u < MT::kSub; ++u)
-              tma_load_3d(b_tile(s, u), &tm_b, &full[s], kx + u * 128, pr.b_row + n0, 0);
-            bulk_load(sf_atom(s, 1), sb + (int64_t)((pr.b_row + n0) >> 7) * sf_stride + (int64_t)kx, 512 * MT::kSub,
-                      &full[s]);
+              tma_load_3d(b_tile(s, u), &tm_b, &full[s], kx + u * 128, tw.b_row, 0);
+            // (a wide tile whose second half lies past the arena's last row
+            // block takes that block's scales again: its columns are dropped)
+            if (atoms) {
+#pragma unroll
+              for (int h = 0; h < BN / 128; ++h)
+                bulk_load(sf_atom(s, 1) + 512 * h,
+                          sb + (int64_t)min((tw.b_row >> 7) + h, sfb_blocks - 1) * sf_stride + (kx >> 9) * 128,
+                          512, &full[s]);
+            }
           } else {
-            tma_load_3d(b_tile(s, 0), &tm_b, &full[s], kx, pr.b_row + n0, 0);
+            tma_load_3d(b_tile(s, 0), &tm_b, &full[s], kx, tw.b_row, 0);
           }
           ++bissued;
         }
@@ -1350,130 +1430,204 @@ __global__ void __launch_bounds__(ModeTraits<MODE>::kThreads, 1)
       *b_issued_slot = bissued;
     }
   } else if (warp == 1) {
-    if (lane == 0 && PAIR && rank != 0) {
+    if (PAIR && rank != 0) {
       // the odd CTA of a pair issues no MMAs: it only keeps its tile ring moving
-      for (int it = 0;; ++it) {
+      for (int it = 0; lane == 0; ++it) {
         const int slot = it % kTileRing, use = it / kTileRing;
         if (!mbar_wait_bounded(&ring_full[slot], use & 1, abort_flag, kWaitLimitNs)) {
           fail();
           break;
         }
-        const int t = ring[slot];
+        const int prob = ring[slot].prob;
         mbar_arrive(&ring_empty[slot]);
-        if (t < 0) break;
+        if (prob < 0) break;
       }
-    } else if (lane == 0) {
+    } else {
+      // The whole warp runs the loop and one elected lane issues, so that
+      // control flow and descriptors stay uniform, and a stage's work beside
+      // the MMAs is kept short: this warp's own time, not the tensor pipe's,
+      // was what bounded the kernel (stages in one lane of divergent code, a
+      // descriptor and a division each, without any loads: 1259 cycles of an
+      // FP8 stage whose MMAs take 512, 1071 of a split-FP16 one, 768).
+      // FP8 at 8192^3 705 -> 630 us on narrow and 693 -> 572 on wide tiles,
+      // 3970 x 3475 x 4050 AUTO 352 -> 344, 512 GEMMs of 32 .. 2048 1115 -> 1071.
+      const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+      auto wait = [&](uint64_t* bar, uint32_t parity) {
+        if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+        const bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, abort_flag, kWaitLimitNs));
+        if (!ok && lane == 0) fail();
+        return ok;
+      };
       // split-BF16 (FP16 pieces for kModeF16); M = 256 for a pair
       constexpr uint32_t idesc = MT::f16 ? idesc_f16_f32(BMT, kBN) : idesc_bf16_f32(BMT, kBN);
       // single CTAs: p0*[q0; q1] as one N = 256 MMA - the q0 and q1 tiles of
       // B^T lie back to back in the stage and the main and correction
       // accumulators side by side in TMEM, so A's p0 is read once for both
       constexpr uint32_t idesc_n256 = MT::f16 ? idesc_f16_f32(kBM, 2 * kBN) : idesc_bf16_f32(kBM, 2 * kBN);
-      int consumed = 0;  // K slices consumed (all tiles)
+      int s = 0;           // stage of the next K slice
+      uint32_t phase = 0;  // and its barrier's phase
+      const uint32_t lo0 = __shfl_sync(0xffffffffu, sw128_kmajor_lo(smem_u32(smem)), 0);
       int chunk_g = 0;   // chunks started (all tiles)
+      int atoms = 0;     // FP8: scale atoms taken (all tiles), and the TMEM slot of the last
+      uint32_t sf_slot = 0;
       bool stop = false;
+      auto advance = [&]() {
+        if (++s == ST) {
+          s = 0;
+          phase ^= 1;
+        }
+      };
       for (int it = 0; !stop; ++it) {
         const int slot = it % kTileRing, use = it / kTileRing;
-        if (!mbar_wait_bounded(&ring_full[slot], use & 1, abort_flag, kWaitLimitNs)) {
-          fail();
-          break;
-        }
-        const int t = ring[slot];
-        mbar_arrive(&ring_empty[slot]);
-        if (t < 0) break;
-        const int num_kt = tile_work<BMT>(probs[find_problem(probs, nprob, t)], t).nkt;
+        if (!wait(&ring_full[slot], use & 1)) break;
+        RingTile tw = ring[slot];
+        const int num_kt = __shfl_sync(0xffffffffu, tw.prob < 0 ? -1 : tw.nkt, 0);
+        tw.kt0 = __shfl_sync(0xffffffffu, tw.kt0, 0);
+        if (lane == 0) mbar_arrive(&ring_empty[slot]);
+        if (num_kt < 0) break;
         for (int kt = 0; kt < num_kt; ++kt) {
-          const int s = consumed % ST, round = consumed / ST;
           const bool chunk_first = (kt % MT::kChunk) == 0;
           const bool chunk_last = ((kt + 1) % MT::kChunk) == 0 || kt + 1 == num_kt;
           if (chunk_first) ++chunk_g;
           const int chunk = chunk_g - 1, b = chunk % MT::kBufs;
-          if (chunk_first && chunk >= MT::kBufs) {  // buffer b must have been drained by the epilogue(s)
-            if (!mbar_wait_bounded(&tempty[b], ((chunk / MT::kBufs) - 1) & 1, abort_flag, kWaitLimitNs)) {
-              fail();
+          if (!MT::wide && chunk_first && chunk >= MT::kBufs) {  // buffer b must have been drained by the epilogue(s)
+            if (!wait(&tempty[b], ((chunk / MT::kBufs) - 1) & 1)) {
               stop = true;
               break;
             }
             tc_fence_after();
           }
-          if (!mbar_wait_bounded(&full[s], round & 1, abort_flag, kWaitLimitNs)) {
-            fail();
+          if (!wait(&full[s], phase)) {
             stop = true;
             break;
           }
           tc_fence_after();
-          const uint32_t acc_main = tmem + (uint32_t)b * MT::kBufCols, acc_corr = acc_main + kBN;
+          const uint32_t acc_main = tm + (uint32_t)b * MT::kBufCols, acc_corr = acc_main + kBN;
+          // the stage's operand tiles (descriptor low words)
           uint32_t a[NT], bb[NT];
 #pragma unroll
           for (int p = 0; p < NT; ++p) {
-            a[p] = smem_u32(a_tile(s, p));
-            bb[p] = smem_u32(b_tile(s, p));
+            a[p] = lo0 + (uint32_t)s * (CF::kStageBytes >> 4) + (uint32_t)p * (CF::kABytes >> 4);
+            bb[p] = lo0 + (uint32_t)s * (CF::kStageBytes >> 4) + ((NT * CF::kABytes + (uint32_t)p * CF::kBBytes) >> 4);
           }
-          // FP8: stage s's TMEM scale slot (8 columns per 128-K block: 4 for
-          // A's scales, 4 for B's).  Its previous user, the stage's previous
-          // round, has finished (the stage came back), so it is free.
-          const uint32_t sf_slot = tmem + MT::kSfCol0 + 8u * MT::kSub * (uint32_t)s;
+          // FP8: the scales of 512 of K into the next of ST TMEM slots (A's in
+          // 4 columns, from kSfB B's).  A slot's last user lies at least ST
+          // stages back, so its MMAs have finished (that stage came back).
           if constexpr (MT::fp8) {
+            if (brings_atoms(tw, kt)) {
+              sf_slot = tm + MT::kSfCol0 + MT::kSfSlot * (uint32_t)(atoms++ % ST);
+              if (elect_one()) {
+                tmem_cp_scales(sf_slot, smem_u32(sf_atom(s, 0)));
 #pragma unroll
-            for (int u = 0; u < MT::kSub; ++u) {
-              tmem_cp_scales(sf_slot + 8u * u, smem_u32(sf_atom(s, 0)) + 512u * u);
-              tmem_cp_scales(sf_slot + 8u * u + 4u, smem_u32(sf_atom(s, 1)) + 512u * u);
+                for (int h = 0; h < BN / 128; ++h)
+                  tmem_cp_scales(sf_slot + MT::kSfB + 4u * h, smem_u32(sf_atom(s, 1)) + 512u * h);
+              }
+              __syncwarp();
             }
+          }
+          // the byte of the scale words that holds the stage's (first) K-block
+          const uint32_t sf_byte = (uint32_t)((tw.kt0 + kt) % MT::kAtomStages) * MT::kSub;
+          if constexpr (MT::wide) {
+            // columns n .. n + 127 (half = true) or all 256 of the stage
+            auto mmas = [&](uint32_t n, bool half, uint32_t acc) {
+#pragma unroll
+              for (int kk = 0; kk < MT::kKSteps; ++kk)
+                mma_mxf8(tm + n, sw128_kmajor_from(a[0] + kk * 2), sw128_kmajor_from(bb[0] + n * 8 + kk * 2),
+                         half ? idesc_mxe4m3(kBM, kBN, sf_byte, sf_byte) : idesc_mxe4m3(kBM, kBNWide, sf_byte, sf_byte),
+                         sf_slot, sf_slot + MT::kSfB + n / 32, kk == 0 ? acc : 1u);
+            };
+            if (chunk_first || chunk_last) {
+#pragma unroll
+              for (uint32_t h = 0; h < 2; ++h) {
+                if (chunk_first && chunk > 0) {  // the half must have been drained
+                  if (!wait(&tempty[h], (chunk - 1) & 1)) {
+                    stop = true;
+                    break;
+                  }
+                  tc_fence_after();
+                }
+                if (elect_one()) {
+                  mmas(h * kBN, true, chunk_first ? 0u : 1u);
+                  if (chunk_last) mma_commit(&tfull[h]);
+                  if (h == 1) mma_commit(&empty[s]);
+                }
+                __syncwarp();
+              }
+              if (stop) break;
+            } else {
+              if (elect_one()) {
+                mmas(0, false, 1u);
+                mma_commit(&empty[s]);
+              }
+              __syncwarp();
+            }
+            advance();
+            continue;
           }
           auto mma = [&](uint32_t d, uint32_t ad, uint32_t bd, uint32_t accumulate) {
             if constexpr (PAIR)
-              mma2_f16(d, sw128_kmajor_desc(ad), sw128_kmajor_desc(bd), idesc, accumulate);
+              mma2_f16(d, sw128_kmajor_from(ad), sw128_kmajor_from(bd), idesc, accumulate);
             else
-              mma_f16(d, sw128_kmajor_desc(ad), sw128_kmajor_desc(bd), idesc, accumulate);
+              mma_f16(d, sw128_kmajor_from(ad), sw128_kmajor_from(bd), idesc, accumulate);
           };
-#pragma unroll
-          for (int kk = 0; kk < MT::kKSteps; ++kk) {
-            // 32 bytes along K per MMA inside the swizzled 128- / 64-byte
-            // row: 16 bf16 (kind::f16) or 32 e4m3 (kind::mxf8f6f4)
-            const uint32_t off = kk * 32;
-            const uint32_t acc = (chunk_first && kk == 0) ? 0u : 1u;
+          if (elect_one()) {
             if constexpr (MT::fp8) {
-              // 32-K sub-block kk of each 128-K scale block: byte kk of each scale word
+              // (along K, as in a wide tile: the same bits)
 #pragma unroll
               for (int u = 0; u < MT::kSub; ++u)
-                mma_mxf8(acc_main, sw128_kmajor_desc(a[u] + off), sw128_kmajor_desc(bb[u] + off),
-                         idesc_mxe4m3(kBM, kBN, kk, kk), sf_slot + 8u * u, sf_slot + 8u * u + 4u,
-                         u == 0 ? acc : 1u);
-            } else {
-              // corrections, largest first: p0p1, p1p0 (+ p0p2, p1p1, p2p0)
-              if constexpr (PAIR) {
-                mma(acc_main, a[0] + off, bb[0] + off, acc);
-                mma(acc_corr, a[0] + off, bb[1] + off, acc);
-              } else {
-                static_assert(CF::kBBytes == kBN * 128, "q1 must follow q0 directly");
-                mma_f16(acc_main, sw128_kmajor_desc(a[0] + off), sw128_kmajor_desc(bb[0] + off), idesc_n256, acc);
-              }
-              mma(acc_corr, a[1] + off, bb[0] + off, 1u);
-              if constexpr (P == 3) {
-                mma(acc_corr, a[0] + off, bb[2] + off, 1u);
-                mma(acc_corr, a[1] + off, bb[1] + off, 1u);
-                mma(acc_corr, a[2] + off, bb[0] + off, 1u);
+#pragma unroll
+                for (int kk = 0; kk < MT::kKSteps; ++kk)
+                  mma_mxf8(acc_main, sw128_kmajor_from(a[u] + kk * 2), sw128_kmajor_from(bb[u] + kk * 2),
+                           idesc_mxe4m3(kBM, kBN, sf_byte + u, sf_byte + u), sf_slot, sf_slot + MT::kSfB,
+                           chunk_first && u + kk == 0 ? 0u : 1u);
+            }
+#pragma unroll
+            for (int kk = 0; kk < MT::kKSteps; ++kk) {
+              // 32 bytes along K per MMA inside the swizzled 128- / 64-byte
+              // row: 16 bf16 (kind::f16) or 32 e4m3 (kind::mxf8f6f4)
+              const uint32_t off = kk * 2;
+              const uint32_t acc = (chunk_first && kk == 0) ? 0u : 1u;
+              if constexpr (!MT::fp8) {
+                // corrections, largest first: p0p1, p1p0 (+ p0p2, p1p1, p2p0)
+                if constexpr (PAIR) {
+                  mma(acc_main, a[0] + off, bb[0] + off, acc);
+                  mma(acc_corr, a[0] + off, bb[1] + off, acc);
+                } else {
+                  static_assert(CF::kBBytes == kBN * 128, "q1 must follow q0 directly");
+                  mma_f16(acc_main, sw128_kmajor_from(a[0] + off), sw128_kmajor_from(bb[0] + off), idesc_n256, acc);
+                }
+                mma(acc_corr, a[1] + off, bb[0] + off, 1u);
+                if constexpr (P == 3) {
+                  mma(acc_corr, a[0] + off, bb[2] + off, 1u);
+                  mma(acc_corr, a[1] + off, bb[1] + off, 1u);
+                  mma(acc_corr, a[2] + off, bb[0] + off, 1u);
+                }
               }
             }
+            if constexpr (PAIR) {
+              mma_commit2(&empty[s], 3);  // both CTAs' stage s
+              if (chunk_last) mma_commit2(&tfull[b], 3);
+            } else {
+              mma_commit(&empty[s]);
+              if (chunk_last) mma_commit(&tfull[b]);
+            }
           }
-          if constexpr (PAIR) {
-            mma_commit2(&empty[s], 3);  // both CTAs' stage s
-            if (chunk_last) mma_commit2(&tfull[b], 3);
-          } else {
-            mma_commit(&empty[s]);
-            if (chunk_last) mma_commit(&tfull[b]);
-          }
-          ++consumed;
+          __syncwarp();
+          advance();
         }
       }
       // accf completes once every MMA issued above has finished, on the
       // normal path and after an abort alike, so TMEM (and, for a pair, the
       // peer's shared memory) is never released under a running MMA.
-      if constexpr (PAIR)
-        mma_commit2(accf, 1);
-      else
-        mma_commit(accf);
-      if (*abort_flag) {
+      __syncwarp();
+      if (elect_one()) {
+        if constexpr (PAIR)
+          mma_commit2(accf, 1);
+        else
+          mma_commit(accf);
+      }
+      __syncwarp();
+      if (lane == 0 && *abort_flag) {
         int never = 0;
         (void)mbar_wait_bounded(accf, 0, &never, kWaitLimitNs);
       }
@@ -1494,12 +1648,11 @@ __global__ void __launch_bounds__(ModeTraits<MODE>::kThreads, 1)
         if (lane == 0) fail();
         break;
       }
-      const int t = ring[slot];
+      const RingTile tw = ring[slot];
       __syncwarp();
       if (lane == 0) mbar_arrive(&ring_empty[slot]);
-      if (t < 0) break;
-      const TcProblem& pr = probs[find_problem(probs, nprob, t)];
-      const TileWork tw = tile_work<BMT>(pr, t);
+      if (tw.prob < 0) break;
+      const TcProblem& pr = probs[tw.prob];
       const int n0 = tw.n0, m0 = tw.m0 + (int)rank * kBM;  // this CTA's rows
       const int nchunks = (tw.nkt + MT::kChunk - 1) / MT::kChunk;
       float acc[kCols];
@@ -1507,17 +1660,19 @@ __global__ void __launch_bounds__(ModeTraits<MODE>::kThreads, 1)
       for (int j = 0; j < kCols; ++j) acc[j] = 0.f;
       bool ok = true;
       for (int c = 0; c < nchunks; ++c, ++chunk_g) {
-        const int b = chunk_g % MT::kBufs;
+        // (in a wide tile this warp's half of the one buffer)
+        const int b = MT::wide ? col0 / kBN : chunk_g % MT::kBufs;
+        const int use_b = MT::wide ? chunk_g : chunk_g / MT::kBufs;
         // tcgen05.ld is warp-collective: make the decision warp-uniform.
         const bool ready =
-            __all_sync(0xffffffffu, mbar_wait_bounded(&tfull[b], (chunk_g / MT::kBufs) & 1, abort_flag, kWaitLimitNs));
+            __all_sync(0xffffffffu, mbar_wait_bounded(&tfull[b], use_b & 1, abort_flag, kWaitLimitNs));
         if (!ready) {
           if (lane == 0) fail();
           ok = false;
           break;
         }
         tc_fence_after();
-        const uint32_t tb = trow + (uint32_t)b * MT::kBufCols;
+        const uint32_t tb = MT::wide ? trow : trow + (uint32_t)b * MT::kBufCols;
         // the fold: FP8 has one accumulator per buffer, the splits two (main,
         // corrections), added with packed round-to-nearest FP32 adds
         if constexpr (MT::fp8) {
@@ -1605,17 +1760,21 @@ __global__ void __launch_bounds__(ModeTraits<MODE>::kThreads, 1)
                 if (skip_row || ((skip_cols >> c) & 1)) acc[c] = -0.0f;
             }
           }
-          float* scr = epi_scratch + (warp - 2) * 1024;
+          constexpr int kRows = CF::kScrRows;
+          float* scr = epi_scratch + (warp - 2) * kRows * 32;
           if (lane == 0) fence_tensormap(&pr.c_map);  // the tables were written after the driver last saw them
 #pragma unroll
-          for (int cb = 0; cb < kCols; cb += 32) {
+          for (int i = 0; i < kCols / 32 * (32 / kRows); ++i) {
+            const int cb = i / (32 / kRows) * 32, r0 = i % (32 / kRows) * kRows;  // the block's columns and rows
+            if (kRows == 32 || lane / kRows == r0 / kRows) {
 #pragma unroll
-            for (int c = 0; c < 8; ++c)
-              *reinterpret_cast<float4*>(scr + lane * 32 + ((c ^ (lane & 7)) * 4)) =
-                  make_float4(acc[cb + 4 * c], acc[cb + 4 * c + 1], acc[cb + 4 * c + 2], acc[cb + 4 * c + 3]);
+              for (int c = 0; c < 8; ++c)
+                *reinterpret_cast<float4*>(scr + (lane % kRows) * 32 + ((c ^ (lane & 7)) * 4)) =
+                    make_float4(acc[cb + 4 * c], acc[cb + 4 * c + 1], acc[cb + 4 * c + 2], acc[cb + 4 * c + 3]);
+            }
             fence_proxy_async_shared();
             __syncwarp();
-            const int bx = n0 + col0 + cb, by = m0 + q * 32;
+            const int bx = n0 + col0 + cb, by = m0 + q * 32 + r0;
             if (lane == 0 && bx < pr.N && by < pr.M) {  // boxes wholly outside C are skipped
               tma_reduce_add_2d(&pr.c_map, smem_u32(scr), bx, by);
               bulk_commit_group();
@@ -1641,28 +1800,35 @@ __global__ void __launch_bounds__(ModeTraits<MODE>::kThreads, 1)
           // shared memory (swizzled as for the TMA update) and the warp
           // updates one row's 32 columns, 128 bytes, per access
           const uint32_t skip_rows = __ballot_sync(0xffffffffu, skip_row);
-          float* scr = epi_scratch + (warp - 2) * 1024;
+          constexpr int kRows = CF::kScrRows;
+          float* scr = epi_scratch + (warp - 2) * kRows * 32;
 #pragma unroll
           for (int cb = 0; cb < kCols; cb += 32) {
-            __syncwarp();
+            auto stage_rows = [&](int r0) {  // rows r0 .. r0 + kRows - 1 of the block into scr
+              __syncwarp();
+              if (kRows == 32 || lane / kRows == r0 / kRows) {
 #pragma unroll
-            for (int c = 0; c < 8; ++c)
-              *reinterpret_cast<float4*>(scr + lane * 32 + ((c ^ (lane & 7)) * 4)) =
-                  make_float4(acc[cb + 4 * c], acc[cb + 4 * c + 1], acc[cb + 4 * c + 2], acc[cb + 4 * c + 3]);
-            __syncwarp();
+                for (int c = 0; c < 8; ++c)
+                  *reinterpret_cast<float4*>(scr + (lane % kRows) * 32 + ((c ^ (lane & 7)) * 4)) =
+                      make_float4(acc[cb + 4 * c], acc[cb + 4 * c + 1], acc[cb + 4 * c + 2], acc[cb + 4 * c + 3]);
+              }
+              __syncwarp();
+            };
+            if (kRows == 32) stage_rows(0);
             const int col = cn + cb + lane;
             // rows r < rows of the block exist for this lane's column
             const int rows = col < pr.N && !(MT::f16 && ((skip_cols >> (cb + lane)) & 1)) ? min(pr.M - row0, 32) : 0;
             float* cp = Cd + (int64_t)row0 * rsc + col;
 #pragma unroll
             for (int r0 = 0; r0 < 32; r0 += 16) {
+              if (kRows == 16) stage_rows(r0);
               float old[16];
               const float* lp = cp;
 #pragma unroll
               for (int r = 0; r < 16; ++r, lp += rsc) old[r] = (add && r0 + r < rows) ? *lp : 0.f;
 #pragma unroll
               for (int r = 0; r < 16; ++r, cp += rsc) {
-                const float v = scr[(r0 + r) * 32 + (((lane >> 2) ^ (r & 7)) * 4) + (lane & 3)];
+                const float v = scr[((r0 + r) % kRows) * 32 + (((lane >> 2) ^ (r & 7)) * 4) + (lane & 3)];
                 if (r0 + r < rows && !((skip_rows >> (r0 + r)) & 1)) *cp = add ? old[r] + v : v;
               }
             }
@@ -1965,6 +2131,7 @@ struct TcGroupPlan {
   CUtensorMap map_a, map_b;
   bool cleared = false;  // the launch's start words are clear already (tc_init_kernel)
   bool pair = false;  // CTA pairs computing 256 x 128 tiles (see gemm_split_kernel)
+  bool wide = false;  // FP8: 128 x 256 tiles (fp8_wide)
   bool guard = false;  // FP16 split with the AUTO guard (F16Guard, f16_guard_fixup_kernel)
   bool row_prep_a = false, row_prep_b = false;  // FP16 split: operand prepared by f16_row_prep_kernel
   bool col_scale_a = false, col_scale_b = false;  // FP16 split: exponents by f16_col_scale_kernel
@@ -1978,14 +2145,32 @@ struct TcGroupPlan {
   bool f16() const { return mode == kModeF16; }
   int planes() const { return fp8() ? 1 : (f16() ? 2 : mode); }
   int slice_k() const {  // K elements per stage
-    return fp8() ? ModeTraits<kModeFp8>::kBKe : (mode == 3 ? ModeTraits<3>::kBKe : ModeTraits<2>::kBKe);
+    return wide ? ModeTraits<kModeFp8, kBNWide>::kBKe
+                : fp8() ? ModeTraits<kModeFp8>::kBKe : (mode == 3 ? ModeTraits<3>::kBKe : ModeTraits<2>::kBKe);
   }
   int pad_k() const { return fp8() ? ModeTraits<kModeFp8>::kBKe : kBK; }  // K padding (multiple of stage and prep tile)
   int row_bytes() const { return mode == 3 ? ModeTraits<3>::kRowBytes : 128; }  // bytes of K per row per sub-tile
+  int64_t sf_stride() const { return (kpad + 511) / 512 * 128; }  // FP8: scale words per 128 rows
   int job_k() const { return fp8() ? 128 : 64; }     // K extent of one preparation tile (PrepTile::TK)
 };
 
 namespace {
+
+// FP8 on 128 x 256 tiles?  The tiles go to the SMs in rounds, and a round of
+// wide tiles takes 1.72 of a narrow round (8192^3: 30.8 against 18.1 us, 14
+// rounds against 27, the call 572 against 630 us; 4096^3 20 against 11.6, 4
+// against 7, 117.3 against 118.6 us; 2048^3 1 against 2, 33.5 against 34.1;
+// 1024^3 1 against 1, 22.7 against 20.4).  The results are the same bits.
+constexpr double kWideRound = 1.72;
+bool fp8_wide(const gbblas_gemm_desc* d, const std::vector<int64_t>& order, int sms) {
+  int64_t narrow = 0, wide = 0;
+  for (int64_t i : order) {
+    const int64_t tm = (d[i].M + kBM - 1) / kBM;
+    narrow += tm * ((d[i].N + kBN - 1) / kBN);
+    wide += tm * ((d[i].N + kBNWide - 1) / kBNWide);
+  }
+  return kWideRound * (double)((wide + sms - 1) / sms) < (double)((narrow + sms - 1) / sms);
+}
 
 // Host-side planning (no device work): problem order (largest K first),
 // arena rows, tile numbering, split jobs, device layout.  opt.split > 1
@@ -1993,7 +2178,7 @@ namespace {
 // each with tiles of its own that store a partial; a reduction then adds
 // the parts into C in order.  opt.pair forces the CTA form (-1: the
 // GBBLAS_TC_PAIR setting).
-gbblas_status plan_group(int mode, const gbblas_gemm_desc* d, int64_t count, TcGroupPlan& pl,
+gbblas_status plan_group(DeviceCtx* c, int mode, const gbblas_gemm_desc* d, int64_t count, TcGroupPlan& pl,
                          const TcLaunchOpts& opt = TcLaunchOpts()) {
   if (mode != 2 && mode != 3 && mode != kModeFp8 && mode != kModeF16 && mode != kModeF16Guard) {
     set_error("tensor-core gemm: unknown mode %d", mode);
@@ -2002,7 +2187,7 @@ gbblas_status plan_group(int mode, const gbblas_gemm_desc* d, int64_t count, TcG
   pl.guard = mode == kModeF16Guard;
   if (pl.guard) mode = kModeF16;
   pl.mode = mode;
-  const int64_t sk = pl.slice_k(), pk = pl.pad_k(), jk = pl.job_k(), jr = 64;
+  const int64_t pk = pl.pad_k(), jk = pl.job_k(), jr = 64;
   std::vector<int64_t> order;
   order.reserve(count);
   for (int64_t i = 0; i < count; ++i) {
@@ -2031,6 +2216,8 @@ gbblas_status plan_group(int mode, const gbblas_gemm_desc* d, int64_t count, TcG
     }
     pl.pair = w2 <= 1.1 * w1;
   }
+  pl.wide = pl.fp8() && opt.split <= 1 && fp8_wide(d, order, c->num_sms);
+  const int64_t sk = pl.slice_k();
   const int64_t bmt = pl.pair ? 2 * kBM : kBM;  // output tile rows
   pl.njobs = (int)order.size();
   pl.ajobs.resize(pl.njobs);
@@ -2055,7 +2242,7 @@ gbblas_status plan_group(int mode, const gbblas_gemm_desc* d, int64_t count, TcG
     p.a_row = (int)pl.a_rows;
     p.b_row = (int)pl.b_rows;
     p.tiles_m = (int)(Mp / bmt);
-    p.tiles_n = (int)(Np / kBN);
+    p.tiles_n = (int)(pl.wide ? (g.N + kBNWide - 1) / kBNWide : Np / kBN);
     p.tile_start = (int)pl.tiles;
     p.C = g.C;
     p.rsc = g.rsc;
@@ -2070,7 +2257,8 @@ gbblas_status plan_group(int mode, const gbblas_gemm_desc* d, int64_t count, TcG
     // (split-K partials are stored by the register path)
     if (!pl.pair && parts == 1 && g.csc == 1 && g.rsc >= g.N && (g.rsc % 4) == 0 &&
         (reinterpret_cast<uintptr_t>(g.C) & 15) == 0 &&
-        make_map_f32_2d(&p.c_map, g.C, (uint64_t)g.N, (uint64_t)g.M, (uint64_t)g.rsc, 32, 32, true) ==
+        make_map_f32_2d(&p.c_map, g.C, (uint64_t)g.N, (uint64_t)g.M, (uint64_t)g.rsc, 32,
+                        pl.wide ? TcCfg<kModeFp8, false, kBNWide>::kScrRows : 32, true) ==
             GBBLAS_STATUS_SUCCESS)
       p.c_tma = 1;
     pl.probs.push_back(p);
@@ -2162,8 +2350,8 @@ gbblas_status plan_group(int mode, const gbblas_gemm_desc* d, int64_t count, TcG
   pl.off_arena = pl.off_red + align256(sizeof(SplitReduce) * pl.reds.size());
   const size_t a_plane = (size_t)(pl.a_rows * pl.pitch), b_plane = (size_t)(pl.b_rows * pl.pitch);
   off = pl.off_arena + align256((size_t)pl.planes() * (a_plane + b_plane) * esize);
-  if (pl.fp8()) {  // FP8: one 4-byte scale word per row and K-block
-    const size_t kb = (size_t)(pl.kpad / 128);
+  if (pl.fp8()) {  // FP8: one 4-byte scale word per row and 512 of K
+    const size_t kb = (size_t)pl.sf_stride() / 128;
     pl.off_sa = off;
     off += align256(kb * (size_t)pl.a_rows * sizeof(uint32_t));
     pl.off_sb = off;
@@ -2223,22 +2411,22 @@ gbblas_status bind_group(TcGroupPlan& pl, char* base, cudaStream_t stream, bool 
   GB_TRY(make_map(&pl.map_a, arena_a(pl), (uint64_t)pl.a_rows, (uint64_t)pl.pitch, (uint64_t)pl.planes(), kBM,
                   pl.fp8(), pl.row_bytes()));
   GB_TRY(make_map(&pl.map_b, arena_b(pl), (uint64_t)pl.b_rows, (uint64_t)pl.pitch, (uint64_t)pl.planes(),
-                  pl.pair ? kBN / 2 : kBN, pl.fp8(), pl.row_bytes()));
+                  pl.pair ? kBN / 2 : (pl.wide ? kBNWide : kBN), pl.fp8(), pl.row_bytes()));
   return GBBLAS_STATUS_SUCCESS;
 }
 
 // Kernel attributes (dynamic shared memory) and how many CTAs (single) or
 // CTA pairs (PAIR) are resident at once on this device; set once per device,
 // before any launch or stream capture.
-template <int MODE, bool PAIR>
+template <int MODE, bool PAIR, int BN = kBN>
 int kernel_setup(DeviceCtx* c) {
-  using CF = TcCfg<MODE, PAIR>;
+  using CF = TcCfg<MODE, PAIR, BN>;
   static std::mutex mu;
   static int resident[64] = {0};
   std::lock_guard<std::mutex> lk(mu);
   int& n = resident[c->device & 63];
   if (n == 0) {
-    cudaFuncSetAttribute(gemm_split_kernel<MODE, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CF::kSmem);
+    cudaFuncSetAttribute(gemm_split_kernel<MODE, PAIR, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CF::kSmem);
     n = c->num_sms;
     if (PAIR) {
       cudaLaunchConfig_t cfg = {};
@@ -2253,7 +2441,7 @@ int kernel_setup(DeviceCtx* c) {
       cfg.attrs = at;
       cfg.numAttrs = 1;
       int k = 0;
-      n = (cudaOccupancyMaxActiveClusters(&k, gemm_split_kernel<MODE, PAIR>, &cfg) == cudaSuccess && k > 0)
+      n = (cudaOccupancyMaxActiveClusters(&k, gemm_split_kernel<MODE, PAIR, BN>, &cfg) == cudaSuccess && k > 0)
               ? k
               : c->num_sms / 2;
       cudaGetLastError();  // a refused query leaves no sticky error behind
@@ -2262,14 +2450,15 @@ int kernel_setup(DeviceCtx* c) {
   return n;
 }
 
-template <int MODE, bool PAIR>
+template <int MODE, bool PAIR, int BN = kBN>
 gbblas_status launch_gemm_kernel(DeviceCtx* c, const TcGroupPlan& pl, cudaStream_t stream, int max_ctas,
                                  int tile_begin, int tile_end, bool chained) {
-  using CF = TcCfg<MODE, PAIR>;
+  using CF = TcCfg<MODE, PAIR, BN>;
+  const int sfb_blocks = (int)(pl.b_rows / 128);
   int* err = reinterpret_cast<int*>(pl.base + kErrWordOffset);
   int* counter = reinterpret_cast<int*>(pl.base + kTileCounterOffset);
   const auto* dprobs = reinterpret_cast<const TcProblem*>(pl.base + pl.off_probs);
-  const int resident = kernel_setup<MODE, PAIR>(c);
+  const int resident = kernel_setup<MODE, PAIR, BN>(c);
   int units = (int)std::min<int64_t>(tile_end - tile_begin, resident);  // CTAs, or CTA pairs
   if (max_ctas > 0) {
     const int cap = PAIR ? std::max(1, max_ctas / 2) : max_ctas;
@@ -2279,12 +2468,12 @@ gbblas_status launch_gemm_kernel(DeviceCtx* c, const TcGroupPlan& pl, cudaStream
     const int* ga = pl.guard ? reinterpret_cast<const int*>(pl.base + pl.off_gflag) : nullptr;
     const int* gb = ga ? ga + pl.a_rows : nullptr;
     if (chained)
-      GB_CUDA_TRY(launch_after(gemm_split_kernel<MODE, false>, dim3(units), ModeTraits<MODE>::kThreads, CF::kSmem,
-                               stream, pl.map_a, pl.map_b, dprobs, pl.nprob, tile_begin, tile_end, pl.kpad, counter,
-                               err, scales_a(pl), scales_b(pl), ga, gb));
+      GB_CUDA_TRY(launch_after(gemm_split_kernel<MODE, false, BN>, dim3(units), CF::MT::kThreads, CF::kSmem,
+                               stream, pl.map_a, pl.map_b, dprobs, pl.nprob, tile_begin, tile_end, pl.sf_stride(),
+                               sfb_blocks, counter, err, scales_a(pl), scales_b(pl), ga, gb));
     else
-      gemm_split_kernel<MODE, false><<<units, ModeTraits<MODE>::kThreads, CF::kSmem, stream>>>(
-          pl.map_a, pl.map_b, dprobs, pl.nprob, tile_begin, tile_end, pl.kpad, counter, err, scales_a(pl), scales_b(pl),
+      gemm_split_kernel<MODE, false, BN><<<units, CF::MT::kThreads, CF::kSmem, stream>>>(
+          pl.map_a, pl.map_b, dprobs, pl.nprob, tile_begin, tile_end, pl.sf_stride(), sfb_blocks, counter, err, scales_a(pl), scales_b(pl),
           ga, gb);
     return check_launch("gemm_split_kernel");
   } else {
@@ -2301,8 +2490,8 @@ gbblas_status launch_gemm_kernel(DeviceCtx* c, const TcGroupPlan& pl, cudaStream
   cfg.attrs = at;
   cfg.numAttrs = 1;
   const cudaError_t e =
-      cudaLaunchKernelEx(&cfg, gemm_split_kernel<MODE, true>, pl.map_a, pl.map_b, dprobs, pl.nprob, tile_begin,
-                         tile_end, pl.kpad, counter, err, (const uint32_t*)scales_a(pl), (const uint32_t*)scales_b(pl),
+      cudaLaunchKernelEx(&cfg, gemm_split_kernel<MODE, true, BN>, pl.map_a, pl.map_b, dprobs, pl.nprob, tile_begin,
+                         tile_end, pl.sf_stride(), sfb_blocks, counter, err, (const uint32_t*)scales_a(pl), (const uint32_t*)scales_b(pl),
                          (const int*)nullptr, (const int*)nullptr);
   if (e != cudaSuccess) {
     count_launch();
@@ -2361,7 +2550,7 @@ gbblas_status launch_bound(DeviceCtx* c, const TcGroupPlan& pl, cudaStream_t str
         const RowFp8Side ra{djobs, ra_rows, reinterpret_cast<uint8_t*>(arena_a(pl)), scales_a(pl)};
         const RowFp8Side rb{djobs + pl.njobs, rb_rows, reinterpret_cast<uint8_t*>(arena_b(pl)), scales_b(pl)};
         GB_CUDA_TRY(
-            launch_chain(chained, fp8_rows_kernel, grid, stream, ra, rb, pl.njobs, pl.pitch, pl.kpad, rpc, kseg));
+            launch_chain(chained, fp8_rows_kernel, grid, stream, ra, rb, pl.njobs, pl.pitch, pl.sf_stride(), rpc, kseg));
         GB_TRY(check_launch("fp8_rows_kernel"));
       } else {
         const RowSplitSide ra{djobs, ra_rows, reinterpret_cast<__nv_bfloat16*>(arena_a(pl)),
@@ -2418,10 +2607,10 @@ gbblas_status launch_bound(DeviceCtx* c, const TcGroupPlan& pl, cudaStream_t str
     const PrepSide pb{djobs + pl.njobs, b_tiles, arena_b(pl), (int64_t)(pl.b_rows * pl.pitch), scales_b(pl), gb};
     if ((a_tiles == 0 || pl.prep_vec_a) && (b_tiles == 0 || pl.prep_vec_b))
       GB_CUDA_TRY(launch_chain(chained, prep_group_kernel<MODE, true>, dim3(prep_ctas), stream, pa, pb, pl.njobs,
-                               pl.pitch, pl.kpad));
+                               pl.pitch, pl.sf_stride()));
     else
       GB_CUDA_TRY(launch_chain(chained, prep_group_kernel<MODE, false>, dim3(prep_ctas), stream, pa, pb, pl.njobs,
-                               pl.pitch, pl.kpad));
+                               pl.pitch, pl.sf_stride()));
     GB_TRY(check_launch("prep_group_kernel"));
   }
   // the GEMM, as `slices` launches over consecutive ranges of whole waves of
@@ -2440,6 +2629,9 @@ gbblas_status launch_bound(DeviceCtx* c, const TcGroupPlan& pl, cudaStream_t str
       GB_CUDA_TRY(cudaMemsetAsync(pl.base + kTileCounterOffset, 0, sizeof(int), stream));
     if constexpr (MODE != kModeFp8 && MODE != kModeF16) {
       st = pl.pair ? launch_gemm_kernel<MODE, true>(c, pl, stream, max_ctas, tb, te, chained)
+                   : launch_gemm_kernel<MODE, false>(c, pl, stream, max_ctas, tb, te, chained && sl == 0);
+    } else if constexpr (MODE == kModeFp8) {
+      st = pl.wide ? launch_gemm_kernel<MODE, false, kBNWide>(c, pl, stream, max_ctas, tb, te, chained && sl == 0)
                    : launch_gemm_kernel<MODE, false>(c, pl, stream, max_ctas, tb, te, chained && sl == 0);
     } else {
       st = launch_gemm_kernel<MODE, false>(c, pl, stream, max_ctas, tb, te, chained && sl == 0);
@@ -2491,7 +2683,7 @@ size_t tc_arena_bytes(int mode, int64_t M, int64_t N, int64_t K) {
   const bool fp8 = mode == kModeFp8;
   const int64_t planes = fp8 ? 1 : (mode == kModeF16 ? 2 : mode), sk = fp8 ? ModeTraits<kModeFp8>::kBKe : kBK;
   const int64_t rows = round_up(M, 2 * kBM) + round_up(N, kBN), Kp = round_up(K, sk);
-  return (size_t)(rows * (Kp * (fp8 ? 1 : 2) + kPitchPadBytes) * planes + (fp8 ? rows * (Kp / 128) * 4 : 0) +
+  return (size_t)(rows * (Kp * (fp8 ? 1 : 2) + kPitchPadBytes) * planes + (fp8 ? rows * ((Kp + 511) / 512) * 4 : 0) +
                   (mode == kModeF16 ? rows * 4 : 0) + (guard ? rows * 12 : 0));
 }
 
@@ -2502,6 +2694,7 @@ void tc_prepare(DeviceCtx* c) {
   kernel_setup<2, false>(c);
   kernel_setup<3, false>(c);
   kernel_setup<kModeFp8, false>(c);
+  kernel_setup<kModeFp8, false, kBNWide>(c);
   kernel_setup<kModeF16, false>(c);
   kernel_setup<2, true>(c);
   kernel_setup<3, true>(c);
@@ -2518,9 +2711,8 @@ gbblas_status tc_group_launch(DeviceCtx* c, const TcGroupPlan* pl, cudaStream_t 
 
 gbblas_status tc_group_create(DeviceCtx* c, int mode, const gbblas_gemm_desc* descs, int64_t count,
                               TcGroupPlan** out) {
-  (void)c;
   TcGroupPlan* pl = new TcGroupPlan();
-  gbblas_status st = plan_group(mode, descs, count, *pl);
+  gbblas_status st = plan_group(c, mode, descs, count, *pl);
   if (st != GBBLAS_STATUS_SUCCESS) {
     delete pl;
     return st;
@@ -2562,7 +2754,7 @@ int* tc_group_error_word(const TcGroupPlan* pl) {
 gbblas_status launch_gemm_tc_group(DeviceCtx* c, int mode, const gbblas_gemm_desc* descs, int64_t count,
                                    cudaStream_t stream, int max_ctas, int slices) {
   TcGroupPlan pl;
-  GB_TRY(plan_group(mode, descs, count, pl));
+  GB_TRY(plan_group(c, mode, descs, count, pl));
   if (pl.nprob == 0) return GBBLAS_STATUS_SUCCESS;
   void* s = nullptr;
   GB_TRY(get_scratch(c, stream, pl.bytes, &s));
@@ -2573,7 +2765,7 @@ gbblas_status launch_gemm_tc_group(DeviceCtx* c, int mode, const gbblas_gemm_des
 gbblas_status launch_gemm_tc_opts(DeviceCtx* c, int mode, const gbblas_gemm_desc& d, const TcLaunchOpts& opt,
                                   cudaStream_t stream) {
   TcGroupPlan pl;
-  GB_TRY(plan_group(mode, &d, 1, pl, opt));
+  GB_TRY(plan_group(c, mode, &d, 1, pl, opt));
   if (pl.nprob == 0) return GBBLAS_STATUS_SUCCESS;
   void* s = nullptr;
   GB_TRY(get_scratch(c, stream, pl.bytes, &s));

@@ -123,6 +123,17 @@ __device__ __forceinline__ void fence_tensormap(const CUtensorMap* map) {
   asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
 
+// One lane of a converged warp, the same one each time.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(one));
+  return one != 0;
+}
+
 // ------------------------------------------------------------ TMEM / MMA
 // Allocate `ncols` (power of two >= 32) TMEM columns; whole warp executes.
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst_smem, uint32_t ncols) {
@@ -157,7 +168,7 @@ __device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64
 // D[tmem] (+)= (A * 2^(sa - 127)) * (B * 2^(sb - 127))^T, kind::mxf8f6f4 with
 // one UE8M0 scale per 32 elements of K (scale_vec::1X; K = 32 per MMA for
 // 8-bit operands, i.e. 32 bytes of each 128-byte swizzled row).  The scales
-// live in TMEM at sfa_tmem / sfb_tmem: for M = N = 128 the scale of A row m
+// live in TMEM at sfa_tmem / sfb_tmem: for M = 128 the scale of A row m
 // is byte (instruction descriptor's A scale id) of column m / 32 in lane m,
 // the scale of B column n is the same byte of column n / 32 in lane
 // n % 32 of each lane quarter (the layout tcgen05.cp 32x128b.warpx4 makes,
@@ -187,9 +198,8 @@ __device__ __forceinline__ uint64_t plain_rows16_desc(uint32_t smem_addr) {
 // Copy one 512-byte scale atom from shared memory into 4 TMEM columns at
 // `taddr` (tcgen05.cp 32x128b.warpx4): atom row i (16 bytes, i < 32) lands in
 // lane i of every lane quarter, its 4-byte word j in column j.  With the
-// scale of operand row r = i + 32 j in word j of atom row i (every byte of the
-// word, one per 32-K sub-block), mma_mxf8 finds each row's scale.  Ordered
-// before later tcgen05.mma of the issuing thread; tcgen05.commit tracks it.
+// scales of operand row r = i + 32 j in word j of atom row i (one byte per
+// K-block), mma_mxf8 finds each row's scale.  Ordered before later tcgen05.mma of the issuing thread; tcgen05.commit tracks it.
 __device__ __forceinline__ void tmem_cp_scales(uint32_t taddr, uint32_t atom_smem) {
   asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(plain_rows16_desc(atom_smem))
                : "memory");
@@ -215,20 +225,19 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// Shared-memory matrix descriptor for a K-major operand tile stored the way
+// Shared-memory matrix descriptor (its low word here) for a K-major operand tile stored the way
 // a 128-byte-swizzled TMA box lands: rows of 128 bytes, 8-row groups
 // 1024 bytes apart (stride byte offset), tile base 1024-byte aligned.
 // Fields: start address >> 4 (bits 0-13), leading byte offset >> 4 (16-29;
 // unused for swizzled K-major, set to 1), stride byte offset >> 4 (32-45),
 // fixed 0b001 (46-48), base offset 0 (49-51), swizzle mode 2 = 128B (61-63).
-__device__ __forceinline__ uint64_t sw128_kmajor_desc(uint32_t smem_addr) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((smem_addr >> 4) & 0x3FFFu);
-  d |= static_cast<uint64_t>(1u) << 16;
-  d |= static_cast<uint64_t>(1024u >> 4) << 32;
-  d |= static_cast<uint64_t>(1u) << 46;
-  d |= static_cast<uint64_t>(2u) << 61;
-  return d;
+__device__ __forceinline__ uint32_t sw128_kmajor_lo(uint32_t smem_addr) {
+  return ((smem_addr >> 4) & 0x3FFFu) | (1u << 16);
+}
+// From the low word (advanced by bytes / 16 within the tiles of a CTA, which
+// never carries out of the address field).
+__device__ __forceinline__ uint64_t sw128_kmajor_from(uint32_t lo) {
+  return (static_cast<uint64_t>((1024u >> 4) | (1u << 14) | (2u << 29)) << 32) | lo;
 }
 
 // The same for a 64-byte-swizzled box: rows of 64 bytes, 8-row groups 512
