@@ -537,7 +537,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   // the limit.)  Either sum is a lower bound; the full one takes a third more
   // shared-memory traffic and keeps operands whose magnitudes spread over
   // many binades, few of them large at once, off the FP64 pipes: exponents of
-  // +-10 at 1531 x 1400 x 1601, 6435 us with the quarter, 275 with all.
+  // +-10 at 1531 x 1400 x 1601, 6435 us with the quarter, 266 with all.
   // The epilogue warps find the two minima while the first stage is under way;
   // the MMA lane and the guard producer wait for them after it (the wait up
   // front took 3 us of every call).
@@ -606,78 +606,99 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      int consumed = 0, chunk_g = 0, g_used = 0;
-      bool stop = false, guard_all = false;
-      for (int w = (int)blockIdx.x; w < items && !stop; w += gridDim.x) {
-        const int nkt = dg_work<CF::kChunk>(p, w).nkt;
-        for (int kt = 0; kt < nkt; ++kt) {
-          const int s = consumed % ST, round = consumed / ST;
-          const bool chunk_first = (kt % CF::kChunk) == 0;
-          const bool chunk_last = ((kt + 1) % CF::kChunk) == 0 || kt + 1 == nkt;
-          if (chunk_first) ++chunk_g;
-          const int chunk = chunk_g - 1, b = chunk & 1;
-          if (chunk_first && chunk >= 2) {  // buffer b drained by the epilogue
-            if (!mbar_wait_bounded(&tempty[b], ((chunk >> 1) - 1) & 1, abort_flag, kWaitLimitNs)) {
-              fail();
-              stop = true;
-              break;
-            }
-            tc_fence_after();
-          }
-          if (!mbar_wait_bounded(&full[s], round & 1, abort_flag, kWaitLimitNs)) {
-            fail();
+    // The whole warp runs the loop and one elected lane issues: control flow
+    // and descriptors stay uniform, and a stage's work beside the MMAs stays
+    // short.  One lane in divergent code, building each descriptor whole, took
+    // longer than the MMAs: seven digits at 1531 x 1400 x 1601 213 -> 202 us,
+    // guarded 241 -> 223; 3000^3 1325 -> 1220, guarded 1468 -> 1329.
+    auto wait = [&](uint64_t* bar, uint32_t parity) {
+      if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+      const bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, abort_flag, kWaitLimitNs));
+      if (!ok && lane == 0) fail();
+      return ok;
+    };
+    const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+    const uint32_t lo0 = __shfl_sync(0xffffffffu, sw64_kmajor_lo(smem_u32(smem)), 0);
+    const uint32_t guard_lo = lo0 + ST * (CF::kStageBytes >> 4);
+    int s = 0;           // stage of the next K slice
+    uint32_t phase = 0;  // and its barrier's phase
+    int chunk_g = 0, g_used = 0;
+    bool stop = false, guard_all = false, first = true;
+    for (int w = (int)blockIdx.x; w < items && !stop; w += gridDim.x) {
+      const int nkt = dg_work<CF::kChunk>(p, w).nkt;
+      for (int kt = 0; kt < nkt; ++kt) {
+        const bool chunk_first = (kt % CF::kChunk) == 0;
+        const bool chunk_last = ((kt + 1) % CF::kChunk) == 0 || kt + 1 == nkt;
+        if (chunk_first) ++chunk_g;
+        const int chunk = chunk_g - 1, b = chunk & 1;
+        if (chunk_first && chunk >= 2) {  // buffer b drained by the epilogue
+          if (!wait(&tempty[b], ((chunk >> 1) - 1) & 1)) {
             stop = true;
             break;
           }
           tc_fence_after();
-          const uint32_t acc = tmem + (uint32_t)b * kBufCols;
-          const uint32_t b0 = smem_u32(b_tile(s));
-          if (G && (guard_all || chunk_first)) {
-            // guard plane x guard plane over these 32 K -> slot S
-            if (!mbar_wait_bounded(gfull, g_used & 1, abort_flag, kWaitLimitNs)) {
-              fail();
-              stop = true;
-              break;
-            }
-            tc_fence_after();
+        }
+        if (!wait(&full[s], phase)) {
+          stop = true;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t acc = tm + (uint32_t)b * kBufCols;
+        const uint32_t a0 = lo0 + (uint32_t)s * (CF::kStageBytes >> 4), b0 = a0 + (CF::kAStage >> 4);
+        if (G && (guard_all || chunk_first)) {
+          // guard plane x guard plane over these 32 K -> slot S
+          if (!wait(gfull, g_used & 1)) {
+            stop = true;
+            break;
+          }
+          tc_fence_after();
+          if (elect_one()) {
 #pragma unroll
             for (int kk = 0; kk < kBK / 16; ++kk)
-              mma_f16(acc + 32u * S, sw64_kmajor_desc(smem_u32(guard_a) + kk * 32),
-                      sw64_kmajor_desc(smem_u32(guard_b) + kk * 32), idesc_bf16_f32(kBM, kBN),
+              mma_f16(acc + 32u * S, sw64_kmajor_from(guard_lo + kk * 2),
+                      sw64_kmajor_from(guard_lo + (CF::kATile >> 4) + kk * 2), idesc_bf16_f32(kBM, kBN),
                       chunk_first && kk == 0 ? 0u : 1u);
             mma_commit(gempty);
-            ++g_used;
           }
+          __syncwarp();
+          ++g_used;
+        }
+        if (elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < kBK / 16; ++kk) {
-            const uint32_t off = kk * 32;  // 16 BF16 of K inside the swizzled 64-byte row
+            const uint32_t off = kk * 2;  // 16 BF16 of K inside the swizzled 64-byte row
 #pragma unroll
             for (int d = 0; d < S; ++d) {
               // digit d of A x digits 0..S-1-d of B (stacked: N = 32 (S - d))
               // -> groups d..S-1; the first MMA of a chunk (N = 32 S) clears all
-              mma_f16(acc + 32u * d, sw64_kmajor_desc(smem_u32(a_tile(s, d)) + off), sw64_kmajor_desc(b0 + off),
+              mma_f16(acc + 32u * d, sw64_kmajor_from(a0 + d * (CF::kATile >> 4) + off), sw64_kmajor_from(b0 + off),
                       idesc_bf16_f32(kBM, kBN * (S - d)), (chunk_first && kk == 0 && d == 0) ? 0u : 1u);
             }
           }
           mma_commit(&empty[s]);
           if (chunk_last) mma_commit(&tfull[b]);
-          if (G && consumed == 0) {  // (the first stage is sampled either way)
-            if (!mbar_wait_bounded(gready, 0, abort_flag, kWaitLimitNs)) {
-              fail();
-              stop = true;
-              break;
-            }
-            guard_all = sample_all();
+        }
+        __syncwarp();
+        if (G && first) {  // (the first stage is sampled either way)
+          if (!wait(gready, 0)) {
+            stop = true;
+            break;
           }
-          ++consumed;
+          guard_all = __shfl_sync(0xffffffffu, (int)sample_all(), 0) != 0;
+        }
+        first = false;
+        if (++s == ST) {
+          s = 0;
+          phase ^= 1;
         }
       }
-      mma_commit(accf);
-      if (*abort_flag) {
-        int never = 0;
-        (void)mbar_wait_bounded(accf, 0, &never, kWaitLimitNs);
-      }
+    }
+    __syncwarp();
+    if (elect_one()) mma_commit(accf);
+    __syncwarp();
+    if (lane == 0 && *abort_flag) {
+      int never = 0;
+      (void)mbar_wait_bounded(accf, 0, &never, kWaitLimitNs);
     }
   } else if (warp >= 2 && warp < 2 + kEpiWarps) {
     // epilogue: TMEM lane quarter q = warp % 4 (tile rows 32q..32q+31), 16

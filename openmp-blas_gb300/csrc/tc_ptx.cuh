@@ -242,14 +242,11 @@ __device__ __forceinline__ uint64_t sw128_kmajor_from(uint32_t lo) {
 
 // The same for a 64-byte-swizzled box: rows of 64 bytes, 8-row groups 512
 // bytes apart, tile base 512-byte aligned, swizzle mode 4 = 64B.
-__device__ __forceinline__ uint64_t sw64_kmajor_desc(uint32_t smem_addr) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((smem_addr >> 4) & 0x3FFFu);
-  d |= static_cast<uint64_t>(1u) << 16;
-  d |= static_cast<uint64_t>(512u >> 4) << 32;
-  d |= static_cast<uint64_t>(1u) << 46;
-  d |= static_cast<uint64_t>(4u) << 61;
-  return d;
+__device__ __forceinline__ uint32_t sw64_kmajor_lo(uint32_t smem_addr) {
+  return ((smem_addr >> 4) & 0x3FFFu) | (1u << 16);
+}
+__device__ __forceinline__ uint64_t sw64_kmajor_from(uint32_t lo) {
+  return (static_cast<uint64_t>((512u >> 4) | (1u << 14) | (4u << 29)) << 32) | lo;
 }
 
 // Instruction descriptor for kind::f16 with BF16 A/B, F32 D, both K-major.
