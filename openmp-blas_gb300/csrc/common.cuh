@@ -306,6 +306,9 @@ namespace gbblas::dev {
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// The line of p into L2.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // Streaming loads: read-only path, no L1 allocation (data is used once).
 __device__ __forceinline__ float4 ld_stream(const float4* p) {
   float4 r;

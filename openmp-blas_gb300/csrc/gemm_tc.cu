@@ -1655,6 +1655,19 @@ __global__ void __launch_bounds__(ModeTraits<MODE, BN>::kThreads, 1)
       const TcProblem& pr = probs[tw.prob];
       const int n0 = tw.n0, m0 = tw.m0 + (int)rank * kBM;  // this CTA's rows
       const int nchunks = (tw.nkt + MT::kChunk - 1) / MT::kChunk;
+      // A column-major C, updated by loads and stores: the tile's lines into L2
+      // while it is computed, as the update holds up the folding (AUTO at
+      // 5000 x 5001 x 130 128 -> 117 us, BF16x3 85 -> 71, FP8 95 -> 80; contiguous
+      // rows gained nothing)
+      if (CF::kTmaC && pr.rsc == 1 && pr.csc != 1 && pr.parts == 1) {
+        const float* at = pr.C + m0 + q * 32 + (int64_t)(n0 + col0) * pr.csc;
+        const int last = min(pr.M - m0 - q * 32, 32) - 1, cols = min(pr.N - n0 - col0, kCols);
+        if (last >= 0)
+          for (int i = lane; i < cols; i += 32) {
+            dev::prefetch_l2(at + i * pr.csc);
+            dev::prefetch_l2(at + i * pr.csc + last);
+          }
+      }
       float acc[kCols];
 #pragma unroll
       for (int j = 0; j < kCols; ++j) acc[j] = 0.f;
@@ -2214,7 +2227,13 @@ gbblas_status plan_group(DeviceCtx* c, int mode, const gbblas_gemm_desc* d, int6
       w1 += (double)round_up(d[i].M, kBM) * nk;
       w2 += (double)round_up(d[i].M, 2 * kBM) * nk;
     }
-    pl.pair = w2 <= 1.1 * w1;
+    // (a pair updates contiguous rows of C that are off the 16-byte grid a
+    // thread per row: 3970 x 3475 x 4050 314 us against 260 in single CTAs,
+    // BF16x6 514 against 467; column-major C 237 against 258)
+    const bool c_ok = std::all_of(order.begin(), order.end(), [&](int64_t i) {
+      return d[i].csc != 1 || ((d[i].rsc & 3) == 0 && (reinterpret_cast<uintptr_t>(d[i].C) & 15) == 0);
+    });
+    pl.pair = w2 <= 1.1 * w1 && c_ok;
   }
   pl.wide = pl.fp8() && opt.split <= 1 && fp8_wide(d, order, c->num_sms);
   const int64_t sk = pl.slice_k();
