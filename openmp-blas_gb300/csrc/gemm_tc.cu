@@ -272,7 +272,9 @@ struct PrepTile {
 };
 
 // For every job, writes its rows_pad x k_pad operand into the arena (row pitch
-// `pitch` elements), zero outside rows x K:
+// `pitch` elements), zero outside rows x K.  (Split-BF16 leaves the padding
+// rows up to the tile's 128 as they are: their outputs do not exist.  A batch
+// of 512 GEMMs of 32 .. 2048 a side wrote 8 % more for them, 1061 -> 1046 us.)
 //  * split-BF16 (MODE 2, 3): MODE pieces p0 = bf16_rn(a), p1 = bf16_rn(a - p0),
 //    ... (piece p at out + p * piece_stride);
 //  * FP8: E4M3 bytes and one power-of-two scale per (row, 128-K block).
@@ -606,6 +608,8 @@ __global__ void __launch_bounds__(256, VEC ? 1 : 4) prep_group_kernel(PrepSide s
   const SplitJob& j = jobs[sjob];
   const int local = t - j.tile_start;
   const int64_t r0 = (int64_t)(local / j.tiles_k) * TR, k0 = (int64_t)(local % j.tiles_k) * TK;
+  constexpr bool kLeavePadding = MODE == 2 || MODE == 3;
+  if (kLeavePadding && r0 >= j.rows) return;
   const bool full = r0 + TR <= j.rows && k0 + TK <= j.K;
   const bool al16 = (reinterpret_cast<uintptr_t>(j.src) & 15) == 0;
   // 128-bit loads along the contiguous dimension: on interior tiles, and on
@@ -732,6 +736,7 @@ __global__ void __launch_bounds__(256, VEC ? 1 : 4) prep_group_kernel(PrepSide s
       const int r = warp * 8 + 2 * i + (lane >> 4), kk = (lane & 15) * 4;
       float4 v = *reinterpret_cast<const float4*>(&tile[prep_slot<LD>(r, kk)]);
       const int64_t base = (j.dst_row + r0 + r) * pitch + k0 + kk;
+      if (kLeavePadding && r0 + r >= j.rows) break;
 #pragma unroll
       for (int p = 0; p < MODE; ++p) {
         const __nv_bfloat162 h01 = __floats2bfloat162_rn(v.x, v.y);
@@ -758,7 +763,7 @@ __global__ void __launch_bounds__(256, VEC ? 1 : 4) prep_group_kernel(PrepSide s
 // `kblk` (kColScaleK) of K; each thread keeps 8 K's loads in flight and its
 // rows' extremes in registers, then atomicMax-es them into e[R] and emin[R]
 // once.  Bound by HBM.  A 4050 x 3475 row-major B: 44 us through
-// f16_scale_kernel's scalar tiles, see the launch rule for this kernel's.
+// f16_scale_kernel's scalar tiles, 22 here.
 // Condition (host side, per operand): every job has rows contiguous.
 constexpr int kColScaleK = 128;
 
@@ -838,8 +843,8 @@ __global__ void __launch_bounds__(256, 4) f16_col_scale_kernel(ScaleSide side_a,
 // column-major B), any alignment: a warp per arena row at a time, each lane 4
 // consecutive K per step (load_row4; four steps' loads in flight), its P
 // pieces written as 8-byte stores - the same pieces as prep_group_kernel,
-// without the shared-memory tile or its barriers.  Padding rows and the K
-// padding get zeros.
+// without the shared-memory tile or its barriers.  The K padding gets zeros, a
+// padding row nothing.
 struct RowSplitSide {
   const SplitJob* jobs;
   int rows;  // arena rows prepared here (0: this operand takes the tile kernel)
@@ -886,8 +891,9 @@ __global__ void __launch_bounds__(256) split_rows_kernel(RowSplitSide side_a, Ro
   const int64_t R = R0 + (threadIdx.x >> 5) * per_warp + rr;  // arena row
   const int64_t local = R - j.dst_row;
   const int64_t kp = (int64_t)j.tiles_k * PrepTile<P>::TK;  // the job's padded K
-  const int64_t K = local < j.rows ? j.K : 0;                // padding rows: all zeros
-  const float* __restrict__ src = j.src + (local < j.rows ? local : 0) * j.rs;
+  if (local >= j.rows) break;  // padding rows
+  const int64_t K = j.K;
+  const float* __restrict__ src = j.src + local * j.rs;
   const int w = row_width(src);
   __nv_bfloat16* __restrict__ dst = sd.out + R * pitch;
   const int64_t kbeg = (int64_t)blockIdx.y * kseg, kend = min(kp, kbeg + kseg);
@@ -926,7 +932,7 @@ __global__ void __launch_bounds__(256) split_rows_kernel(RowSplitSide side_a, Ro
 // arena row, a 128-K block per step, four steps' loads in flight - the same
 // bytes and scales as prep_group_kernel, without the shared-memory tile.
 // Grid as split_rows_kernel's.  Bound by HBM (4 B read, 1 written per element):
-// of an 8192^2 pair's 192 us by tiles A's half took 90, see launch_bound.
+// 8192^2 in 56 us, 90 by tiles.
 struct RowFp8Side {
   const SplitJob* jobs;
   int rows;  // arena rows prepared here (0: this operand takes the tile kernel)
