@@ -760,12 +760,18 @@ __global__ void __launch_bounds__(256, VEC ? 1 : 4) prep_group_kernel(PrepSide s
 // a column reduction.  A CTA covers 1024 consecutive rows (4 per thread: one
 // float4 where every column of the job starts on a 16-byte boundary and the
 // row count is a multiple of 4, else rows tid, tid + 256, ... one by one) and
-// `kblk` (kColScaleK) of K; each thread keeps 8 K's loads in flight and its
+// `kblk` (col_scale_k) of K; each thread keeps 8 K's loads in flight and its
 // rows' extremes in registers, then atomicMax-es them into e[R] and emin[R]
 // once.  Bound by HBM.  A 4050 x 3475 row-major B: 44 us through
 // f16_scale_kernel's scalar tiles, 22 here.
 // Condition (host side, per operand): every job has rows contiguous.
-constexpr int kColScaleK = 128;
+// K per CTA where few CTAs take the whole.  A thread's eight loads in flight need three or four CTAs on an SM
+// to stream, but each CTA ends in an atomic per row, and past some hundred on
+// one row they queue.  AUTO calls with 128 / 64 / 32 / 16 of K per CTA, us:
+// 2048^3 87 / 78 / 74 / 77, 3970 x 3475 x 4050 329 / 323 / 319 / 319,
+// 64 x 8192 x 500 39 / 33 / 30 / 30, 32 x 4096^2 72 / 67 / 69 / 80,
+// 512^2 x 8192 53 / 48 / 50 / 59, 8192^3 the same.
+int col_scale_k(int64_t longest_k) { return longest_k <= 4096 ? 32 : (longest_k <= 8192 ? 64 : 128); }
 
 __global__ void __launch_bounds__(256, 4) f16_col_scale_kernel(ScaleSide side_a, ScaleSide side_b, int njobs,
                                                                int kblk) {
@@ -2156,7 +2162,7 @@ struct TcGroupPlan {
   bool col_scale_a = false, col_scale_b = false;  // FP16 split: exponents by f16_col_scale_kernel
   bool row_split_a = false, row_split_b = false;  // BF16 split, FP8: operand prepared row by row
   bool prep_vec_a = false, prep_vec_b = false;    // prep_group_kernel: 128-bit loads for every job of the operand
-  int a_col_ctas = 0, b_col_ctas = 0, col_kblk = 128;
+  int a_col_ctas = 0, b_col_ctas = 0, col_kblk = 32;
   size_t off_gmin = 0, off_gflag = 0, off_glist = 0;  // guard arrays: A rows then B rows each
   size_t off_init_end = 0;  // the launch clears [kTileCounterOffset, off_init_end)
   std::vector<char> tables;  // host image of [off_probs, off_arena), copied with one memcpy
@@ -2341,9 +2347,13 @@ gbblas_status plan_group(DeviceCtx* c, int mode, const gbblas_gemm_desc* d, int6
     };
     pl.col_scale_a = !pl.row_prep_a && std::all_of(pl.ajobs.begin(), pl.ajobs.end(), col_ok);
     pl.col_scale_b = !pl.row_prep_b && std::all_of(pl.bjobs.begin(), pl.bjobs.end(), col_ok);
-    // (shorter K ranges for more CTAs measured slower: 28.6 against 24.5 us
-    // for a 4096^2 operand with 16 instead of 128 of K per CTA)
-    pl.col_kblk = kColScaleK;
+    // (128 of K per CTA where that fills the SMs: 512 GEMMs of 32 .. 2048 a
+    // side 2279 us, 2291 with shorter ranges)
+    auto col_ctas = [&](int kblk) {
+      pl.col_kblk = kblk;
+      return (pl.col_scale_a ? number(pl.ajobs, kblk) : 0) + (pl.col_scale_b ? number(pl.bjobs, kblk) : 0);
+    };
+    if (col_ctas(128) < 4 * (int64_t)c->num_sms) col_ctas(col_scale_k(pl.kpad));
     const int64_t na = pl.col_scale_a ? number(pl.ajobs, pl.col_kblk) : 0,
                   nb = pl.col_scale_b ? number(pl.bjobs, pl.col_kblk) : 0;
     if (na + nb >= (1ll << 31)) pl.col_scale_a = pl.col_scale_b = false;
