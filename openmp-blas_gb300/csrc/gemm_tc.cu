@@ -1819,43 +1819,42 @@ __global__ void __launch_bounds__(ModeTraits<MODE, BN>::kThreads, 1)
       float* Cd = add ? pr.C : pr.ws + (int64_t)tw.part * pr.ws_plane;
       const int64_t rsc = add ? pr.rsc : pr.ws_rs, csc = add ? pr.csc : pr.ws_cs;
       const int row0 = m0 + q * 32, cn = n0 + col0;
-      if constexpr (CF::kTmaC) {
+      if constexpr (CF::kTmaC && !MT::wide) {  // (wide tiles: never, see plan_group)
         if (csc == 1) {
           // contiguous C rows of any alignment: the 32 x 32 blocks go through
           // shared memory (swizzled as for the TMA update) and the warp
           // updates one row's 32 columns, 128 bytes, per access
           const uint32_t skip_rows = __ballot_sync(0xffffffffu, skip_row);
-          constexpr int kRows = CF::kScrRows;
-          float* scr = epi_scratch + (warp - 2) * kRows * 32;
+          float* scr = epi_scratch + (warp - 2) * 1024;
 #pragma unroll
           for (int cb = 0; cb < kCols; cb += 32) {
-            auto stage_rows = [&](int r0) {  // rows r0 .. r0 + kRows - 1 of the block into scr
-              __syncwarp();
-              if (kRows == 32 || lane / kRows == r0 / kRows) {
+            __syncwarp();
 #pragma unroll
-                for (int c = 0; c < 8; ++c)
-                  *reinterpret_cast<float4*>(scr + (lane % kRows) * 32 + ((c ^ (lane & 7)) * 4)) =
-                      make_float4(acc[cb + 4 * c], acc[cb + 4 * c + 1], acc[cb + 4 * c + 2], acc[cb + 4 * c + 3]);
-              }
-              __syncwarp();
-            };
-            if (kRows == 32) stage_rows(0);
+            for (int c = 0; c < 8; ++c)
+              *reinterpret_cast<float4*>(scr + lane * 32 + ((c ^ (lane & 7)) * 4)) =
+                  make_float4(acc[cb + 4 * c], acc[cb + 4 * c + 1], acc[cb + 4 * c + 2], acc[cb + 4 * c + 3]);
+            __syncwarp();
             const int col = cn + cb + lane;
             // rows r < rows of the block exist for this lane's column
             const int rows = col < pr.N && !(MT::f16 && ((skip_cols >> (cb + lane)) & 1)) ? min(pr.M - row0, 32) : 0;
             float* cp = Cd + (int64_t)row0 * rsc + col;
 #pragma unroll
             for (int r0 = 0; r0 < 32; r0 += 16) {
-              if (kRows == 16) stage_rows(r0);
               float old[16];
               const float* lp = cp;
 #pragma unroll
               for (int r = 0; r < 16; ++r, lp += rsc) old[r] = (add && r0 + r < rows) ? *lp : 0.f;
+              // all 16 out of shared memory before the first store, since the
+              // compiler keeps loads and stores in order (8191 x 8191 x 512: FP8
+              // 321 -> 274 us, BF16x3 207 -> 197)
 #pragma unroll
-              for (int r = 0; r < 16; ++r, cp += rsc) {
-                const float v = scr[((r0 + r) % kRows) * 32 + (((lane >> 2) ^ (r & 7)) * 4) + (lane & 3)];
-                if (r0 + r < rows && !((skip_rows >> (r0 + r)) & 1)) *cp = add ? old[r] + v : v;
+              for (int r = 0; r < 16; ++r) {
+                const float v = scr[(r0 + r) * 32 + (((lane >> 2) ^ (r & 7)) * 4) + (lane & 3)];
+                old[r] = add ? old[r] + v : v;
               }
+#pragma unroll
+              for (int r = 0; r < 16; ++r, cp += rsc)
+                if (r0 + r < rows && !((skip_rows >> (r0 + r)) & 1)) *cp = old[r];
             }
           }
           continue;
@@ -2232,6 +2231,10 @@ gbblas_status plan_group(DeviceCtx* c, int mode, const gbblas_gemm_desc* d, int6
   bool want_pair = opt.pair == 1;
   if (opt.pair < 0)
     if (const char* e = std::getenv("GBBLAS_TC_PAIR"); e && e[0] == '1') want_pair = true;
+  // no contiguous rows of C off the 16-byte grid
+  const bool c_ok = std::all_of(order.begin(), order.end(), [&](int64_t i) {
+    return d[i].csc != 1 || ((d[i].rsc & 3) == 0 && (reinterpret_cast<uintptr_t>(d[i].C) & 15) == 0);
+  });
   if (want_pair && mode != kModeFp8 && mode != kModeF16) {
     double w1 = 0, w2 = 0;
     for (int64_t i : order) {
@@ -2242,12 +2245,11 @@ gbblas_status plan_group(DeviceCtx* c, int mode, const gbblas_gemm_desc* d, int6
     // (a pair updates contiguous rows of C that are off the 16-byte grid a
     // thread per row: 3970 x 3475 x 4050 314 us against 260 in single CTAs,
     // BF16x6 514 against 467; column-major C 237 against 258)
-    const bool c_ok = std::all_of(order.begin(), order.end(), [&](int64_t i) {
-      return d[i].csc != 1 || ((d[i].rsc & 3) == 0 && (reinterpret_cast<uintptr_t>(d[i].C) & 15) == 0);
-    });
     pl.pair = w2 <= 1.1 * w1 && c_ok;
   }
-  pl.wide = pl.fp8() && opt.split <= 1 && fp8_wide(d, order, c->num_sms);
+  // (wide tiles would update such rows in halves of a block, with registers
+  // spilled: 3970 x 3475 x 4050 164 us against 142, 8191 x 8191 x 512 390 against 273)
+  pl.wide = pl.fp8() && opt.split <= 1 && c_ok && fp8_wide(d, order, c->num_sms);
   const int64_t sk = pl.slice_k();
   const int64_t bmt = pl.pair ? 2 * kBM : kBM;  // output tile rows
   pl.njobs = (int)order.size();
