@@ -462,8 +462,14 @@ gbblas_status launch_gemv_rows(DeviceCtx* c, int64_t rows, int64_t cols, const T
   const int64_t ctas = cdiv(groups, kWarps >> lwc);
   // split the columns while the CTAs do not fill the SMs and each warp has
   // more than 8 vectors a lane
+  // (up to 60 MB only where they are fewer than two an SM, 1.5 for double: the
+  // finish of a split in two costs more than the idle warps do.  Split and not,
+  // us, f32 312 x 23256 17.4 and 14.3, 600 x 23256 21.2 and 18.4, 312 x 200001
+  // 57 and 64; f64 312 x 8192 17.2 and 14.4, 256 x 16000 22.5 and 18.4, 312 x
+  // 50000 42 and 47)
   int64_t ksplit = 1;
-  if (ctas * kWarps < 32 * sms) ksplit = std::min(cdiv(48 * sms, ctas * kWarps), nv >> (lwc + 8));
+  const int64_t warps_enough = (double)rows * cols * sizeof(T) > 60.0e6 ? 32 : (sizeof(T) == 8 ? 12 : 16);
+  if (ctas * kWarps < warps_enough * sms) ksplit = std::min(cdiv(48 * sms, ctas * kWarps), nv >> (lwc + 8));
   ksplit = std::max<int64_t>(1, std::min<int64_t>(ksplit, 65535));
   const int64_t vps = cdiv(cdiv(nv, ksplit), 32) * 32;
   if (vps > 0) ksplit = std::max<int64_t>(1, cdiv(nv, vps));
