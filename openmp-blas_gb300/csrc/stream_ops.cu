@@ -319,17 +319,20 @@ template <typename T>
 gbblas_status launch_transpose(DeviceCtx* c, int64_t M, int64_t N, const T* A, int64_t rsa, int64_t csa, T* C,
                                int64_t rsc, int64_t csc, cudaStream_t s) {
   if (M == 0 || N == 0) return GBBLAS_STATUS_SUCCESS;
-  // Large matrices whose written rows do not all start on a line: strips, 12
-  // CTAs per SM.  From 200 MB moved (below it the writes of neighbouring tiles
+  // Large matrices whose written rows do not all start on a multiple of four
+  // elements (where they do, few sectors are written in two parts: by tiles and
+  // in strips, us, f32 9877 rows of 6901 116 and 107.5, of 6902 113 and 107, of
+  // 6900 104 and 107, of 6904 95 and 107; f64 6901 193 and 177, 6902 191 and
+  // 177, 6900 175 and 176): strips, 12 CTAs per SM.  From 200 MB moved (below it the writes of neighbouring tiles
   // meet in L2 before they leave it: 4501 x 4499 f32, 162 MB, 33.5 us by tiles
   // and 35.0 in strips; 6001 x 5003, 240 MB, 51.2 and 47.4).
   const bool c_rows = csc == 1;
   const int64_t ldc = c_rows ? rsc : csc, ra = c_rows ? rsa : csa, ca = c_rows ? csa : rsa;
   const int64_t m = c_rows ? M : N, n = c_rows ? N : M;  // C has n contiguous rows of m
-  constexpr int TJ = TransCfg<T>::kTJ, LINE = TransCfg<T>::kLine;
+  constexpr int TJ = TransCfg<T>::kTJ;
   const int64_t jblocks = (n + TJ - 1) / TJ, chunks = (m + kCI - 1) / kCI;
   if ((c_rows || rsc == 1) && (ra == 1 || ca == 1) && 2.0 * (double)M * (double)N * sizeof(T) >= 200e6 &&
-      (ldc % LINE != 0 || (reinterpret_cast<uintptr_t>(C) & 127) != 0) && jblocks * chunks <= 0x7fffffff / kCI) {
+      (ldc % 4 != 0 || reinterpret_cast<uintptr_t>(C) % (4 * sizeof(T)) != 0) && jblocks * chunks <= 0x7fffffff / kCI) {
     const int64_t strips = std::min(chunks, std::max<int64_t>(1, (12 * (int64_t)c->num_sms + jblocks - 1) / jblocks));
     const int64_t strip = (chunks + strips - 1) / strips;
     const unsigned lgrid = (unsigned)(jblocks * ((chunks + strip - 1) / strip));
