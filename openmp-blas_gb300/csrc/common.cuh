@@ -370,8 +370,12 @@ __device__ __forceinline__ unsigned cluster_rank() {
 }
 // Barrier over every thread of every CTA of the cluster (release / acquire:
 // shared-memory writes before it are visible to the cluster's CTAs after).
-// Each thread must reach it: kernels that use it exit no thread early.
+// Each thread must reach it: kernels that use it exit no thread early.  The
+// .aligned form is defined only for a converged warp, and nothing else brings
+// the lanes of a divergent loop or branch before it (ragged columns, a block's
+// one summing thread) together again.
 __device__ __forceinline__ void cluster_sync() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // Load the object at shared address `p` of this CTA as it sits in the shared

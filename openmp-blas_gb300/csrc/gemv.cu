@@ -203,14 +203,12 @@ __global__ void __launch_bounds__(kRowsThreads, R == 4 ? 3 : 4)
       partials[(int64_t)blockIdx.y * rows + r] = sum;
   }
   if constexpr (CL) {
-    __syncwarp();
     dev::cluster_sync();
     if (blockIdx.y == 0 && r < rows) {  // rank 0 of the cluster: splits in order
       T s = T(0);
       for (unsigned k = 0; k < gridDim.y; ++k) s += dev::dsmem_ld(&split_part[threadIdx.x], k);
       y[r] = accumulate ? y[r] + s : s;
     }
-    __syncwarp();
     dev::cluster_sync();  // the other splits stay resident until rank 0 has read them
   }
 }
@@ -364,7 +362,6 @@ __global__ void __launch_bounds__(256, 3)
       partials[(int64_t)blockIdx.y * rows + r] = sum;
   }
   if constexpr (CL) {
-    __syncwarp();  // lanes past the last row rejoin before the aligned cluster barrier
     dev::cluster_sync();
     if (blockIdx.y == 0) {  // rank 0 of the cluster: splits in order
       for (int t = threadIdx.x; t < rw * CF::kRows && cta_rb + t < rows; t += kRowsThreads) {
@@ -373,7 +370,6 @@ __global__ void __launch_bounds__(256, 3)
         y[cta_rb + t] = accumulate ? y[cta_rb + t] + s : s;
       }
     }
-    __syncwarp();
     dev::cluster_sync();  // the other splits stay resident until rank 0 has read them
   }
 }

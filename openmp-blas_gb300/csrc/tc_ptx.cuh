@@ -283,8 +283,9 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
-// Every thread of both CTAs of the cluster.
+// Every thread of both CTAs of the cluster (each warp converged for it).
 __device__ __forceinline__ void cluster_sync_all() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // Shared-memory address of the same object in CTA `rank` of the cluster.
