@@ -281,6 +281,10 @@ namespace gbblas {
 // (about 1 us) off a chain of short kernels.  Only for a kernel whose every
 // CTA calls dev::grid_wait() before it touches memory, and only directly
 // behind a kernel of this library that does the same or was launched plainly.
+// Such a kernel is resident while the ones before it still write, so what they
+// write (tables, exponents, flags, lists, counts, partials) is not constant for
+// as long as it runs: it takes those by plain pointers (no `const __restrict__`)
+// and plain or __ldcg loads.  The read-only path is for the caller's operands.
 template <typename... P, typename... A>
 cudaError_t launch_after(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream, A&&... args) {
   cudaLaunchConfig_t cfg = {};

@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(256) digits_kernel(const DgOperand oa, const D
   const int blk = is_a ? (int)blockIdx.x : (int)blockIdx.x - oa.blocks;
   const double* __restrict__ src = o.src;
   const int64_t rows = o.rows, K = o.K, rs = o.rs, cs = o.cs, plane_stride = o.plane_stride, pitch = o.pitch;
-  const int* __restrict__ e_row = o.e;
+  const int* e_row = o.e;
   unsigned* __restrict__ gsum_row = o.gsum;
   __nv_bfloat16* __restrict__ out = o.out;
   const int tid = threadIdx.x;

@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(256) f16_scale_kernel(ScaleSide side_a, ScaleS
   __shared__ int sjob;
   const bool on_b = (int)blockIdx.x >= side_a.tiles;
   const ScaleSide sd = on_b ? side_b : side_a;
-  const SplitJob* __restrict__ jobs = sd.jobs;
+  const SplitJob* jobs = sd.jobs;
   const int t = (int)blockIdx.x - (on_b ? side_a.tiles : 0), tid = threadIdx.x;
   if (tid == 0) {
     int lo = 0, hi = njobs - 1;
@@ -586,7 +586,7 @@ __global__ void __launch_bounds__(256, VEC ? 1 : 4) prep_group_kernel(PrepSide s
   __shared__ int sjob;
   const bool on_b = (int)blockIdx.x >= side_a.tiles;
   const PrepSide sd = on_b ? side_b : side_a;
-  const SplitJob* __restrict__ jobs = sd.jobs;
+  const SplitJob* jobs = sd.jobs;
   void* __restrict__ out = sd.out;
   const int64_t piece_stride = sd.piece_stride;
   uint32_t* __restrict__ scales = sd.scales;
@@ -1144,7 +1144,7 @@ __global__ void __launch_bounds__(256) f16_row_prep_kernel(RowPrepSide side_a, R
 }
 
 // ---------------------------------------------------------------- GEMM
-__device__ __forceinline__ int find_problem(const TcProblem* __restrict__ probs, int nprob, int t) {
+__device__ __forceinline__ int find_problem(const TcProblem* probs, int nprob, int t) {
   int lo = 0, hi = nprob - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
@@ -1216,10 +1216,9 @@ __device__ __forceinline__ TileWork tile_work(const TcProblem& p, int t) {
 template <int MODE, bool PAIR, int BN>
 __global__ void __launch_bounds__(ModeTraits<MODE, BN>::kThreads, 1)
     gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
-                      const TcProblem* __restrict__ probs, int nprob, int tile_begin, int total_tiles,
+                      const TcProblem* probs, int nprob, int tile_begin, int total_tiles,
                       int64_t sf_stride, int sfb_blocks, int* __restrict__ tile_counter, int* __restrict__ err,
-                      const uint32_t* __restrict__ sa, const uint32_t* __restrict__ sb,
-                      const int* __restrict__ guard_a, const int* __restrict__ guard_b) {
+                      const uint32_t* sa, const uint32_t* sb, const int* guard_a, const int* guard_b) {
   using MT = ModeTraits<MODE, BN>;
   using CF = TcCfg<MODE, PAIR, BN>;
   constexpr int P = MT::P;
@@ -1758,7 +1757,7 @@ __global__ void __launch_bounds__(ModeTraits<MODE, BN>::kThreads, 1)
           skip_row = guard_a[(int64_t)pr.a_row + m0 + q * 32 + lane] != 0;
 #pragma unroll
           for (int c = 0; c < kCols; ++c)
-            if (__ldg(guard_b + (int64_t)pr.b_row + n0 + col0 + c)) skip_cols |= uint64_t(1) << c;
+            if (guard_b[(int64_t)pr.b_row + n0 + col0 + c]) skip_cols |= uint64_t(1) << c;
           // a split-K partial takes -0.0 there, which leaves C as it was when
           // the parts are added into it
           if (pr.parts > 1 && (skip_row || skip_cols)) {
@@ -1961,12 +1960,9 @@ __global__ void __launch_bounds__(ModeTraits<MODE, BN>::kThreads, 1)
 // (K / 32 + 5) eps32 (|A||B|)_ij, order fixed: the same bits on every run.
 // CTAs take the listed rows in turn; with empty lists every CTA returns at
 // once.  jobs: the A jobs then the B^T jobs of a group (problem i = job i).
-__global__ void __launch_bounds__(256) f16_guard_fixup_kernel(const SplitJob* __restrict__ jobs, int njobs,
-                                                              const TcProblem* __restrict__ probs,
-                                                              const int* __restrict__ list_a,
-                                                              const int* __restrict__ list_b,
-                                                              const int* __restrict__ counts,
-                                                              const int* __restrict__ flags_a) {
+__global__ void __launch_bounds__(256) f16_guard_fixup_kernel(const SplitJob* jobs, int njobs, const TcProblem* probs,
+                                                              const int* list_a, const int* list_b, const int* counts,
+                                                              const int* flags_a) {
   dev::grid_release();
   dev::grid_wait();
   const int na = counts[0], nb = counts[1];
@@ -2016,7 +2012,7 @@ __global__ void __launch_bounds__(256) f16_guard_fixup_kernel(const SplitJob* __
 // Split-K: C += part[0] + part[1] + ... (in that order) for every element of
 // every split problem; blockIdx.y = problem, warps walk its rows' 32-column
 // blocks.  Bound by the L2 the partials were just written to.
-__global__ void __launch_bounds__(256) splitk_reduce_kernel(const SplitReduce* __restrict__ jobs) {
+__global__ void __launch_bounds__(256) splitk_reduce_kernel(const SplitReduce* jobs) {
   dev::grid_release();
   dev::grid_wait();
   const SplitReduce j = jobs[blockIdx.y];

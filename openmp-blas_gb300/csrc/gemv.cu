@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(kRowsThreads, R == 4 ? 3 : 4)
 __device__ __forceinline__ int finish_group(int ksplit) { return ksplit > 16 ? 8 : 1; }
 
 template <typename T>
-__global__ void __launch_bounds__(256) finish_splits_kernel(int64_t rows, int ksplit, const T* __restrict__ partials,
+__global__ void __launch_bounds__(256) finish_splits_kernel(int64_t rows, int ksplit, const T* partials,
                                                             T* __restrict__ y, bool accumulate) {
   dev::grid_wait();
   __shared__ T part[256];

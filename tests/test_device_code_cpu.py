@@ -36,3 +36,39 @@ def test_aligned_cluster_barriers_follow_a_warp_barrier():
             assert "__syncwarp();" in body, f"{name}: {body}"
             found += 1
     assert found == 2
+
+
+def kernels(text):
+    """(name, parameters, body) of each __global__ function."""
+    for m in re.finditer(r"__global__\s+void\s+(?:__launch_bounds__\([^)]*(?:\([^)]*\)[^)]*)*\)\s*)?(\w+)\s*\(", text):
+        depth, i = 1, m.end()
+        while depth:
+            depth += {"(": 1, ")": -1}.get(text[i], 0)
+            i += 1
+        yield m.group(1), text[m.end():i - 1], block(text, i)
+
+
+def test_chained_kernels_take_the_chains_results_by_plain_loads():
+    """A kernel launched behind the one before it (grid_wait) is resident while
+    that one writes: what it reads of it must not be promised constant for the
+    kernel's lifetime (const __restrict__, __ldg, ld_stream), or the loads may
+    be served from the read-only path or moved ahead of the wait.  The caller's
+    operands, reached through a job's or an operand's `src`, may be."""
+    found = []
+    for name, text in sources().items():
+        assert not re.search(r"\b(TcProblem|SplitJob|SplitReduce)\s*\*\s*__restrict__", text), name
+        for kernel, params, body in kernels(text):
+            if "grid_wait()" not in body:
+                continue
+            found.append(kernel)
+            assert not re.search(r"const\s+[\w:]+\s*\*\s*__restrict__", params), f"{kernel}({params})"
+            operands = {"j.src", "src"}
+            for local, value in re.findall(r"const\s+[\w:]+\s*\*\s*__restrict__\s+(\w+)\s*=\s*([\w.]+)", body):
+                assert value in ("j.src", "o.src"), f"{kernel}: {local} = {value}"
+                operands.add(local)
+            for local, value in re.findall(r"const\s+(?:float|double)\s*\*\s*(\w+)\s*=\s*([\w.]+)", body):
+                if value in operands:
+                    operands.add(local)
+            for arg in re.findall(r"(?:__ldg|ld_stream)\(\s*(?:reinterpret_cast<[^>]*>\(\s*)?\(?\s*([\w.]+)", body):
+                assert arg in operands, f"{kernel}: read-only load of {arg}"
+    assert len(found) >= 12 and {"gemm_split_kernel", "dgemm_digits_kernel", "finish_splits_kernel"} <= set(found)
