@@ -696,10 +696,6 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncwarp();
     if (elect_one()) mma_commit(accf);
     __syncwarp();
-    if (lane == 0 && *abort_flag) {
-      int never = 0;
-      (void)mbar_wait_bounded(accf, 0, &never, kWaitLimitNs);
-    }
   } else if (warp >= 2 && warp < 2 + kEpiWarps) {
     // epilogue: TMEM lane quarter q = warp % 4 (tile rows 32q..32q+31), 16
     // columns (half h) of each group's 32
@@ -876,13 +872,17 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 
   // ---- teardown: drain in-flight copies if the pipeline stopped early, make
-  // sure every MMA finished (warp 1 waited on accf after an abort), free TMEM
+  // sure every MMA finished, free TMEM.  Any role may be the one that gives
+  // up, also after the others have done their part, so the flag is looked at
+  // once all of them have stopped.
+  __syncthreads();
   if (warp == 0 && lane == 0 && *abort_flag) {
     int never = 0;
+    (void)mbar_wait_bounded(accf, 0, &never, kWaitLimitNs);
     const int from = issued > ST ? issued - ST : 0;
     for (int k = from; k < issued; ++k) (void)mbar_wait_bounded(&full[k % ST], (k / ST) & 1, &never, kWaitLimitNs / 2);
-    // copies of B the A producer did not match complete on no barrier it
-    // waits for: give them 100 us to land
+    // copies of B the A producer did not match, and the guard's, complete on
+    // no barrier it waits for: give them 100 us to land
     const uint64_t t0 = global_timer_ns();
     while (global_timer_ns() - t0 < 100000ull) {
     }

@@ -72,3 +72,14 @@ def test_chained_kernels_take_the_chains_results_by_plain_loads():
             for arg in re.findall(r"(?:__ldg|ld_stream)\(\s*(?:reinterpret_cast<[^>]*>\(\s*)?\(?\s*([\w.]+)", body):
                 assert arg in operands, f"{kernel}: read-only load of {arg}"
     assert len(found) >= 12 and {"gemm_split_kernel", "dgemm_digits_kernel", "finish_splits_kernel"} <= set(found)
+
+
+def test_digit_gemm_looks_at_the_abort_flag_behind_a_barrier():
+    """A role that gives up after the others have finished must still find its
+    copies and MMAs waited for before the CTA leaves: the teardown reads the
+    flag after a barrier of the whole CTA."""
+    body = dict((k, b) for k, _, b in kernels(sources()["gemm_f64_tc.cu"]))["dgemm_digits_kernel"]
+    checks = [m.start() for m in re.finditer(r"if \([^)]*lane == 0 && \*abort_flag\)", body)]
+    assert len(checks) == 1
+    stores = body.rindex("crow[")  # the epilogue's last store into C
+    assert stores < body.index("__syncthreads();", stores) < checks[0]
