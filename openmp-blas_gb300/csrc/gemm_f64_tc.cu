@@ -36,9 +36,8 @@
 //
 // The guard (7 digits, G = 1; what AUTO runs): one more plane per operand,
 // P = max(|D_0| - 1, 0) <= |x| 2^7, whose products summed over the first
-// 32 of K of every 128-K chunk (over all of K where that sample is too thin)
-// bound sum_k |a_ik||b_kj| from below.  An
-// epilogue warp keeps its 32 x 16 block only where that bound makes the
+// 32 of K of every 128-K chunk (over all of K in tiles where that sample is
+// too thin) bound sum_k |a_ik||b_kj| from below.  An epilogue warp keeps its 32 x 16 block only where that bound makes the
 // digit error smaller than the FP64 pipes' bound; other blocks leave C
 // alone and are recomputed on the FP64 pipes by dgemm_fixup_kernel.
 //
@@ -125,7 +124,7 @@ struct DgCfg {
   static_assert(kStages >= 2, "need a double-buffered stage ring");
   static_assert((uint64_t)S * kChunk * kBK * 16384 < (1u << 24), "chunk sums must stay exact in FP32");
   static_assert(kStageBytes % 1024 == 0, "stages stay 1024-byte aligned");
-  static_assert((2 * 4 + 2 * 2 + 2 + 1) * 8 + 8 + 8 <= kBarBytes, "barrier area too small");
+  static_assert((2 * 4 + 2 * 2 + 2 + 1) * 8 + 8 <= kBarBytes, "barrier area too small");
 };
 
 // One GEMM (device-side view).
@@ -160,6 +159,9 @@ struct DgProblem {
 // inside the FP64 pipes' bound 2 K eps (|A||B| + |C|).
 constexpr int kGuardMin = 1 << 14;
 constexpr int kGuardCap = 1 << 30;  // the guard sums saturate here (int32)
+// Sampled row sum of a row left out of the sampling's choice: above any real
+// one (127 x 32 per 128 of K, below 2^25 at the longest K).
+constexpr unsigned kNoGuardSum = 1u << 30;
 
 // ------------------------------------------------------ operand preparation
 // Row scales: e[r] = the exponent frexp gives for max_k |src(r, k)| (so the
@@ -354,7 +356,7 @@ __global__ void __launch_bounds__(256) digits_kernel(const DgOperand oa, const D
   }
   __syncthreads();
   const int r = tid >> 3, kq = (tid & 7) * 4;
-  const int e = e_row[r0 + r] == kBadExp ? kBadExp : used_exp(e_row[r0 + r]);
+  const int er = e_row[r0 + r], e = er == kBadExp ? kBadExp : used_exp(er);
   int d[4][S];
 #pragma unroll
   for (int j = 0; j < 4; ++j) f64_digits<S>(tile[r][kq + j], e, d[j]);
@@ -377,11 +379,14 @@ __global__ void __launch_bounds__(256) digits_kernel(const DgOperand oa, const D
     w.y = *reinterpret_cast<const uint32_t*>(&h23);
     *reinterpret_cast<uint2*>(dst + S * plane_stride) = w;
     // the row's sum over the first 32 of every 128 K (8 threads a row), for the
-    // GEMM's choice of how much of K the guard samples
+    // GEMM's choice of how much of K the guard samples.  The guard rejects the
+    // blocks of a zero row, or one with Inf or NaN, however much is sampled:
+    // its sum is set beyond any other, so that it does not weigh in the choice.
     if (k0 % 128 == 0) {
       int sum = (int)(g(d[0][0]) + g(d[1][0]) + g(d[2][0]) + g(d[3][0]));
 #pragma unroll
       for (int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      if (er == kZeroExp || er == kBadExp) sum = k0 == 0 ? (int)kNoGuardSum : 0;
       if ((tid & 7) == 0 && r0 + r < rows && sum) atomicAdd(gsum_row + r0 + r, (unsigned)sum);
     }
   }
@@ -488,8 +493,6 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint64_t* accf = gempty + 1;   // [1]  every MMA of this CTA finished
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accf + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  uint64_t* gready = accf + 2;   // [1] the guard's minima are in `least`
-  __shared__ unsigned least[2];  // guard: smallest row sum of A, column sum of B
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
@@ -504,8 +507,6 @@ __global__ void __launch_bounds__(kThreads, 1)
     mbar_init(gfull, 1);
     mbar_init(gempty, 1);
     mbar_init(accf, 1);
-    mbar_init(gready, kEpiWarps);
-    least[0] = least[1] = 0xFFFFFFFFu;
     *abort_flag = 0;
     fence_mbar_init();
     prefetch_tensormap(&tm_a);
@@ -530,19 +531,41 @@ __global__ void __launch_bounds__(kThreads, 1)
   };
 
   const int items = dg_items(p);
-  // The guard's sampling: the first 32 of every 128 K, or, where the guard
-  // planes' sums over those say that some output's lower bound may fall short,
-  // all of K.  (The smallest row sum times the smallest column sum over the
-  // number of K sampled estimates an output's sum; it has to be four times
-  // the limit.)  Either sum is a lower bound; the full one takes a third more
-  // shared-memory traffic and keeps operands whose magnitudes spread over
-  // many binades, few of them large at once, off the FP64 pipes: exponents of
-  // +-10 at 1531 x 1400 x 1601, 6435 us with the quarter, 266 with all.
-  // The epilogue warps find the two minima while the first stage is under way;
-  // the MMA lane and the guard producer wait for them after it (the wait up
-  // front took 3 us of every call).
-  auto sample_all = [&]() {
-    return (float)least[0] * (float)least[1] < 4.0f * (float)kGuardMin * 32.0f * (float)((p.K + 127) / 128);
+  // The guard's sampling of a tile: the first 32 of every 128 K, or, where the
+  // guard planes' sums over those say that some output's lower bound may fall
+  // short, all of K.  (The smallest row sum of the tile times its smallest
+  // column sum over the number of K sampled estimates an output's sum; it has
+  // to be four times the limit.)  Either sum is a lower bound; the full one
+  // takes a third more shared-memory traffic and keeps operands whose
+  // magnitudes spread over many binades, few of them large at once, off the
+  // FP64 pipes: exponents of +-10 at 1531 x 1400 x 1601, 6435 us with the
+  // quarter, 266 with all.  By tile, so that a few thin rows cost no more than
+  // their own tiles, and no CTA reads more than 160 sums at a time (one choice
+  // for the product, from all M + N sums in every CTA: 10^6 x 32 x 1000 10.11
+  // ms, now 9.82; 1531 x 1400 x 1601 224 us, now 221, with a zero row 955 and
+  // 909, the rest being that row's blocks on the pipes).  The MMA warp and the guard producer each read the sums when they
+  // come to a tile and need them after its first stage, which is sampled
+  // either way.
+  struct TileSums {
+    unsigned a[kBM / 32], b;
+  };
+  auto tile_sums = [&](int m0, int n0) {  // lane l: rows l, l + 32, ..., column l
+    TileSums t;
+#pragma unroll
+    for (int i = 0; i < kBM / 32; ++i) {
+      const int row = m0 + 32 * i + lane;
+      t.a[i] = row < p.M ? __ldcg(p.ga + row) - kArrivedBase : kNoGuardSum;
+    }
+    t.b = n0 + lane < p.N ? __ldcg(p.gb + n0 + lane) - kArrivedBase : kNoGuardSum;
+    return t;
+  };
+  auto sample_all = [&](const TileSums& t) {
+    unsigned la = t.a[0];
+#pragma unroll
+    for (int i = 1; i < kBM / 32; ++i) la = min(la, t.a[i]);
+    la = __reduce_min_sync(0xffffffffu, la);
+    const unsigned lb = __reduce_min_sync(0xffffffffu, t.b);
+    return (float)la * (float)lb < 4.0f * (float)kGuardMin * 32.0f * (float)((p.K + 127) / 128);
   };
   int issued = 0;  // A producer: stages whose copies were issued
   if ((warp == 0 || warp == kBProdWarp) && lane == 0) {
@@ -577,32 +600,28 @@ __global__ void __launch_bounds__(kThreads, 1)
     // guard producer: the guard planes' 32 K of every sampled stage into the
     // guard slot, once the guard product before has read it.  A warp of its
     // own, so that waiting for the one slot does not hold back the stages.
-    if (lane == 0) {
-      int g_issued = 0;
-      bool stop = false, guard_all = false;
-      for (int w = (int)blockIdx.x; w < items && !stop; w += gridDim.x) {
-        const DgWork dw = dg_work<CF::kChunk>(p, w);
-        int m0, n0;
-        dg_tile(p, dw.tile, m0, n0);
-        for (int kt = 0; kt < dw.nkt; kt += guard_all ? 1 : CF::kChunk, ++g_issued) {
-          if (g_issued > 0 && !mbar_wait_bounded(gempty, (g_issued - 1) & 1, abort_flag, kWaitLimitNs)) {
-            fail();
-            stop = true;
-            break;
-          }
+    int g_issued = 0;
+    bool stop = false;
+    for (int w = (int)blockIdx.x; w < items && !stop; w += gridDim.x) {
+      const DgWork dw = dg_work<CF::kChunk>(p, w);
+      int m0, n0;
+      dg_tile(p, dw.tile, m0, n0);
+      const TileSums sums = tile_sums(m0, n0);
+      bool guard_all = false;
+      for (int kt = 0; kt < dw.nkt; kt += guard_all ? 1 : CF::kChunk, ++g_issued) {
+        if (g_issued > 0 && !__all_sync(0xffffffffu, mbar_wait_bounded(gempty, (g_issued - 1) & 1, abort_flag, kWaitLimitNs))) {
+          if (lane == 0) fail();
+          stop = true;
+          break;
+        }
+        if (lane == 0) {
           const int kx = (dw.kt0 + kt) * kBK;
           mbar_arrive_expect_tx(gfull, CF::kATile + CF::kBTile);
           tma_load_3d(guard_a, &tm_ga, gfull, kx, m0, 0);
           tma_load_3d(guard_b, &tm_gb, gfull, kx, n0, 0);
-          if (g_issued == 0) {  // (the first stage is sampled either way)
-            if (!mbar_wait_bounded(gready, 0, abort_flag, kWaitLimitNs)) {
-              fail();
-              stop = true;
-              break;
-            }
-            guard_all = sample_all();
-          }
         }
+        __syncwarp();
+        if (kt == 0) guard_all = sample_all(sums);
       }
     }
   } else if (warp == 1) {
@@ -623,9 +642,17 @@ __global__ void __launch_bounds__(kThreads, 1)
     int s = 0;           // stage of the next K slice
     uint32_t phase = 0;  // and its barrier's phase
     int chunk_g = 0, g_used = 0;
-    bool stop = false, guard_all = false, first = true;
+    bool stop = false;
     for (int w = (int)blockIdx.x; w < items && !stop; w += gridDim.x) {
-      const int nkt = dg_work<CF::kChunk>(p, w).nkt;
+      const DgWork dw = dg_work<CF::kChunk>(p, w);
+      const int nkt = dw.nkt;
+      bool guard_all = false;
+      TileSums sums;
+      if constexpr (G) {
+        int m0, n0;
+        dg_tile(p, dw.tile, m0, n0);
+        sums = tile_sums(m0, n0);
+      }
       for (int kt = 0; kt < nkt; ++kt) {
         const bool chunk_first = (kt % CF::kChunk) == 0;
         const bool chunk_last = ((kt + 1) % CF::kChunk) == 0 || kt + 1 == nkt;
@@ -679,14 +706,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           if (chunk_last) mma_commit(&tfull[b]);
         }
         __syncwarp();
-        if (G && first) {  // (the first stage is sampled either way)
-          if (!wait(gready, 0)) {
-            stop = true;
-            break;
-          }
-          guard_all = __shfl_sync(0xffffffffu, (int)sample_all(), 0) != 0;
-        }
-        first = false;
+        if (G && kt == 0) guard_all = __shfl_sync(0xffffffffu, (int)sample_all(sums), 0) != 0;
         if (++s == ST) {
           s = 0;
           phase ^= 1;
@@ -701,21 +721,6 @@ __global__ void __launch_bounds__(kThreads, 1)
     // columns (half h) of each group's 32
     const int q = warp & 3, h = (warp - 2) >> 2;
     const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(16 * h);
-    if constexpr (G) {
-      unsigned la = 0xFFFFFFFFu, lb = 0xFFFFFFFFu;
-      const int tid = threadIdx.x - 64;
-#pragma unroll 8
-      for (int i = tid; i < p.M; i += 32 * kEpiWarps) la = min(la, __ldcg(p.ga + i) - kArrivedBase);
-#pragma unroll 8
-      for (int i = tid; i < p.N; i += 32 * kEpiWarps) lb = min(lb, __ldcg(p.gb + i) - kArrivedBase);
-      la = __reduce_min_sync(0xffffffffu, la);
-      lb = __reduce_min_sync(0xffffffffu, lb);
-      if (lane == 0) {
-        atomicMin(&least[0], la);
-        atomicMin(&least[1], lb);
-        mbar_arrive(gready);  // release: the waiters see both
-      }
-    }
     int chunk_g = 0;
     bool ok = true;
     for (int wk = (int)blockIdx.x; wk < items && ok; wk += gridDim.x) {
