@@ -229,14 +229,20 @@ void tc_prepare(DeviceCtx* c);
 // kernels' launch attributes (set by tc_prepare).
 int dgemm_digits_count(gbblas_accuracy acc);
 int64_t dgemm_digits_max_k(int digits);
-size_t dgemm_digits_scratch_bytes(int digits, bool guarded, int64_t M, int64_t N, int64_t K);
+// How much scratch a digit GEMM takes beside its planes: all it has a use for;
+// none for cutting the last round's tiles along K (the same bits, slower); nor
+// for the guard's sampled sums (a quarter of K is sampled throughout: blocks of
+// operands whose magnitudes spread widely go to the FP64 pipes).
+enum class DgScratch { kCut, kWhole, kLeast };
+size_t dgemm_digits_scratch_bytes(int sms, int digits, bool guarded, int64_t M, int64_t N, int64_t K, int max_ctas,
+                                  DgScratch level);
 // AUTO for a double GEMM: the guarded digits for this shape (else the FP64 pipes).
 bool dgemm_auto_digits(int64_t M, int64_t N, int64_t K, int num_sms);
 void dgemm_digits_prepare(DeviceCtx* c);
 gbblas_status launch_dgemm_digits(DeviceCtx* c, int digits, bool guarded, int64_t M, int64_t N, int64_t K,
                                   const double* A, int64_t rsa, int64_t csa, const double* B, int64_t rsb,
                                   int64_t csb, double* C, int64_t rsc, int64_t csc, cudaStream_t stream,
-                                  int max_ctas = 0, int slices = 1);
+                                  int max_ctas = 0, int slices = 1, DgScratch level = DgScratch::kCut);
 
 // Grouped GEMV: row-streaming problems in one persistent launch, the rest
 // per problem (batch.cu).

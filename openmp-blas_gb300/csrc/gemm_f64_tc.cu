@@ -95,6 +95,8 @@ constexpr int kBadExp = INT_MAX;                  // scale marker: the row / col
 constexpr int kZeroExp = (int)0x80808080;          // scale of an all-zero row (the fill byte 0x80)
 constexpr unsigned kArrivedBase = 0x80808080u;     // where counts start: the fill byte 0x80
 
+constexpr int chunk_stages(int digits) { return digits <= 7 ? 4 : 2; }  // stages per TMEM chunk, see DgCfg
+
 // S digits; G = 1 adds the guard plane (P = max(|D_0| - 1, 0), whose
 // product sum bounds sum_k |a_ik||b_kj| from below) and its accumulator in
 // TMEM column slot S.
@@ -113,7 +115,7 @@ struct DgCfg {
   static constexpr uint32_t kGuardBytes = G ? kATile + kBTile : 0;
   // stages per TMEM chunk: a group's sum over the chunk stays below 2^24
   // (S * chunk * 2^14 with chunk = 128 K for S <= 7, 64 K for S = 8)
-  static constexpr int kChunk = S <= 7 ? 4 : 2;
+  static constexpr int kChunk = chunk_stages(S);
   // longest K: the 64-bit accumulators stay below 2^62 (each chunk adds
   // less than 2^48 to hi and to lo)
   static constexpr int64_t kMaxK = 1 << 20;
@@ -140,7 +142,7 @@ struct DgProblem {
   int64_t rsc, csc;
   const int* ea;  // [rows of A, padded] row scales
   const int* eb;  // [columns of B, padded] column scales
-  const unsigned* ga;  // guarded form: the rows' (columns') sampled sums of the guard plane, from kArrivedBase
+  const unsigned* ga;  // guarded form: the rows' (columns') sampled sums of the guard plane, from kArrivedBase (or null)
   const unsigned* gb;
   // guarded form: the 32 x 16 blocks the guard rejected (block b of tile t
   // = t * 8 + epilogue warp), recomputed on the FP64 pipes from A and B
@@ -382,7 +384,7 @@ __global__ void __launch_bounds__(256) digits_kernel(const DgOperand oa, const D
     // GEMM's choice of how much of K the guard samples.  The guard rejects the
     // blocks of a zero row, or one with Inf or NaN, however much is sampled:
     // its sum is set beyond any other, so that it does not weigh in the choice.
-    if (k0 % 128 == 0) {
+    if (k0 % 128 == 0 && gsum_row) {
       int sum = (int)(g(d[0][0]) + g(d[1][0]) + g(d[2][0]) + g(d[3][0]));
 #pragma unroll
       for (int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
@@ -550,7 +552,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     unsigned a[kBM / 32], b;
   };
   auto tile_sums = [&](int m0, int n0) {  // lane l: rows l, l + 32, ..., column l
-    TileSums t;
+    TileSums t = {{kNoGuardSum, kNoGuardSum, kNoGuardSum, kNoGuardSum}, kNoGuardSum};
+    if (p.ga == nullptr) return t;  // no room for them (DgScratch::kLeast): the quarter
 #pragma unroll
     for (int i = 0; i < kBM / 32; ++i) {
       const int row = m0 + 32 * i + lane;
@@ -949,6 +952,42 @@ inline int rest_parts(int64_t rest, int64_t chunks, int ctas) {
   return rest > 0 ? (int)std::max<int64_t>(1, std::min<int64_t>(ctas / rest, chunks / 2)) : 1;
 }
 
+// Where a call's arrays lie in its scratch, and its size.
+struct DgLayout {
+  int64_t mp, np, kp, tiles, rest;
+  int ctas, parts;                      // CTAs of the grid, K parts of the last round's tiles
+  size_t arr, ea, eb, ga, gb, a, b, fix;  // arr .. a: filled with 0x80
+  size_t slots, gslots, bytes;
+};
+DgLayout dg_layout(int sms, int digits, bool guarded, int64_t M, int64_t N, int64_t K, int max_ctas, DgScratch level) {
+  DgLayout l;
+  const int64_t planes = digits + (guarded ? 1 : 0);
+  l.mp = round_up(M, kBM);
+  l.np = round_up(N, kBN);
+  l.kp = round_up(K, kBK);
+  l.tiles = (l.mp / kBM) * (l.np / kBN);
+  l.ctas = std::min(sms, kMaxCtas);
+  if (max_ctas > 0 && l.ctas > max_ctas) l.ctas = max_ctas;
+  l.rest = l.tiles % l.ctas;
+  const int64_t chunk = chunk_stages(digits), chunks = (l.kp / kBK + chunk - 1) / chunk;
+  l.parts = level == DgScratch::kCut ? rest_parts(l.rest, chunks, l.ctas) : 1;
+  const size_t rows = align256(sizeof(int) * (size_t)l.mp), cols = align256(sizeof(int) * (size_t)l.np);
+  const bool sums = guarded && level != DgScratch::kLeast;
+  l.arr = kScratchZeroBytes;
+  l.ea = l.arr + (l.parts > 1 ? kArrivedBytes : 0);
+  l.eb = l.ea + rows;
+  l.ga = l.eb + cols;
+  l.gb = l.ga + (sums ? rows : 0);
+  l.a = l.gb + (sums ? cols : 0);
+  l.b = l.a + align256((size_t)(planes * l.mp * l.kp) * sizeof(__nv_bfloat16));
+  l.fix = l.b + align256((size_t)(planes * l.np * l.kp) * sizeof(__nv_bfloat16));
+  l.slots = l.fix + (guarded ? align256(sizeof(int) * (size_t)(1 + l.tiles * kEpiWarps)) : 0);
+  const size_t n = l.parts > 1 ? (size_t)l.rest * l.parts : 0;
+  l.gslots = l.slots + n * kSlotBytes;
+  l.bytes = l.gslots + (guarded ? n * kGSlotBytes : 0);
+  return l;
+}
+
 template <int S, int G>
 void dg_setup(DeviceCtx* c) {
   static std::mutex mu;
@@ -964,7 +1003,7 @@ void dg_setup(DeviceCtx* c) {
 template <int S, int G>
 gbblas_status launch_digits(DeviceCtx* c, int64_t M, int64_t N, int64_t K, const double* A, int64_t rsa,
                             int64_t csa, const double* B, int64_t rsb, int64_t csb, double* C, int64_t rsc,
-                            int64_t csc, cudaStream_t stream, int max_ctas, int slices) {
+                            int64_t csc, cudaStream_t stream, int max_ctas, int slices, DgScratch level) {
   using CF = DgCfg<S, G>;
   constexpr int NP = CF::NP;
   if (K > CF::kMaxK) {
@@ -975,44 +1014,41 @@ gbblas_status launch_digits(DeviceCtx* c, int64_t M, int64_t N, int64_t K, const
     set_error("dgemm (FP64 digits): problem too large for the tile grid");
     return GBBLAS_STATUS_NOT_SUPPORTED;
   }
-  const int64_t Mp = round_up(M, kBM), Np = round_up(N, kBN), Kp = round_up(K, kBK);
-  const size_t off_arr = kScratchZeroBytes;  // arrival counts of cut tiles, filled with 0x80 as the scales are
-  const size_t off_ea = off_arr + kArrivedBytes;
-  const size_t off_eb = off_ea + align256(sizeof(int) * (size_t)Mp);
-  const size_t off_ga = off_eb + align256(sizeof(int) * (size_t)Np);
-  const size_t off_gb = off_ga + (G ? align256(sizeof(int) * (size_t)Mp) : 0);
-  const size_t off_a = off_gb + (G ? align256(sizeof(int) * (size_t)Np) : 0);
-  const size_t a_plane = (size_t)(Mp * Kp), b_plane = (size_t)(Np * Kp);
-  const size_t off_b = off_a + align256((size_t)NP * a_plane * sizeof(__nv_bfloat16));
-  const int64_t tiles = (Mp / kBM) * (Np / kBN);
-  const size_t off_fix = off_b + align256((size_t)NP * b_plane * sizeof(__nv_bfloat16));
-  const size_t off_slots = off_fix + (G ? align256(sizeof(int) * (size_t)(1 + tiles * kEpiWarps)) : 0);
-  int ctas = std::min(c->num_sms, kMaxCtas);
-  if (max_ctas > 0 && ctas > max_ctas) ctas = max_ctas;
-  const int64_t chunks = (Kp / kBK + CF::kChunk - 1) / CF::kChunk, rest = tiles % ctas;
-  const int parts = rest_parts(rest, chunks, ctas);
-  const size_t nslots = parts > 1 ? (size_t)rest * parts : 0;
-  const size_t bytes = off_slots + nslots * (kSlotBytes + (G ? kGSlotBytes : 0));
+  DgLayout l = dg_layout(c->num_sms, S, G != 0, M, N, K, max_ctas, level);
   void* scratch = nullptr;
-  GB_TRY(get_scratch(c, stream, bytes, &scratch));
+  gbblas_status got = get_scratch(c, stream, l.bytes, &scratch);
+  // no room: without what only makes the call faster
+  while (got == GBBLAS_STATUS_ALLOC_FAILED && level != DgScratch::kLeast) {
+    level = level == DgScratch::kCut ? DgScratch::kWhole : DgScratch::kLeast;
+    const size_t asked = l.bytes;
+    l = dg_layout(c->num_sms, S, G != 0, M, N, K, max_ctas, level);
+    if (l.bytes == asked) continue;
+    cudaGetLastError();
+    got = get_scratch(c, stream, l.bytes, &scratch);
+  }
+  GB_TRY(got);
+  const int64_t Mp = l.mp, Np = l.np, Kp = l.kp, tiles = l.tiles;
+  const int ctas = l.ctas;
   char* base = static_cast<char*>(scratch);
-  int* ea = reinterpret_cast<int*>(base + off_ea);
-  int* eb = reinterpret_cast<int*>(base + off_eb);
-  auto* da = reinterpret_cast<__nv_bfloat16*>(base + off_a);
-  auto* db = reinterpret_cast<__nv_bfloat16*>(base + off_b);
+  int* ea = reinterpret_cast<int*>(base + l.ea);
+  int* eb = reinterpret_cast<int*>(base + l.eb);
+  auto* da = reinterpret_cast<__nv_bfloat16*>(base + l.a);
+  auto* db = reinterpret_cast<__nv_bfloat16*>(base + l.b);
+  const size_t a_plane = (size_t)(Mp * Kp), b_plane = (size_t)(Np * Kp);
   int* err = reinterpret_cast<int*>(base + kErrWordOffset);
 
   // scales: rows of A over K; columns of B (element (n, k) = B[k*rsb + n*csb])
-  int* fix_count = G ? reinterpret_cast<int*>(base + off_fix) : nullptr;
+  int* fix_count = G ? reinterpret_cast<int*>(base + l.fix) : nullptr;
   // kZeroExp everywhere (ea and eb), and kArrivedBase
-  const int words = (int)((off_a - off_arr) / sizeof(uint4));
+  const int words = (int)((l.a - l.arr) / sizeof(uint4));
   dg_init_kernel<<<std::min((words + 255) / 256, c->num_sms), 256, 0, stream>>>(
-      reinterpret_cast<uint4*>(base + off_arr), words);
+      reinterpret_cast<uint4*>(base + l.arr), words);
   GB_TRY(check_launch("dg_init_kernel"));
   const int stk = (int)((K + kScaleTK - 1) / kScaleTK);
   const int tiles_k = (int)(Kp / 32);
-  unsigned* gsa = reinterpret_cast<unsigned*>(base + off_ga);
-  unsigned* gsb = reinterpret_cast<unsigned*>(base + off_gb);
+  const bool sums = G && level != DgScratch::kLeast;
+  unsigned* gsa = sums ? reinterpret_cast<unsigned*>(base + l.ga) : nullptr;
+  unsigned* gsb = sums ? reinterpret_cast<unsigned*>(base + l.gb) : nullptr;
   DgOperand oa{A, M, K, rsa, csa, ea, gsa, da, (int64_t)a_plane, Kp, stk, (int)((Mp / 32) * stk)};
   DgOperand ob{B, N, K, csb, rsb, eb, gsb, db, (int64_t)b_plane, Kp, stk, (int)((Np / 32) * stk)};
   if ((double)(Mp + Np) / 32 * tiles_k >= 2.0e9) {
@@ -1064,9 +1100,9 @@ gbblas_status launch_digits(DeviceCtx* c, int64_t M, int64_t N, int64_t K, const
   p.csb = csb;
   p.K = K;
   dg_setup<S, G>(c);
-  p.slots = reinterpret_cast<longlong2*>(base + off_slots);
-  p.gslots = reinterpret_cast<int*>(base + off_slots + nslots * kSlotBytes);
-  p.arrived = reinterpret_cast<unsigned*>(base + off_arr);
+  p.slots = reinterpret_cast<longlong2*>(base + l.slots);
+  p.gslots = reinterpret_cast<int*>(base + l.gslots);
+  p.arrived = reinterpret_cast<unsigned*>(base + l.arr);
   // slices: consecutive tile ranges of whole waves, one launch each (higher-
   // priority work on other streams gets the SMs between them); the tiles of
   // the last, incomplete wave are cut along K (dg_work)
@@ -1077,7 +1113,7 @@ gbblas_status launch_digits(DeviceCtx* c, int64_t M, int64_t N, int64_t K, const
     p.tile_begin = (int)tb;
     p.full = (int)((te - tb) / ctas * ctas);
     p.rest = (int)(te - tb - p.full);
-    p.parts = p.rest ? parts : 1;
+    p.parts = p.rest ? l.parts : 1;
     const int grid = (int)std::min<int64_t>(ctas, p.full + (int64_t)p.rest * p.parts);
     if (sl == 0)
       GB_CUDA_TRY(launch_after(dgemm_digits_kernel<S, G>, dim3(grid), kThreads, CF::kSmem, stream, ma, mb, mga, mgb, p, err));
@@ -1102,16 +1138,9 @@ int dgemm_digits_count(gbblas_accuracy acc) {
 
 int64_t dgemm_digits_max_k(int digits) { return digits == 8 ? DgCfg<8, 0>::kMaxK : DgCfg<7, 0>::kMaxK; }
 
-// Scratch one call takes (scales, digit planes, fix-up list), as launch_digits lays it out.
-size_t dgemm_digits_scratch_bytes(int digits, bool guarded, int64_t M, int64_t N, int64_t K) {
-  const int64_t Mp = round_up(M, kBM), Np = round_up(N, kBN), Kp = round_up(K, kBK);
-  const int64_t np = digits + (guarded ? 1 : 0);
-  const int64_t tiles = (Mp / kBM) * (Np / kBN);
-  return kScratchZeroBytes + kArrivedBytes + (size_t)kMaxCtas * (kSlotBytes + kGSlotBytes) +
-         (guarded ? align256(sizeof(int) * (size_t)Mp) + align256(sizeof(int) * (size_t)Np) : 0) + align256(sizeof(int) * (size_t)Mp) +
-         align256(sizeof(int) * (size_t)Np) +
-         align256((size_t)(np * Mp * Kp) * 2) + align256((size_t)(np * Np * Kp) * 2) +
-         (guarded ? align256(sizeof(int) * (size_t)(1 + tiles * kEpiWarps)) : 0);
+size_t dgemm_digits_scratch_bytes(int sms, int digits, bool guarded, int64_t M, int64_t N, int64_t K, int max_ctas,
+                                  DgScratch level) {
+  return dg_layout(sms, digits, guarded, M, N, K, max_ctas, level).bytes;
 }
 
 void dgemm_digits_prepare(DeviceCtx* c) {
@@ -1123,14 +1152,14 @@ void dgemm_digits_prepare(DeviceCtx* c) {
 gbblas_status launch_dgemm_digits(DeviceCtx* c, int digits, bool guarded, int64_t M, int64_t N, int64_t K,
                                   const double* A, int64_t rsa, int64_t csa, const double* B, int64_t rsb,
                                   int64_t csb, double* C, int64_t rsc, int64_t csc, cudaStream_t stream, int max_ctas,
-                                  int slices) {
+                                  int slices, DgScratch level) {
   if (M == 0 || N == 0 || K == 0) return GBBLAS_STATUS_SUCCESS;
   if (guarded && digits == 7)
-    return launch_digits<7, 1>(c, M, N, K, A, rsa, csa, B, rsb, csb, C, rsc, csc, stream, max_ctas, slices);
+    return launch_digits<7, 1>(c, M, N, K, A, rsa, csa, B, rsb, csb, C, rsc, csc, stream, max_ctas, slices, level);
   if (!guarded && digits == 7)
-    return launch_digits<7, 0>(c, M, N, K, A, rsa, csa, B, rsb, csb, C, rsc, csc, stream, max_ctas, slices);
+    return launch_digits<7, 0>(c, M, N, K, A, rsa, csa, B, rsb, csb, C, rsc, csc, stream, max_ctas, slices, level);
   if (!guarded && digits == 8)
-    return launch_digits<8, 0>(c, M, N, K, A, rsa, csa, B, rsb, csb, C, rsc, csc, stream, max_ctas, slices);
+    return launch_digits<8, 0>(c, M, N, K, A, rsa, csa, B, rsb, csb, C, rsc, csc, stream, max_ctas, slices, level);
   set_error("dgemm (FP64 digits): %d digits%s not supported", digits, guarded ? " with the guard" : "");
   return GBBLAS_STATUS_INVALID_VALUE;
 }

@@ -43,6 +43,8 @@ struct Req {
   bool heavy = false;
   int f64_digits = 0;         // double GEMM on tensor-core digits (0: the FP64 pipes)
   bool f64_guarded = false;   // ... in the guarded form
+  DgScratch f64_scratch = DgScratch::kWhole;  // ... and the scratch it takes
+  int64_t cut_bytes = 0;      // bytes more for cutting its last tiles along K, taken where the budget has them
   Clock::time_point t_submit, t_round, t_enqueued, t_done;
   int round_size = 0;
   bool done = false;
@@ -96,15 +98,15 @@ int server_f64_digits(const gbblas_request& r, int sms, bool* guarded) {
 }
 
 // Device bytes a request holds while in flight: operands, result, and the
-// operand arena (BF16 pieces or FP8 values and scales) of a tensor-core GEMM.
-int64_t working_set(const gbblas_request& r, int f64_digits, bool f64_guarded) {
+// operand arena (BF16 pieces, FP8 values and scales) of a tensor-core GEMM;
+// the scratch of a double GEMM on digits comes on top.
+int64_t working_set(const gbblas_request& r) {
   const int64_t s = r.dtype == GBBLAS_F64 ? 8 : 4;
   switch (r.op) {
     case GBBLAS_OP_MTM: {
       int64_t b = (r.M * r.K + r.K * r.N + r.M * r.N) * s;
       if (r.dtype == GBBLAS_F32 && r.accuracy != GBBLAS_ACCURACY_FP32 && !server_auto_fma(r))
         b += (int64_t)tc_arena_bytes(server_mode(r.accuracy), r.M, r.N, r.K);
-      if (f64_digits) b += (int64_t)dgemm_digits_scratch_bytes(f64_digits, f64_guarded, r.M, r.N, r.K);
       return b;
     }
     case GBBLAS_OP_MTV:
@@ -202,6 +204,34 @@ void CUDART_CB on_round_done(void* p) {
   s->cv.notify_one();
 }
 
+// Whether a heavy request runs on the whole GPU in slices, and the SM cap of one that does not.
+bool sliced(const gbblas_server_s* s, const Req& q) {
+  return s->cfg.slice_us > 0 && q.r.op == GBBLAS_OP_MTM &&
+         (q.f64_digits || (q.r.dtype == GBBLAS_F32 && q.r.accuracy != GBBLAS_ACCURACY_FP32));
+}
+int heavy_ctas(const gbblas_server_s* s) { return std::max(1, s->ctx->num_sms * s->cfg.heavy_sm_percent / 100); }
+
+// A double GEMM on digits: the scratch it is admitted with.  What only makes it
+// faster (dgemm_digits_scratch_bytes) never keeps a request out: the cut of its
+// last tiles is left to the moment its round is formed, the guard's sums go
+// where they alone would put the request over the budget.
+void add_f64_scratch(const gbblas_server_s* s, Req* q) {
+  if (!q->f64_digits) return;
+  const int cap = q->heavy && !sliced(s, *q) ? heavy_ctas(s) : 0;
+  auto scratch = [&](DgScratch level) {
+    return (int64_t)dgemm_digits_scratch_bytes(s->ctx->num_sms, q->f64_digits, q->f64_guarded, q->r.M, q->r.N, q->r.K,
+                                               cap, level);
+  };
+  const int64_t whole = scratch(DgScratch::kWhole);
+  if (q->bytes + whole <= s->cfg.budget_bytes) {
+    q->bytes += whole;
+    q->cut_bytes = scratch(DgScratch::kCut) - whole;
+  } else {
+    q->f64_scratch = DgScratch::kLeast;
+    q->bytes += scratch(DgScratch::kLeast);
+  }
+}
+
 // Enqueue one round on `st` (scheduler thread, no lock held).
 gbblas_status launch_round(gbblas_server_s* s, Round* rd, cudaStream_t st) {
   DeviceCtx* c = s->ctx;
@@ -222,7 +252,7 @@ gbblas_status launch_round(gbblas_server_s* s, Round* rd, cudaStream_t st) {
       if (q->f64_digits) {
         note(launch_dgemm_digits(c, q->f64_digits, q->f64_guarded, r.M, r.N, r.K,
                                  static_cast<const double*>(r.A), rsa, csa, static_cast<const double*>(r.B), rsb, csb,
-                                 static_cast<double*>(r.C), rsc, csc, st, cap, rd->slices));
+                                 static_cast<double*>(r.C), rsc, csc, st, cap, rd->slices, q->f64_scratch));
       } else if (r.dtype == GBBLAS_F64) {
         note(launch_gemm_fma<double>(c, r.M, r.N, r.K, static_cast<const double*>(r.A), rsa, csa,
                                      static_cast<const double*>(r.B), rsb, csb, static_cast<double*>(r.C), rsc,
@@ -339,6 +369,10 @@ void scheduler_main(gbblas_server_s* s) {
           if (s->inflight_bytes + r->bytes > s->cfg.budget_bytes) break;  // wait for memory
           if (!rd->reqs.empty() && est + r->est_us > (double)s->cfg.heavy_us) break;
           q.pop_front();
+          if (r->cut_bytes > 0 && s->inflight_bytes + r->bytes + r->cut_bytes <= s->cfg.budget_bytes) {
+            r->f64_scratch = DgScratch::kCut;
+            r->bytes += r->cut_bytes;
+          }
           rd->reqs.push_back(r);
           rd->bytes += r->bytes;
           est += r->est_us;
@@ -371,12 +405,10 @@ void scheduler_main(gbblas_server_s* s) {
           // the high-priority light streams first.  Other heavy requests keep
           // the SM cap.
           Req* h = rd->reqs[0];
-          const bool sliceable = h->r.op == GBBLAS_OP_MTM &&
-                                 (h->f64_digits || (h->r.dtype == GBBLAS_F32 && h->r.accuracy != GBBLAS_ACCURACY_FP32));
-          if (sliceable && s->cfg.slice_us > 0)
+          if (sliced(s, *h))
             rd->slices = (int)std::max(1.0, std::ceil(h->est_us / (double)s->cfg.slice_us));
           else
-            rd->max_ctas = std::max(1, s->ctx->num_sms * s->cfg.heavy_sm_percent / 100);
+            rd->max_ctas = heavy_ctas(s);
         }
         cudaStream_t st = heavy ? s->heavy_streams[slot] : s->streams[slot];
         const auto t_round = Clock::now();
@@ -519,9 +551,10 @@ gbblas_status gbblas_server_submit(gbblas_server s, const gbblas_request* r, uin
   auto q = std::make_unique<Req>();
   q->r = *r;
   q->f64_digits = server_f64_digits(*r, s->ctx->num_sms, &q->f64_guarded);
-  q->bytes = working_set(*r, q->f64_digits, q->f64_guarded);
+  q->bytes = working_set(*r);
   q->est_us = estimate_us(*r, q->f64_digits);
   q->heavy = q->est_us > (double)s->cfg.heavy_us;
+  add_f64_scratch(s, q.get());
   if (q->bytes > s->cfg.budget_bytes) {
     set_error("gbblas_server_submit: request needs %lld bytes, the budget is %lld", (long long)q->bytes,
               (long long)s->cfg.budget_bytes);
