@@ -2801,7 +2801,13 @@ gbblas_status launch_gemm_tc_opts(DeviceCtx* c, int mode, const gbblas_gemm_desc
   GB_TRY(plan_group(c, mode, &d, 1, pl, opt));
   if (pl.nprob == 0) return GBBLAS_STATUS_SUCCESS;
   void* s = nullptr;
-  GB_TRY(get_scratch(c, stream, pl.bytes, &s));
+  const gbblas_status got = get_scratch(c, stream, pl.bytes, &s);
+  if (got == GBBLAS_STATUS_ALLOC_FAILED && !pl.reds.empty()) {
+    // no room for the parts' sums: K in one piece
+    cudaGetLastError();
+    return launch_gemm_tc_opts(c, mode, d, TcLaunchOpts{1, opt.pair}, stream);
+  }
+  GB_TRY(got);
   GB_TRY(bind_group(pl, static_cast<char*>(s), stream, true));
   return tc_group_launch(c, &pl, stream, 0, gemm_slices_env());
 }

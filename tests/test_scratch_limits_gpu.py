@@ -61,3 +61,21 @@ got = run(s, *ops, {accuracy})
 assert torch.equal(got, want)
 assert gbblas.kernel_launches() - n >= 4, "not the digits"
 """)
+
+
+@pytest.mark.parametrize("accuracy", ["ACCURACY_AUTO", "ACCURACY_FP16X3"])
+def test_tensor_core_gemm_without_room_for_the_parts(cuda, accuracy):
+    """20 MB of FP16 pieces, 8 of partial sums for K in two parts."""
+    child(f"""
+import os
+acc = gbblas.{accuracy}
+os.environ["GBBLAS_GEMM_AUTO"] = "1"
+ops = operands(1024, 1024, 2400, torch.float32)
+os.environ["GBBLAS_TC_SPLITK"] = "1"
+want = run(torch.cuda.Stream(), *ops, acc)
+del os.environ["GBBLAS_TC_SPLITK"]
+cut = run(torch.cuda.Stream(), *ops, acc)
+assert not torch.equal(cut, want), "K is not cut here"
+limit_pool()
+assert torch.equal(run(torch.cuda.Stream(), *ops, acc), want)
+""")
