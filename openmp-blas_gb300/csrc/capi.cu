@@ -286,7 +286,7 @@ gbblas_status gemm_any(DeviceCtx* c, int64_t M, int64_t N, int64_t K, const T* A
     // whichever FP32-accurate path the autotuner measured faster for this
     // shape bucket (FMA kernel or the guarded FP16 split).
     int mode = tc_mode(acc);
-    if (acc == GBBLAS_ACCURACY_AUTO && tuned_gemm_auto(c, M, N, K) == 1) mode = kTcModeF16Guard;
+    if (acc == GBBLAS_ACCURACY_AUTO && tuned_gemm_auto(c, M, N, K, s) == 1) mode = kTcModeF16Guard;
     if (mode != 0) return launch_gemm_tc(c, mode, M, N, K, A, rsa, csa, B, rsb, csb, C, rsc, csc, s);
     // FP32 on the FMA pipe: the tile shape the autotuner measured faster
     return launch_gemm_fma<T>(c, M, N, K, A, rsa, csa, B, rsb, csb, C, rsc, csc, s, 0,

@@ -249,7 +249,7 @@ gbblas_status launch_dgemm_digits(DeviceCtx* c, int digits, bool guarded, int64_
 gbblas_status launch_gemv_group(DeviceCtx* c, const gbblas_gemv_desc* d, int64_t count, cudaStream_t s);
 
 // Autotuner (tune.cu): AUTO accuracy -> 1 = the guarded FP16 split (kTcModeF16Guard), 0 = FMA.
-int tuned_gemm_auto(DeviceCtx* c, int64_t M, int64_t N, int64_t K);
+int tuned_gemm_auto(DeviceCtx* c, int64_t M, int64_t N, int64_t K, cudaStream_t stream);
 // Autotuner: split-K parts and CTA form of one tensor-core GEMM.
 TcLaunchOpts tuned_tc_opts(DeviceCtx* c, int mode, int64_t M, int64_t N, int64_t K, cudaStream_t stream);
 // Autotuner: FP32 FMA tile (launch_gemm_fma's `tile`).

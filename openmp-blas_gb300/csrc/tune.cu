@@ -283,9 +283,9 @@ int tuned_gemv_group_rows(DeviceCtx* c, const gbblas_gemv_desc* d, int64_t count
   return best;
 }
 
-// 1 = split-BF16 (six products), 0 = FP32 FMA, for an AUTO-accuracy GEMM of
-// this shape.  Without tuning: the tensor cores once the work fills them.
-int tuned_gemm_auto(DeviceCtx* c, int64_t M, int64_t N, int64_t K) {
+// 1 = the guarded FP16 split, 0 = FP32 FMA, for an AUTO-accuracy GEMM of this
+// shape on `stream`.  Without tuning: the tensor cores once the work fills them.
+int tuned_gemm_auto(DeviceCtx* c, int64_t M, int64_t N, int64_t K, cudaStream_t stream) {
   if (const char* e = std::getenv("GBBLAS_GEMM_AUTO"); e && (e[0] == '0' || e[0] == '1')) return e[0] - '0';
   const int fallback = (M >= 256 && N >= 256 && K >= 256 && (double)M * N * K >= 1.0e9) ? 1 : 0;
   Tuner& t = Tuner::get();
@@ -296,7 +296,7 @@ int tuned_gemm_auto(DeviceCtx* c, int64_t M, int64_t N, int64_t K) {
                           "|k" + std::to_string(bk) + "|f32";
   int v = t.lookup(key);
   if (v >= 0) return t.remember(packed, v);
-  if (!t.enabled()) return fallback;
+  if (!t.enabled() || capturing(stream)) return fallback;
   // representative shape of the bucket, capped so tuning stays cheap
   const int64_t m = std::min<int64_t>(int64_t(1) << bm, 8192), n = std::min<int64_t>(int64_t(1) << bn, 8192),
                 k = std::min<int64_t>(int64_t(1) << bk, 8192);
