@@ -189,6 +189,13 @@ struct TcLaunchOpts {
   int pair = -1;
 };
 
+// Contiguous rows of C, if it has such, all start on 16-byte boundaries: where
+// they do not, CTA pairs (and FP8's wide tiles) would update them slowly and
+// are not used.
+inline bool tc_c_on_grid(const gbblas_gemm_desc& d) {
+  return d.csc != 1 || ((d.rsc & 3) == 0 && aligned16(d.C));
+}
+
 // One problem with the autotuner's launch shape for it.
 gbblas_status launch_gemm_tc(DeviceCtx* c, int mode, int64_t M, int64_t N, int64_t K, const float* A, int64_t rsa,
                              int64_t csa, const float* B, int64_t rsb, int64_t csb, float* C, int64_t rsc,
@@ -251,7 +258,7 @@ gbblas_status launch_gemv_group(DeviceCtx* c, const gbblas_gemv_desc* d, int64_t
 // Autotuner (tune.cu): AUTO accuracy -> 1 = the guarded FP16 split (kTcModeF16Guard), 0 = FMA.
 int tuned_gemm_auto(DeviceCtx* c, int64_t M, int64_t N, int64_t K, cudaStream_t stream);
 // Autotuner: split-K parts and CTA form of one tensor-core GEMM.
-TcLaunchOpts tuned_tc_opts(DeviceCtx* c, int mode, int64_t M, int64_t N, int64_t K, cudaStream_t stream);
+TcLaunchOpts tuned_tc_opts(DeviceCtx* c, int mode, const gbblas_gemm_desc& g, cudaStream_t stream);
 // Autotuner: FP32 FMA tile (launch_gemm_fma's `tile`).
 int tuned_fma_tile(DeviceCtx* c, const gbblas_gemm_desc& g, cudaStream_t stream);
 

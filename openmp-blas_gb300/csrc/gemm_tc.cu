@@ -2227,10 +2227,7 @@ gbblas_status plan_group(DeviceCtx* c, int mode, const gbblas_gemm_desc* d, int6
   bool want_pair = opt.pair == 1;
   if (opt.pair < 0)
     if (const char* e = std::getenv("GBBLAS_TC_PAIR"); e && e[0] == '1') want_pair = true;
-  // no contiguous rows of C off the 16-byte grid
-  const bool c_ok = std::all_of(order.begin(), order.end(), [&](int64_t i) {
-    return d[i].csc != 1 || ((d[i].rsc & 3) == 0 && (reinterpret_cast<uintptr_t>(d[i].C) & 15) == 0);
-  });
+  const bool c_ok = std::all_of(order.begin(), order.end(), [&](int64_t i) { return tc_c_on_grid(d[i]); });
   if (want_pair && mode != kModeFp8 && mode != kModeF16) {
     double w1 = 0, w2 = 0;
     for (int64_t i : order) {
@@ -2817,7 +2814,7 @@ gbblas_status launch_gemm_tc(DeviceCtx* c, int mode, int64_t M, int64_t N, int64
                              int64_t csc, cudaStream_t stream) {
   if (M == 0 || N == 0 || K == 0) return GBBLAS_STATUS_SUCCESS;
   gbblas_gemm_desc d{M, N, K, A, rsa, csa, B, rsb, csb, C, rsc, csc};
-  return launch_gemm_tc_opts(c, mode, d, tuned_tc_opts(c, mode, d.M, d.N, d.K, stream), stream);
+  return launch_gemm_tc_opts(c, mode, d, tuned_tc_opts(c, mode, d, stream), stream);
 }
 
 }  // namespace gbblas

@@ -377,7 +377,8 @@ static int split_parts(DeviceCtx* c, int mode, int64_t M, int64_t N, int64_t K) 
   return best;
 }
 
-TcLaunchOpts tuned_tc_opts(DeviceCtx* c, int mode, int64_t M, int64_t N, int64_t K, cudaStream_t stream) {
+TcLaunchOpts tuned_tc_opts(DeviceCtx* c, int mode, const gbblas_gemm_desc& g, cudaStream_t stream) {
+  const int64_t M = g.M, N = g.N, K = g.K;
   TcLaunchOpts def;
   if (const char* e = std::getenv("GBBLAS_TC_SPLITK"); e && std::atoi(e) > 0) {
     def.split = std::atoi(e);
@@ -385,13 +386,14 @@ TcLaunchOpts tuned_tc_opts(DeviceCtx* c, int mode, int64_t M, int64_t N, int64_t
   }
   def.split = split_parts(c, mode, M, N, K);
   // GBBLAS_TC_PAIR, when set, fixes the CTA form; otherwise the tuner picks it
-  // (pairs only where padding M to 256 rows adds at most 10 % of the work)
+  // (pairs only where padding M to 256 rows adds at most 10 % of the work, and
+  // where C admits them: elsewhere the plan would drop the pairs and the split
+  // with them)
   const char* pe = std::getenv("GBBLAS_TC_PAIR");
   const bool pair_env = pe && pe[0];
   def.pair = pair_env ? -1 : 0;
   const bool pairs = !pair_env && mode != tc_mode(GBBLAS_ACCURACY_FP8) && mode != tc_mode(GBBLAS_ACCURACY_FP16X3) &&
-                     mode != kTcModeF16Guard &&
-                     M >= 256 &&
+                     mode != kTcModeF16Guard && tc_c_on_grid(g) && M >= 256 &&
                      (double)((M + 255) / 256 * 256) <= 1.1 * (double)((M + 127) / 128 * 128);
   if (!pairs) return def;
   Tuner& t = Tuner::get();
