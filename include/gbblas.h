@@ -225,8 +225,8 @@ gbblas_status gbblas_dgemv(gbblas_layout la, int transpose, int64_t M, int64_t N
 /* *result = sum_i a[i] * b[i] over n elements; result is a DEVICE pointer.
  *                                             replaces amt::dot_prod,
  * reference include/dot.hpp:176-224 (helper 143-174).  Single precision
- * keeps Kahan-compensated FP32 partials and combines them in FP64, so it is
- * at least as accurate as the reference's blocked OpenMP reduction.
+ * keeps Kahan-compensated FP32 partials, combines them as unevaluated pairs of
+ * floats (46 bits) within a warp and in FP64 beyond it, so it is at least as accurate as the reference's blocked OpenMP reduction.
  * n == 0 writes 0. */
 gbblas_status gbblas_sdot(int64_t n, const float* a, const float* b, float* result, void* stream);
 gbblas_status gbblas_ddot(int64_t n, const double* a, const double* b, double* result, void* stream);
@@ -236,7 +236,7 @@ gbblas_status gbblas_ddot(int64_t n, const double* a, const double* b, double* r
  * point exists for GPU callers that cannot allocate device memory when they
  * call (a caller-owned memory pool or a pre-reserved serving loop that must
  * not grow, or a foreign-language binding without access to cudaMalloc).
- * It computes the same result as gbblas_sdot but calls no cudaMalloc,
+ * It computes the same result, bit for bit, as gbblas_sdot but calls no cudaMalloc,
  * cudaFree or other allocating routine: its reduction scratch is one fixed
  * 33,024-byte device array inside the library (room for 4096 per-CTA
  * partials; a GB300 uses at most 608), which every GPU that loads the

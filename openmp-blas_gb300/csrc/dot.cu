@@ -3,14 +3,15 @@
 // Reference: include/dot.hpp:143-174 picks one of three CPU regimes by size
 // (serial SIMD below 2*L1, OpenMP-static L1/2 blocks below L3, L2/2 x L1/2
 // two-level blocks above) and combines per-thread partials with an OpenMP
-// reduction.  On the GPU one regime fits every size: a grid of
-// (SMs x resident CTAs) threads streams both vectors once with 128-bit
-// read-only loads, each thread keeps its own partial sums, CTAs reduce with
-// warp shuffles, the CTAs of each thread-block cluster (kDotCluster CTAs)
-// add their totals through distributed shared memory in rank order, and the
-// last cluster to finish adds the per-cluster partials in index order.  The
-// order of every addition is fixed by n and the grid size, so results are
-// bit-reproducible run to run.
+// reduction.  On the GPU one kernel serves every size: a grid of threads
+// streams both vectors once with 128-bit read-only loads, each thread keeps its
+// own partial sums, and CTAs reduce with warp shuffles.  Short vectors go to
+// one CTA, or to one thread-block cluster whose rank 0 adds the CTAs' totals
+// through distributed shared memory in rank order; longer ones to up to (SMs x
+// resident CTAs) CTAs - in clusters of kDotCluster once those are reached -
+// whose totals the last to finish adds in index order (dot_shape).  The order of every
+// addition is fixed by n and the number of SMs, so results are bit-reproducible
+// run to run, and gbblas_sdot_noalloc's are gbblas_sdot's.
 //
 // Accuracy: FP32 partials are Kahan-compensated (products and sums rounded
 // with __fmul_rn / __fadd_rn so the compiler cannot contract them into FMAs
@@ -281,28 +282,53 @@ cudaError_t launch_dot_kernel(bool vec, int grid, int cluster, cudaStream_t stre
 
 }  // namespace
 
+namespace {
+
+// The CTAs of a dot over n elements.  `brief`: kDotOneThreads threads each,
+// one CTA or one cluster, no scratch; else kDotThreads, with grid / cluster
+// partials.
+struct DotShape {
+  bool brief;
+  int64_t grid;
+  int cluster;
+};
 template <typename T>
-gbblas_status launch_dot(DeviceCtx* c, int64_t n, const T* a, const T* b, T* result, cudaStream_t stream) {
-  const bool vec = aligned16(a) && aligned16(b);
+DotShape dot_shape(int64_t n, int num_sms) {
   const int64_t bytes = n * (int64_t)sizeof(T);
   if (bytes <= 8 * kDotOne<T>) {
     const int ctas = (int)std::max<int64_t>(1, (bytes + kDotOne<T> - 1) / kDotOne<T>);
-    GB_CUDA_TRY((launch_dot_kernel<T, kDotOneThreads>(vec, ctas, ctas, stream, a, b, n, nullptr, nullptr, result)));
-    return check_launch("dot_kernel");
+    return {true, ctas, ctas};
   }
   const int64_t per_cta = (int64_t)kDotThreads * kDotUnroll * Vec<T>::width;
-  int64_t want = (n + per_cta - 1) / per_cta;
-  const int64_t full = (int64_t)c->num_sms * kDotCtasPerSm;
+  const int64_t want = (n + per_cta - 1) / per_cta, full = (int64_t)num_sms * kDotCtasPerSm;
   // clusters only once the grid is full (fewer partials for the last one to
   // add); below that their barriers only add latency
   const int cluster = want >= full ? kDotCluster : 1;
-  int grid = (int)std::min(want, full);
-  grid = (grid + cluster - 1) / cluster * cluster;  // whole clusters
-  void* s = nullptr;
-  GB_TRY(get_scratch(c, stream, kScratchZeroBytes + sizeof(double) * (grid / cluster), &s));
-  unsigned* counter = reinterpret_cast<unsigned*>(s);
-  double* partials = reinterpret_cast<double*>(static_cast<char*>(s) + kScratchZeroBytes);
-  GB_CUDA_TRY(launch_dot_kernel<T>(vec, grid, cluster, stream, a, b, n, partials, counter, result));
+  return {false, (std::min(want, full) + cluster - 1) / cluster * cluster, cluster};  // whole clusters
+}
+
+template <typename T>
+cudaError_t launch_dot_shape(const DotShape& d, cudaStream_t stream, const T* a, const T* b, int64_t n,
+                             double* partials, unsigned* counter, T* result) {
+  const bool vec = aligned16(a) && aligned16(b);
+  return d.brief ? launch_dot_kernel<T, kDotOneThreads>(vec, (int)d.grid, d.cluster, stream, a, b, n, nullptr, nullptr, result)
+                 : launch_dot_kernel<T>(vec, (int)d.grid, d.cluster, stream, a, b, n, partials, counter, result);
+}
+
+}  // namespace
+
+template <typename T>
+gbblas_status launch_dot(DeviceCtx* c, int64_t n, const T* a, const T* b, T* result, cudaStream_t stream) {
+  const DotShape d = dot_shape<T>(n, c->num_sms);
+  unsigned* counter = nullptr;
+  double* partials = nullptr;
+  if (!d.brief) {
+    void* s = nullptr;
+    GB_TRY(get_scratch(c, stream, kScratchZeroBytes + sizeof(double) * (d.grid / d.cluster), &s));
+    counter = reinterpret_cast<unsigned*>(s);
+    partials = reinterpret_cast<double*>(static_cast<char*>(s) + kScratchZeroBytes);
+  }
+  GB_CUDA_TRY(launch_dot_shape<T>(d, stream, a, b, n, partials, counter, result));
   return check_launch("dot_kernel");
 }
 
@@ -393,21 +419,16 @@ extern "C" gbblas_status gbblas_sdot_noalloc(int64_t n, const float* a, const fl
   NoAllocDev* d = nullptr;
   GB_TRY(noalloc_setup(&d));
   cudaStream_t s = as_stream(stream);
-  const bool vec = aligned16(a) && aligned16(b);
-  const int64_t per_cta = (int64_t)kDotThreads * kDotUnroll * 4;
-  const int64_t want = (n + per_cta - 1) / per_cta;
-  const int64_t full = (int64_t)d->num_sms * kDotCtasPerSm;
-  int64_t grid = want < full ? (want < 1 ? 1 : want) : full;
-  grid = (grid + kDotCluster - 1) / kDotCluster * kDotCluster;  // whole clusters
-  if (grid > kNoAllocMaxCtas) {
+  const DotShape shape = dot_shape<float>(n, d->num_sms);
+  if (shape.grid > kNoAllocMaxCtas) {
     set_error("gbblas_sdot_noalloc: needs %lld reduction slots, the fixed scratch holds %d",
-              (long long)grid, kNoAllocMaxCtas);
+              (long long)shape.grid, kNoAllocMaxCtas);
     return GBBLAS_STATUS_NOT_SUPPORTED;
   }
   unsigned* counter = static_cast<unsigned*>(d->scratch);
   double* partials = reinterpret_cast<double*>(static_cast<char*>(d->scratch) + kScratchZeroBytes);
   // The counter must start at zero; partials are fully rewritten by each call.
-  GB_CUDA_TRY(cudaMemsetAsync(counter, 0, sizeof(unsigned), s));
-  GB_CUDA_TRY(launch_dot_kernel<float>(vec, (int)grid, kDotCluster, s, a, b, n, partials, counter, result));
+  if (!shape.brief) GB_CUDA_TRY(cudaMemsetAsync(counter, 0, sizeof(unsigned), s));
+  GB_CUDA_TRY(launch_dot_shape<float>(shape, s, a, b, n, partials, counter, result));
   return check_launch("dot_kernel (noalloc)");
 }

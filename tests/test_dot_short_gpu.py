@@ -52,3 +52,17 @@ def test_not_finite_stays_not_finite(cuda, bad, n):
     a[n // 3] = bad
     assert not np.isfinite(gpu_dot(cuda, a, b))
     assert not np.isfinite(gpu_dot(cuda, a.astype(np.float64), b.astype(np.float64)))
+
+
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("n", [0, 1] + EDGES + [2500000, 2600001])  # (... and the full grid, in clusters)
+def test_allocation_free_form_gives_the_same_bits(cuda, n, offset):
+    import gbblas
+    torch = cuda
+    g = torch.Generator(device="cuda").manual_seed(n)
+    a, b = (torch.rand(n + offset, generator=g, device="cuda") * 2 - 1 for _ in range(2))
+    out = torch.full((2,), 7.0, device="cuda")
+    for i, fn in enumerate(("gbblas_sdot", "gbblas_sdot_noalloc")):
+        gbblas.call(fn, n, a[offset:].data_ptr(), b[offset:].data_ptr(), out[i:].data_ptr(), None)
+    torch.cuda.synchronize()
+    assert out[0].item() == out[1].item()
