@@ -347,7 +347,10 @@ gbblas_status launch_cfg(DeviceCtx* c, int64_t M, int64_t N, int64_t K, const T*
   const int la = mode(A, rsa, csa), lb = mode(B, csb, rsb);
   const int64_t tiles_n = (N + BN - 1) / BN, ntiles = tiles_n * ((M + BM - 1) / BM);
   int64_t g = ntiles;
-  if (max_ctas > 0) g = std::min<int64_t>(g, std::max(1, max_ctas / parts));
+  if (max_ctas > 0) {
+    parts = std::min(parts, max_ctas);
+    g = std::min<int64_t>(g, max_ctas / parts);
+  }
   if (g > 0x7fffffff) g = 0x7fffffff;
   set_attributes<T, BM, BN, TM, TN>(c);
   cudaLaunchConfig_t cfg = {};

@@ -75,3 +75,21 @@ def test_split_within_bound_and_repeats(cuda, monkeypatch, dtype, tile, M, N, K)
         got = gemm(cuda, A, B, C0, la, lb, lc, 1)
         assert np.all(np.abs(got - exact) <= tol)
         np.testing.assert_array_equal(gemm(cuda, A, B, C0, la, lb, lc, 1), got)
+
+
+def test_split_stays_within_the_servers_cta_cap(cuda, monkeypatch):
+    """A heavy request capped to one CTA takes its tiles whole: the unsplit
+    form's bits, not those of K cut over a cluster of eight."""
+    import gbblas
+    A, B, C0 = operands(37, 70, 5000, np.float32, 5)
+    monkeypatch.setenv("GBBLAS_FMA_TILE", "0")
+    whole = gemm(cuda, A, B, C0, 1, 1, 1)
+    monkeypatch.setenv("GBBLAS_FMA_TILE", "5")
+    assert not np.array_equal(gemm(cuda, A, B, C0, 1, 1, 1), whole)
+    monkeypatch.delenv("GBBLAS_FMA_TILE")
+    a, b, c = (cuda.from_numpy(x.copy()).cuda() for x in (A, B, C0))
+    srv = gbblas.Server(streams=1, heavy_us=1, heavy_sm_percent=1, slice_us=-1)
+    srv.wait(srv.submit(gbblas.Request(gbblas.OP_MTM, gbblas.F32, gbblas.ACCURACY_FP32, gbblas.LAST_ORDER, 37, 70, 5000,
+                                       a.data_ptr(), b.data_ptr(), c.data_ptr())))
+    srv.close()
+    np.testing.assert_array_equal(c.cpu().numpy(), whole)
