@@ -142,8 +142,8 @@ struct DgProblem {
   int64_t rsc, csc;
   const int* ea;  // [rows of A, padded] row scales
   const int* eb;  // [columns of B, padded] column scales
-  const unsigned* ga;  // guarded form: the rows' (columns') sampled sums of the guard plane, from kArrivedBase (or null)
-  const unsigned* gb;
+  const unsigned long long* ga;  // guarded form: the rows' (columns') sampled sums of the guard plane, or null
+  const unsigned long long* gb;
   // guarded form: the 32 x 16 blocks the guard rejected (block b of tile t
   // = t * 8 + epilogue warp), recomputed on the FP64 pipes from A and B
   int* fix_count;
@@ -161,9 +161,12 @@ struct DgProblem {
 // inside the FP64 pipes' bound 2 K eps (|A||B| + |C|).
 constexpr int kGuardMin = 1 << 14;
 constexpr int kGuardCap = 1 << 30;  // the guard sums saturate here (int32)
-// Sampled row sum of a row left out of the sampling's choice: above any real
-// one (127 x 32 per 128 of K, below 2^25 at the longest K).
-constexpr unsigned kNoGuardSum = 1u << 30;
+// A row's sampled sums of the guard plane: the sum in the low word, that of the
+// squares, in sixteens, in the high one (at most 2^25 and 2^28 at the longest
+// K), from the fill byte 0x80 on.  kNoGuardSum, above any real sum and without
+// squares: a row left out of the sampling's choice.
+constexpr unsigned long long kGuardSumBase = 0x8080808080808080ull;
+constexpr unsigned long long kNoGuardSum = 1ull << 30;
 
 // ------------------------------------------------------ operand preparation
 // Row scales: e[r] = the exponent frexp gives for max_k |src(r, k)| (so the
@@ -181,7 +184,7 @@ struct DgOperand {
   const double* src;
   int64_t rows, K, rs, cs;  // element (r, k) at src[r*rs + k*cs]
   int* e;                   // row scales
-  unsigned* gsum;           // guard: the rows' sampled sums of the guard plane (start at kArrivedBase)
+  unsigned long long* gsum; // guard: the rows' sampled sums of the guard plane (start at kGuardSumBase)
   __nv_bfloat16* out;       // digit planes
   int64_t plane_stride, pitch;
   int tiles_k;              // CTAs per 32 rows (K tiles of the kernel at hand)
@@ -339,7 +342,7 @@ __global__ void __launch_bounds__(256) digits_kernel(const DgOperand oa, const D
   const double* __restrict__ src = o.src;
   const int64_t rows = o.rows, K = o.K, rs = o.rs, cs = o.cs, plane_stride = o.plane_stride, pitch = o.pitch;
   const int* e_row = o.e;
-  unsigned* __restrict__ gsum_row = o.gsum;
+  unsigned long long* __restrict__ gsum_row = o.gsum;
   __nv_bfloat16* __restrict__ out = o.out;
   const int tid = threadIdx.x;
   const int64_t r0 = (int64_t)(blk / o.tiles_k) * 32, k0 = (int64_t)(blk % o.tiles_k) * 32;
@@ -380,16 +383,23 @@ __global__ void __launch_bounds__(256) digits_kernel(const DgOperand oa, const D
     w.x = *reinterpret_cast<const uint32_t*>(&h01);
     w.y = *reinterpret_cast<const uint32_t*>(&h23);
     *reinterpret_cast<uint2*>(dst + S * plane_stride) = w;
-    // the row's sum over the first 32 of every 128 K (8 threads a row), for the
-    // GEMM's choice of how much of K the guard samples.  The guard rejects the
-    // blocks of a zero row, or one with Inf or NaN, however much is sampled:
-    // its sum is set beyond any other, so that it does not weigh in the choice.
+    // the row's sum and sum of squares (in sixteens) over the first 32 of every
+    // 128 K (8 threads a row), for the GEMM's choice of how much of K the guard
+    // samples.  The guard rejects the blocks of a zero row, or one with Inf or
+    // NaN, however much is sampled: its sum is set beyond any other, so that it
+    // does not weigh in the choice.
     if (k0 % 128 == 0 && gsum_row) {
-      int sum = (int)(g(d[0][0]) + g(d[1][0]) + g(d[2][0]) + g(d[3][0]));
+      unsigned both = 0;  // sum below bit 13 (at most 32 x 127), squares from it (at most 32 x 127^2)
 #pragma unroll
-      for (int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-      if (er == kZeroExp || er == kBadExp) sum = k0 == 0 ? (int)kNoGuardSum : 0;
-      if ((tid & 7) == 0 && r0 + r < rows && sum) atomicAdd(gsum_row + r0 + r, (unsigned)sum);
+      for (int j = 0; j < 4; ++j) {
+        const unsigned v = (unsigned)max(abs(d[j][0]) - 1, 0);
+        both += v * v << 13 | v;
+      }
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) both += __shfl_xor_sync(0xffffffffu, both, o);
+      unsigned long long sum = (unsigned long long)(both >> 17) << 32 | (both & 0x1FFFu);
+      if (er == kZeroExp || er == kBadExp) sum = k0 == 0 ? kNoGuardSum : 0;
+      if ((tid & 7) == 0 && r0 + r < rows && sum) atomicAdd(gsum_row + r0 + r, sum);
     }
   }
 }
@@ -533,23 +543,31 @@ __global__ void __launch_bounds__(kThreads, 1)
   };
 
   const int items = dg_items(p);
-  // The guard's sampling of a tile: the first 32 of every 128 K, or, where the
-  // guard planes' sums over those say that some output's lower bound may fall
-  // short, all of K.  (The smallest row sum of the tile times its smallest
-  // column sum over the number of K sampled estimates an output's sum; it has
-  // to be four times the limit.)  Either sum is a lower bound; the full one
-  // takes a third more shared-memory traffic and keeps operands whose
-  // magnitudes spread over many binades, few of them large at once, off the
-  // FP64 pipes: exponents of +-10 at 1531 x 1400 x 1601, 6435 us with the
-  // quarter, 266 with all.  By tile, so that a few thin rows cost no more than
-  // their own tiles, and no CTA reads more than 160 sums at a time (one choice
-  // for the product, from all M + N sums in every CTA: 10^6 x 32 x 1000 10.11
-  // ms, now 9.82; 1531 x 1400 x 1601 224 us, now 221, with a zero row 955 and
-  // 909, the rest being that row's blocks on the pipes).  The MMA warp and the guard producer each read the sums when they
-  // come to a tile and need them after its first stage, which is sampled
-  // either way.
+  // The guard's sampling of a tile: the first 32 of every 128 K, or all of K.
+  // Either sum is a lower bound; the full one takes a third more shared-memory
+  // traffic and keeps operands whose magnitudes spread over many binades, few of
+  // them large at once, off the FP64 pipes (exponents of +-10 at 1531 x 1400 x
+  // 1601: 6435 us with the quarter, 268 with all), where a single block costs
+  // more than a tile.  The quarter is taken where no output should fall short of
+  // the limit L by it.  The tile's smallest row sum times its smallest column
+  // sum over the number n of sampled K estimates the smallest output sum, R in
+  // units of L, and n times the largest ratios of squares' sum to square of the
+  // sum the output sums' relative variance s^2: R has to be 4, or 1 + 2.75
+  // deviations, (1 - 1/R) >= 2.75 s.  Over thirteen distributions of operands
+  // (uniform, normal, exponential, log-normal, exponents of +-2 to +-10, 50 to
+  // 80 % zeros), by model: of 19000 tiles with 2.75 deviations one had an output
+  // below L, of 13000 with 2.5 to 2.75 five.  The estimate alone, R >= 4, made
+  // operands that the quarter serves pay for all: normal ones at 2048 x 2048 x
+  // 1500 437 us, now 360, exponential ones over K = 4000 1104, now 878.
+  // By tile, so that a few thin rows cost no more than their own tiles, and no
+  // CTA reads more than 160 sums at a time (one choice for the product, from all
+  // M + N sums in every CTA: 10^6 x 32 x 1000 10.11 ms, by tile 9.82; 1531 x 1400
+  // x 1601 with a zero row 955 us and 909, the rest being that row's blocks on
+  // the pipes).  The MMA warp and the guard producer each read the sums when they
+  // come to a tile and need them after its first stage, which is sampled either
+  // way.
   struct TileSums {
-    unsigned a[kBM / 32], b;
+    unsigned long long a[kBM / 32], b;
   };
   auto tile_sums = [&](int m0, int n0) {  // lane l: rows l, l + 32, ..., column l
     TileSums t = {{kNoGuardSum, kNoGuardSum, kNoGuardSum, kNoGuardSum}, kNoGuardSum};
@@ -557,18 +575,31 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
     for (int i = 0; i < kBM / 32; ++i) {
       const int row = m0 + 32 * i + lane;
-      t.a[i] = row < p.M ? __ldcg(p.ga + row) - kArrivedBase : kNoGuardSum;
+      if (row < p.M) t.a[i] = __ldcg(p.ga + row) - kGuardSumBase;
     }
-    t.b = n0 + lane < p.N ? __ldcg(p.gb + n0 + lane) - kArrivedBase : kNoGuardSum;
+    if (n0 + lane < p.N) t.b = __ldcg(p.gb + n0 + lane) - kGuardSumBase;
     return t;
   };
   auto sample_all = [&](const TileSums& t) {
-    unsigned la = t.a[0];
+    unsigned la = (unsigned)t.a[0];
 #pragma unroll
-    for (int i = 1; i < kBM / 32; ++i) la = min(la, t.a[i]);
+    for (int i = 1; i < kBM / 32; ++i) la = min(la, (unsigned)t.a[i]);
     la = __reduce_min_sync(0xffffffffu, la);
-    const unsigned lb = __reduce_min_sync(0xffffffffu, t.b);
-    return (float)la * (float)lb < 4.0f * (float)kGuardMin * 32.0f * (float)((p.K + 127) / 128);
+    const unsigned lb = __reduce_min_sync(0xffffffffu, (unsigned)t.b);
+    const float n = 32.0f * (float)((p.K + 127) / 128), nl = n * (float)kGuardMin, est = (float)la * (float)lb;
+    if (est >= 4.0f * nl) return false;
+    if (est <= nl) return true;
+    auto ratio = [](unsigned long long v) {  // (the sum is not zero here)
+      const float sum = (float)(unsigned)v;
+      return __float_as_uint(__fdividef(16.0f * (float)(unsigned)(v >> 32), sum * sum));
+    };
+    unsigned ca = ratio(t.a[0]);
+#pragma unroll
+    for (int i = 1; i < kBM / 32; ++i) ca = max(ca, ratio(t.a[i]));
+    ca = __reduce_max_sync(0xffffffffu, ca);
+    const unsigned cb = __reduce_max_sync(0xffffffffu, ratio(t.b));
+    const float x = 1.0f - __fdividef(nl, est), var = n * __uint_as_float(ca) * __uint_as_float(cb);
+    return x * x < 2.75f * 2.75f * var;
   };
   int issued = 0;  // A producer: stages whose copies were issued
   if ((warp == 0 || warp == kBProdWarp) && lane == 0) {
@@ -972,13 +1003,15 @@ DgLayout dg_layout(int sms, int digits, bool guarded, int64_t M, int64_t N, int6
   const int64_t chunk = chunk_stages(digits), chunks = (l.kp / kBK + chunk - 1) / chunk;
   l.parts = level == DgScratch::kCut ? rest_parts(l.rest, chunks, l.ctas) : 1;
   const size_t rows = align256(sizeof(int) * (size_t)l.mp), cols = align256(sizeof(int) * (size_t)l.np);
+  const size_t row_sums = align256(sizeof(unsigned long long) * (size_t)l.mp),
+               col_sums = align256(sizeof(unsigned long long) * (size_t)l.np);
   const bool sums = guarded && level != DgScratch::kLeast;
   l.arr = kScratchZeroBytes;
   l.ea = l.arr + (l.parts > 1 ? kArrivedBytes : 0);
   l.eb = l.ea + rows;
   l.ga = l.eb + cols;
-  l.gb = l.ga + (sums ? rows : 0);
-  l.a = l.gb + (sums ? cols : 0);
+  l.gb = l.ga + (sums ? row_sums : 0);
+  l.a = l.gb + (sums ? col_sums : 0);
   l.b = l.a + align256((size_t)(planes * l.mp * l.kp) * sizeof(__nv_bfloat16));
   l.fix = l.b + align256((size_t)(planes * l.np * l.kp) * sizeof(__nv_bfloat16));
   l.slots = l.fix + (guarded ? align256(sizeof(int) * (size_t)(1 + l.tiles * kEpiWarps)) : 0);
@@ -1047,8 +1080,8 @@ gbblas_status launch_digits(DeviceCtx* c, int64_t M, int64_t N, int64_t K, const
   const int stk = (int)((K + kScaleTK - 1) / kScaleTK);
   const int tiles_k = (int)(Kp / 32);
   const bool sums = G && level != DgScratch::kLeast;
-  unsigned* gsa = sums ? reinterpret_cast<unsigned*>(base + l.ga) : nullptr;
-  unsigned* gsb = sums ? reinterpret_cast<unsigned*>(base + l.gb) : nullptr;
+  auto* gsa = sums ? reinterpret_cast<unsigned long long*>(base + l.ga) : nullptr;
+  auto* gsb = sums ? reinterpret_cast<unsigned long long*>(base + l.gb) : nullptr;
   DgOperand oa{A, M, K, rsa, csa, ea, gsa, da, (int64_t)a_plane, Kp, stk, (int)((Mp / 32) * stk)};
   DgOperand ob{B, N, K, csb, rsb, eb, gsb, db, (int64_t)b_plane, Kp, stk, (int)((Np / 32) * stk)};
   if ((double)(Mp + Np) / 32 * tiles_k >= 2.0e9) {

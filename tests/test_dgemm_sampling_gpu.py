@@ -69,3 +69,21 @@ def test_choices_mixed_over_tiles(cuda, M, N, K):
     exact = A.astype(np.longdouble) @ B.astype(np.longdouble) + 0.25
     assert np.all(np.abs(got - exact) <= 2 * K * 2.0 ** -52 * (np.abs(A) @ np.abs(B) + 0.25))
     np.testing.assert_array_equal(product(cuda, A, B), got)
+
+
+def test_the_quarter_where_its_sums_vary_little(cuda):
+    """Sums whose smallest product is three times the limit and varies by a
+    twentieth: the quarter is taken.  Shown on operands built so that it rejects
+    every block (never large at the same sampled k), which are then sums of
+    fused multiply-adds in order of k, as the pipes add them."""
+    from fractions import Fraction
+    M, N, K = 128, 32, 16384
+    A, B = turns_on_the_choice(M, N, K, np.random.default_rng(3))
+    A, B = A / 8, B / 8
+    A[:, 100], B[101, :] = 0.75, 0.75  # (not sampled) the rows' and columns' largest, digits of 96
+    got = product(cuda, A, B)
+    for i, j in ((0, 0), (77, 13), (127, 31)):
+        s = 0.0
+        for x, y in zip(A[i].tolist(), B[:, j].tolist()):
+            s = float(Fraction(x) * Fraction(y) + Fraction(s))
+        assert got[i, j] == s + 0.25
