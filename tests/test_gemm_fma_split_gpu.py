@@ -93,3 +93,13 @@ def test_split_stays_within_the_servers_cta_cap(cuda, monkeypatch):
                                        a.data_ptr(), b.data_ptr(), c.data_ptr())))
     srv.close()
     np.testing.assert_array_equal(c.cpu().numpy(), whole)
+
+
+@pytest.mark.parametrize("la,lb,lc", [(1, 1, 1), (0, 1, 0), (1, 0, 1)])
+@pytest.mark.parametrize("K", [1, 2, 7, 15, 16, 17, 31, 33])
+def test_double_adds_nothing_beyond_k(cuda, K, la, lb, lc):
+    """Products that underflow to -0 into a C of -0: every sum is -0, unless a
+    k that does not exist adds its +0 (and takes the time of one that does)."""
+    A, B = np.full((70, K), -1e-200), np.full((K, 67), 1e-200)
+    got = gemm(cuda, A, B, np.full((70, 67), -0.0), la, lb, lc, 1)
+    assert np.all(got == 0) and np.all(np.signbit(got))
