@@ -13,8 +13,9 @@
 //              simd_loop.hpp:52-78, accumulates into y) and vtm with
 //              row-major A.
 //
-// Both stream A from HBM once with 128-bit read-only loads at any leading
-// dimension and keep x in L1 / shared memory.  When the grid would be too
+// Both stream A from HBM once, with 128-bit read-only loads (columns off the
+// 16-byte grid: of single elements, except for large float matrices), and keep x
+// in L1 / shared memory.  When the grid would be too
 // small to fill the 152 SMs the reduction dimension is split across CTAs.
 // Up to 8 splits of a small matrix run as one thread-block cluster per row
 // block: each CTA leaves its partials in its shared memory and the
@@ -106,12 +107,16 @@ __device__ __forceinline__ T warp_totals(const T (&v)[4], int lane) {
 // elements up to it and its last few are added one by one, everything between
 // by 128-bit loads, and x is read once for all R rows (by vectors where it
 // shares their alignment).  grid = (groups / groups per CTA, ksplit); split p
-// covers vectors p * vps .. + vps - 1.
+// covers vectors p * vps .. + vps - 1.  The last vectors of a row, fewer than U
+// a lane, are loaded together too: one after another they cost a round trip to
+// memory each (f32 4096 x 512, four vectors a row and lane: 5.8 us, 4.3 so).
+// AL: every row and x start on 16-byte boundaries; CTAS: resident CTAs an SM.
 // CL: the ksplit CTAs of a row block form a cluster (1, ksplit, 1).
-template <typename T, int R, bool CL>
-__global__ void __launch_bounds__(kRowsThreads, R == 4 ? 3 : 4)
+template <typename T, int R, bool AL, bool CL, int CTAS>
+__global__ void __launch_bounds__(kRowsThreads, CTAS)
     gemv_rows_kernel(int64_t rows, int64_t cols, const T* __restrict__ A, int64_t lda, const T* __restrict__ x,
-                     T* __restrict__ y, bool accumulate, T* __restrict__ partials, int64_t vps, int lperiod, int lwc) {
+                     T* __restrict__ y, bool accumulate, T* __restrict__ partials, int64_t vps, int lp, int lwc) {
+  const int lperiod = AL ? 0 : lp;
   using VT = typename V<T>::t;
   constexpr int W = V<T>::w;
   constexpr int U = R == 4 ? 2 : 4;  // vectors per row and lane in flight
@@ -130,60 +135,90 @@ __global__ void __launch_bounds__(kRowsThreads, R == 4 ? 3 : 4)
   const int nr = r0 < rows ? (int)min((rows - r0 + period - 1) >> lperiod, (int64_t)R) : 0;
   const T* __restrict__ row = A + (nr > 0 ? r0 : 0) * lda;
   const int64_t rstep = lda << lperiod;
-  int64_t head = (int64_t)(((16 - (reinterpret_cast<uintptr_t>(row) & 15)) & 15) / sizeof(T));
+  int64_t head = AL ? 0 : (int64_t)(((16 - (reinterpret_cast<uintptr_t>(row) & 15)) & 15) / sizeof(T));
   if (head > cols) head = cols;
   const int64_t nv = (cols - head) / W;
   const int64_t v1 = min(((int64_t)blockIdx.y + 1) * vps, nv);
   const T* __restrict__ xb = x + head;
-  const bool xvec = (reinterpret_cast<uintptr_t>(xb) & 15) == 0;
-  auto xload = [&](int64_t v) {
-    VT r;
-    if (xvec) {
-      r = ldg_vec(reinterpret_cast<const VT*>(xb) + v);
-    } else {
-      T* e = reinterpret_cast<T*>(&r);
+  const bool xvec = AL || (reinterpret_cast<uintptr_t>(xb) & 15) == 0;
+  // the elements before the first vector and after the last (R = 1, whose
+  // calls are short: loaded ahead of the rest)
+  T ex = T(0), ea[R];
+  int64_t edge = -1;
+  auto load_edge = [&]() {
+    if (blockIdx.y == 0 && wi == 0) {
+      const int64_t tail = cols - head - nv * W;
+      edge = lane < head ? lane : (lane >= 8 && lane - 8 < tail ? head + nv * W + lane - 8 : -1);
+      if (edge >= 0) {
+        ex = __ldg(x + edge);
 #pragma unroll
-      for (int i = 0; i < W; ++i) e[i] = __ldg(xb + v * W + i);
+        for (int j = 0; j < R; ++j)
+          if (j < nr) ea[j] = dev::ld_stream(row + j * rstep + edge);
+      }
     }
-    return r;
   };
+  if (R == 1) load_edge();
+
   T acc[R];
 #pragma unroll
   for (int j = 0; j < R; ++j) acc[j] = T(0);
-
-  const int64_t step = 32 * wc;
-  int64_t v = (int64_t)blockIdx.y * vps + wi * 32 + lane;
+  const int step = 32 * wc;
+  const int64_t v = (int64_t)blockIdx.y * vps + wi * 32 + lane;
+  const VT* q = reinterpret_cast<const VT*>(row + head) + v;  // this lane's next vector of the first row
+  const T* xq = xb + v * W;                                    // and of x
+  const int64_t rv = rstep / W;                                // the next row's vectors lie this far on
+  int left = (int)(v1 - v) + lane;                             // of the warp's range (32 vectors every `step`), from lane 0 on
+  auto xload = [&](int u) {
+    VT r;
+    if (xvec) {
+      r = ldg_vec(reinterpret_cast<const VT*>(xq) + u * step);
+    } else {
+      T* e = reinterpret_cast<T*>(&r);
+#pragma unroll
+      for (int i = 0; i < W; ++i) e[i] = __ldg(xq + u * step * W + i);
+    }
+    return r;
+  };
   if (nr == R) {
-    for (; v + (U - 1) * step < v1; v += U * step) {
+    for (; left > (U - 1) * step + 31; left -= U * step, q += U * step, xq += U * step * W) {
       VT a[U][R], xv[U];
 #pragma unroll
       for (int u = 0; u < U; ++u)
 #pragma unroll
-        for (int j = 0; j < R; ++j)
-          a[u][j] = dev::ld_stream(reinterpret_cast<const VT*>(row + head + j * rstep) + v + u * step);
+        for (int j = 0; j < R; ++j) a[u][j] = dev::ld_stream(q + j * rv + u * step);
 #pragma unroll
-      for (int u = 0; u < U; ++u) xv[u] = xload(v + u * step);
+      for (int u = 0; u < U; ++u) xv[u] = xload(u);
 #pragma unroll
       for (int u = 0; u < U; ++u)
 #pragma unroll
         for (int j = 0; j < R; ++j) acc[j] = vdot(a[u][j], xv[u], acc[j]);
     }
   }
-  for (; v < v1; v += step) {
-    const VT xv = xload(v);
+  // what is left (of all rows, where they are fewer than R): under predicates,
+  // with its loads in flight together
+  for (; left > 0; left -= U * step, q += U * step, xq += U * step * W) {
+    VT a[U][R], xv[U];
 #pragma unroll
-    for (int j = 0; j < R; ++j)
-      if (j < nr) acc[j] = vdot(dev::ld_stream(reinterpret_cast<const VT*>(row + head + j * rstep) + v), xv, acc[j]);
-  }
-  if (blockIdx.y == 0 && wi == 0) {  // the elements before the first vector and after the last
-    const int64_t tail = cols - head - nv * W;
-    const int64_t c = lane < head ? lane : (lane >= 8 && lane - 8 < tail ? head + nv * W + lane - 8 : -1);
-    if (c >= 0) {
-      const T xc = __ldg(x + c);
+    for (int u = 0; u < U; ++u)
 #pragma unroll
       for (int j = 0; j < R; ++j)
-        if (j < nr) acc[j] = fma(dev::ld_stream(row + j * rstep + c), xc, acc[j]);
+        if (j < nr && left - lane > u * step) a[u][j] = dev::ld_stream(q + j * rv + u * step);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (left - lane > u * step) xv[u] = xload(u);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (left <= u * step) break;  // (the whole warp: no FP64 work on absent vectors)
+#pragma unroll
+      for (int j = 0; j < R; ++j)
+        if (j < nr && left - lane > u * step) acc[j] = vdot(a[u][j], xv[u], acc[j]);
     }
+  }
+  if (R > 1) load_edge();
+  if (edge >= 0) {
+#pragma unroll
+    for (int j = 0; j < R; ++j)
+      if (j < nr) acc[j] = fma(ea[j], ex, acc[j]);
   }
   dev::grid_release();  // a chained finish_splits_kernel may be set up
 
@@ -211,6 +246,50 @@ __global__ void __launch_bounds__(kRowsThreads, R == 4 ? 3 : 4)
     }
     dev::cluster_sync();  // the other splits stay resident until rank 0 has read them
   }
+}
+
+// Row-streaming form of a small matrix, all latency: a warp per row, every load
+// of the row in flight at once - vectors (AL: rows and x on 16-byte boundaries)
+// or elements - and no barrier.  cols at most kShortCols.  us back to back in a
+// graph, by the general form (before its remainder had its loads in flight
+// together) and here: f32 310 x 448 4.1 and 1.7, 64 x 67 2.0 and 1.1, 1000 x 512
+// 2.3 and 1.9; f64 64 x 67 2.5 and 1.8.
+template <typename T>
+constexpr int kShortCols = sizeof(T) == 4 ? 512 : 256;
+template <typename T, bool AL>
+__global__ void __launch_bounds__(kRowsThreads) gemv_rows_short_kernel(int rows, int cols, const T* __restrict__ A,
+                                                                       int64_t lda, const T* __restrict__ x,
+                                                                       T* __restrict__ y, bool accumulate) {
+  using VT = std::conditional_t<AL, typename V<T>::t, T>;
+  constexpr int W = AL ? V<T>::w : 1, U = kShortCols<T> / (32 * W);
+  const int lane = threadIdx.x & 31, r = (int)blockIdx.x * kWarps + (int)(threadIdx.x >> 5);
+  if (r >= rows) return;
+  const T* __restrict__ row = A + r * lda;
+  VT a[U], xv[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+    if (lane + 32 * u < cols / W) {
+      a[u] = dev::ld_stream(reinterpret_cast<const VT*>(row) + lane + 32 * u);
+      xv[u] = __ldg(reinterpret_cast<const VT*>(x) + lane + 32 * u);
+    }
+  const int c = cols / W * W + lane;  // AL: the elements after the last vector
+  T ea = T(0), ex = T(0);
+  if (AL && c < cols) {
+    ea = dev::ld_stream(row + c);
+    ex = __ldg(x + c);
+  }
+  T s = T(0);
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+    if (lane + 32 * u < cols / W) {
+      if constexpr (AL)
+        s = vdot(a[u], xv[u], s);
+      else
+        s = fma(a[u], xv[u], s);
+    }
+  if (AL && c < cols) s = fma(ea, ex, s);
+  s = dev::warp_sum(s);
+  if (lane == 0) y[r] = accumulate ? y[r] + s : s;
 }
 
 // y[r] = (accumulate ? y[r] : 0) + sum_s partials[s*rows + r].  Up to 16
@@ -444,37 +523,61 @@ gbblas_status launch_gemv_rows(DeviceCtx* c, int64_t rows, int64_t cols, const T
   constexpr int W = V<T>::w;
   const int64_t nv = cols / W, sms = c->num_sms;
   const int odd = align_period<T>(lda);
-  // warps per row group: as many as leave each 2 vectors a lane (4 where the
-  // rows are few and the call is all latency: 944 x 1024 f32 4.1 us, 6.2 with 1)
-  const int64_t least = rows >= 16 * sms ? 64 : 128;
-  int lwc = 3;
-  while (lwc > 0 && (nv >> lwc) < least) --lwc;
-  // 4 rows a group once those groups make 3 CTAs per SM (2 where the 4 rows
-  // share x read element by element, or the FP64 additions of their sums):
-  // 1488 x 16384 f32 takes 21 us as 372 CTAs of 4 rows, 18-20 as 1488 of one
-  const int R = (rows << lwc) >= (odd > 0 || sizeof(T) == 8 ? 64 : 96) * sms ? 4 : 1;
+  const bool al = odd == 0 && aligned16(A) && aligned16(x);
+  if (rows <= 1024 && cols <= kShortCols<T>) {
+    const dim3 grid((unsigned)cdiv(rows, kWarps));
+    if (al)
+      gemv_rows_short_kernel<T, true><<<grid, kRowsThreads, 0, stream>>>((int)rows, (int)cols, A, lda, x, y, accumulate);
+    else
+      gemv_rows_short_kernel<T, false><<<grid, kRowsThreads, 0, stream>>>((int)rows, (int)cols, A, lda, x, y, accumulate);
+    return check_launch("gemv_rows_short_kernel");
+  }
+  // Rows per group, warps per group (2^lwc) and column ranges, from a sweep of
+  // 300 shapes of 48 .. 32768 rows and columns, both types, aligned and not, over
+  // every choice, on cold operands back to back in a graph (calls timed from the
+  // host start 4 us apart at best, which hid what small ones take): 2.5-4 % off
+  // the best choice of each shape in the mean.  Four rows a group once the rows
+  // make enough of them; more warps a group while a warp has more than `most`
+  // vectors of a row, or there are few warps and each keeps 32 vectors; fewer
+  // again where the CTAs would be one round of four an SM and a part of another
+  // (double, bound by its FP64 work, up to several); then the columns in ranges
+  // while the CTAs do not fill the SMs and a warp keeps 256 vectors (128, float
+  // and under half a CTA an SM).  us, a CTA per row group / the rule that left
+  // each warp 64 or 128 vectors / now: f32 707 x 3824 4.0 / 5.1 / 4.4, 4096 x 512
+  // 4.1 / 5.7 / 3.4, 32768 x 2048 39.3 / 42.7 / 40.4; f64 740 x 2083 7.3 / 9.8 /
+  // 7.4, 4096 x 1024 21.5 / 15.9 / 12.1, 32768 x 1024 146 / 95 / 66.
+  constexpr bool kF32 = sizeof(T) == 4;
+  const int R = rows >= (kF32 ? 1024 : 3000) ? 4 : 1;
   const int lperiod = R == 1 ? 0 : odd;
   const int64_t groups = cdiv(rows, (int64_t)R << lperiod) << lperiod;
-  const int64_t ctas = cdiv(groups, kWarps >> lwc);
-  // split the columns while the CTAs do not fill the SMs and each warp has
-  // more than 8 vectors a lane
-  // (up to 60 MB only where they are fewer than two an SM, 1.5 for double: the
-  // finish of a split in two costs more than the idle warps do.  Split and not,
-  // us, f32 312 x 23256 17.4 and 14.3, 600 x 23256 21.2 and 18.4, 312 x 200001
-  // 57 and 64; f64 312 x 8192 17.2 and 14.4, 256 x 16000 22.5 and 18.4, 312 x
-  // 50000 42 and 47)
+  const int64_t most = kF32 ? 128 : 256, few = (kF32 ? 8 : 4) * sms;
+  int lwc = 0;
+  while (lwc < 3 && ((nv >> lwc) > most || ((nv >> (lwc + 1)) >= 32 && (groups << lwc) < few))) ++lwc;
+  auto ctas_of = [&](int l) { return cdiv(groups, kWarps >> l); };
+  const int64_t over = (kF32 ? 4 : (R == 1 ? 3 : 8)) * sms, upto = (kF32 ? 6 : 20) * sms;
+  while (lwc > 0 && ctas_of(lwc) > over && ctas_of(lwc) <= upto && (nv >> (lwc - 1)) <= (kF32 ? 2048 : 1024)) --lwc;
+  const int64_t ctas = ctas_of(lwc);
+  // (single rows beyond 60 MB: an incomplete round of CTAs costs more than the
+  // second kernel: f32 312 x 200001 57 us in ranges and 64 whole, 312 x 23256 17.4
+  // and 14.3; f64 312 x 50000 42 and 47, 312 x 8192 17.2 and 14.4)
+  const double bytes = (double)rows * cols * sizeof(T);
+  const int64_t enough = R == 1 && bytes > 60.0e6 ? 5 * sms / 2 : (kF32 ? 3 * sms / 2 : sms);
   int64_t ksplit = 1;
-  const int64_t warps_enough = (double)rows * cols * sizeof(T) > 60.0e6 ? 32 : (sizeof(T) == 8 ? 12 : 16);
-  if (ctas * kWarps < warps_enough * sms) ksplit = std::min(cdiv(48 * sms, ctas * kWarps), nv >> (lwc + 8));
+  if (ctas < enough) ksplit = std::min(cdiv(4 * sms, ctas), nv >> (lwc + (kF32 && ctas < sms / 2 ? 7 : 8)));
   ksplit = std::max<int64_t>(1, std::min<int64_t>(ksplit, 65535));
   const int64_t vps = cdiv(cdiv(nv, ksplit), 32) * 32;
   if (vps > 0) ksplit = std::max<int64_t>(1, cdiv(nv, vps));
   const dim3 grid((unsigned)ctas, (unsigned)ksplit);
-  if (R == 4)
-    return launch_split<T>(c, gemv_rows_kernel<T, 4, true>, gemv_rows_kernel<T, 4, false>, grid, rows, cols, y,
-                           accumulate, stream, "gemv_rows_kernel", A, lda, x, vps, lperiod, lwc);
-  return launch_split<T>(c, gemv_rows_kernel<T, 1, true>, gemv_rows_kernel<T, 1, false>, grid, rows, cols, y,
-                         accumulate, stream, "gemv_rows_kernel", A, lda, x, vps, lperiod, lwc);
+  // (CTAs an SM: float's four rows on boundaries fit four, and take them except
+  // from 300 MB on, where three read DRAM better: 16384^2 157 us with four, 151
+  // with three; 16384 x 8192 81 and 78; 2048 x 32768 42 and 47, 8192 x 1024 7.0 and 7.9)
+  const bool huge = kF32 && bytes > 300.0e6;
+#define GB_ROWS(R_, AL_, CTAS_)                                                                                   \
+  launch_split<T>(c, gemv_rows_kernel<T, R_, AL_, true, CTAS_>, gemv_rows_kernel<T, R_, AL_, false, CTAS_>, grid, \
+                  rows, cols, y, accumulate, stream, "gemv_rows_kernel", A, lda, x, vps, lperiod, lwc)
+  if (R == 4) return !al ? GB_ROWS(4, false, 3) : (kF32 && !huge ? GB_ROWS(4, true, (kF32 ? 4 : 3)) : GB_ROWS(4, true, 3));
+  return al ? GB_ROWS(1, true, 4) : GB_ROWS(1, false, 4);
+#undef GB_ROWS
 }
 
 template <typename T>
@@ -483,31 +586,37 @@ gbblas_status launch_gemv_cols(DeviceCtx* c, int64_t rows, int64_t cols, const T
   if (rows <= 0) return GBBLAS_STATUS_SUCCESS;
   constexpr int W = V<T>::w;
   const bool vec = aligned16(A) && (lda % W) == 0;
-  // unaligned columns: shifted vectors for float; for double, bound by the
-  // FP64 pipes, one row a lane (no row is computed twice)
-  constexpr bool kShift = sizeof(T) == 4;
-  using Odd = ColsCfg<kShift ? W : 1, kShift>;
+  // unaligned columns: one row a lane, or, for a float matrix beyond 100 MB,
+  // shifted vectors (16387 x 4096 48 us, 53 by elements; 8195 x 256 6.6 and 5.1,
+  // 259 x 128 4.0 and 2.7: their four sets of sums weigh there); double is bound
+  // by the FP64 pipes, and no row is to be computed twice
+  constexpr bool kF32 = sizeof(T) == 4;
+  const double bytes = (double)rows * cols * sizeof(T);
+  const bool shift = kF32 && !vec && bytes > 100.0e6;
+  const int64_t span = vec ? ColsCfg<W, false>::kRows : (shift ? ColsCfg<W, true>::kRows : 32);
   // two row blocks a CTA from 2048 rows (their pieces of a column adjoin: at
   // 16384^2 f32 159 us with one, 154-156 with two, 160 with eight), one below
   const int rw = rows > 2048 ? 2 : 1;
-  const int64_t blocks = cdiv(rows, (vec ? ColsCfg<W, false>::kRows : Odd::kRows) * (int64_t)rw);
-  // columns per CTA: enough CTAs for 16 per SM, at least 64 columns, a whole
+  const int64_t blocks = cdiv(rows, span * rw);
+  // columns per CTA: enough CTAs for 16 per SM (5 of single rows up to 20 MB: shapes
+  // of 8 .. 20 MB 6 % faster in the mean), at least 64 columns, a whole
   // number of rounds (8 columns a warp); double, whose time is its FP64 work,
   // shares short rows out evenly instead (20069 x 264: 20 us, 23 in 64s and a
   // rest; float 11.0 and 10.3)
-  const int64_t want = std::min<int64_t>(cdiv(16 * (int64_t)c->num_sms, blocks), 65535), round = 8 * (kWarps / rw);
+  const int64_t per_sm = kF32 && !vec && bytes < 20.0e6 ? 5 : 16;
+  const int64_t want = std::min<int64_t>(cdiv(per_sm * c->num_sms, blocks), 65535), round = 8 * (kWarps / rw);
   const int64_t even = cdiv(cols, std::max<int64_t>(1, std::min(want, cols / 64)));
-  const int64_t cps = cdiv(sizeof(T) == 8 ? even : std::max<int64_t>(cdiv(cols, want), 64), round) * round;
+  const int64_t cps = cdiv(!kF32 ? even : std::max<int64_t>(cdiv(cols, want), 64), round) * round;
   const dim3 grid((unsigned)blocks, (unsigned)std::max<int64_t>(1, cdiv(cols, cps)));
   if (vec)
     return launch_split<T>(c, gemv_cols_kernel<T, W, false, true>, gemv_cols_kernel<T, W, false, false>, grid, rows,
                            cols, y, accumulate, stream, "gemv_cols_kernel", A, lda, x, cps, rw);
-  if constexpr (kShift)
-    return launch_split<T>(c, gemv_cols_kernel<T, W, true, true>, gemv_cols_kernel<T, W, true, false>, grid, rows,
-                           cols, y, accumulate, stream, "gemv_cols_kernel", A, lda, x, cps, rw);
-  else
-    return launch_split<T>(c, gemv_cols_kernel<T, 1, false, true>, gemv_cols_kernel<T, 1, false, false>, grid, rows,
-                           cols, y, accumulate, stream, "gemv_cols_kernel", A, lda, x, cps, rw);
+  if constexpr (kF32)
+    if (shift)
+      return launch_split<T>(c, gemv_cols_kernel<T, W, true, true>, gemv_cols_kernel<T, W, true, false>, grid, rows,
+                             cols, y, accumulate, stream, "gemv_cols_kernel", A, lda, x, cps, rw);
+  return launch_split<T>(c, gemv_cols_kernel<T, 1, false, true>, gemv_cols_kernel<T, 1, false, false>, grid, rows,
+                         cols, y, accumulate, stream, "gemv_cols_kernel", A, lda, x, cps, rw);
 }
 
 #define GB_INST(T)                                                                                          \
