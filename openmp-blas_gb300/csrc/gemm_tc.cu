@@ -1958,11 +1958,15 @@ __global__ void __launch_bounds__(ModeTraits<MODE, BN>::kThreads, 1)
 // products, one warp per output: lane l sums k = l, l + 32, ... in order,
 // then the lanes' sums meet in a fixed shuffle tree.  Error at most
 // (K / 32 + 5) eps32 (|A||B|)_ij, order fixed: the same bits on every run.
-// CTAs take the listed rows in turn; with empty lists every CTA returns at
-// once.  jobs: the A jobs then the B^T jobs of a group (problem i = job i).
+// CTAs take kFixOutputs outputs of a listed row in turn (a whole row a CTA made
+// one row of 4096 outputs cost 140 us beside a GEMM of 38, 1158 x 4096 x 201;
+// now 49 in all; with a row-major B 822, now under 80); `chunks` of them cover the longest row.  With empty lists every CTA
+// returns at once.  jobs: the A jobs then the B^T jobs of a group (problem i =
+// job i).
+constexpr int kFixOutputs = 64;
 __global__ void __launch_bounds__(256) f16_guard_fixup_kernel(const SplitJob* jobs, int njobs, const TcProblem* probs,
                                                               const int* list_a, const int* list_b, const int* counts,
-                                                              const int* flags_a) {
+                                                              const int* flags_a, int chunks) {
   dev::grid_release();
   dev::grid_wait();
   const int na = counts[0], nb = counts[1];
@@ -1985,7 +1989,8 @@ __global__ void __launch_bounds__(256) f16_guard_fixup_kernel(const SplitJob* jo
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     return s;
   };
-  for (int e = blockIdx.x; e < na + nb; e += gridDim.x) {
+  for (int64_t it = blockIdx.x; it < (int64_t)(na + nb) * chunks; it += gridDim.x) {
+    const int e = (int)(it / chunks), first = (int)(it % chunks) * kFixOutputs;
     const bool row_entry = e < na;
     const int64_t r = row_entry ? list_a[e] : list_b[e - na];
     const int ji = job_of(row_entry ? jobs : jobs + njobs, r);
@@ -1994,13 +1999,15 @@ __global__ void __launch_bounds__(256) f16_guard_fixup_kernel(const SplitJob* jo
     const TcProblem& p = probs[ji];
     if (row_entry) {
       const int64_t i = r - ja.dst_row;  // every column of row i
-      for (int64_t jc = warp; jc < p.N; jc += nwarps) {
+      const int last = min(p.N, first + kFixOutputs);
+      for (int64_t jc = first + warp; jc < last; jc += nwarps) {
         const float v = dot(ja, i, jb, jc);
         if (lane == 0) p.C[i * p.rsc + jc * p.csc] += v;
       }
     } else {
       const int64_t jc = r - jb.dst_row;  // every row of column jc, but the out-of-span rows' (done above)
-      for (int64_t i = warp; i < p.M; i += nwarps) {
+      const int last = min(p.M, first + kFixOutputs);
+      for (int64_t i = first + warp; i < last; i += nwarps) {
         if (flags_a[ja.dst_row + i]) continue;
         const float v = dot(ja, i, jb, jc);
         if (lane == 0) p.C[i * p.rsc + jc * p.csc] += v;
@@ -2676,9 +2683,11 @@ gbblas_status launch_bound(DeviceCtx* c, const TcGroupPlan& pl, cudaStream_t str
     st = check_launch("splitk_reduce_kernel");
   }
   if (st == GBBLAS_STATUS_SUCCESS && pl.guard) {
+    int most = 1;  // outputs of the longest row
+    for (const TcProblem& p : pl.probs) most = std::max({most, p.M, p.N});
     GB_CUDA_TRY(launch_chain(chained, f16_guard_fixup_kernel, dim3(2 * c->num_sms), stream, djobs, pl.njobs,
                              reinterpret_cast<const TcProblem*>(pl.base + pl.off_probs), ga.list, gb.list, gcounts,
-                             ga.flags));
+                             ga.flags, (most + kFixOutputs - 1) / kFixOutputs));
     st = check_launch("f16_guard_fixup_kernel");
   }
   return st;
