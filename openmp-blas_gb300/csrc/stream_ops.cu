@@ -124,8 +124,8 @@ __global__ void __launch_bounds__(kThreads, 3) transpose_kernel(int64_t M, int64
 // chunk leaves of a row's last line waits for the next chunk.  94 us; 16383 x
 // 16001 f32 529 -> 375, f64 838 -> 677 (chunks of 32 rows and twice the CTAs:
 // 98 us for the first).
-// KCONTIG: A's columns are contiguous as C's rows are (rsa = 1): no exchange
-// of indexes, the pieces run along i.
+// (A and C contiguous along the same index, no exchange, stay with the tiles:
+// 9001 x 7003 f32 86 us, 100 in strips.)
 constexpr int kCI = 64;
 
 template <typename T>
@@ -134,10 +134,10 @@ struct TransCfg {
   static constexpr int kLine = 128 / (int)sizeof(T);  // elements per line
 };
 
-template <typename T, bool KCONTIG>
+template <typename T>
 __global__ void __launch_bounds__(kThreads, 4) transpose_lines_kernel(int64_t M, int64_t N, const T* __restrict__ A,
-                                                                int64_t rsa, int64_t csa, T* __restrict__ C,
-                                                                int64_t rsc, int64_t jblocks, int strip) {
+                                                                int64_t rsa, T* __restrict__ C, int64_t rsc,
+                                                                int64_t jblocks, int strip) {
   constexpr int TJ = TransCfg<T>::kTJ, LINE = TransCfg<T>::kLine;
   constexpr int PER = kCI * TJ / kThreads;  // elements of a chunk per thread
   __shared__ T ring[2 * kCI][TJ + 1];
@@ -146,18 +146,18 @@ __global__ void __launch_bounds__(kThreads, 4) transpose_lines_kernel(int64_t M,
   const int64_t i0 = (int64_t)(blockIdx.x / jblocks) * strip * kCI;
   const int64_t i1 = min(i0 + (int64_t)strip * kCI, M);  // the strip's rows
   // element e of this thread lies at (ii(e), jj(e)) of a chunk
-  auto ii = [&](int e) { return KCONTIG ? tx + 32 * (e % (kCI / 32)) : ty + 8 * (e / (TJ / 32)); };
-  auto jj = [&](int e) { return KCONTIG ? ty + 8 * (e / (kCI / 32)) : tx + 32 * (e % (TJ / 32)); };
+  auto ii = [&](int e) { return ty + 8 * (e / (TJ / 32)); };
+  auto jj = [&](int e) { return tx + 32 * (e % (TJ / 32)); };
   T r[PER];
   auto load = [&](int64_t ic) {
-    const T* p = A + ic * rsa + j0 * csa;
+    const T* p = A + ic * rsa + j0;
     if (ic + kCI <= i1 && j0 + TJ <= N) {
 #pragma unroll
-      for (int e = 0; e < PER; ++e) r[e] = p[ii(e) * rsa + jj(e) * csa];
+      for (int e = 0; e < PER; ++e) r[e] = p[ii(e) * rsa + jj(e)];
     } else {
 #pragma unroll
       for (int e = 0; e < PER; ++e)
-        r[e] = (ic + ii(e) < i1 && j0 + jj(e) < N) ? p[ii(e) * rsa + jj(e) * csa] : T(0);
+        r[e] = (ic + ii(e) < i1 && j0 + jj(e) < N) ? p[ii(e) * rsa + jj(e)] : T(0);
     }
   };
   load(i0);
@@ -331,15 +331,12 @@ gbblas_status launch_transpose(DeviceCtx* c, int64_t M, int64_t N, const T* A, i
   const int64_t m = c_rows ? M : N, n = c_rows ? N : M;  // C has n contiguous rows of m
   constexpr int TJ = TransCfg<T>::kTJ;
   const int64_t jblocks = (n + TJ - 1) / TJ, chunks = (m + kCI - 1) / kCI;
-  if ((c_rows || rsc == 1) && (ra == 1 || ca == 1) && 2.0 * (double)M * (double)N * sizeof(T) >= 200e6 &&
+  if ((c_rows || rsc == 1) && ca == 1 && 2.0 * (double)M * (double)N * sizeof(T) >= 200e6 &&
       (ldc % 4 != 0 || reinterpret_cast<uintptr_t>(C) % (4 * sizeof(T)) != 0) && jblocks * chunks <= 0x7fffffff / kCI) {
     const int64_t strips = std::min(chunks, std::max<int64_t>(1, (12 * (int64_t)c->num_sms + jblocks - 1) / jblocks));
     const int64_t strip = (chunks + strips - 1) / strips;
     const unsigned lgrid = (unsigned)(jblocks * ((chunks + strip - 1) / strip));
-    if (ca != 1)
-      transpose_lines_kernel<T, true><<<lgrid, kThreads, 0, s>>>(m, n, A, ra, ca, C, ldc, jblocks, (int)strip);
-    else
-      transpose_lines_kernel<T, false><<<lgrid, kThreads, 0, s>>>(m, n, A, ra, ca, C, ldc, jblocks, (int)strip);
+    transpose_lines_kernel<T><<<lgrid, kThreads, 0, s>>>(m, n, A, ra, C, ldc, jblocks, (int)strip);
     return check_launch("transpose_lines_kernel");
   }
   constexpr int TILE = 64;  // 16 (f32) / 32 (f64) KB of shared memory per CTA

@@ -31,3 +31,26 @@ def test_lines(cuda, dt, la, lc, M, N, pad, off):
     assert torch.equal(got.contiguous().view(I), want.contiguous().view(I))
     # C^T's other half: nothing beside C changed
     assert bool((C[:, (M if lc else N):] == -3.0).all()) and bool((buf[:off] == -3.0).all()) and bool((buf[-9:] == -3.0).all())
+
+
+def test_no_exchange_is_no_slower_than_one(cuda):
+    """A and C contiguous along the same index: a copy, without an exchange
+    through shared memory and so not slower than the transpose of that size."""
+    import gbblas
+    torch = cuda
+    M, N = 9001, 7003
+    A, C, flush = (torch.rand(n, device="cuda") for n in (M * N, M * N, 64 << 20))
+
+    def best(rsc, csc):
+        times = []
+        for _ in range(15):
+            flush.fill_(1.0)
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            gbblas.call("gbblas_stranspose", M, N, A.data_ptr(), N, 1, C.data_ptr(), rsc, csc, None)
+            e1.record()
+            torch.cuda.synchronize()
+            times.append(e0.elapsed_time(e1))
+        return min(times)
+
+    assert best(1, N) <= best(M, 1)
