@@ -1960,9 +1960,9 @@ __global__ void __launch_bounds__(ModeTraits<MODE, BN>::kThreads, 1)
 // (K / 32 + 5) eps32 (|A||B|)_ij, order fixed: the same bits on every run.
 // CTAs take kFixOutputs outputs of a listed row in turn (a whole row a CTA made
 // one row of 4096 outputs cost 140 us beside a GEMM of 38, 1158 x 4096 x 201;
-// now 49 in all; with a row-major B 822, now under 80); `chunks` of them cover the longest row.  With empty lists every CTA
-// returns at once.  jobs: the A jobs then the B^T jobs of a group (problem i =
-// job i).
+// now 49 in all; with a row-major B 822, now under 80); `chunks` of them cover
+// the longest row.  With empty lists every CTA returns at once.  jobs: the A
+// jobs then the B^T jobs of a group (problem i = job i).
 constexpr int kFixOutputs = 64;
 __global__ void __launch_bounds__(256) f16_guard_fixup_kernel(const SplitJob* jobs, int njobs, const TcProblem* probs,
                                                               const int* list_a, const int* list_b, const int* counts,

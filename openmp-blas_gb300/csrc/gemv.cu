@@ -29,7 +29,7 @@
 // loads at odd leading dimensions, a CTA per four rows, a thread per row of a
 // column) and now: rows f32 16384^2 153.9 -> 148, 8191 x 6001 48.3 -> 35.4,
 // 25596 x 256 16.4 -> 8.5; f64 18652 x 947 86 -> 45, 25596 x 256 82 -> 20;
-// columns f32 16384^2 156.4 -> 154, 10001 x 10003 166 -> 69, 256 x 25596 36 -> 12;
+// columns f32 16384^2 156.4 -> 154, 10001 x 10003 166 -> 69, 256 x 25596 36 -> 11;
 // f64 8191 x 6001 95 -> 92, 10001 x 10003 205 -> 177, 512 x 6552 33 -> 15.
 #include <algorithm>
 #include <type_traits>

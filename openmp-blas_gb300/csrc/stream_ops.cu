@@ -323,9 +323,10 @@ gbblas_status launch_transpose(DeviceCtx* c, int64_t M, int64_t N, const T* A, i
   // elements (where they do, few sectors are written in two parts: by tiles and
   // in strips, us, f32 9877 rows of 6901 116 and 107.5, of 6902 113 and 107, of
   // 6900 104 and 107, of 6904 95 and 107; f64 6901 193 and 177, 6902 191 and
-  // 177, 6900 175 and 176): strips, 12 CTAs per SM.  From 200 MB moved (below it the writes of neighbouring tiles
-  // meet in L2 before they leave it: 4501 x 4499 f32, 162 MB, 33.5 us by tiles
-  // and 35.0 in strips; 6001 x 5003, 240 MB, 51.2 and 47.4).
+  // 177, 6900 175 and 176): strips, 12 CTAs per SM.  From 200 MB moved (below it
+  // the writes of neighbouring tiles meet in L2 before they leave it: 4501 x 4499
+  // f32, 162 MB, 33.5 us by tiles and 35.0 in strips; 6001 x 5003, 240 MB, 51.2
+  // and 47.4).
   const bool c_rows = csc == 1;
   const int64_t ldc = c_rows ? rsc : csc, ra = c_rows ? rsa : csa, ca = c_rows ? csa : rsa;
   const int64_t m = c_rows ? M : N, n = c_rows ? N : M;  // C has n contiguous rows of m
